@@ -18,9 +18,17 @@
 // Two tile configurations:
 //   PAIR  : a cluster of two CTAs computes a 256 x 256 tile with cta_group::2 MMAs.  Each
 //           CTA stages its own 128 rows of A and half (128 rows) of B, so a k-block costs
-//           32 KB of loads per SM instead of 48 KB: the kernel is bound by the L2-to-SM
-//           path, and this raises FLOPs per loaded byte by 1.5x.  No multicast load is used.
+//           32 KB of loads per SM instead of 48 KB.  No multicast load is used.
 //   single: one CTA computes 128 x BN (BN = 128 or 256).
+//
+// What bounds it.  A k-block (64 of K) of a pair tile is 512 clocks of MMA, reads 32 KB and receives 32 KB of shared
+// memory per SM, which together is the full 128 bytes per clock of its port.  Loads from L2 are not the limit (a
+// load-only kernel draws 60 bytes per clock into every SM at once, 128 into one alone; a k-block needs 63).  What kept
+// the pipe waiting were the single threads of the roles: one TMA producer took 400 to 590 clocks to issue the copies of
+// a k-block, the MMA thread 390 to issue and 190 to wait, and both read the tile list and the problem table (two
+// dependent L2 reads) between tiles.  Two producers, a warp-uniform MMA loop and a scheduler warp that keeps a ring
+// of decoded tiles in shared memory took a k-block from 690-900 to 560-715 clocks; Newton-Schulz of GPT-2 XL,
+// sustained under the 1000 W cap, from 46.2 to 40.8 ms.
 //
 // Three ways to launch the loop (the template parameter CHAINED separates the first from the other two):
 //   per phase : one launch per GEMM flavour and iteration, tiles dealt round-robin, launches chained with
@@ -53,13 +61,14 @@ struct Cfg {
     static constexpr int kBRows = PAIR ? 128 : BN;   // rows of B this CTA stages per k-block
     static constexpr int kBBytes = (kBRows / 64) * kBoxBytes;
     static constexpr int kStageBytes = kABytes + kBBytes;
-    // warp 0: TMA producer, warp 1: MMA issuer, then four epilogue warps (one per TMEM lane
-    // quarter) for every 64 columns of the tile
+    // warp 0: TMA producer of A, warp 1: MMA issuer, then four epilogue warps (one per TMEM lane quarter) for every
+    // 64 columns of the tile, the TMA producer of B and the tile scheduler
     static constexpr int kEpiWarps = 4 * (BN / 64);
-    static constexpr int kThreads = 32 * (2 + kEpiWarps);
+    static constexpr int kProducerA = 0, kMmaWarp = 1, kEpiWarp0 = 2, kProducerB = 2 + kEpiWarps, kSchedulerWarp = 3 + kEpiWarps;
+    static constexpr int kThreads = 32 * (4 + kEpiWarps);
     static constexpr int kStagingBytes = kEpiWarps * kSlabBytes;
     static constexpr int kTmemCols = 2 * BN;
-    static constexpr int kBarrierBytes = 512;   // mbarriers, flags, and the tile ring of the chained launch
+    static constexpr int kBarrierBytes = 768;   // mbarriers, flags, the tile ring and the hand-over ring of the chained launch
     static constexpr int kStages = (kSmemLimit - kStagingBytes - kBarrierBytes - 1024) / kStageBytes;
     static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
     static constexpr int kTileM = PAIR ? 256 : 128;  // rows of the (cluster) tile
@@ -88,6 +97,9 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // arrive on a barrier given by its shared::cluster address (own or peer CTA)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
@@ -121,7 +133,7 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 }
 // Bounded wait (about two seconds of wall clock).  Returns false when the limit ran out or
 // another role of this CTA already gave up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag) {
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag) {
 #pragma unroll 1
     for (int it = 0; it < 128; ++it)
         if (mbar_try_wait(bar, parity)) return true;
@@ -135,6 +147,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
     *abort_flag = 1;
     return false;
+}
+
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag) {
+    return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity, abort_flag);
 }
 
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
@@ -183,29 +199,26 @@ __device__ __forceinline__ bool chain_wait(const uint32_t *counter, uint32_t nee
     return false;
 }
 
-// Chained launch: which tile a CTA (pair) works on next is decided at run time (an atomic ticket over the work
-// list, claimed by the leader's producer thread), so the roles of the CTA, and the peer CTA of a pair, learn it
-// through a small ring in shared memory: entry k holds (k + 1) << 32 | tile for the k-th tile of this CTA.  No
-// role is ever more than stages + 2 tiles behind the producer, far less than the ring's length.
-constexpr uint32_t kTileRing = 16;
+// Chained launch: which tile a CTA pair works on next is decided at run time (an atomic ticket over the work list,
+// claimed by the leader's scheduler), so the peer CTA learns it through a small ring in its shared memory: entry k
+// holds (k + 1) << 32 | tile for the k-th tile of the pair.  The leader's scheduler is never more than the tile ring
+// and the pipeline ahead of the peer's, far less than this ring's length.
+constexpr uint32_t kHandRing = 16;
 constexpr uint32_t kNoTile = 0xffffffffu;
-__device__ __forceinline__ void ring_put_local(volatile uint64_t *ring, uint32_t seq, uint32_t tile) {
-    ring[seq % kTileRing] = ((uint64_t)(seq + 1u) << 32) | tile;
-}
-__device__ __forceinline__ void ring_put_remote(uint32_t ring_cluster_addr, uint32_t seq, uint32_t tile) {
+__device__ __forceinline__ void hand_put(uint32_t hand_cluster_addr, uint32_t seq, uint32_t tile) {
     const uint64_t v = ((uint64_t)(seq + 1u) << 32) | tile;
-    asm volatile("st.volatile.shared::cluster.u64 [%0], %1;" ::"r"(ring_cluster_addr + 8u * (seq % kTileRing)), "l"(v)
+    asm volatile("st.volatile.shared::cluster.u64 [%0], %1;" ::"r"(hand_cluster_addr + 8u * (seq % kHandRing)), "l"(v)
                  : "memory");
 }
 // Bounded: gives kNoTile when the CTA is aborting or nothing arrives within the wait limit.
-__device__ __forceinline__ uint32_t ring_get(volatile uint64_t *ring, uint32_t seq, volatile uint32_t *abort_flag) {
+__device__ __forceinline__ uint32_t hand_get(volatile uint64_t *ring, uint32_t seq, volatile uint32_t *abort_flag) {
     const uint64_t want = (uint64_t)(seq + 1u);
-    uint64_t v = ring[seq % kTileRing];
+    uint64_t v = ring[seq % kHandRing];
     if ((v >> 32) == want) return (uint32_t)v;
     const uint64_t start = global_timer_ns();
 #pragma unroll 1
     for (uint32_t it = 0; it < kSpinLimit; ++it) {
-        v = ring[seq % kTileRing];
+        v = ring[seq % kHandRing];
         if ((v >> 32) == want) return (uint32_t)v;
         if (*abort_flag) return kNoTile;
         if (global_timer_ns() - start > kWaitLimitNs) break;
@@ -258,6 +271,11 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t
             ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
             : "memory");
 }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(r));
+    return r != 0u;
+}
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp receives row (lane base + i).
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t *r) {
     asm volatile(
@@ -306,65 +324,53 @@ __device__ __forceinline__ uint32_t instr_desc(int m, int n, int f16, uint32_t a
            ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// What one role needs to know about the tile it works on.  Plain launch: one GEMM flavour for the whole grid
-// (epilogue, coefficients and scaling are launch arguments).  Chained launch: every entry of the list carries
-// its own flavour, iteration and the progress count of its matrix that must be reached before its operands
-// may be read.
-struct TileWork {
-    uint32_t problem, tile_m, tile_n, mirror, epilogue, slot, need, scale_pow, iter;
-    uint32_t problem2, need2;   // second part of a kEpiGramPoly entry
+// What the roles of a CTA need to know about the tile they work on, written by the CTA's scheduler warp into a
+// small ring in shared memory.  The tile list and the problem table are two dependent reads of L2 (about 700 clocks
+// each); with the ring they are off the path of the roles, which read an entry in a few tens of clocks.
+struct alignas(16) TileEntry {
+    uint64_t map_a, map_b;   // tensor maps of the operands
+    uint64_t out;            // 16-bit result, or the FP32 one (kEpiApplyLast)
+    uint64_t frag;
+    uint32_t M, N, num_kb, pitch_bytes;
+    uint32_t tile;           // tile_m | tile_n << 16
+    uint32_t flags;
+    uint32_t tiles_n, slot;
 };
-// A work-list entry runs as one GEMM, or (kEpiGramPoly) as two on the same CTA (pair): part 0 the Gram tile,
-// whose accumulator stays in tensor memory, part 1 the polynomial tile that consumes it.
-struct TilePart {
-    uint32_t problem, epilogue, need;
-};
-__device__ __forceinline__ uint32_t tile_parts(const TileWork &w) { return w.epilogue == kEpiGramPoly ? 2u : 1u; }
-__device__ __forceinline__ TilePart tile_part(const TileWork &w, uint32_t part) {
-    TilePart p;
-    if (w.epilogue != kEpiGramPoly) {
-        p.problem = w.problem; p.epilogue = w.epilogue; p.need = w.need;
-    } else if (part == 0u) {
-        p.problem = w.problem; p.epilogue = kEpiGramHold; p.need = w.need;
-    } else {
-        p.problem = w.problem2; p.epilogue = kEpiPolyFused; p.need = w.need2;
-    }
-    return p;
-}
-template <bool CHAINED>
-__device__ __forceinline__ TileWork tile_work(const void *tiles, uint32_t t, uint32_t epilogue, uint32_t scale_pow) {
-    TileWork w;
-    w.problem2 = 0;
-    w.need2 = 0;
-    if (CHAINED) {
-        const uint4 c = __ldg(reinterpret_cast<const uint4 *>(tiles) + 2 * (size_t)t);
-        w.problem = c.x;
-        w.tile_m = c.y & 0xffffu;
-        w.tile_n = c.y >> 16;
-        w.slot = c.z & 0xffffu;
-        w.epilogue = (c.z >> 16) & 0xffu;
-        w.mirror = (c.z >> 24) & 1u;
-        w.scale_pow = (c.z >> 25) & 3u;
-        w.iter = (c.z >> 27) & 31u;
-        w.need = c.w;
-        if (w.epilogue == kEpiGramPoly) {
-            const uint4 d = __ldg(reinterpret_cast<const uint4 *>(tiles) + 2 * (size_t)t + 1);
-            w.problem2 = d.x;
-            w.need2 = d.y;
-        }
-    } else {
-        const GemmTile tl = reinterpret_cast<const GemmTile *>(tiles)[t];
-        w.problem = tl.problem;
-        w.tile_m = tl.tile_m;
-        w.tile_n = tl.tile_n;
-        w.mirror = tl.reserved;
-        w.epilogue = epilogue;
-        w.slot = tl.problem;
-        w.need = 0;
-        w.scale_pow = scale_pow;
-        w.iter = 0;
-    }
-    return w;
+static_assert(sizeof(TileEntry) == 64, "an entry is read as four 16-byte words");
+constexpr uint32_t kRing = 4;
+// flags of an entry
+constexpr uint32_t kTileAMn = 1u, kTileBMn = 2u, kTileMirror = 4u;
+constexpr uint32_t kTileShared = 8u;      // B is the A tile: loaded once, read twice
+constexpr uint32_t kTileDependent = 16u;  // the operands were written by this launch
+constexpr uint32_t kTileEnd = 32u;        // no more tiles
+constexpr int kTileEpiShift = 8, kTileScaleShift = 12, kTileIterShift = 16, kTileNShift = 24;
+
+// Fills in everything but `flags` bits that come from the list entry.  The MMA's N is the width of the tile that
+// exists, rounded up: a 1600-wide output has a last tile column of 64, which a 256-wide MMA would spend four times as
+// long on.  K-major B: steps of 64 (a pair splits N in two halves of at least 32 rows); MN-major B: steps of 128, so
+// that each half is made of whole 64-element swizzle atoms.
+template <int BN, bool PAIR>
+__device__ __forceinline__ void fill_entry(TileEntry &e, const GemmProblem *p, uint32_t tile_m, uint32_t tile_n, uint32_t epilogue,
+                                           uint32_t flags) {
+    e.map_a = p->map_a;
+    e.map_b = p->map_b;
+    e.frag = p->frag32;
+    e.M = p->M;
+    e.N = p->N;
+    e.num_kb = (p->K + kGemmBlockK - 1) / kGemmBlockK;
+    e.tiles_n = p->tiles_n;
+    const bool last = epilogue == kEpiApplyLast;
+    e.out = last ? p->out32 : p->out16;
+    e.pitch_bytes = last ? p->pitch32 * 4u : p->pitch16 * 2u;
+    e.tile = tile_m | (tile_n << 16);
+    const uint32_t a_mn = p->a_mn_major, b_mn = p->b_mn_major;
+    const uint32_t step = b_mn ? 128u : 64u;
+    const uint32_t left = e.N - tile_n * BN;
+    const uint32_t n_mma = min((uint32_t)BN, (left + step - 1u) / step * step);
+    // a diagonal tile of X X^T or G G: this CTA's 128 rows of B are its 128 rows of A, in the same shared-memory layout
+    const bool shared = PAIR && tile_m == tile_n && e.map_a == e.map_b && a_mn == b_mn && n_mma == (uint32_t)BN;
+    e.flags = flags | (a_mn ? kTileAMn : 0u) | (b_mn ? kTileBMn : 0u) | (shared ? kTileShared : 0u) |
+              (epilogue << kTileEpiShift) | ((n_mma / 32u) << kTileNShift);
 }
 
 template <int BN, bool PAIR, bool CHAINED>
@@ -372,27 +378,21 @@ __global__ void __launch_bounds__((Cfg<BN, PAIR>::kThreads), 1)
 k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ tiles,
           uint32_t tile_count, uint32_t epilogue_arg, int f16, GemmCoefficients coef,
           const float *__restrict__ slot_scale, uint32_t scale_pow_arg, uint32_t *status, ChainSync *sync,
-          uint32_t slot_count, uint32_t debug_flags) {
+          uint32_t slot_count) {
     using C = Cfg<BN, PAIR>;
-#ifdef B2_MEASURE
-    const bool dbg_no_store = debug_flags & 1u;   // drop every epilogue store
-    const bool dbg_no_global = debug_flags & 8u;  // stage in shared memory but issue no global store
-#else
-    constexpr bool dbg_no_store = false, dbg_no_global = false;
-    (void)debug_flags;
-#endif
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *stage_base = smem;
     uint8_t *staging = smem + C::kStages * C::kStageBytes;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(staging + C::kStagingBytes);
-    // bars[0..S) full, [S..2S) empty, [2S..2S+2) tmem_full, [2S+2..2S+4) tmem_empty
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * C::kStages + 4);
+    uint8_t *control = staging + C::kStagingBytes;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(control);
+    // bars: full[S], empty[S], tmem_full[2], tmem_empty[2], ring_full[kRing], ring_empty[kRing]
+    constexpr int kBars = 2 * C::kStages + 4 + 2 * (int)kRing;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kBars);
     volatile uint32_t *abort_flag = tmem_slot + 1;
-    // chained: one more than the index of the last tile whose dependency wait this CTA's producer has passed
-    volatile uint32_t *passed_tile = tmem_slot + 2;
-    volatile uint64_t *tile_ring = reinterpret_cast<volatile uint64_t *>(reinterpret_cast<uint8_t *>(bars) + 256);
-    static_assert((2 * C::kStages + 4) * 8 + 16 <= 256 && 256 + kTileRing * 8 <= C::kBarrierBytes, "barrier region layout");
+    TileEntry *ring = reinterpret_cast<TileEntry *>(control + 256);
+    volatile uint64_t *hand = reinterpret_cast<volatile uint64_t *>(control + 256 + kRing * sizeof(TileEntry));
+    static_assert(kBars * 8 + 8 <= 256 && 256 + kRing * sizeof(TileEntry) + kHandRing * 8 <= C::kBarrierBytes, "control region layout");
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -400,27 +400,34 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
     const uint32_t first_tile = PAIR ? blockIdx.x / 2 : blockIdx.x;
     const uint32_t tile_stride = PAIR ? gridDim.x / 2 : gridDim.x;
     const uint32_t bar0 = smem_u32(bars);
-    auto full_bar = [&](int s) { return bar0 + 8u * s; };
-    auto empty_bar = [&](int s) { return bar0 + 8u * (C::kStages + s); };
-    auto tfull_bar = [&](int a) { return bar0 + 8u * (2 * C::kStages + a); };
-    auto tempty_bar = [&](int a) { return bar0 + 8u * (2 * C::kStages + 2 + a); };
+    auto full_bar = [&](uint32_t s) { return bar0 + 8u * s; };
+    auto empty_bar = [&](uint32_t s) { return bar0 + 8u * (C::kStages + s); };
+    auto tfull_bar = [&](uint32_t a) { return bar0 + 8u * (2 * C::kStages + a); };
+    auto tempty_bar = [&](uint32_t a) { return bar0 + 8u * (2 * C::kStages + 2 + a); };
+    auto ring_full = [&](uint32_t k) { return bar0 + 8u * (2 * C::kStages + 4 + k % kRing); };
+    auto ring_empty = [&](uint32_t k) { return bar0 + 8u * (2 * C::kStages + 4 + kRing + k % kRing); };
+    auto ring_parity = [&](uint32_t k) { return (k / kRing) & 1u; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kStages; ++s) {
-            mbar_init(full_bar(s), 1);
+            mbar_init(full_bar(s), 2);    // one arrival from each of the leader's two TMA producers
             mbar_init(empty_bar(s), 1);
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(tfull_bar(a), 1);
             mbar_init(tempty_bar(a), PAIR ? 2 * C::kEpiWarps : C::kEpiWarps);
         }
+        for (uint32_t k = 0; k < kRing; ++k) {
+            mbar_init(ring_full(k), 1);
+            mbar_init(ring_empty(k), C::kEpiWarps + 2 + (rank == 0 ? 1 : 0));
+        }
         *abort_flag = 0;
-        *passed_tile = 0;
-        for (uint32_t k = 0; k < kTileRing; ++k) tile_ring[k] = 0;
+        if (CHAINED)
+            for (uint32_t k = 0; k < kHandRing; ++k) hand[k] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
     }
-    if (warp == 1) {
+    if (warp == C::kMmaWarp) {
         if (PAIR) {
             asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                          "r"((uint32_t)C::kTmemCols) : "memory");
@@ -436,182 +443,189 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
     if (PAIR) cluster_sync_all();  // the peer's barriers are initialised before anything signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // Programmatic dependent launch: the next launch of the stream may start its own prologue on
-    // SMs this grid has left; nothing above reads what the previous launch wrote, everything
-    // below may, so the wait for that launch (a no-op without the launch attribute) sits here.
+    // Programmatic dependent launch: the next launch of the stream may start its own prologue on SMs this grid has
+    // left.  What the previous launch wrote may be read only below the wait (a no-op without the launch attribute);
+    // the tile list, the problem table and the tensor maps belong to the plan, so the scheduler warp of a plain launch
+    // does not wait and has the first entries in the ring, and their tensor maps fetched, by then.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (CHAINED || warp != C::kSchedulerWarp) asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer
+    if (warp == C::kSchedulerWarp) {
+        // ------------------------------------------------------------------ tile scheduler
         if (lane == 0) {
-            uint32_t stage = 0, phase = 0;
+            uint32_t k = 0;   // ring sequence number
             bool ok = true;
-            // Plain launch: tile first_tile + k * tile_stride.  Chained launch: the leader claims list entries in
-            // order with an atomic ticket (a tile only ever waits for tiles with smaller tickets, which running
-            // CTAs hold, so the launch makes progress however many CTAs are resident; the CTAs stay within one
-            // wave of each other in the list, which keeps a matrix's operands in L2 while its tiles are worked
-            // on; and a slower SM simply takes fewer tiles).  The ticket for the tile after next is claimed, and
-            // the next tile's description and progress count fetched, while this tile's copies are issued.
-            uint32_t seq = 0, t = first_tile, t_next = kNoTile;
-            const bool claims = CHAINED && (!PAIR || rank == 0);
-            // A list with fused Gram + polynomial entries: their second part waits for tiles with larger tickets, so
-            // a CTA must not sit on a ticket it has not started.  The next ticket is then drawn only once the last
-            // wait of the current tile has passed, and looked at after the tile's copies have been issued.
-            const bool fused_list = CHAINED && epilogue_arg != 0u;
-            const uint32_t peer_ring = (CHAINED && PAIR) ? map_to_cta(smem_u32(const_cast<uint64_t *>(tile_ring)), 1) : 0u;
-            auto announce = [&](uint32_t tile) {   // leader: tell this CTA's roles (and the peer CTA) the seq-th tile
-                ring_put_local(tile_ring, seq, tile);
-                if (PAIR) ring_put_remote(peer_ring, seq, tile);
+            auto claim_slot = [&]() { return mbar_wait(ring_empty(k), ring_parity(k) ^ 1u, abort_flag); };
+            auto publish_entry = [&]() {
+                mbar_arrive(ring_full(k));
+                ++k;
             };
-            if (CHAINED) {
-                if (claims) {
-                    t = atomicAdd(&sync->ticket, 1u);
-                    announce(t);
-                    if (!fused_list && t < tile_count) t_next = atomicAdd(&sync->ticket, 1u);
-                } else {
-                    t = ring_get(tile_ring, seq, abort_flag);
+            if (!CHAINED) {
+                // tile first_tile + i * tile_stride; the list is read one tile ahead
+                const GemmTile *list = reinterpret_cast<const GemmTile *>(tiles);
+                uint32_t t = first_tile;
+                GemmTile next = {};
+                if (t < tile_count) next = list[t];
+                while (t < tile_count) {
+                    const GemmTile tl = next;
+                    t += tile_stride;
+                    if (t < tile_count) next = list[t];
+                    if (!claim_slot()) { ok = false; break; }
+                    TileEntry &e = ring[k % kRing];
+                    fill_entry<BN, PAIR>(e, problems + tl.problem, tl.tile_m, tl.tile_n, epilogue_arg,
+                                         (tl.reserved ? kTileMirror : 0u) | (scale_pow_arg << kTileScaleShift));
+                    e.slot = tl.problem;
+                    if (k < 2) {
+                        asm volatile("prefetch.tensormap [%0];" ::"l"(e.map_a) : "memory");
+                        asm volatile("prefetch.tensormap [%0];" ::"l"(e.map_b) : "memory");
+                    }
+                    publish_entry();
+                }
+            } else {
+                // The leader claims list entries in order with an atomic ticket (a tile only ever waits for tiles with
+                // smaller tickets, which running CTAs hold, so the launch makes progress however many CTAs are
+                // resident; the CTAs stay within a few tiles of each other in the list, which keeps a matrix's
+                // operands in L2 while its tiles are worked on; and a slower SM simply takes fewer tiles) and hands
+                // them to the peer CTA.  An entry goes into the ring once the tiles it reads from have been stored and
+                // published.  A fused Gram + polynomial entry becomes two; its second part waits for tiles with LARGER
+                // tickets, and the next ticket is drawn only after that wait, so a CTA never sits on a ticket it has
+                // not started while it waits for one.
+                const bool claims = !PAIR || rank == 0;
+                const uint32_t peer_hand = PAIR ? map_to_cta(smem_u32(const_cast<uint64_t *>(hand)), 1) : 0u;
+                for (uint32_t seq = 0; ok; ++seq) {
+                    uint32_t t;
+                    if (claims) {
+                        t = atomicAdd(&sync->ticket, 1u);
+                        if (PAIR) hand_put(peer_hand, seq, t);
+                    } else {
+                        t = hand_get(hand, seq, abort_flag);
+                    }
+                    if (t >= tile_count) break;
+                    const uint4 c = __ldg(reinterpret_cast<const uint4 *>(tiles) + 2 * (size_t)t);
+                    const uint4 d = __ldg(reinterpret_cast<const uint4 *>(tiles) + 2 * (size_t)t + 1);
+                    const uint32_t slot = c.z & 0xffffu, epilogue = (c.z >> 16) & 0xffu;
+                    const bool two = epilogue == kEpiGramPoly;
+                    const uint32_t flags = (((c.z >> 24) & 1u) ? kTileMirror : 0u) | (((c.z >> 25) & 3u) << kTileScaleShift) |
+                                           (((c.z >> 27) & 31u) << kTileIterShift);
+                    for (uint32_t part = 0; ok && part < (two ? 2u : 1u); ++part) {
+                        const uint32_t need = part ? d.y : c.w;
+                        if (need != 0u) {
+                            if (!chain_wait(&sync->progress[slot], need, &sync->abort, abort_flag)) { ok = false; break; }
+                            (void)ld_acquire_gpu(&sync->progress[slot]);
+                        }
+                        if (!claim_slot()) { ok = false; break; }
+                        TileEntry &e = ring[k % kRing];
+                        fill_entry<BN, PAIR>(e, problems + (part ? d.x : c.x), c.y & 0xffffu, c.y >> 16,
+                                             two ? (part ? kEpiPolyFused : kEpiGramHold) : epilogue,
+                                             flags | (need != 0u ? kTileDependent : 0u));
+                        e.slot = slot;
+                        publish_entry();
+                    }
                 }
             }
-            TileWork next = {};
-            uint32_t next_seen = 0;
-            auto describe_next = [&]() {
-                if (t < tile_count) {
-                    next = tile_work<CHAINED>(tiles, t, epilogue_arg, scale_pow_arg);
-                    if (CHAINED && next.need != 0u) next_seen = ld_relaxed_gpu(&sync->progress[next.slot]);
-                }
-            };
-            describe_next();
-            while (ok && t < tile_count) {
-                const TileWork tl = next;
-                const uint32_t seen = next_seen;
-                const uint32_t t_now = t;
-                const uint32_t parts = CHAINED ? tile_parts(tl) : 1u;
-                // the tile after this one
-                if (!CHAINED) {
-                    t += tile_stride;
-                    describe_next();
-                } else if (!fused_list) {
-                    if (claims) {
-                        t = t_next;
-                        ++seq;
-                        announce(t);
-                        if (t < tile_count) t_next = atomicAdd(&sync->ticket, 1u);
-                    } else {
-                        ++seq;
-                        t = ring_get(tile_ring, seq, abort_flag);
-                    }
-                    describe_next();
-                }
-                uint32_t drawn = kNoTile;
-                for (uint32_t part = 0; ok && part < parts; ++part) {
-                    TilePart tp;
-                    if (CHAINED) {
-                        tp = tile_part(tl, part);
-                    } else {
-                        tp.problem = tl.problem; tp.epilogue = tl.epilogue; tp.need = 0u;
-                    }
-                    const GemmProblem *p = problems + tp.problem;
-                    const uint64_t map_a = p->map_a, map_b = p->map_b;
-                    const uint32_t a_mn = p->a_mn_major, b_mn = p->b_mn_major, K = p->K;
-                    const int m0 = tl.tile_m * C::kTileM + (int)rank * 128;
-                    const int n0 = tl.tile_n * BN + (PAIR ? (int)rank * 128 : 0);
-                    const int num_kb = (int)((K + kGemmBlockK - 1) / kGemmBlockK);
-                    // A diagonal tile of X X^T or G G: this CTA's 128 rows of B are its 128 rows of A, in
-                    // the same shared-memory layout.  They are loaded once and the MMA reads them twice.
-                    const bool shared_operand = PAIR && tl.tile_m == tl.tile_n && map_a == map_b && a_mn == b_mn;
-                    if (CHAINED && tp.need != 0u) {
-                        // the operands are the outputs of the matrix's previous phase: every tile of that phase
-                        // has been stored and published before the first copy is issued
-                        if ((part != 0u || seen < tp.need) &&
-                            !chain_wait(&sync->progress[tl.slot], tp.need, &sync->abort, abort_flag)) { ok = false; break; }
-                        (void)ld_acquire_gpu(&sync->progress[tl.slot]);
-                        fence_proxy_async_all();
-                    }
-                    if (CHAINED && part == 0u) *passed_tile = t_now + 1u;
-                    if (fused_list && claims && part + 1u == parts) drawn = atomicAdd(&sync->ticket, 1u);
-                    const uint32_t stage_tx = shared_operand ? 2u * (uint32_t)kABytes
-                                                             : (uint32_t)C::kStageBytes * (PAIR ? 2u : 1u);
-                    for (int kb = 0; kb < num_kb; ++kb) {
+            if (ok && claim_slot()) {
+                ring[k % kRing].flags = kTileEnd;
+                publish_entry();
+            }
+        }
+    } else if (warp == C::kProducerA || warp == C::kProducerB) {
+        // ------------------------------------------------------------------ TMA producers, one per operand
+        // Issuing one TMA copy takes a thread 70 to 100 clocks, so one thread for both operands was the slowest role of
+        // the pipeline (400 to 590 clocks of the 512 a k-block's MMAs take).
+        if (lane == 0) {
+            const bool for_b = warp == C::kProducerB;
+            const uint32_t leader_full = PAIR ? map_to_cta(full_bar(0), 0) : full_bar(0);
+            uint32_t stage = 0, phase = 0, turn = 0;   // turn: parity of the k-blocks so far, over all tiles
+            bool ok = true;
+            for (uint32_t k = 0; ok; ++k) {
+                if (!mbar_wait(ring_full(k), ring_parity(k), abort_flag)) break;
+                const TileEntry &e = ring[k % kRing];
+                const uint32_t flags = e.flags, tile = e.tile;
+                const int num_kb = (int)e.num_kb;
+                const uint64_t map_a = e.map_a, map_b = e.map_b;
+                mbar_arrive(ring_empty(k));
+                if (flags & kTileEnd) break;
+                // the operands were stored by other CTAs of this launch: the scheduler has seen their counts
+                if (CHAINED && (flags & kTileDependent)) fence_proxy_async_all();
+                // A tile whose B is its A: the two producers take every other k-block.  (Both have to take part: a
+                // producer that the pipeline could do without might fall two phases of a stage's barrier behind, or run
+                // two ahead, and a parity wait cannot tell two phases apart.)
+                const bool shared = (flags & kTileShared) != 0u;
+                const bool as_b = for_b && !shared;
+                const uint64_t map = as_b ? map_b : map_a;
+                const bool mn = (flags & (as_b ? kTileBMn : kTileAMn)) != 0u;
+                const int n_half = (int)(flags >> kTileNShift) * 16;   // half of the MMA's N
+                const int row0 = as_b ? (int)(tile >> 16) * BN + (PAIR ? (int)rank * n_half : 0)
+                                      : (int)(tile & 0xffffu) * C::kTileM + (int)rank * 128;
+                // PAIR: both CTAs' copies complete on the leader's barrier, which expects the bytes of both
+                const uint32_t bytes = (as_b ? (uint32_t)C::kBBytes : (uint32_t)kABytes) * (PAIR ? 2u : 1u);
+                const uint32_t dst0 = smem_u32(stage_base) + (as_b ? (uint32_t)kABytes : 0u);
+                const int boxes = as_b ? C::kBRows / 128 : 1;
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    turn ^= 1u;
+                    if (!shared || turn == (for_b ? 1u : 0u)) {
                         if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { ok = false; break; }
-                        // PAIR: both CTAs' copies complete on the leader's barrier, which expects
-                        // the bytes of both
-                        const uint32_t fb = PAIR ? map_to_cta(full_bar(stage), 0) : full_bar(stage);
-                        if (!PAIR || rank == 0) mbar_expect_tx(full_bar(stage), stage_tx);
-                        const uint32_t sa = smem_u32(stage_base + stage * C::kStageBytes);
-                        const uint32_t sb = sa + kABytes;
+                        if (!PAIR || rank == 0) {
+                            mbar_expect_tx(full_bar(stage), bytes);
+                            if (shared) mbar_arrive(full_bar(stage));   // in the other producer's place
+                        }
+                        const uint32_t fb = leader_full + 8u * stage, dst = dst0 + stage * (uint32_t)C::kStageBytes;
                         const int k0 = kb * kGemmBlockK;
-                        if (a_mn) {  // 64 x 64 boxes: x = M index, y = K index
-                            tma_load_2d<PAIR>(sa, map_a, fb, m0, k0);
-                            tma_load_2d<PAIR>(sa + kBoxBytes, map_a, fb, m0 + 64, k0);
-                        } else {     // one 64 (K) x 128 (rows) box
-                            tma_load_2d<PAIR>(sa, map_a, fb, k0, m0);
-                        }
-#pragma unroll
-                        for (int j = 0; j < C::kBRows / 128; ++j) {
-                            if (shared_operand) break;
-                            if (b_mn) {
-                                tma_load_2d<PAIR>(sb + (2 * j) * kBoxBytes, map_b, fb, n0 + 128 * j, k0);
-                                tma_load_2d<PAIR>(sb + (2 * j + 1) * kBoxBytes, map_b, fb, n0 + 128 * j + 64, k0);
-                            } else {
-                                tma_load_2d<PAIR>(sb + (2 * j) * kBoxBytes, map_b, fb, k0, n0 + 128 * j);
+                        if (mn) {   // 64 x 64 boxes: x = M or N index, y = K index
+                            for (int j = 0; j < boxes; ++j) {
+                                tma_load_2d<PAIR>(dst + (2 * j) * kBoxBytes, map, fb, row0 + 128 * j, k0);
+                                tma_load_2d<PAIR>(dst + (2 * j + 1) * kBoxBytes, map, fb, row0 + 128 * j + 64, k0);
                             }
+                        } else {    // 64 (K) x 128 (rows) boxes
+                            for (int j = 0; j < boxes; ++j)
+                                tma_load_2d<PAIR>(dst + (2 * j) * kBoxBytes, map, fb, k0, row0 + 128 * j);
                         }
-                        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
                     }
-                }
-                if (fused_list && ok) {
-                    ++seq;
-                    if (claims) {
-                        t = drawn;
-                        announce(t);
-                    } else {
-                        t = ring_get(tile_ring, seq, abort_flag);
-                    }
-                    describe_next();
+                    if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
                 }
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == C::kMmaWarp) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0 && rank == 0) {
+        // The whole warp walks the loop and one elected lane issues: with warp-uniform control flow and operands the
+        // issue of a k-block is about 100 clocks shorter than from a single diverged lane.
+        if (rank == 0) {
+            const uint64_t desc0 = smem_desc(__shfl_sync(0xffffffffu, smem_u32(stage_base), 0), 0, 1024);
+            const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
-            uint32_t seq = 0;
-            for (uint32_t t = CHAINED ? ring_get(tile_ring, 0u, abort_flag) : first_tile; ok && t < tile_count;
-                 t = CHAINED ? ring_get(tile_ring, ++seq, abort_flag) : t + tile_stride) {
-                const TileWork tl = tile_work<CHAINED>(tiles, t, epilogue_arg, scale_pow_arg);
-                const uint32_t parts = CHAINED ? tile_parts(tl) : 1u;
-                for (uint32_t part = 0; ok && part < parts; ++part) {
-                    const GemmProblem *p = problems + (CHAINED ? tile_part(tl, part).problem : tl.problem);
-                    const uint32_t a_mn = p->a_mn_major, b_mn = p->b_mn_major, K = p->K;
-                    const int num_kb = (int)((K + kGemmBlockK - 1) / kGemmBlockK);
-                    const uint32_t idesc = instr_desc(C::kTileM, BN, f16, a_mn, b_mn);
-                    const bool shared_operand = PAIR && tl.tile_m == tl.tile_n && p->map_a == p->map_b && a_mn == b_mn;
-                    if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) { ok = false; break; }
+            for (uint32_t k = 0; ok; ++k) {
+                if (!__all_sync(0xffffffffu, mbar_wait(ring_full(k), ring_parity(k), abort_flag))) break;
+                const uint32_t flags = __shfl_sync(0xffffffffu, ring[k % kRing].flags, 0);
+                const uint32_t num_kb = __shfl_sync(0xffffffffu, ring[k % kRing].num_kb, 0);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ring_empty(k));
+                if (flags & kTileEnd) break;
+                const uint32_t a_mn = flags & kTileAMn ? 1u : 0u, b_mn = flags & kTileBMn ? 1u : 0u;
+                const uint32_t idesc = instr_desc(C::kTileM, (int)(flags >> kTileNShift) * 32, f16, a_mn, b_mn);
+                // leading byte offset (unused by a K-major operand) and the step of 16 in K, in units of 16 bytes
+                const uint64_t a0 = desc0 + ((uint64_t)(a_mn ? kBoxBytes >> 4 : 1) << 16);
+                const uint64_t b0 = desc0 + ((uint64_t)(b_mn ? kBoxBytes >> 4 : 1) << 16) + (flags & kTileShared ? 0u : (uint32_t)(kABytes >> 4));
+                const uint32_t a_step = a_mn ? 128u : 2u, b_step = b_mn ? 128u : 2u;
+                if (!__all_sync(0xffffffffu, mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag))) break;
+                tc_fence_after();
+                const uint32_t d_tmem = tmem + acc * BN;
+                for (uint32_t kb = 0; kb < num_kb; ++kb) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(full_bar(stage), phase, abort_flag))) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + acc * BN;
-                    for (int kb = 0; kb < num_kb; ++kb) {
-                        if (!mbar_wait(full_bar(stage), phase, abort_flag)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t sa = smem_u32(stage_base + stage * C::kStageBytes);
-                        const uint32_t sb = shared_operand ? sa : sa + kABytes;
+                    const uint64_t ad = a0 + stage * (uint32_t)(C::kStageBytes >> 4), bd = b0 + stage * (uint32_t)(C::kStageBytes >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                        for (int k = 0; k < kGemmBlockK / 16; ++k) {
-                            const uint64_t ad = a_mn ? smem_desc(sa + k * 2048, kBoxBytes, 1024)
-                                                     : smem_desc(sa + k * 32, 16, 1024);
-                            const uint64_t bd = b_mn ? smem_desc(sb + k * 2048, kBoxBytes, 1024)
-                                                     : smem_desc(sb + k * 32, 16, 1024);
-                            tc_mma<PAIR>(d_tmem, ad, bd, idesc, (uint32_t)((kb | k) != 0));
-                        }
+                        for (uint32_t j = 0; j < kGemmBlockK / 16; ++j)
+                            tc_mma<PAIR>(d_tmem, ad + j * a_step, bd + j * b_step, idesc, j != 0 ? 1u : (uint32_t)(kb != 0));
                         tc_commit<PAIR>(empty_bar(stage));
-                        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
+                        if (kb + 1 == num_kb) tc_commit<PAIR>(tfull_bar(acc));
                     }
-                    if (!ok) break;
-                    tc_commit<PAIR>(tfull_bar(acc));
-                    acc ^= 1u;
-                    if (acc == 0) acc_phase ^= 1u;
+                    __syncwarp();
+                    if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
                 }
+                acc ^= 1u;
+                if (acc == 0) acc_phase ^= 1u;
             }
         }
     } else {
@@ -620,14 +634,14 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
         // one 64-column chunk of the tile, so an accumulator buffer is free again after ONE chunk
         // has been read and a tile's epilogue takes a quarter of the time it would on one warp.
         const int q = warp & 3;
-        const int chunk = (warp - 2) >> 2;
+        const int chunk = (warp - C::kEpiWarp0) >> 2;
         const int c0 = chunk * 64;
         // Results leave through a per-warp 4 KB slab in shared memory and plain 128-bit global stores: the warp
         // writes its 32 rows into the slab (one row per lane, 16-byte chunks XOR-swizzled by the row so that the
         // fill and the copy-out are both conflict-free), then copies it out with eight lanes per row, so every
         // store instruction writes whole 128-byte lines.  Plain stores need no bulk-group wait before the slab
         // is refilled or the launch ends, and a fence orders them before the progress count of a chained launch.
-        uint8_t *slab = staging + (size_t)(warp - 2) * kSlabBytes;
+        uint8_t *slab = staging + (size_t)(warp - C::kEpiWarp0) * kSlabBytes;
         // 32 rows x 128 bytes, swizzled -> row-major tensor; rows >= row_limit and bytes >= byte_limit are dropped
         auto slab_to_global = [&](uint8_t *base, size_t pitch_bytes, int row0, int row_limit, int byte0, int byte_limit) {
 #pragma unroll 2
@@ -665,76 +679,66 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
             if (lane == 0) atomicAdd(&sync->progress[unpublished], 1u);
             unpublished = kNoSlot;
         };
-        uint32_t seq = 0;
-        bool alive = true;
-        for (uint32_t t = CHAINED ? ring_get(tile_ring, 0u, abort_flag) : first_tile; alive && t < tile_count;
-             t = CHAINED ? ring_get(tile_ring, ++seq, abort_flag) : t + tile_stride) {
-            const TileWork tl = tile_work<CHAINED>(tiles, t, epilogue_arg, scale_pow_arg);
+        for (uint32_t k = 0;; ++k) {
+            if (CHAINED && unpublished != kNoSlot && !__all_sync(0xffffffffu, mbar_test(ring_full(k), ring_parity(k)))) publish();
+            if (!__all_sync(0xffffffffu, mbar_wait(ring_full(k), ring_parity(k), abort_flag))) break;
+            const TileEntry &entry = ring[k % kRing];
+            const uint32_t flags = entry.flags, M = entry.M, N = entry.N, slot = entry.slot;
+            uint8_t *out = reinterpret_cast<uint8_t *>(entry.out);
+            const size_t pitch = entry.pitch_bytes;
+            const float4 *frag = reinterpret_cast<const float4 *>(entry.frag);
+            const int tile_m = (int)(entry.tile & 0xffffu), tile_n = (int)(entry.tile >> 16);
+            // fragment scratch is indexed by 128-row sub-tiles
+            const uint32_t tile_lin = (PAIR ? (uint32_t)tile_m * 2 + rank : (uint32_t)tile_m) * entry.tiles_n + tile_n;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ring_empty(k));
+            if (flags & kTileEnd) break;
+            const uint32_t epilogue = CHAINED ? (flags >> kTileEpiShift) & 15u : epilogue_arg;
+            const uint32_t scale_pow = (flags >> kTileScaleShift) & 3u;
             // the iteration's coefficient triple, picked without indexing the argument block by a register
             float ca = coef.v[0], cb = coef.v[1], cc = coef.v[2];
             if (CHAINED) {
+                const uint32_t iter = (flags >> kTileIterShift) & 31u;
 #pragma unroll
                 for (uint32_t i = 1; i < kMaxChainIterations; ++i)
-                    if (tl.iter == i) { ca = coef.v[3 * i]; cb = coef.v[3 * i + 1]; cc = coef.v[3 * i + 2]; }
+                    if (iter == i) { ca = coef.v[3 * i]; cb = coef.v[3 * i + 1]; cc = coef.v[3 * i + 2]; }
             }
-            const uint32_t parts = CHAINED ? tile_parts(tl) : 1u;
-#pragma unroll 1
-            for (uint32_t part = 0; part < parts; ++part) {
-            const uint32_t epilogue = CHAINED ? tile_part(tl, part).epilogue : tl.epilogue;
-            const GemmProblem *p = problems + (CHAINED ? tile_part(tl, part).problem : tl.problem);
             const bool hold = CHAINED && epilogue == kEpiGramHold;    // the accumulator stays for the next part
             const bool fused = CHAINED && epilogue == kEpiPolyFused;  // combines with the held accumulator
-            const uint32_t M = p->M, N = p->N;
-            uint8_t *out16 = reinterpret_cast<uint8_t *>(p->out16), *out32 = reinterpret_cast<uint8_t *>(p->out32);
-            const size_t pitch16 = (size_t)p->pitch16 * 2, pitch32 = (size_t)p->pitch32 * 4;
             // symmetric outputs (Gram, Poly): tiles below the diagonal are not computed; the tile
             // above writes them as its transpose (reference: tiles/symmetric.rs:76-92)
-            const bool mirror = tl.mirror != 0;
-            const float4 *frag = reinterpret_cast<const float4 *>(p->frag32);
-            // fragment scratch is indexed by 128-row sub-tiles
-            const uint32_t sub_m = PAIR ? (uint32_t)tl.tile_m * 2 + rank : tl.tile_m;
-            const uint32_t tile_lin = sub_m * p->tiles_n + tl.tile_n;
-            const int m0 = tl.tile_m * C::kTileM + (int)rank * 128, n0 = tl.tile_n * BN;
+            const bool mirror = (flags & kTileMirror) != 0u;
+            const int m0 = tile_m * C::kTileM + (int)rank * 128, n0 = tile_n * BN;
             const int row_in_tile = 32 * q + lane;
             const int grow = m0 + row_in_tile;
             const int slab_row0 = m0 + 32 * q;
             // fragment order: [128-row sub-tile][32-column unit][float4 index][row]
             const size_t unit0 = ((size_t)tile_lin * (BN / 32) + (size_t)(c0 / 32)) * 8;
 
-            // The polynomial epilogue needs the FP32 Gram tile: fetch the first 32 columns before
-            // the accumulator is ready so the latency hides behind the MMAs.
+            // The polynomial epilogue needs the FP32 Gram tile: fetch the first 32 columns before the accumulator is
+            // ready so the latency hides behind the MMAs.  (Chained: an entry is in the ring only once the matrix's
+            // Gram phase is complete.)
             float4 g[8];
-            // chained: the Gram tile may be read early only if the matrix's Gram phase is already complete
-            bool g_fetched = epilogue == kEpiPoly && !dbg_no_store;
-            if (CHAINED && g_fetched) g_fetched = *passed_tile > t;   // this CTA's producer has seen the phase complete
-            if (g_fetched) {
+            if (epilogue == kEpiPoly) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) g[j] = __ldcg(frag + (unit0 + j) * kGemmBlockM + row_in_tile);
             }
-            if (CHAINED && unpublished != kNoSlot && !mbar_test(tfull_bar(acc), acc_phase)) publish();
-
-            bool ready = mbar_wait(tfull_bar(acc), acc_phase, abort_flag);
-            ready = __all_sync(0xffffffffu, ready);
-            if (!ready) { alive = false; break; }
+            if (CHAINED && unpublished != kNoSlot && !__all_sync(0xffffffffu, mbar_test(tfull_bar(acc), acc_phase))) publish();
+            if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), acc_phase, abort_flag))) break;
             tc_fence_after();
-            if (CHAINED && epilogue == kEpiPoly && !dbg_no_store && !g_fetched) {
-                // the accumulator is complete, so the producer has seen the Gram phase complete
-#pragma unroll
-                for (int j = 0; j < 8; ++j) g[j] = __ldcg(frag + (unit0 + j) * kGemmBlockM + row_in_tile);
-            }
             const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + acc * BN + c0;
             // fused: the Gram accumulator of this tile sits in the other buffer
             const uint32_t held_taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (acc ^ 1u) * BN + c0;
             const uint32_t tempty = tempty_leader0 + 8u * acc;
             const uint32_t held_tempty = tempty_leader0 + 8u * (acc ^ 1u);
-            const bool in_range = n0 + c0 < (int)N && slab_row0 < (int)M && !dbg_no_store;   // warp-uniform
+            const bool in_range = n0 + c0 < (int)N && slab_row0 < (int)M;   // warp-uniform
             // One-pass prepare: the operand of the first iteration is the un-normalised update, and
             // s = 1 / (1.01 |u| + 1e-7) of the tile's matrix enters here: G = (s s) X X^T, X1 = s (Q X).
             // (A fused polynomial part scales the held Gram accumulator, not its own.)
             float out_scale = 1.0f;
-            if (slot_scale != nullptr && tl.scale_pow != 0u && epilogue != kEpiPoly) {
-                const float sv = __ldcg(slot_scale + tl.slot);
-                out_scale = tl.scale_pow == 2u ? sv * sv : sv;
+            if (slot_scale != nullptr && scale_pow != 0u && epilogue != kEpiPoly) {
+                const float sv = __ldcg(slot_scale + slot);
+                out_scale = scale_pow == 2u ? sv * sv : sv;
             }
             const bool scaled = out_scale != 1.0f;   // warp-uniform
 
@@ -763,8 +767,7 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                         *reinterpret_cast<uint4 *>(slab + lane * 128 + ((j ^ (lane & 7)) << 4)) = w;
                     }
                     __syncwarp();
-                    if (!dbg_no_global)
-                        slab_to_global(out32, pitch32, slab_row0, (int)M, (n0 + c0 + 32 * sub) * 4, (int)pitch32);
+                    slab_to_global(out, pitch, slab_row0, (int)M, (n0 + c0 + 32 * sub) * 4, (int)pitch);
                 }
             } else {
                 // 16-bit result: the chunk's 64 columns are read in two halves of 32 and packed
@@ -810,17 +813,15 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * out_scale);
                     }
-                    if ((epilogue == kEpiGram || epilogue == kEpiPoly) && !dbg_no_store) {
+                    if (epilogue == kEpiGram || epilogue == kEpiPoly) {
                         const size_t unit = unit0 + 8 * sub;
                         if (epilogue == kEpiGram) {
-                            if (!dbg_no_global) {
-                                float4 *fw = const_cast<float4 *>(frag);
+                            float4 *fw = const_cast<float4 *>(frag);
 #pragma unroll
-                                for (int j = 0; j < 8; ++j)
-                                    __stcg(fw + (unit + j) * kGemmBlockM + row_in_tile,
-                                           make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                                       __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
-                            }
+                            for (int j = 0; j < 8; ++j)
+                                __stcg(fw + (unit + j) * kGemmBlockM + row_in_tile,
+                                       make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                   __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
                         } else {
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
@@ -854,7 +855,7 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                         *reinterpret_cast<uint4 *>(slab + lane * 128 + ((j ^ (lane & 7)) << 4)) = w;
                     }
                     __syncwarp();
-                    if (!dbg_no_global) slab_to_global(out16, pitch16, slab_row0, (int)M, (n0 + c0) * 2, (int)pitch16);
+                    slab_to_global(out, pitch, slab_row0, (int)M, (n0 + c0) * 2, (int)pitch);
                     if (mirror) {
                         // transposed 64 x 32 block (rows = this chunk's columns), plain row-major
                         // 64-byte rows: lanes pair up so every lane stores two rows of one column
@@ -867,20 +868,18 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                             *reinterpret_cast<uint32_t *>(slab + (c + (lane & 1)) * 64 + (lane & ~1) * 2) = out;
                         }
                         __syncwarp();
-                        if (!dbg_no_global)
-                            slab_t_to_global(out16, pitch16, n0 + c0, (int)M, slab_row0 * 2, (int)pitch16);
+                        slab_t_to_global(out, pitch, n0 + c0, (int)M, slab_row0 * 2, (int)pitch);
                     }
                 }
             }
             if (CHAINED) {
                 if (unpublished != kNoSlot) publish();   // (a tile whose stores were all skipped)
-                unpublished = tl.slot;
+                unpublished = slot;
                 // the other CTAs wait for a held Gram tile before they can go on: publish it at once
                 if (hold) publish();
             }
             acc ^= 1u;
             if (acc == 0) acc_phase ^= 1u;
-            }
         }
         if (CHAINED && unpublished != kNoSlot) publish();
     }
@@ -905,7 +904,7 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
             sync->exited = 0;
         }
     }
-    if (warp == 1) {
+    if (warp == C::kMmaWarp) {
         if (PAIR)
             asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                          "r"((uint32_t)C::kTmemCols) : "memory");
@@ -952,7 +951,7 @@ cudaError_t launch_impl(const GemmProblem *problems, const void *tiles, uint32_t
     cfg.dynamicSmemBytes = Cfg<BN, PAIR>::kSmemBytes;
     cfg.stream = s;
     return cudaLaunchKernelEx(&cfg, k_ns_gemm<BN, PAIR, CHAINED>, problems, tiles, tile_count, epilogue, f16, coef,
-                              slot_scale, scale_pow, status, static_cast<ChainSync *>(sync), slot_count, debug_flags);
+                              slot_scale, scale_pow, status, static_cast<ChainSync *>(sync), slot_count);
 }
 
 template <bool CHAINED>
