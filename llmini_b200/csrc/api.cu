@@ -275,7 +275,7 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
     L.off_gp = take((size_t)std::max(3u * L.gp_tiles, 1u) * sizeof(ChainTile));
     L.off_meta_end = off;
     // ---- per-step scratch ----
-    L.off_partials = take((size_t)std::max(chunks, 1u) * B2_ONE_PASS_PARTIALS * sizeof(double));
+    L.off_partials = take((size_t)std::max(chunks, 1u) * B2_CHUNK_PARTIALS * sizeof(double));
     L.off_inv_norm = take(count * sizeof(float));
     L.off_amax_x = take(count * sizeof(float));
     L.off_status = take(sizeof(uint32_t));
@@ -622,22 +622,11 @@ int b2_muon_prepare_polar(b2_muon_plan *plan, const b2_muon_slot_descriptor *d_s
     const Layout &L = plan->layout;
     cudaStream_t s = as_stream(stream);
     SlotView v = plan->view(d_slots);
-    double *partials = plan->at<double>(L.off_partials);
-    float *inv = plan->at<float>(L.off_inv_norm);
-    const MomentumParams mp = momentum_params(a);
-    if (plan->options.normalize_mode == B2_NORMALIZE_DEFERRED) {
-        // one pass over the gradients; the scalar goes to the first Newton-Schulz iteration (b2_muon_polar)
-        cudaError_t e = launch_muon_momentum_sumsq(v, mp, plan->at<uint64_t>(L.off_x0_ptrs), partials,
-                                                   plan->at<float>(L.off_amax_x), s);
-        if (e == cudaSuccess) e = launch_muon_inv_norm(v, partials, inv, B2_ONE_PASS_PARTIALS, s);
-        return (int)e;
-    }
-    cudaError_t e = launch_muon_sumsq(v, mp, partials, plan->at<float>(L.off_amax_x), s);
-    if (e == cudaSuccess) e = launch_muon_inv_norm(v, partials, inv, 1u, s);
-    if (e == cudaSuccess)
-        e = launch_muon_momentum_normalize(v, mp, inv, plan->at<uint64_t>(L.off_x0_ptrs),
-                                           plan->options.operand_format == B2_OPERAND_F16, s);
-    return (int)e;
+    // after the one-pass form the scalar goes to the first Newton-Schulz iteration (b2_muon_polar)
+    return (int)launch_muon_prepare(v, momentum_params(a), plan->options.normalize_mode == B2_NORMALIZE_DEFERRED,
+                                    plan->at<uint64_t>(L.off_x0_ptrs), plan->at<uint64_t>(L.off_u_ptrs),
+                                    plan->options.operand_format == B2_OPERAND_F16, plan->at<double>(L.off_partials),
+                                    plan->at<float>(L.off_inv_norm), plan->at<float>(L.off_amax_x), s);
 }
 
 int b2_muon_polar(b2_muon_plan *plan, const b2_muon_step_args *a, void *stream) {

@@ -44,17 +44,12 @@ struct UpdateParams {
     float symexp_beta;             // > 0: SymExpLin forward on y, scales from the slot table (or unit)
     const b2_symexp_lin_slot_descriptor *symexp_slots;
 };
-cudaError_t launch_muon_sumsq(const SlotView &v, const MomentumParams &mp, double *partials, float *amax_x,
-                              cudaStream_t s);
-// One-pass form of stages M+N: momentum state, un-normalised BF16 operand and the chunk sums in one launch.
-cudaError_t launch_muon_momentum_sumsq(const SlotView &v, const MomentumParams &mp, const uint64_t *x0_ptrs,
-                                       double *partials, float *amax_x, cudaStream_t s);
-// `partials_per_chunk`: 1 after launch_muon_sumsq, B2_ONE_PASS_PARTIALS after launch_muon_momentum_sumsq.
-#define B2_ONE_PASS_PARTIALS 8
-cudaError_t launch_muon_inv_norm(const SlotView &v, const double *partials, float *inv_norm,
-                                 uint32_t partials_per_chunk, cudaStream_t s);
-cudaError_t launch_muon_momentum_normalize(const SlotView &v, const MomentumParams &mp, const float *inv_norm,
-                                           const uint64_t *x0_ptrs, int f16, cudaStream_t s);
+// Stages M+N.  `one_pass`: the operand is left un-normalised (BF16 only); otherwise with the reference's rounding point.
+// `u_ptrs`: the slots' FP32 result buffers, used as scratch by the variance-adaptive two-pass form.
+#define B2_CHUNK_PARTIALS 8   // f64 partial sums per chunk
+cudaError_t launch_muon_prepare(const SlotView &v, const MomentumParams &mp, bool one_pass, const uint64_t *x0_ptrs,
+                                const uint64_t *u_ptrs, int f16, double *partials, float *inv_norm, float *amax_x,
+                                cudaStream_t s);
 cudaError_t launch_muon_update(const SlotView &v, const uint64_t *u_ptrs, float *amax_x, const UpdateParams &up,
                                cudaStream_t s);
 // Stages U and Q in one launch over an item list (bit 31: encode span of B2_FUSED_ENCODE_SPAN chunks, else update

@@ -42,20 +42,35 @@ __device__ __forceinline__ float momentum_update_vs(float graw, float pm, float 
     const float numerator = nesterov ? g + (mu / one_minus_mu) * corrected : corrected;
     return numerator / (sqrtf(fmaxf(next_v * bias_correction_inv, 0.0f)) + 1.0e-8f);
 }
-// Four consecutive elements of stage M in either variant.
+// Four consecutive elements of stage M in either variant: loads and arithmetic apart, because a kernel has to issue the
+// loads of all its quads before the first store (which could alias them as far as the compiler knows, so it would not
+// hoist them itself, and each quad would wait out a round trip to memory).
 struct Quad { float u[4], m[4], v[4]; };
 template <int VS>
-__device__ __forceinline__ Quad momentum_quad(const float *grad, const uint16_t *mom, const uint16_t *var, uint32_t i,
-                                              const MomentumParams &mp, bool streaming) {
+struct QuadRaw {
+    float4 g;
+    uint2 m;
+    uint2 v[1];   // VS only
+};
+template <int VS>
+__device__ __forceinline__ QuadRaw<VS> quad_load(const float *grad, const uint16_t *mom, const uint16_t *var, uint32_t i,
+                                                 bool streaming) {
+    QuadRaw<VS> r;
+    r.g = streaming ? __ldcs(reinterpret_cast<const float4 *>(grad + i)) : *reinterpret_cast<const float4 *>(grad + i);
+    r.m = *reinterpret_cast<const uint2 *>(mom + i);
+    if (VS) r.v[0] = *reinterpret_cast<const uint2 *>(var + i);
+    return r;
+}
+template <int VS>
+__device__ __forceinline__ Quad momentum_quad(const QuadRaw<VS> &r, const MomentumParams &mp) {
     Quad q;
-    const float4 g = streaming ? __ldcs(reinterpret_cast<const float4 *>(grad + i))
-                               : *reinterpret_cast<const float4 *>(grad + i);
-    const uint2 m = *reinterpret_cast<const uint2 *>(mom + i);
+    const float4 g = r.g;
+    const uint2 m = r.m;
     const float gr[4] = {g.x, g.y, g.z, g.w};
     const float pm[4] = {bf16_bits_to_f32(m.x & 0xffffu), bf16_bits_to_f32(m.x >> 16),
                          bf16_bits_to_f32(m.y & 0xffffu), bf16_bits_to_f32(m.y >> 16)};
     if (VS) {
-        const uint2 v = *reinterpret_cast<const uint2 *>(var + i);
+        const uint2 v = r.v[0];
         const float pv[4] = {bf16_bits_to_f32(v.x & 0xffffu), bf16_bits_to_f32(v.x >> 16),
                              bf16_bits_to_f32(v.y & 0xffffu), bf16_bits_to_f32(v.y >> 16)};
 #pragma unroll
@@ -104,173 +119,100 @@ __device__ __forceinline__ ChunkCtx chunk_ctx(const b2_muon_slot_descriptor *slo
     return x;
 }
 
-// Pass 1 of stages M+N: sum of u^2 per chunk: an f32 fma chain over a thread's eight values,
-// then f64 across threads, warps and chunks, so the grid shape does not change the result.  Also clears the two amax
-// words the update kernel later raises with atomicMax.
-template <int VS>
-__global__ void __launch_bounds__(kThreads, VS ? 4 : 6)
-k_muon_sumsq(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint32_t slot_count,
-             uint32_t total_chunks, MomentumParams mp, double *partials, float *amax_x) {
-    // Two chunks per trip: both chunks' loads are in flight together and one pair of barriers
-    // serves both block reductions.  Every chunk still leaves its own partial, summed in the same
-    // order as before, so the result does not depend on the pairing.
-    __shared__ double warp_part[2][kThreads / 32];
-    const int tid = threadIdx.x;
-    if (mp.d_grad_scale) mp.grad_scale = __ldg(mp.d_grad_scale);
-    for (uint32_t c0 = 2 * blockIdx.x; c0 < total_chunks; c0 += 2 * gridDim.x) {
-        float local[2] = {0.0f, 0.0f};
-        uint32_t reset_slot[2] = {0xffffffffu, 0xffffffffu};
-        uint64_t reset_amax[2] = {0, 0};
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const uint32_t c = c0 + k;
-            if (c >= total_chunks) break;   // CTA-uniform
-            ChunkCtx cx = chunk_ctx(slots, prefix, slot_count, c);
-            const float *grad = reinterpret_cast<const float *>(cx.d.grad);
-            const uint16_t *mom = reinterpret_cast<const uint16_t *>(cx.d.momentum);
-            const uint16_t *var = reinterpret_cast<const uint16_t *>(cx.d.variance);
-            const uint32_t base = cx.local_chunk * kChunk;
-            if (cx.local_chunk == 0) {
-                reset_slot[k] = cx.slot;
-                reset_amax[k] = cx.d.schedule_amax;
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t i = base + h * (kChunk / 2) + tid * 4;
-                if (i < cx.len) {
-                    const Quad q = momentum_quad<VS>(grad, mom, var, i, mp, false);
-                    // per-thread chain as in the reference (momentum.rs:63: fma(update, update, sum));
-                    // eight terms at most, so the chain's rounding stays below 1e-7 relative
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) local[k] = fmaf(q.u[e], q.u[e], local[k]);
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const double acc = warp_sum((double)local[k]);
-            if ((tid & 31) == 0) warp_part[k][tid >> 5] = acc;
-        }
-        __syncthreads();
-        if (tid < 2 && c0 + tid < total_chunks) {
-            double s = 0.0;
-#pragma unroll
-            for (int w = 0; w < kThreads / 32; ++w) s += warp_part[tid][w];
-            partials[c0 + tid] = s;
-            const uint32_t rs = tid == 0 ? reset_slot[0] : reset_slot[1];
-            const uint64_t ra = tid == 0 ? reset_amax[0] : reset_amax[1];
-            if (rs != 0xffffffffu) {
-                amax_x[rs] = 0.0f;
-                *reinterpret_cast<float *>(ra) = 0.0f;
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// One CTA per slot: fixed-order sum of the slot's chunk partials, then
-// inv = 1 / (sqrt(S) * 1.01 + 1e-7)
-// (crates/cuda-kernels/src/gpt/optimizer/muon/polar/fused/normalize.rs:8-9,82-86).
-__global__ void __launch_bounds__(kThreads)
-k_muon_inv_norm(const uint32_t *prefix, const double *partials, float *inv_norm, uint32_t per_chunk) {
-    __shared__ double warp_part[kThreads / 32];
+constexpr uint32_t kWarpsPerCta = kThreads / 32;
+static_assert(kWarpsPerCta == B2_CHUNK_PARTIALS, "partial sums per chunk");
+// One CTA per slot: fixed-order sum of the slot's partials, then inv = 1 / (sqrt(S) * 1.01 + 1e-7)
+// (crates/cuda-kernels/src/gpt/optimizer/muon/polar/fused/normalize.rs:8-9,82-86).  The loads of a slot are a chain of
+// round trips of one CTA, so it is as wide as a CTA can be.
+constexpr int kNormThreads = 1024;
+__global__ void __launch_bounds__(kNormThreads)
+k_muon_inv_norm(const uint32_t *prefix, const double *partials, float *inv_norm) {
+    __shared__ double warp_part[kNormThreads / 32];
     const uint32_t s = blockIdx.x;
-    const uint32_t begin = prefix[s] * per_chunk, end = prefix[s + 1] * per_chunk;
+    const uint32_t begin = prefix[s] * kWarpsPerCta, end = prefix[s + 1] * kWarpsPerCta;
     double acc = 0.0;
-    for (uint32_t c = begin + threadIdx.x; c < end; c += kThreads) acc += partials[c];
+#pragma unroll 8
+    for (uint32_t c = begin + threadIdx.x; c < end; c += kNormThreads) acc += partials[c];
     acc = warp_sum(acc);
     if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-#pragma unroll
-        for (int w = 0; w < kThreads / 32; ++w) t += warp_part[w];
-        float sum = (float)t;
-        inv_norm[s] = 1.0f / (sqrtf(sum) * 1.01f + 1.0e-7f);
+    if (threadIdx.x < 32) {
+        const float sum = (float)warp_sum(warp_part[threadIdx.x]);
+        if (threadIdx.x == 0) inv_norm[s] = 1.0f / (sqrtf(sum) * 1.01f + 1.0e-7f);
     }
 }
 
-// Pass 2 of stages M+N: stores the BF16 momentum state and X0 = r16(u * inv) in the storage
-// layout [rows][cols] (momentum.rs:56-63 and normalize.rs:137-143; operand rounding
-// .../polar/fused/stage.rs:51-55).  No transpose: the GEMMs read either orientation.
-template <int VS>
-__global__ void __launch_bounds__(kThreads, VS ? 4 : 8)
-k_muon_momentum_normalize(const b2_muon_slot_descriptor *slots, const uint32_t *prefix,
-                          uint32_t slot_count, uint32_t total_chunks, MomentumParams mp,
-                          const float *inv_norm, const uint64_t *x0_ptrs, int f16) {
-    const int tid = threadIdx.x;
-    if (mp.d_grad_scale) mp.grad_scale = __ldg(mp.d_grad_scale);
-    for (uint32_t c = blockIdx.x; c < total_chunks; c += gridDim.x) {
-        ChunkCtx cx = chunk_ctx(slots, prefix, slot_count, c);
-        const float *grad = reinterpret_cast<const float *>(cx.d.grad);
-        uint16_t *mom = reinterpret_cast<uint16_t *>(cx.d.momentum);
-        uint16_t *var = reinterpret_cast<uint16_t *>(cx.d.variance);
-        uint16_t *x0 = reinterpret_cast<uint16_t *>(x0_ptrs[cx.slot]);
-        const float inv = inv_norm[cx.slot];
-        const uint32_t base = cx.local_chunk * kChunk;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t i = base + h * (kChunk / 2) + tid * 4;
-            if (i < cx.len) {
-                const Quad q = momentum_quad<VS>(grad, mom, var, i, mp, true);
-                *reinterpret_cast<uint2 *>(mom + i) = pack_bf16x4(q.m);
-                if (VS) *reinterpret_cast<uint2 *>(var + i) = pack_bf16x4(q.v);
-                uint2 xo;
-                xo.x = pack_operands(q.u[0] * inv, q.u[1] * inv, f16);
-                xo.y = pack_operands(q.u[2] * inv, q.u[3] * inv, f16);
-                *reinterpret_cast<uint2 *>(x0 + i) = xo;
-            }
-        }
-    }
-}
-
-// Stages M+N in ONE pass over the gradients: BF16 momentum state, the UN-normalised 16-bit operand
-// X0 = r16(u) in the storage layout, and the sum of u^2 (taken over the FP32 u, as normalize.rs:35-79 does).
-// The Frobenius scale s = 1 / (1.01 |u| + 1e-7) is not known until every chunk of the matrix has been
-// summed, so it is left to the first Newton-Schulz iteration, which is linear in it: G = (s s) X0 X0^T and
-// X1 = s (Q X0) (the Gram and Apply epilogues multiply by the slot's scalar).  10 bytes per element cross
-// the memory interface instead of 16.  The operand is rounded before instead of after the scaling, which is
-// not the reference's rounding point; the two-pass kernels above keep that one.  BF16 operands only: an
-// un-normalised F16 operand could leave F16's range.
-// Every warp leaves its own f64 partial per chunk (kThreads / 32 per chunk, summed in a fixed order by
-// k_muon_inv_norm), so no CTA-wide barrier sits between a chunk's loads and the next chunk's.  Two chunks
-// per trip keep eight 128-bit loads per thread in flight.  Also clears the two amax words of each slot.
-constexpr uint32_t kWarpsPerCta = kThreads / 32;
-static_assert(kWarpsPerCta == B2_ONE_PASS_PARTIALS, "partials per chunk of the one-pass prepare");
-template <int VS>
-__global__ void __launch_bounds__(kThreads, VS ? 4 : 8)
+// First pass of stages M+N: the sum of u^2 (taken over the FP32 u, normalize.rs:35-79: an f32 fma chain over a thread's
+// eight values of a chunk, then f64 across lanes, warps and chunks), and what OUT says:
+//   kOutNothing : nothing else.  The reference's rounding point X0 = r16(u * s), s = 1 / (1.01 |u| + 1e-7), needs the norm
+//                 before the first element can be stored, so k_muon_normalize<0> reads gradient and momentum again:
+//                 16 bytes per element in all.
+//   kOutUpdate  : the BF16 states, and u in FP32 in the matrix's result buffer (free until the last Newton-Schulz launch);
+//                 k_muon_normalize<1> only scales it.  For the variance-adaptive update, whose square root and division
+//                 per element bounded both passes when both evaluated them: 22 bytes per element instead of 20, one
+//                 evaluation instead of two.
+//   kOutOperand : the BF16 states and the UN-normalised operand X0 = r16(u).  There is no second pass: the first
+//                 Newton-Schulz iteration is linear in s, G = (s s) X0 X0^T and X1 = s (Q X0) (the Gram and Apply
+//                 epilogues multiply by the slot's scalar).  10 bytes per element.  The operand is rounded before instead
+//                 of after the scaling.  BF16 operands only: an un-normalised F16 operand could leave F16's range.
+// Every warp leaves its own f64 partial per chunk (summed in a fixed order by k_muon_inv_norm), so no CTA-wide barrier
+// sits between a chunk's loads and the next chunk's.  Two chunks per trip, all of whose loads go out first.  Also clears
+// the two amax words that the update kernel later raises with atomicMax.
+enum { kOutNothing, kOutUpdate, kOutOperand };
+template <int VS, int OUT>
+__global__ void __launch_bounds__(kThreads, VS ? 3 : 4)
 k_muon_momentum_sumsq(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint32_t slot_count,
-                      uint32_t total_chunks, MomentumParams mp, const uint64_t *x0_ptrs, double *partials,
+                      uint32_t total_chunks, MomentumParams mp, const uint64_t *out_ptrs, double *partials,
                       float *amax_x) {
     const int tid = threadIdx.x;
     if (mp.d_grad_scale) mp.grad_scale = __ldg(mp.d_grad_scale);
     for (uint32_t c0 = 2 * blockIdx.x; c0 < total_chunks; c0 += 2 * gridDim.x) {
         float local[2] = {0.0f, 0.0f};
+        QuadRaw<VS> raw[2][2];
+        uint32_t base[2] = {0, 0}, len[2] = {0, 0};   // len 0: no such chunk
+        uint16_t *mom[2], *var[2];
+        uint64_t out[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const uint32_t c = c0 + k;
             if (c >= total_chunks) break;   // CTA-uniform
-            ChunkCtx cx = chunk_ctx(slots, prefix, slot_count, c);
-            const float *grad = reinterpret_cast<const float *>(cx.d.grad);
-            uint16_t *mom = reinterpret_cast<uint16_t *>(cx.d.momentum);
-            uint16_t *var = reinterpret_cast<uint16_t *>(cx.d.variance);
-            uint16_t *x0 = reinterpret_cast<uint16_t *>(x0_ptrs[cx.slot]);
-            const uint32_t base = cx.local_chunk * kChunk;
-            if (cx.local_chunk == 0 && tid == 0) {
-                amax_x[cx.slot] = 0.0f;
-                *reinterpret_cast<float *>(cx.d.schedule_amax) = 0.0f;
+            const uint32_t slot = find_slot(prefix, slot_count, c);
+            const b2_muon_slot_descriptor *d = slots + slot;
+            const float *grad = reinterpret_cast<const float *>(d->grad);
+            mom[k] = reinterpret_cast<uint16_t *>(d->momentum);
+            var[k] = reinterpret_cast<uint16_t *>(d->variance);
+            if (OUT != kOutNothing) out[k] = out_ptrs[slot];
+            len[k] = d->rows * d->cols;
+            base[k] = (c - prefix[slot]) * kChunk;
+            if (base[k] == 0 && tid == 0) {
+                amax_x[slot] = 0.0f;
+                *reinterpret_cast<float *>(d->schedule_amax) = 0.0f;
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const uint32_t i = base + h * (kChunk / 2) + tid * 4;
-                if (i < cx.len) {
-                    const Quad q = momentum_quad<VS>(grad, mom, var, i, mp, true);
-                    *reinterpret_cast<uint2 *>(mom + i) = pack_bf16x4(q.m);
-                    if (VS) *reinterpret_cast<uint2 *>(var + i) = pack_bf16x4(q.v);
-                    uint2 xo;
-                    xo.x = pack_operands(q.u[0], q.u[1], 0);
-                    xo.y = pack_operands(q.u[2], q.u[3], 0);
-                    *reinterpret_cast<uint2 *>(x0 + i) = xo;
+                const uint32_t i = base[k] + h * (kChunk / 2) + tid * 4;
+                if (i < len[k]) raw[k][h] = quad_load<VS>(grad, mom[k], var[k], i, OUT != kOutNothing);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t i = base[k] + h * (kChunk / 2) + tid * 4;
+                if (i < len[k]) {
+                    const Quad q = momentum_quad<VS>(raw[k][h], mp);
+                    if (OUT != kOutNothing) {
+                        *reinterpret_cast<uint2 *>(mom[k] + i) = pack_bf16x4(q.m);
+                        if (VS) *reinterpret_cast<uint2 *>(var[k] + i) = pack_bf16x4(q.v);
+                    }
+                    if (OUT == kOutUpdate)
+                        *reinterpret_cast<float4 *>(reinterpret_cast<float *>(out[k]) + i) = make_float4(q.u[0], q.u[1], q.u[2], q.u[3]);
+                    if (OUT == kOutOperand) {
+                        uint2 xo;
+                        xo.x = pack_operands(q.u[0], q.u[1], 0);
+                        xo.y = pack_operands(q.u[2], q.u[3], 0);
+                        *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(out[k]) + i) = xo;
+                    }
 #pragma unroll
                     for (int e = 0; e < 4; ++e) local[k] = fmaf(q.u[e], q.u[e], local[k]);
                 }
@@ -281,6 +223,50 @@ k_muon_momentum_sumsq(const b2_muon_slot_descriptor *slots, const uint32_t *pref
             if (c0 + k >= total_chunks) break;
             const double acc = warp_sum((double)local[k]);
             if ((tid & 31) == 0) partials[(size_t)(c0 + k) * kWarpsPerCta + (tid >> 5)] = acc;
+        }
+    }
+}
+
+// Second pass: X0 = r16(u * inv) in the storage layout [rows][cols] (momentum.rs:56-63 and normalize.rs:137-143; operand
+// rounding .../polar/fused/stage.rs:51-55).  No transpose: the GEMMs read either orientation.  STORED = 0 computes u
+// again and stores the BF16 momentum; STORED = 1 reads the u that the first pass left.
+template <int STORED>
+__global__ void __launch_bounds__(kThreads, 6)
+k_muon_normalize(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint32_t slot_count, uint32_t total_chunks,
+                 MomentumParams mp, const float *inv_norm, const uint64_t *x0_ptrs, const uint64_t *u_ptrs, int f16) {
+    const int tid = threadIdx.x;
+    if (mp.d_grad_scale) mp.grad_scale = __ldg(mp.d_grad_scale);
+    for (uint32_t c = blockIdx.x; c < total_chunks; c += gridDim.x) {
+        const uint32_t slot = find_slot(prefix, slot_count, c);
+        const b2_muon_slot_descriptor *d = slots + slot;
+        const uint32_t len = d->rows * d->cols, base = (c - prefix[slot]) * kChunk + tid * 4;
+        const float *grad = reinterpret_cast<const float *>(d->grad);
+        uint16_t *mom = reinterpret_cast<uint16_t *>(d->momentum);
+        uint16_t *x0 = reinterpret_cast<uint16_t *>(x0_ptrs[slot]);
+        const float inv = inv_norm[slot];
+        QuadRaw<0> raw[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t i = base + h * (kChunk / 2);
+            if (i >= len) continue;
+            if (STORED) raw[h].g = ld_stream(reinterpret_cast<const float *>(u_ptrs[slot]) + i);
+            else raw[h] = quad_load<0>(grad, mom, nullptr, i, true);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t i = base + h * (kChunk / 2);
+            if (i >= len) continue;
+            float u[4] = {raw[h].g.x, raw[h].g.y, raw[h].g.z, raw[h].g.w};
+            if (!STORED) {
+                const Quad q = momentum_quad<0>(raw[h], mp);
+                *reinterpret_cast<uint2 *>(mom + i) = pack_bf16x4(q.m);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) u[e] = q.u[e];
+            }
+            uint2 xo;
+            xo.x = pack_operands(u[0] * inv, u[1] * inv, f16);
+            xo.y = pack_operands(u[2] * inv, u[3] * inv, f16);
+            *reinterpret_cast<uint2 *>(x0 + i) = xo;
         }
     }
 }
@@ -1595,43 +1581,32 @@ static inline int clamp_grid(uint32_t chunks, int cap) {
     return (int)(chunks < (uint32_t)cap ? chunks : (uint32_t)cap);
 }
 
-cudaError_t launch_muon_sumsq(const SlotView &v, const MomentumParams &mp, double *partials, float *amax_x,
-                              cudaStream_t s) {
-    if (v.total_chunks == 0) return cudaSuccess;
-    if (mp.variance_adaptive)
-        k_muon_sumsq<1><<<clamp_grid((v.total_chunks + 1) / 2, v.grid), kThreads, 0, s>>>(
-            v.slots, v.chunk_prefix, v.slot_count, v.total_chunks, mp, partials, amax_x);
-    else
-        k_muon_sumsq<0><<<clamp_grid((v.total_chunks + 1) / 2, v.grid), kThreads, 0, s>>>(
-            v.slots, v.chunk_prefix, v.slot_count, v.total_chunks, mp, partials, amax_x);
-    return cudaGetLastError();
-}
-cudaError_t launch_muon_momentum_sumsq(const SlotView &v, const MomentumParams &mp, const uint64_t *x0_ptrs,
-                                       double *partials, float *amax_x, cudaStream_t s) {
-    if (v.total_chunks == 0) return cudaSuccess;
-    if (mp.variance_adaptive)
-        k_muon_momentum_sumsq<1><<<clamp_grid((v.total_chunks + 1) / 2, v.grid), kThreads, 0, s>>>(
-            v.slots, v.chunk_prefix, v.slot_count, v.total_chunks, mp, x0_ptrs, partials, amax_x);
-    else
-        k_muon_momentum_sumsq<0><<<clamp_grid((v.total_chunks + 1) / 2, v.grid), kThreads, 0, s>>>(
-            v.slots, v.chunk_prefix, v.slot_count, v.total_chunks, mp, x0_ptrs, partials, amax_x);
-    return cudaGetLastError();
-}
-cudaError_t launch_muon_inv_norm(const SlotView &v, const double *partials, float *inv_norm,
-                                 uint32_t partials_per_chunk, cudaStream_t s) {
+cudaError_t launch_muon_prepare(const SlotView &v, const MomentumParams &mp, bool one_pass, const uint64_t *x0_ptrs,
+                                const uint64_t *u_ptrs, int f16, double *partials, float *inv_norm, float *amax_x,
+                                cudaStream_t s) {
     if (v.slot_count == 0) return cudaSuccess;
-    k_muon_inv_norm<<<v.slot_count, kThreads, 0, s>>>(v.chunk_prefix, partials, inv_norm, partials_per_chunk);
-    return cudaGetLastError();
-}
-cudaError_t launch_muon_momentum_normalize(const SlotView &v, const MomentumParams &mp, const float *inv_norm,
-                                           const uint64_t *x0_ptrs, int f16, cudaStream_t s) {
-    if (v.total_chunks == 0) return cudaSuccess;
+    if (v.total_chunks != 0) {
+        const int grid = clamp_grid((v.total_chunks + 1) / 2, v.grid);
+#define B2_LAUNCH_SUMSQ(VS, OUT, PTRS)                                                                              \
+    k_muon_momentum_sumsq<VS, OUT><<<grid, kThreads, 0, s>>>(v.slots, v.chunk_prefix, v.slot_count, v.total_chunks, \
+                                                             mp, PTRS, partials, amax_x)
+        if (one_pass) { if (mp.variance_adaptive) B2_LAUNCH_SUMSQ(1, kOutOperand, x0_ptrs); else B2_LAUNCH_SUMSQ(0, kOutOperand, x0_ptrs); }
+        else if (mp.variance_adaptive) B2_LAUNCH_SUMSQ(1, kOutUpdate, u_ptrs);
+        else B2_LAUNCH_SUMSQ(0, kOutNothing, nullptr);
+#undef B2_LAUNCH_SUMSQ
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    k_muon_inv_norm<<<v.slot_count, kNormThreads, 0, s>>>(v.chunk_prefix, partials, inv_norm);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || one_pass || v.total_chunks == 0) return e;
+    const int grid = clamp_grid(v.total_chunks, v.grid);
     if (mp.variance_adaptive)
-        k_muon_momentum_normalize<1><<<clamp_grid(v.total_chunks, v.grid), kThreads, 0, s>>>(
-            v.slots, v.chunk_prefix, v.slot_count, v.total_chunks, mp, inv_norm, x0_ptrs, f16);
+        k_muon_normalize<1><<<grid, kThreads, 0, s>>>(v.slots, v.chunk_prefix, v.slot_count, v.total_chunks, mp, inv_norm,
+                                                      x0_ptrs, u_ptrs, f16);
     else
-        k_muon_momentum_normalize<0><<<clamp_grid(v.total_chunks, v.grid), kThreads, 0, s>>>(
-            v.slots, v.chunk_prefix, v.slot_count, v.total_chunks, mp, inv_norm, x0_ptrs, f16);
+        k_muon_normalize<0><<<grid, kThreads, 0, s>>>(v.slots, v.chunk_prefix, v.slot_count, v.total_chunks, mp, inv_norm,
+                                                      x0_ptrs, u_ptrs, f16);
     return cudaGetLastError();
 }
 cudaError_t launch_muon_update(const SlotView &v, const uint64_t *u_ptrs, float *amax_x, const UpdateParams &up,
