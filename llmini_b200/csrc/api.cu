@@ -125,7 +125,7 @@ struct Layout {
     uint32_t total_chunks = 0;
     int bn = 256;
     int pair = 0;   // 1: two-CTA 256 x 256 tiles
-    int symmetric = 0;  // 1: Gram / Poly compute the upper triangle of tiles only
+    int symmetric = 0;  // 1: Gram / Poly compute the upper triangle of tiles only (square tiles)
     int tile_m = 128;
     size_t off_prefix, off_partials, off_inv_norm, off_amax_x, off_status, off_x0_ptrs, off_x1_ptrs, off_u_ptrs, off_maps,
         off_problems, off_tiles_nn, off_tiles_out, off_unit_prefix, off_factor_ptrs, off_unit_partials, off_slot_stats,
@@ -143,32 +143,60 @@ bool valid_shape(uint32_t rows, uint32_t cols, const b2_muon_options &o) {
     return true;
 }
 
-// Tile configuration: reserved[0] = 128 / 256 forces the single-CTA kernel with that width,
-// 512 forces the two-CTA pair; 0 picks the cheapest by padded tensor work, weighted by how
-// well each configuration feeds the tensor core (measured: the pair streams 1.5x fewer bytes
-// per FLOP than 128 x 256, which in turn beats 128 x 128).
-void pick_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t count, const b2_muon_options &o, int &bn,
-                int &pair) {
+// G and Q are symmetric: with square tiles, those below the diagonal can be written as transposes of those above instead
+// of being computed.  Pairs always do that.  With 128 x 128 tiles the transposed store makes a tile's epilogue longer,
+// which pays only where the tiles are more than one wave: one 3072 x 768 (36 tiles) 166 us in full, 176 as a triangle;
+// six layers of width 384 (216 tiles) 216 us in full, 189 as a triangle.
+constexpr uint32_t kTileRuleSms = 148;   // of a B200; not asked of the device, because the workspace size depends on it
+bool triangle_of_128(const uint32_t *rows, const uint32_t *cols, uint32_t count) {
+    uint64_t full = 0;
+    for (uint32_t s = 0; s < count; ++s) {
+        if ((uint64_t)rows[s] * cols[s] == 0) continue;
+        const uint64_t t = (std::min(rows[s], cols[s]) + 127u) / 128u;
+        full += t * t;
+    }
+    return full > kTileRuleSms;
+}
+// Tile configuration: tile_override = 128 / 256 forces the single-CTA kernel with that width, 512 the two-CTA pair; 0
+// picks the cheapest by estimated time.  A phase (one launch) takes a fixed time (launch, prologue, pipeline fill, last
+// epilogue) plus the longer of its longest tile and its share of all tiles; a tile takes so long per k-block (64 of K)
+// and for its epilogue.  Few tiles: the longest one decides, and small tiles on many SMs win; many tiles: the pair, which
+// loads half as many bytes per FLOP, wins.  The constants (us) are fitted to the Newton-Schulz stage of 24 plans of 1 to
+// 48 matrices, 64 to 6400 wide, in each configuration (mostly within 15 %).
+// Measured, pairs -> 128 x 128 (us): one 3072 x 768 242 -> 166, one layer of width 384 173 -> 119, 768 267 -> 206, 1024
+// 345 -> 325, the six largest matrices of a layer pair of width 768 298 -> 253; on the other side of the line two layers
+// of width 768 308 -> 318, four 494 -> 526, four of width 1024 883 -> 959.
+void pick_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t count, const b2_muon_options &o, int &bn, int &pair) {
     if (o.tile_override == 128 || o.tile_override == 256) { bn = (int)o.tile_override; pair = 0; return; }
     if (o.tile_override == 512) { bn = 256; pair = 1; return; }
-    const int tm[3] = {128, 128, 256}, tn[3] = {128, 256, 256};
-    const double weight[3] = {1.9, 1.45, 1.0};
-    double cost[3] = {0, 0, 0};
+    struct Config { uint32_t tm, tn; double groups; bool triangle; double fixed, per_k_block, epilogue; };
+    const Config config[3] = {{128, 128, kTileRuleSms, triangle_of_128(rows, cols, count), 5.0, 0.27, 1.9},
+                              {128, 256, kTileRuleSms, false, 7.0, 0.39, 2.5},
+                              {256, 256, kTileRuleSms / 2, true, 7.0, 0.37, 2.5}};
+    double best_time = 0.0;
+    int best = -1;
     for (int ci = 0; ci < 3; ++ci) {
+        const Config &c = config[ci];
+        double longest[3] = {0, 0, 0}, total[3] = {0, 0, 0};   // Gram, polynomial, apply
         for (uint32_t s = 0; s < count; ++s) {
             if ((uint64_t)rows[s] * cols[s] == 0) continue;
-            double n = std::min(rows[s], cols[s]), m = std::max(rows[s], cols[s]);
-            auto pad = [](double v, double t) { return std::ceil(v / t) * t; };
-            bool tall = rows[s] > cols[s];
-            double nn = pad(n, tm[ci]) * pad(n, tn[ci]);
-            double out = tall ? pad(m, tm[ci]) * pad(n, tn[ci]) : pad(n, tm[ci]) * pad(m, tn[ci]);
-            cost[ci] += weight[ci] * (nn * m + nn * n + out * n);
+            const uint32_t n = std::min(rows[s], cols[s]), m = std::max(rows[s], cols[s]);
+            auto tiles = [](uint32_t v, uint32_t t) { return (double)((v + t - 1) / t); };
+            const bool tall = rows[s] > cols[s];
+            const double a = tiles(n, c.tm), nn = c.triangle ? a * (a + 1.0) / 2.0 : a * tiles(n, c.tn);
+            const double out = tall ? tiles(m, c.tm) * tiles(n, c.tn) : a * tiles(m, c.tn);
+            const double k_gram = c.per_k_block * tiles(m, kGemmBlockK), k_rest = c.per_k_block * tiles(n, kGemmBlockK);
+            longest[0] = std::max(longest[0], k_gram);
+            longest[1] = longest[2] = std::max(longest[1], k_rest);
+            total[0] += nn * (k_gram + c.epilogue);
+            total[1] += nn * (k_rest + c.epilogue);
+            total[2] += out * (k_rest + c.epilogue);
         }
+        double time = 0.0;
+        for (int k = 0; k < 3; ++k) time += c.fixed + std::max(longest[k], total[k] / c.groups);
+        if (best < 0 || time < best_time) { best = ci; best_time = time; }
     }
-    int best = 0;
-    for (int ci = 1; ci < 3; ++ci)
-        if (cost[ci] < cost[best]) best = ci;
-    bn = tn[best];
+    bn = (int)config[best].tn;
     pair = best == 2;
 }
 
@@ -208,7 +236,7 @@ void build_items(Layout &L, const std::vector<uint32_t> &first) {
 bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, const b2_muon_options &o, Layout &L) {
     pick_tiles(rows, cols, count, o, L.bn, L.pair);
     L.tile_m = L.pair ? 256 : 128;
-    L.symmetric = (L.pair && L.bn == 256) ? 1 : 0;
+    L.symmetric = L.pair || (L.bn == 128 && triangle_of_128(rows, cols, count)) ? 1 : 0;
 #ifdef B2_MEASURE
     if (o.measure_flags & 4u) L.symmetric = 0;   // all tiles of the symmetric outputs
 #endif
@@ -490,7 +518,7 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
         const SlotLayout &sl = L.slots[s];
         for (uint32_t i = 0; i < sl.tiles_m_nn; ++i)
             for (uint32_t j = 0; j < sl.tiles_n_nn; ++j) {
-                // square 256 x 256 tiles: G and Q are symmetric, so only tiles on or above the
+                // square tiles: G and Q are symmetric, so only tiles on or above the
                 // diagonal are computed and the others are written as transposes
                 if (L.symmetric && j < i) continue;
                 tnn[inn++] = GemmTile{(uint16_t)s, (uint16_t)i, (uint16_t)j, (uint16_t)((L.symmetric && j > i) ? 1 : 0)};

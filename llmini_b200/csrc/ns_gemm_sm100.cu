@@ -368,7 +368,7 @@ __device__ __forceinline__ void fill_entry(TileEntry &e, const GemmProblem *p, u
     const uint32_t left = e.N - tile_n * BN;
     const uint32_t n_mma = min((uint32_t)BN, (left + step - 1u) / step * step);
     // a diagonal tile of X X^T or G G: this CTA's 128 rows of B are its 128 rows of A, in the same shared-memory layout
-    const bool shared = PAIR && tile_m == tile_n && e.map_a == e.map_b && a_mn == b_mn && n_mma == (uint32_t)BN;
+    const bool shared = (PAIR || BN == 128) && tile_m == tile_n && e.map_a == e.map_b && a_mn == b_mn && n_mma == (uint32_t)BN;
     e.flags = flags | (a_mn ? kTileAMn : 0u) | (b_mn ? kTileBMn : 0u) | (shared ? kTileShared : 0u) |
               (epilogue << kTileEpiShift) | ((n_mma / 32u) << kTileNShift);
 }

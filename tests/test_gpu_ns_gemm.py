@@ -158,3 +158,21 @@ def test_steps_with_fewer_iterations_take_the_per_phase_launches():
         assert torch.equal(plan.scratch(i, 1), plan5.scratch(i, 1))
     plan.close()
     plan5.close()
+
+
+def test_tile_choice_agrees_with_the_oracle_on_both_sides_of_the_line():
+    """One layer of width 512 takes 128 x 128 tiles, three of width 768 take pairs; mixed with odd row counts."""
+    rng = np.random.default_rng(3)
+    for shapes in ([(1536, 512), (333, 512)], [(2304, 768)] * 9 + [(701, 768)]):
+        xs = [_x0(rng, r, c, b2.OPERAND_BF16) for r, c in shapes]
+        plan = _run(shapes, b2.OPERAND_BF16, 1, o.fixed_coefficients(1), 0, xs)
+        for i in (0, len(shapes) - 1):
+            x = xs[i].astype(np.float64)
+            n_major = x if shapes[i][0] <= shapes[i][1] else x.T
+            a, b, c = (float(v) for v in o.fixed_coefficients(1)[0])
+            g = n_major @ n_major.T
+            u = (a * np.eye(len(g)) + b * g + c * g @ g) @ n_major
+            u = u if shapes[i][0] <= shapes[i][1] else u.T
+            got = host(plan.scratch(i, 1)).reshape(shapes[i])
+            # G, Q and X are BF16 operands (2^-9 relative each); Q is dominated by its rounded diagonal
+            assert np.linalg.norm(got - u) <= 4.0 * 2.0 ** -9 * np.linalg.norm(u)
