@@ -127,6 +127,7 @@ struct Layout {
     int pair = 0;   // 1: two-CTA 256 x 256 tiles
     int symmetric = 0;  // 1: Gram / Poly compute the upper triangle of tiles only (square tiles)
     int tile_m = 128;
+    uint32_t small_smem = 0;   // shared memory of the one-CTA-per-matrix loop, 0 where some matrix is too large for it
     size_t off_prefix, off_partials, off_inv_norm, off_amax_x, off_status, off_x0_ptrs, off_x1_ptrs, off_u_ptrs, off_maps,
         off_problems, off_tiles_nn, off_tiles_out, off_unit_prefix, off_factor_ptrs, off_unit_partials, off_slot_stats,
         off_items, off_fused_sync, off_chain, off_gp, off_chain_sync, off_meta_end, total;
@@ -240,6 +241,17 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
 #ifdef B2_MEASURE
     if (o.measure_flags & 4u) L.symmetric = 0;   // all tiles of the symmetric outputs
 #endif
+    // One CTA per matrix runs the whole loop where every matrix fits it and neither a tile shape nor another schedule was
+    // asked for (Newton-Schulz stage, per phase -> one CTA each: three of 64 x 64 at most 66 -> 20 us, one layer of width
+    // 128 84 -> 57, twelve 89 -> 58).
+    L.small_smem = 0;
+    if (o.tile_override == 0 && o.ns_schedule == B2_NS_PER_PHASE) {
+        for (uint32_t s = 0; s < count; ++s) {
+            if ((uint64_t)rows[s] * cols[s] == 0) continue;
+            if (!ns_small_fits(rows[s], cols[s])) { L.small_smem = 0; break; }
+            L.small_smem = std::max(L.small_smem, ns_small_smem(rows[s], cols[s]));
+        }
+    }
     L.slots.resize(count);
     L.chunk_prefix.assign(count + 1, 0);
     size_t off = 0;
@@ -430,6 +442,10 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
     p->ws = static_cast<uint8_t *>(d_workspace);
     e = gemm_configure(L.bn, L.pair);
     if (e != cudaSuccess) { delete p; return (int)e; }
+    if (L.small_smem) {
+        e = ns_small_configure(L.small_smem);
+        if (e != cudaSuccess) { delete p; return (int)e; }
+    }
     p->resident_groups = (uint32_t)std::max(gemm_resident_groups(L.bn, L.pair, p->dev.sm_count), 0);
 
     p->meta.assign(L.off_meta_end, 0);
@@ -670,11 +686,12 @@ int b2_muon_polar(b2_muon_plan *plan, const b2_muon_step_args *a, void *stream) 
     const int grid = plan->dev.sm_count;
     cudaError_t e = cudaSuccess;
     bool whole_loop = L.chain_tiles != 0 && a->iterations == L.chain_iterations;
+    bool small = L.small_smem != 0 && a->iterations <= kMaxChainIterations;
 #ifdef B2_MEASURE
-    if (plan->options.measure_phase_mask) whole_loop = false;
+    if (plan->options.measure_phase_mask) whole_loop = small = false;
 #endif
-    if (whole_loop) {
-        // every GEMM of every iteration as one grid, ordered by per-matrix progress counts
+    if (whole_loop || small) {
+        // every GEMM of every iteration as one grid: a CTA per matrix, or tiles ordered by per-matrix progress counts
         GemmCoefficients coef = {};
         for (uint32_t it = 0; it < a->iterations; ++it) {
             if (a->coefficients) {
@@ -684,6 +701,10 @@ int b2_muon_polar(b2_muon_plan *plan, const b2_muon_step_args *a, void *stream) 
             }
         }
         const float *scale = plan->options.normalize_mode == B2_NORMALIZE_DEFERRED ? plan->at<float>(L.off_inv_norm) : nullptr;
+        if (small)
+            return (int)launch_ns_small(probs + (size_t)kGram0 * count, probs + (size_t)kPoly * count, probs + (size_t)kApply0 * count,
+                                        probs + (size_t)kApply1 * count, probs + (size_t)kLast0 * count, count, a->iterations, f16,
+                                        plan->options.update_input == B2_UPDATE_16BIT, coef, scale, L.small_smem, status, s);
         return (int)launch_ns_chain(L.bn, L.pair, probs, plan->at<ChainTile>(L.off_chain), L.chain_tiles, f16, coef, scale,
                                     status, plan->ws + L.off_chain_sync, count, plan->options.measure_flags, grid, s);
     }

@@ -40,6 +40,8 @@
 //
 // Every mbarrier wait, ring read and dependency wait is bounded: on expiry the CTA raises a status word, drains
 // and frees its TMEM before returning.
+#include <algorithm>
+
 #include <cuda.h>
 
 #include "common.cuh"
@@ -914,6 +916,249 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
     }
 }
 
+// ---- the whole Newton-Schulz loop of a small matrix in one CTA ---------------------------------------------------
+// A matrix whose smaller dimension is at most 128 and whose larger one at most 512 fits one SM: the operand (up to
+// 128 KB), G and Q (32 KB each) stay in shared memory over all iterations, and the FP32 accumulators of a phase in
+// tensor memory (the result of the Apply phase fills its 512 columns).  With one launch per phase such a matrix spends
+// its time on launches and on the way through L2 between them (4.4 to 5.6 us per phase whose MMAs take well below one);
+// here a phase costs its MMAs, one commit, the accumulator's way through registers and two barriers.
+// The operand keeps its storage orientation: panels of 64 columns x 128-row blocks as TMA delivers them (128-byte
+// swizzle), read K-major along a row and MN-major across rows, so one copy serves both GEMMs it takes part in:
+//   wide (rows <= cols)  Gram K-major,  X' = Q X with X as an MN-major B;   tall  Gram MN-major,  X' = X Q with X as a
+//   K-major A.
+// What TMA fills in beyond the matrix is zero and stays zero, so nothing needs a bound but the stores.  Rounding points,
+// operand values and the order of every sum are those of k_ns_gemm.
+constexpr int kSmallThreads = 256;
+constexpr uint32_t kSmallPanel = 128 * 128;   // bytes: 128 rows x 64 16-bit values
+constexpr uint32_t kSmallTmemCols = 512;
+
+struct SmallLoop {
+    uint32_t iterations;
+    int f16;
+    int last16;           // the last result leaves in the operand type (into the operand buffer that is its turn)
+    GemmCoefficients coef;
+};
+
+__device__ __forceinline__ uint32_t small_swizzled(uint32_t row, uint32_t chunk) { return row * 128u + ((chunk ^ (row & 7u)) << 4); }
+
+__global__ void __launch_bounds__(kSmallThreads, 1)
+k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__ poly, const GemmProblem *__restrict__ apply0,
+           const GemmProblem *__restrict__ apply1, const GemmProblem *__restrict__ last, SmallLoop loop,
+           const float *__restrict__ slot_scale, uint32_t *status) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t *g_panels = smem, *q_panels = smem + 2 * kSmallPanel, *x_panels = smem + 4 * kSmallPanel;
+    __shared__ uint64_t bars[2];              // operand loaded; MMAs of a phase retired
+    __shared__ uint32_t tmem_slot, abort_word;
+    volatile uint32_t *abort_flag = &abort_word;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t slot = blockIdx.x;
+    const uint32_t load_bar = smem_u32(bars), mma_bar = load_bar + 8;
+    const GemmProblem *ap = apply0 + slot;
+    const uint32_t rows = ap->M, cols = ap->N;   // of the storage layout
+    const bool empty = rows == 0u;
+    const bool tall = gram[slot].a_mn_major != 0u;
+    const uint32_t n = tall ? cols : rows;
+    const uint32_t panels = tall ? 2u : (cols + 63u) / 64u, blocks = tall ? (rows + 127u) / 128u : 1u;
+
+    if (threadIdx.x == 0) {
+        mbar_init(load_bar, 1);
+        mbar_init(mma_bar, 1);
+        abort_word = 0;
+        fence_async_smem();
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(kSmallTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    if (!empty) {
+        if (threadIdx.x == 0) {
+            const uint64_t map = tall ? ap->map_a : gram[slot].map_a;   // 64 x 128 boxes of the first operand buffer
+            mbar_expect_tx(load_bar, panels * blocks * kSmallPanel);
+            for (uint32_t p = 0; p < panels; ++p)
+                for (uint32_t j = 0; j < blocks; ++j)
+                    tma_load_2d<false>(smem_u32(x_panels) + (p * blocks + j) * kSmallPanel, map, load_bar, (int)(64 * p), (int)(128 * j));
+        }
+        const float slot_s = slot_scale != nullptr ? __ldcg(slot_scale + slot) : 1.0f;
+        const int f16 = loop.f16;
+        const uint32_t q = warp & 3, half = warp >> 2;
+        const uint32_t row = 32 * q + lane;                          // TMEM lane
+        const uint32_t lane_base = tmem + ((32u * q) << 16);
+        const uint32_t g_addr = smem_u32(g_panels), q_addr = smem_u32(q_panels), x_addr = smem_u32(x_panels);
+        const uint32_t k16_n = (n + 15u) / 16u;                       // steps of 16 over the smaller dimension
+        uint32_t phase = 0;
+        (void)mbar_wait(load_bar, 0, abort_flag);   // on expiry the flag ends the loop at its next barrier
+        // MMAs of a phase by one thread of warp 0, then everybody waits for them
+        auto run = [&](auto &&issue) {
+            if (warp == 0 && elect_one()) {
+                tc_fence_after();
+                issue();
+                tc_commit<false>(mma_bar);
+            }
+            __syncwarp();
+            (void)mbar_wait(mma_bar, phase, abort_flag);
+            phase ^= 1u;
+            tc_fence_after();
+        };
+        // what this thread stored to shared memory is visible to the next phase's MMAs, and its TMEM reads are done
+        auto hand_over = [&]() {
+            fence_async_smem();
+            tc_fence_before();
+            __syncthreads();
+        };
+        __syncthreads();
+        // coefficients without indexing the argument block by a register
+        for (uint32_t it = 0; it < loop.iterations; ++it) {
+            float ca = loop.coef.v[0], cb = loop.coef.v[1], cc = loop.coef.v[2];
+#pragma unroll
+            for (uint32_t i = 1; i < kMaxChainIterations; ++i)
+                if (it == i) { ca = loop.coef.v[3 * i]; cb = loop.coef.v[3 * i + 1]; cc = loop.coef.v[3 * i + 2]; }
+            const bool final = it + 1 == loop.iterations;
+            const float s1 = it == 0 ? slot_s : 1.0f, s2 = s1 * s1;
+            // ---- Gram: columns 0 .. 127 of tensor memory
+            run([&] {
+                const uint32_t idesc = instr_desc(128, 128, f16, tall ? 1u : 0u, tall ? 1u : 0u);
+                if (tall) {
+                    const uint32_t steps = (rows + 15u) / 16u;
+                    for (uint32_t k = 0; k < steps; ++k) {
+                        const uint64_t d = smem_desc(x_addr + k * 2048u, blocks * kSmallPanel, 1024);
+                        tc_mma<false>(tmem, d, d, idesc, k != 0);
+                    }
+                } else {
+                    const uint32_t steps = (cols + 15u) / 16u;
+                    for (uint32_t k = 0; k < steps; ++k) {
+                        const uint64_t d = smem_desc(x_addr + (k >> 2) * kSmallPanel + (k & 3u) * 32u, 16, 1024);
+                        tc_mma<false>(tmem, d, d, idesc, k != 0);
+                    }
+                }
+            });
+            // each warp takes 64 columns of its 32 rows: one panel of G (and of Q)
+            uint8_t *g_out = reinterpret_cast<uint8_t *>(gram[slot].out16), *q_out = reinterpret_cast<uint8_t *>(poly[slot].out16);
+            const uint32_t pitch = gram[slot].pitch16;
+            auto store_nn = [&](uint8_t *panel0, uint8_t *global, uint32_t col, const uint32_t *v) {   // 32 columns from `col`
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint4 w;
+                    w.x = pack_operands(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]), f16);
+                    w.y = pack_operands(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]), f16);
+                    w.z = pack_operands(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]), f16);
+                    w.w = pack_operands(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]), f16);
+                    const uint32_t c = col + 8 * j;
+                    *reinterpret_cast<uint4 *>(panel0 + (c >> 6) * kSmallPanel + small_swizzled(row, (c & 63u) >> 3)) = w;
+                    if (final && row < n && c < pitch) *reinterpret_cast<uint4 *>(global + ((size_t)row * pitch + c) * 2) = w;
+                }
+            };
+#pragma unroll 1
+            for (uint32_t sub = 0; sub < 2; ++sub) {
+                const uint32_t col = 64 * half + 32 * sub;
+                uint32_t v[32];
+                tc_ld32(lane_base + col, v);
+                tc_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * s2);
+                store_nn(g_panels, g_out, col, v);
+            }
+            hand_over();
+            // ---- Poly: columns 128 .. 255; the Gram accumulator stays where it is
+            run([&] {
+                const uint32_t idesc = instr_desc(128, 128, f16, 0u, 0u);
+                for (uint32_t k = 0; k < k16_n; ++k) {
+                    const uint64_t d = smem_desc(g_addr + (k >> 2) * kSmallPanel + (k & 3u) * 32u, 16, 1024);
+                    tc_mma<false>(tmem + 128u, d, d, idesc, k != 0);
+                }
+            });
+#pragma unroll 1
+            for (uint32_t sub = 0; sub < 2; ++sub) {
+                const uint32_t col = 64 * half + 32 * sub;
+                uint32_t v[32], h[32];
+                tc_ld32(lane_base + 128u + col, v);
+                tc_ld32(lane_base + col, h);
+                tc_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    // rows and columns beyond the matrix stay zero
+                    const float ident = (col + j == row && row < n) ? ca : 0.0f;
+                    // store/plain.rs:175-178: fma(c, acc, fma(b, base, identity))
+                    v[j] = __float_as_uint(fmaf(cc, __uint_as_float(v[j]), fmaf(cb, __uint_as_float(h[j]) * s2, ident)));
+                }
+                store_nn(q_panels, q_out, col, v);
+            }
+            hand_over();
+            // ---- Apply: one 128 x 128 block of the result per 128 columns of tensor memory
+            run([&] {
+                if (tall) {
+                    const uint32_t idesc = instr_desc(128, 128, f16, 0u, 0u);
+                    for (uint32_t j = 0; j < blocks; ++j)
+                        for (uint32_t k = 0; k < k16_n; ++k)
+                            tc_mma<false>(tmem + 128u * j,
+                                          smem_desc(x_addr + ((k >> 2) * blocks + j) * kSmallPanel + (k & 3u) * 32u, 16, 1024),
+                                          smem_desc(q_addr + (k >> 2) * kSmallPanel + (k & 3u) * 32u, 16, 1024), idesc, k != 0);
+                } else {
+                    for (uint32_t p = 0; p < panels; p += 2) {
+                        const uint32_t idesc = instr_desc(128, p + 1 < panels ? 128 : 64, f16, 0u, 1u);
+                        for (uint32_t k = 0; k < k16_n; ++k)
+                            tc_mma<false>(tmem + 64u * p, smem_desc(q_addr + (k >> 2) * kSmallPanel + (k & 3u) * 32u, 16, 1024),
+                                          smem_desc(x_addr + p * kSmallPanel + k * 2048u, kSmallPanel, 1024), idesc, k != 0);
+                    }
+                }
+            });
+            const uint32_t columns = tall ? 128u * blocks : 64u * panels;
+            const bool out32 = final && !loop.last16;
+            uint8_t *out = reinterpret_cast<uint8_t *>(out32 ? last[slot].out32 : ((it & 1u) ? apply1 + slot : ap)->out16);
+            // the operand buffers in memory hold the last three operands of the loop, as with a launch per phase
+            const bool to_global = it + 3 >= loop.iterations;
+#pragma unroll 1
+            for (uint32_t t = 32 * half; t < columns; t += 64) {
+                uint32_t v[32];
+                tc_ld32(lane_base + t, v);
+                tc_ld_wait();
+                const uint32_t c0 = tall ? (t & 127u) : t, r = tall ? (t >> 7) * 128u + row : row;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * s1);
+                if (out32) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (r < rows && c0 + 4 * j < cols)
+                            *reinterpret_cast<uint4 *>(out + ((size_t)r * cols + c0 + 4 * j) * 4) =
+                                make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                } else {
+                    uint8_t *panel0 = x_panels + (tall ? (t >> 7) * kSmallPanel : 0u);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        uint4 w;
+                        w.x = pack_operands(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]), f16);
+                        w.y = pack_operands(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]), f16);
+                        w.z = pack_operands(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]), f16);
+                        w.w = pack_operands(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]), f16);
+                        const uint32_t c = c0 + 8 * j;
+                        *reinterpret_cast<uint4 *>(panel0 + (c >> 6) * blocks * kSmallPanel + small_swizzled(row, (c & 63u) >> 3)) = w;
+                        if (to_global && r < rows && c < cols) *reinterpret_cast<uint4 *>(out + ((size_t)r * cols + c) * 2) = w;
+                    }
+                }
+            }
+            hand_over();
+            if (*abort_flag) break;   // a wait ran out: written before the barrier, so every thread sees it
+        }
+        if (*abort_flag) {
+            // copies or MMAs may still be in flight: give them time to land before the memory is released
+            for (int i = 0; i < 4096; ++i) __nanosleep(512);
+            if (threadIdx.x == 0) atomicExch(status, 1u);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kSmallTmemCols) : "memory");
+}
+
 template <int BN, bool PAIR, bool CHAINED>
 cudaError_t launch_impl(const GemmProblem *problems, const void *tiles, uint32_t tile_count, uint32_t epilogue,
                         int f16, const GemmCoefficients &coef, const float *slot_scale, uint32_t scale_pow,
@@ -1034,6 +1279,31 @@ cudaError_t launch_ns_gemm(int block_n, int pair, const GemmProblem *problems, c
     coef.v[0] = ca; coef.v[1] = cb; coef.v[2] = cc;
     return dispatch<false>(block_n, pair, problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow, status,
                            nullptr, 0u, debug_flags, grid, s);
+}
+bool ns_small_fits(uint32_t rows, uint32_t cols) { return std::min(rows, cols) <= 128u && std::max(rows, cols) <= 512u; }
+uint32_t ns_small_smem(uint32_t rows, uint32_t cols) {
+    const uint32_t x = rows > cols ? 2u * ((rows + 127u) / 128u) : (cols + 63u) / 64u;
+    return 1024u + (4u + x) * kSmallPanel;
+}
+cudaError_t ns_small_configure(uint32_t smem_bytes) {
+    return cudaFuncSetAttribute(k_ns_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+}
+cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, const GemmProblem *apply0, const GemmProblem *apply1,
+                            const GemmProblem *last, uint32_t slot_count, uint32_t iterations, int f16, int last16,
+                            const GemmCoefficients &coef, const float *slot_scale, uint32_t smem_bytes, uint32_t *status,
+                            cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(slot_count, 1, 1);
+    cfg.blockDim = dim3(kSmallThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem_bytes;
+    cfg.stream = s;
+    SmallLoop loop = {iterations, f16, last16, coef};
+    return cudaLaunchKernelEx(&cfg, k_ns_small, gram, poly, apply0, apply1, last, loop, slot_scale, status);
 }
 size_t chain_sync_bytes(uint32_t slot_count) { return sizeof(ChainSync) + sizeof(uint32_t) * slot_count; }
 uint32_t chain_epilogue_warps(int block_n, int pair) { return (uint32_t)(4 * (block_n / 64)) * (pair ? 2u : 1u); }

@@ -160,6 +160,40 @@ def test_steps_with_fewer_iterations_take_the_per_phase_launches():
     plan5.close()
 
 
+SMALL = [(16, 16), (64, 64), (128, 128), (128, 512), (512, 128), (100, 112), (129, 128), (127, 144), (512, 16), (16, 512),
+         (1, 496), (384, 80), (65, 64), (128, 48), (80, 448)]   # one SM holds each of them
+
+
+@pytest.mark.parametrize("fmt", [b2.OPERAND_BF16, b2.OPERAND_F16])
+@pytest.mark.parametrize("iterations,deferred,update16", [(1, False, False), (2, False, True), (5, False, False), (5, True, True)])
+def test_one_cta_loop_equals_the_per_phase_launches_bit_for_bit(fmt, iterations, deferred, update16):
+    """Plans whose matrices all fit one SM take the one-CTA loop; a forced tile shape keeps the launches per phase."""
+    if deferred and fmt == b2.OPERAND_F16:
+        return   # refused by the plan
+    rng = np.random.default_rng(iterations)
+    shapes = SMALL[:7] + [(0, 0)] + SMALL[7:]
+    live = [(i, s) for i, s in enumerate(shapes) if s[0]]
+    xs = {i: _x0(rng, r, c, fmt) for i, (r, c) in live}
+    co = o.polar_express_coefficients(iterations) if fmt == b2.OPERAND_F16 else o.fixed_coefficients(iterations)
+    results = []
+    for tile_n in (0, 128):
+        plan = b2.MuonPlan(shapes, operand_format=fmt, scale_layout=b2.SCALES_RAW, tile_n=tile_n, max_iterations=iterations,
+                           normalize_mode=b2.NORMALIZE_DEFERRED if deferred else b2.NORMALIZE_TWO_PASS,
+                           update_input=b2.UPDATE_16BIT if update16 else b2.UPDATE_F32)
+        for i, (r, c) in live:
+            for w in (0, 1, 5, 6, 7):
+                plan.scratch(i, w).zero_()
+            plan.scratch(i, 0).copy_(dev(xs[i]).to(plan.scratch(i, 0).dtype))
+            plan.scratch(i, 2).view(torch.float32).fill_(0.75)   # read by a one-pass plan only
+        b2.OptimizerModule().muon_polar(plan, b2.MuonMegaUpdateArgs(iterations=iterations, coefficients=co))
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        results.append([[host(plan.scratch(i, w).float()).copy() for w in (0, 1, 5, 6, 7)] for i, _ in live])
+    for (_, shape), a, b in zip(live, *results):
+        for w, u, v in zip(("operand 0", "U", "G", "Q", "operand 1"), a, b):
+            assert np.array_equal(u, v), (shape, w, float(np.abs(u - v).max()))
+
+
 def test_tile_choice_agrees_with_the_oracle_on_both_sides_of_the_line():
     """One layer of width 512 takes 128 x 128 tiles, three of width 768 take pairs; mixed with odd row counts."""
     rng = np.random.default_rng(3)
