@@ -210,3 +210,39 @@ def test_tile_choice_agrees_with_the_oracle_on_both_sides_of_the_line():
             got = host(plan.scratch(i, 1)).reshape(shapes[i])
             # G, Q and X are BF16 operands (2^-9 relative each); Q is dominated by its rounded diagonal
             assert np.linalg.norm(got - u) <= 4.0 * 2.0 ** -9 * np.linalg.norm(u)
+
+
+@pytest.mark.parametrize("deferred", [False, True])
+@pytest.mark.parametrize("shapes", [
+    [(3072, 768)],                              # four shares of twelve k-blocks
+    [(77, 1040), (1999, 64), (130, 16)],        # shares of unequal length, one matrix not split, ragged everywhere
+    [(200, 1536)],                              # shares of a wide matrix, tiles clipped in both directions
+])
+def test_split_gram_tiles(shapes, deferred):
+    """Few 128 x 128 Gram tiles with a long K are split; the shares add up to the product, launch after launch."""
+    rng = np.random.default_rng(17)
+    xs = [_x0(rng, r, c, b2.OPERAND_BF16) for r, c in shapes]
+    s = 0.75 if deferred else 1.0
+    plan = b2.MuonPlan(shapes, scale_layout=b2.SCALES_RAW, tile_n=128, max_iterations=1,
+                       normalize_mode=b2.NORMALIZE_DEFERRED if deferred else b2.NORMALIZE_TWO_PASS)
+    first = None
+    for _ in range(3):
+        for i, x in enumerate(xs):
+            plan.scratch(i, 0).copy_(dev(x).to(torch.bfloat16))
+            plan.scratch(i, 2).view(torch.float32).fill_(0.75)   # read by a one-pass plan only
+            plan.scratch(i, 5).zero_()
+        b2.OptimizerModule().muon_polar(plan, b2.MuonMegaUpdateArgs(iterations=1, coefficients=o.fixed_coefficients(1)))
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        got = [[host(plan.scratch(i, w).float()).copy() for w in (5, 6, 1)] for i in range(len(shapes))]
+        if first is not None:   # which share comes last must not matter
+            assert all(np.array_equal(u, v) for a, b in zip(first, got) for u, v in zip(a, b))
+        first = got
+    for x, (r, c), (g16, q16, u) in zip(xs, shapes, got):
+        n = min(r, c)
+        xd = (x if r <= c else x.T).astype(np.float64)
+        G = xd @ xd.T * s * s
+        g16 = g16.reshape(n, -1)[:, :n]
+        # one rounding to BF16 (half a unit in the last place, 2^-9 .. 2^-8 relative) on top of FP32 sums of max(r, c) products
+        bound = 2.0 ** -8 * np.abs(G) + max(r, c) * 2.0 ** -24 * s * s * (np.abs(xd) @ np.abs(xd).T)
+        assert np.all(np.abs(g16 - G) <= bound)
