@@ -209,6 +209,13 @@ __device__ __forceinline__ void atomic_max_nonneg(float *addr, float v) {
     atomicMax(reinterpret_cast<unsigned int *>(addr), __float_as_uint(v));
 }
 
+// First statement of every streaming kernel: the next launch of the stream may begin, and this one goes on once the launch
+// in front of it has ended and its stores are visible (programmatic dependent launch; a no-op without the attribute).
+__device__ __forceinline__ void stream_enter() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---- streaming loads/stores ------------------------------------------------------------------
 __device__ __forceinline__ float4 ld_stream(const float *p) {
     return __ldcs(reinterpret_cast<const float4 *>(p));
