@@ -336,8 +336,7 @@ __device__ __forceinline__ float4 load_update16(const uint16_t *U, uint32_t i, i
                        bf16_bits_to_f32(w.y >> 16));
 }
 template <int EXT, int UFMT = 0>
-__device__ __forceinline__ void update_chunk(const ChunkCtx &cx, const uint64_t *u_ptrs, float *amax_x,
-                                             const UpdateParams &up, bool keep_y, float *warp_ax, float *warp_ay) {
+__device__ __forceinline__ void update_chunk(const ChunkCtx &cx, const uint64_t *u_ptrs, const UpdateParams &up, bool keep_y, float *warp_ax, float *warp_ay) {
     const float lr = up.lr, wd = up.wd, c_avg = up.c_avg, beta = up.beta;
     const int tid = threadIdx.x;
     const float *U = reinterpret_cast<const float *>(u_ptrs[cx.slot]);
@@ -426,17 +425,18 @@ __device__ __forceinline__ void update_chunk(const ChunkCtx &cx, const uint64_t 
         warp_ax[tid >> 5] = ax;
         warp_ay[tid >> 5] = ay;
     }
-    __syncthreads();
-    if (tid == 0) {
-        float mx = 0.0f, my = 0.0f;
+}
+// One thread, behind a barrier after update_chunk: raises the slot's two maxima.
+__device__ __forceinline__ void raise_amax(const b2_muon_slot_descriptor *slots, float *amax_x, uint32_t slot,
+                                           const float *warp_ax, const float *warp_ay) {
+    float mx = 0.0f, my = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kThreads / 32; ++w) {
-            mx = fmaxf(mx, warp_ax[w]);
-            my = fmaxf(my, warp_ay[w]);
-        }
-        atomic_max_nonneg(amax_x + cx.slot, mx);
-        atomic_max_nonneg(reinterpret_cast<float *>(cx.d.schedule_amax), my);
+    for (int w = 0; w < kThreads / 32; ++w) {
+        mx = fmaxf(mx, warp_ax[w]);
+        my = fmaxf(my, warp_ay[w]);
     }
+    atomic_max_nonneg(amax_x + slot, mx);
+    atomic_max_nonneg(reinterpret_cast<float *>(slots[slot].schedule_amax), my);
 }
 
 template <int EXT, int UFMT>
@@ -444,11 +444,14 @@ __global__ void __launch_bounds__(kThreads, 5)
 k_muon_update(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint32_t slot_count,
               uint32_t total_chunks, const uint64_t *u_ptrs, float *amax_x, UpdateParams up) {
     stream_enter();
-    __shared__ float warp_ax[kThreads / 32], warp_ay[kThreads / 32];
-    for (uint32_t c = blockIdx.x; c < total_chunks; c += gridDim.x) {
+    // two sets of warp maxima: one barrier per chunk
+    __shared__ float warp_ax[2][kThreads / 32], warp_ay[2][kThreads / 32];
+    uint32_t turn = 0;
+    for (uint32_t c = blockIdx.x; c < total_chunks; c += gridDim.x, turn ^= 1u) {
         ChunkCtx cx = chunk_ctx(slots, prefix, slot_count, c);
-        update_chunk<EXT, UFMT>(cx, u_ptrs, amax_x, up, false, warp_ax, warp_ay);
+        update_chunk<EXT, UFMT>(cx, u_ptrs, up, false, warp_ax[turn], warp_ay[turn]);
         __syncthreads();
+        if (threadIdx.x == 0) raise_amax(slots, amax_x, cx.slot, warp_ax[turn], warp_ay[turn]);
     }
 }
 
@@ -1101,8 +1104,9 @@ k_muon_update_encode(const b2_muon_slot_descriptor *slots, const uint32_t *prefi
                      UpdateParams up, int quantize_y, int scale_layout, FusedSync *sync, uint32_t *status,
                      uint64_t wait_ns) {
     stream_enter();
-    __shared__ float warp_ax[kThreads / 32], warp_ay[kThreads / 32];
-    __shared__ uint32_t s_ticket[2], s_ok;
+    // One barrier per item: every word that crosses it exists twice, and a thread is never a second barrier ahead.
+    __shared__ float warp_ax[2][kThreads / 32], warp_ay[2][kThreads / 32];
+    __shared__ uint32_t s_ticket[2], s_ok[2];
     const int tid = threadIdx.x;
     if (tid == 0) s_ticket[0] = atomicAdd(&sync->ticket, 1u);
     __syncthreads();
@@ -1116,12 +1120,13 @@ k_muon_update_encode(const b2_muon_slot_descriptor *slots, const uint32_t *prefi
         const uint32_t c = item & ~kItemEncode;
         ChunkCtx cx = chunk_ctx(slots, prefix, slot_count, c);
         if (!(item & kItemEncode)) {
-            update_chunk<0, UFMT>(cx, u_ptrs, amax_x, up, quantize_y != 0, warp_ax, warp_ay);
+            update_chunk<0, UFMT>(cx, u_ptrs, up, quantize_y != 0, warp_ax[it & 1], warp_ay[it & 1]);
             // Publish.  The barrier orders every thread's stores before thread 0's fence, which is
-            // cumulative; thread 0 raised the two maxima before it.  (Letting the other warps run
-            // ahead of the fence, or publishing one item late, both measured slower.)
+            // cumulative; thread 0 raises the two maxima before it, while the other warps go on.
+            if (tid == 0) s_ticket[(it + 1) & 1] = next_ticket;
             __syncthreads();
             if (tid == 0) {
+                raise_amax(slots, amax_x, cx.slot, warp_ax[it & 1], warp_ay[it & 1]);
                 __threadfence();
                 atomicAdd(&sync->done[cx.slot], 1u);
             }
@@ -1144,10 +1149,11 @@ k_muon_update_encode(const b2_muon_slot_descriptor *slots, const uint32_t *prefi
                     atomicExch(status, 1u);
                 }
                 __threadfence();
-                s_ok = ok;
+                s_ok[it & 1] = ok;
+                s_ticket[(it + 1) & 1] = next_ticket;
             }
             __syncthreads();
-            if (!s_ok) break;   // uniform: s_ok is shared
+            if (!s_ok[it & 1]) break;   // uniform: s_ok is shared
             const float *src = reinterpret_cast<const float *>(quantize_y ? cx.d.grad : cx.d.x_master);
             const float amax = __ldcg(quantize_y ? reinterpret_cast<const float *>(cx.d.schedule_amax)
                                                  : amax_x + cx.slot);
@@ -1171,8 +1177,6 @@ k_muon_update_encode(const b2_muon_slot_descriptor *slots, const uint32_t *prefi
                                                     reinterpret_cast<uint8_t *>(cx.d.bytes), scales, scale_layout, k, rows);
             }
         }
-        if (tid == 0) s_ticket[(it + 1) & 1] = next_ticket;
-        __syncthreads();
     }
     // leave the words as the next launch expects them (a memset node per step costs more)
     if (tid == 0) {
