@@ -458,17 +458,20 @@ k_muon_update(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint
 // NorMuon second moment per neuron, and the Hyperball statistics when `hyperball` is set:
 // crates/cuda-kernels/src/gpt/optimizer/muon/fused/tma_split.rs:285-443.  U is in the storage
 // layout here, so a neuron's values are one row (rows >= cols: a warp per row) or one column
-// (rows < cols: 128 columns per CTA, the eight warps striding over the rows); both read whole
-// 512-byte row segments.  Per unit four partial sums leave the CTA: raw, scaled, parameter, dot.
-// COLS = 0 handles the row-neuron units, COLS = 1 the column-neuron ones; each instance skips the
+// (rows < cols: COLS columns per CTA, the threads striding over the rows); both read whole 128-byte lines or more.  Per
+// unit four partial sums leave the CTA: raw, scaled, parameter, dot.
+// COLS = 0 handles the row-neuron units, the others the column-neuron ones; each instance skips the
 // other's units, so the register-hungry column form (eight loads in flight per thread) does not
 // take the occupancy of the row form down with it.
+// COLS = 128 where that gives every SM a unit, else 32: a matrix of a thousand columns is nine units of 128, each a chain
+// of round trips over its rows (ragged plan of 5 matrices: 19 us, with 32 columns 9; GPT-2 medium: 80 us, with 32 103).
 template <int COLS>
 __global__ void __launch_bounds__(kThreads, COLS ? 2 : 4)
 k_normuon_stats(const b2_muon_slot_descriptor *slots, uint32_t slot_count, NeuronView nv, const uint64_t *u_ptrs,
                 int hyperball) {
     stream_enter();
-    __shared__ float col_raw[COLS ? kThreads / 32 : 1][128], col_dot[COLS ? kThreads / 32 : 1][128];
+    constexpr uint32_t kUnitCols = COLS ? COLS : 4, kQuads = kUnitCols / 4, kRowLanes = kThreads / kQuads;
+    __shared__ float col_raw[COLS ? kRowLanes : 1][kUnitCols], col_dot[COLS ? kRowLanes : 1][kUnitCols];
     __shared__ double part[kThreads / 32][4];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint32_t unit = blockIdx.x; unit < nv.total_units; unit += gridDim.x) {
@@ -525,17 +528,17 @@ k_normuon_stats(const b2_muon_slot_descriptor *slots, uint32_t slot_count, Neuro
                 }
             }
         } else {
-            const uint32_t c0 = local * 128 + lane * 4;
+            const uint32_t quad = tid % kQuads, row_lane = tid / kQuads;
+            const uint32_t c0 = local * kUnitCols + quad * 4;
             float raw[4] = {0.f, 0.f, 0.f, 0.f}, dot[4] = {0.f, 0.f, 0.f, 0.f}, param = 0.0f;
             if (c0 < d.cols) {
-                // eight rows per step and warp: eight independent 128-bit loads in flight per thread
-                // (one at a time left each 128-column unit latency-bound at about 100 us)
-                constexpr uint32_t kRowsInFlight = 8, kWarps = kThreads / 32;
-                for (uint32_t r0 = warp; r0 < d.rows; r0 += kWarps * kRowsInFlight) {
+                // eight independent 128-bit loads in flight per thread
+                constexpr uint32_t kRowsInFlight = 8;
+                for (uint32_t r0 = row_lane; r0 < d.rows; r0 += kRowLanes * kRowsInFlight) {
                     float4 u[kRowsInFlight], p[kRowsInFlight];
 #pragma unroll
                     for (uint32_t k = 0; k < kRowsInFlight; ++k) {
-                        const uint32_t r = r0 + k * kWarps;
+                        const uint32_t r = r0 + k * kRowLanes;
                         const size_t at = (size_t)r * d.cols + c0;
                         u[k] = r < d.rows ? *reinterpret_cast<const float4 *>(U + at) : make_float4(0.f, 0.f, 0.f, 0.f);
                         if (hyperball)
@@ -559,16 +562,16 @@ k_normuon_stats(const b2_muon_slot_descriptor *slots, uint32_t slot_count, Neuro
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                col_raw[warp][lane * 4 + e] = raw[e];
-                col_dot[warp][lane * 4 + e] = dot[e];
+                col_raw[row_lane][quad * 4 + e] = raw[e];
+                col_dot[row_lane][quad * 4 + e] = dot[e];
             }
             s_param = (double)param;
             __syncthreads();
-            const uint32_t col = local * 128 + tid;
-            if (tid < 128 && col < d.cols) {
+            const uint32_t col = local * kUnitCols + tid;
+            if (tid < kUnitCols && col < d.cols) {
                 double r = 0.0, dd = 0.0;
-#pragma unroll
-                for (int w = 0; w < kThreads / 32; ++w) {
+#pragma unroll 8
+                for (uint32_t w = 0; w < kRowLanes; ++w) {
                     r += (double)col_raw[w][tid];
                     dd += (double)col_dot[w][tid];
                 }
@@ -1809,7 +1812,10 @@ cudaError_t launch_normuon_stats(const SlotView &v, const NeuronView &nv, const 
                                  cudaStream_t s) {
     if (nv.total_units == 0) return cudaSuccess;
     stream_launch(kPlain, k_normuon_stats<0>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
-    stream_launch(kOverlapped, k_normuon_stats<1>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
+    if (nv.unit_cols == 128)
+        stream_launch(kOverlapped, k_normuon_stats<128>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
+    else
+        stream_launch(kOverlapped, k_normuon_stats<32>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
     stream_launch(kOverlapped, k_normuon_reduce, v.slot_count, kThreads, s, v.slots, nv);
     return cudaGetLastError();
 }
