@@ -240,8 +240,11 @@ void pick_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t count, cons
 // update work instead of arriving as a block (measured 390 us against 405 us; with kLag 4000, or a feed slower
 // than the arrival, the weights have left L2 and it is 420 us).  A group's list ends with the encode spans still
 // pending, so every group is complete in itself and the total length does not depend on the grouping.
+// A matrix of more than kLargeChunks chunks (48 KB of traffic each, 96 MB of the 126 MB of L2) is encoded last span first:
+// its most recent values are still in L2 then and its oldest have left it either way (half of the layers of GPT-2 XL,
+// alone: 3580 -> 3486 us).
 void build_items(Layout &L, const std::vector<uint32_t> &first) {
-    const uint32_t kLag = 1200, kEvery = 3, kEncodeFlag = 0x80000000u;
+    const uint32_t kLag = 1200, kEvery = 3, kLargeChunks = 2000, kEncodeFlag = 0x80000000u;
     L.items.clear();
     L.group_item_begin.assign(1, 0u);
     for (size_t g = 0; g + 1 < first.size(); ++g) {
@@ -257,7 +260,11 @@ void build_items(Layout &L, const std::vector<uint32_t> &first) {
                     since = 0;
                 }
             }
-            for (uint32_t c = lo; c < hi; c += B2_FUSED_ENCODE_SPAN) pending.emplace_back(hi - 1 + kLag, kEncodeFlag | c);
+            const uint32_t spans = (hi - lo + B2_FUSED_ENCODE_SPAN - 1) / B2_FUSED_ENCODE_SPAN;
+            for (uint32_t k = 0; k < spans; ++k) {
+                const uint32_t span = hi - lo > kLargeChunks ? spans - 1 - k : k;
+                pending.emplace_back(hi - 1 + kLag, kEncodeFlag | (lo + span * B2_FUSED_ENCODE_SPAN));
+            }
         }
         while (head < pending.size()) L.items.push_back(pending[head++].second);
         L.group_item_begin.push_back((uint32_t)L.items.size());
