@@ -19,7 +19,8 @@
 //   PAIR  : a cluster of two CTAs computes a 256 x 256 tile with cta_group::2 MMAs.  Each
 //           CTA stages its own 128 rows of A and half (128 rows) of B, so a k-block costs
 //           32 KB of loads per SM instead of 48 KB.  No multicast load is used.
-//   single: one CTA computes 128 x BN (BN = 128 or 256).
+//   single: one CTA computes 128 x BN (BN = 128 or 256).  128 x 128 is for plans of few tiles (the rule is in api.cu), whose
+//           Gram tiles may also be split along K.
 //
 // What bounds it.  A k-block (64 of K) of a pair tile is 512 clocks of MMA, reads 32 KB and receives 32 KB of shared
 // memory per SM, which together is the full 128 bytes per clock of its port.  Loads from L2 are not the limit (a
@@ -30,7 +31,8 @@
 // of decoded tiles in shared memory took a k-block from 690-900 to 560-715 clocks; Newton-Schulz of GPT-2 XL,
 // sustained under the 1000 W cap, from 46.2 to 40.8 ms.
 //
-// Three ways to launch the loop (the template parameter CHAINED separates the first from the other two):
+// Three ways to launch the loop (the template parameter CHAINED separates the first from the other two), and a fourth for
+// matrices that fit one SM (k_ns_small below):
 //   per phase : one launch per GEMM flavour and iteration, tiles dealt round-robin, launches chained with
 //               programmatic dependent launch.  The default.
 //   chained   : one persistent grid over a work list of every tile of every iteration; CTAs draw tiles with an
