@@ -1213,7 +1213,7 @@ k_quantize_flat(const float *src, const float *z, const float *xm, float beta, c
         if (blockIdx.x == 0 && threadIdx.x == 0) out_gs[0] = gs;
         return;
     }
-    encode_pipeline<MODE, 16>(chunks, beta, sx, [&](uint32_t c) {
+    encode_pipeline<MODE, MODE == 0 ? 16 : 0>(chunks, beta, sx, [&](uint32_t c) {
         return EncodeTarget{src, z, xm, fp4, scales, out_gs, len, c * kChunk, k, rows, magic, gs, scale_layout, false};
     });
 }
