@@ -1363,7 +1363,8 @@ cudaError_t launch_ns_gemm(int block_n, int pair, const GemmProblem *problems, c
 bool ns_small_fits(uint32_t rows, uint32_t cols) { return std::min(rows, cols) <= 128u && std::max(rows, cols) <= 512u; }
 uint32_t ns_small_smem(uint32_t rows, uint32_t cols) {
     const uint32_t x = rows > cols ? 2u * ((rows + 127u) / 128u) : (cols + 63u) / 64u;
-    return 1024u + (4u + x) * kSmallPanel;
+    // at least half of an SM's: a second CTA on it would only wait for the first one's tensor memory, all of which it takes
+    return std::max(1024u + (4u + x) * kSmallPanel, 116u * 1024u);
 }
 cudaError_t ns_small_configure(uint32_t smem_bytes) {
     return cudaFuncSetAttribute(k_ns_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);

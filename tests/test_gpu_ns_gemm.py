@@ -246,3 +246,15 @@ def test_split_gram_tiles(shapes, deferred):
         # one rounding to BF16 (half a unit in the last place, 2^-9 .. 2^-8 relative) on top of FP32 sums of max(r, c) products
         bound = 2.0 ** -8 * np.abs(G) + max(r, c) * 2.0 ** -24 * s * s * (np.abs(xd) @ np.abs(xd).T)
         assert np.all(np.abs(g16 - G) <= bound)
+
+
+def test_one_cta_loop_with_more_matrices_than_sms():
+    rng = np.random.default_rng(9)
+    shapes = [(64, 96), (96, 64), (128, 256)] * 110   # 330 CTAs, more than two waves of one per SM
+    xs = [_x0(rng, r, c, b2.OPERAND_BF16) for r, c in shapes[:3]]
+    results = []
+    for tile_n in (0, 128):
+        plan = _run(shapes, b2.OPERAND_BF16, 5, o.fixed_coefficients(5), tile_n, [xs[i % 3] for i in range(len(shapes))])
+        results.append([host(plan.scratch(i, 1)).copy() for i in range(len(shapes))])
+    for i, (a, b) in enumerate(zip(*results)):
+        assert np.array_equal(a, b) and np.array_equal(a, results[0][i % 3]), i
