@@ -133,10 +133,6 @@ struct Layout {
         off_problems, off_tiles_nn, off_tiles_out, off_unit_prefix, off_factor_ptrs, off_unit_partials, off_slot_stats,
         off_items, off_fused_sync, off_chain, off_gp, off_chain_sync, off_meta_end, total;
     uint32_t tiles_nn = 0, tiles_out = 0;
-    uint32_t gram_share = 0;     // k-blocks of a share of a split Gram tile, 0: the Gram phase takes the plain list
-    uint32_t tiles_gram = 0;     // entries of the split Gram list
-    size_t off_tiles_gram, off_split_partials, off_split_counters;
-    uint32_t shares(uint32_t s) const { return ((slots[s].m + 63u) / 64u + gram_share - 1u) / gram_share; }
 };
 
 bool valid_shape(uint32_t rows, uint32_t cols, const b2_muon_options &o) {
@@ -163,29 +159,6 @@ bool triangle_of_128(const uint32_t *rows, const uint32_t *cols, uint32_t count)
     }
     return full > kTileRuleSms;
 }
-// 128 x 128 Gram tiles that are few leave SMs idle while each runs through all of K: they are split into shares of at most
-// `share` k-blocks, one CTA each, where all shares together are still one wave.  A share's accumulator goes through L2
-// (about 2 us), so a split has to take at least 12 k-blocks (2.9 us) off the longest tile.  Returns the k-blocks of a share,
-// or 0 for no split.
-uint32_t gram_share(const uint32_t *rows, const uint32_t *cols, uint32_t count) {
-    uint32_t longest = 0;
-    for (uint32_t s = 0; s < count; ++s)
-        if ((uint64_t)rows[s] * cols[s] != 0) longest = std::max(longest, (std::max(rows[s], cols[s]) + 63u) / 64u);
-    if (longest > 0xffffu) return 0;
-    for (uint32_t share = 4; share + 12u <= longest; ++share) {
-        uint64_t entries = 0;
-        bool deep = false;
-        for (uint32_t s = 0; s < count && entries <= kTileRuleSms; ++s) {
-            if ((uint64_t)rows[s] * cols[s] == 0) continue;
-            const uint64_t t = (std::min(rows[s], cols[s]) + 127u) / 128u;
-            const uint32_t shares = ((std::max(rows[s], cols[s]) + 63u) / 64u + share - 1u) / share;
-            deep = deep || shares > kMaxSplit;
-            entries += t * t * shares;
-        }
-        if (entries <= kTileRuleSms && !deep) return share;
-    }
-    return 0;
-}
 // Tile configuration: tile_override = 128 / 256 forces the single-CTA kernel with that width, 512 the two-CTA pair; 0
 // picks the cheapest by estimated time.  A phase (one launch) takes a fixed time (launch, prologue, pipeline fill, last
 // epilogue) plus the longer of its longest tile and its share of all tiles; a tile takes so long per k-block (64 of K)
@@ -202,7 +175,6 @@ void pick_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t count, cons
     const Config config[3] = {{128, 128, kTileRuleSms, triangle_of_128(rows, cols, count), 5.0, 0.27, 1.9},
                               {128, 256, kTileRuleSms, false, 7.0, 0.39, 2.5},
                               {256, 256, kTileRuleSms / 2, true, 7.0, 0.37, 2.5}};
-    const uint32_t share = gram_share(rows, cols, count);
     double best_time = 0.0;
     int best = -1;
     for (int ci = 0; ci < 3; ++ci) {
@@ -222,7 +194,6 @@ void pick_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t count, cons
             total[1] += nn * (k_rest + c.epilogue);
             total[2] += out * (k_rest + c.epilogue);
         }
-        if (ci == 0 && share != 0) longest[0] = c.per_k_block * share + 2.0;
         double time = 0.0;
         for (int k = 0; k < 3; ++k) time += c.fixed + std::max(longest[k], total[k] / c.groups);
         if (best < 0 || time < best_time) { best = ci; best_time = time; }
@@ -289,7 +260,6 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
             L.small_smem = std::max(L.small_smem, ns_small_smem(rows[s], cols[s]));
         }
     }
-    L.gram_share = (L.bn == 128 && L.small_smem == 0 && o.ns_schedule == B2_NS_PER_PHASE) ? gram_share(rows, cols, count) : 0u;
     L.slots.resize(count);
     L.chunk_prefix.assign(count + 1, 0);
     size_t off = 0;
@@ -327,7 +297,7 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
     L.off_factor_ptrs = take(count * sizeof(uint64_t));
     L.off_maps = take((size_t)count * kMapsPerSlot * sizeof(CUtensorMap));
     L.off_problems = take((size_t)kProblemTypes * count * sizeof(GemmProblem));
-    L.tiles_nn = L.tiles_out = L.tiles_gram = 0;
+    L.tiles_nn = L.tiles_out = 0;
     for (uint32_t s = 0; s < count; ++s) {
         SlotLayout &sl = L.slots[s];
         sl.rows = rows[s]; sl.cols = cols[s];
@@ -339,13 +309,11 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
         sl.sub_m_nn = sl.tiles_m_nn * (L.tile_m / kGemmBlockM);  // 128-row sub-tiles (fragment scratch)
         if (sl.len == 0) continue;
         L.tiles_nn += L.symmetric ? sl.tiles_m_nn * (sl.tiles_m_nn + 1) / 2 : sl.tiles_m_nn * sl.tiles_n_nn;
-        if (L.gram_share) L.tiles_gram += sl.tiles_m_nn * sl.tiles_n_nn * L.shares(s);
         uint32_t M = rows[s] > cols[s] ? sl.m : sl.n, N = rows[s] > cols[s] ? sl.n : sl.m;
         L.tiles_out += ((M + L.tile_m - 1) / L.tile_m) * ((N + L.bn - 1) / L.bn);
     }
     L.off_tiles_nn = take((size_t)std::max(L.tiles_nn, 1u) * sizeof(GemmTile));
     L.off_tiles_out = take((size_t)std::max(L.tiles_out, 1u) * sizeof(GemmTile));
-    L.off_tiles_gram = take((size_t)std::max(L.tiles_gram, 1u) * sizeof(GemmTile));
     // the whole Newton-Schulz loop as one work list, for the iteration count the plan is made for
     L.chain_iterations = 0;
     L.chain_tiles = 0;
@@ -367,8 +335,6 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
     L.off_slot_stats = take((size_t)count * 4 * sizeof(float));
     L.off_fused_sync = take(fused_sync_bytes(count));
     L.off_chain_sync = take(chain_sync_bytes(count));
-    L.off_split_counters = take((size_t)std::max(L.tiles_gram, 1u) * kSplitCounters * sizeof(uint32_t));
-    L.off_split_partials = take((size_t)L.tiles_gram * kSplitTileBytes);
     for (uint32_t s = 0; s < count; ++s) {
         SlotLayout &sl = L.slots[s];
         if (sl.len == 0) continue;
@@ -587,17 +553,6 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
                 tnn[inn++] = GemmTile{(uint16_t)s, (uint16_t)i, (uint16_t)j, (uint16_t)((L.symmetric && j > i) ? 1 : 0)};
             }
     }
-    if (L.gram_share) {
-        GemmTile *tg = reinterpret_cast<GemmTile *>(h + L.off_tiles_gram);
-        uint32_t at = 0;
-        for (uint32_t i = 0; i < inn; ++i) {
-            const uint32_t shares = L.shares(tnn[i].problem);
-            for (uint32_t k = 0; k < shares; ++k) {
-                tg[at] = tnn[i];
-                tg[at++].reserved = (uint16_t)(tnn[i].reserved | k << 1 | (shares - 1u) << 4);
-            }
-        }
-    }
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return L.slots[a].n > L.slots[b].n; });
     for (uint32_t s : order) {
         const SlotLayout &sl = L.slots[s];
@@ -677,8 +632,6 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
         e = cudaMemsetAsync(p->ws + L.off_chain_sync, 0, chain_sync_bytes(slot_count), as_stream(stream));
     if (e == cudaSuccess)
         e = cudaMemsetAsync(p->ws + L.off_fused_sync, 0, fused_sync_bytes(slot_count), as_stream(stream));
-    if (e == cudaSuccess && L.tiles_gram)
-        e = cudaMemsetAsync(p->ws + L.off_split_counters, 0, (size_t)L.tiles_gram * kSplitCounters * sizeof(uint32_t), as_stream(stream));
     if (e != cudaSuccess) { delete p; return (int)e; }
     *out = p;
     return B2_SUCCESS;
@@ -795,11 +748,8 @@ int b2_muon_polar(b2_muon_plan *plan, const b2_muon_step_args *a, void *stream) 
                                 f16, coef, scale, status, plan->ws + L.off_chain_sync, count, dbg, grid, s, true);
         } else {
             if (mask & 1u)
-                e = launch_ns_gemm(L.bn, L.pair, probs + (size_t)(kGram0 + b) * count,
-                                   L.gram_share ? plan->at<GemmTile>(L.off_tiles_gram) : tnn,
-                                   L.gram_share ? L.tiles_gram : L.tiles_nn, kEpiGram, f16, ca, cb, cc, scale, 2u, status, dbg,
-                                   grid, s,
-                                   SplitScratch{plan->at<float>(L.off_split_partials), plan->at<uint32_t>(L.off_split_counters)});
+                e = launch_ns_gemm(L.bn, L.pair, probs + (size_t)(kGram0 + b) * count, tnn, L.tiles_nn, kEpiGram, f16, ca, cb,
+                                   cc, scale, 2u, status, dbg, grid, s);
             if (e == cudaSuccess && (mask & 2u))
                 e = launch_ns_gemm(L.bn, L.pair, probs + (size_t)kPoly * count, tnn, L.tiles_nn, kEpiPoly, f16, ca, cb, cc,
                                    nullptr, 0u, status, dbg, grid, s);

@@ -145,11 +145,8 @@ struct GemmTile {
     uint16_t problem;
     uint16_t tile_m;
     uint16_t tile_n;
-    // bit 0: also store the transposed tile (symmetric output, tile above the diagonal).  Gram lists may split K: bits 1-3
-    // the share of this entry, bits 4-6 the number of shares less one; the shares of a tile are consecutive entries.
-    uint16_t reserved;
+    uint16_t reserved;   // 1: also store the transposed tile (symmetric output, tile above the diagonal)
 };
-constexpr uint32_t kMaxSplit = 8;
 
 constexpr int kGemmBlockM = 128;
 constexpr int kGemmBlockK = 64;
@@ -180,14 +177,6 @@ struct alignas(16) ChainTile {
 };
 static_assert(sizeof(ChainTile) == 32, "ChainTile is read as two 16-byte words");
 
-// Scratch of a list with split tiles (128 x 128 tiles only): per entry an FP32 tile and a word per epilogue warp.  The
-// words are zeroed once by the owner; every launch leaves them zeroed.
-struct SplitScratch {
-    float *partials = nullptr;
-    uint32_t *counters = nullptr;
-};
-constexpr size_t kSplitTileBytes = 128 * 128 * 4;
-constexpr uint32_t kSplitCounters = 8;
 cudaError_t gemm_configure(int block_n, int pair);
 // CTAs (pairs of CTAs when `pair`) of the ticketed kernel that the device runs at the same time, 0 if unknown.
 // Call after gemm_configure.
@@ -198,7 +187,7 @@ int gemm_resident_groups(int block_n, int pair, int sm_count);
 cudaError_t launch_ns_gemm(int block_n, int pair, const GemmProblem *problems, const GemmTile *tiles,
                            uint32_t tile_count, uint32_t epilogue, int f16, float ca, float cb,
                            float cc, const float *slot_scale, uint32_t scale_pow, uint32_t *status,
-                           uint32_t debug_flags, int grid, cudaStream_t s, const SplitScratch &split = {});
+                           uint32_t debug_flags, int grid, cudaStream_t s);
 
 // The whole loop of every matrix in one launch, one CTA per matrix: for plans all of whose matrices pass ns_small_fits.
 // The problem arrays are those of the plan's first slot (`apply0` writes the second operand buffer, `apply1` the first);

@@ -19,8 +19,10 @@
 //   PAIR  : a cluster of two CTAs computes a 256 x 256 tile with cta_group::2 MMAs.  Each
 //           CTA stages its own 128 rows of A and half (128 rows) of B, so a k-block costs
 //           32 KB of loads per SM instead of 48 KB.  No multicast load is used.
-//   single: one CTA computes 128 x BN (BN = 128 or 256).  128 x 128 is for plans of few tiles (the rule is in api.cu), whose
-//           Gram tiles may also be split along K.
+//   single: one CTA computes 128 x BN (BN = 128 or 256).  128 x 128 is for plans of few tiles (the rule is in api.cu).
+// In every configuration a tile's sum runs over all of K in one order, so a matrix's result does not depend on which
+// other matrices share its plan: a sharded run and a single GPU compute the same bits.  (Splitting K of the long Gram
+// tiles of a small plan over several CTAs took one 3072 x 768 from 166 to 150 us and broke that.)
 //
 // What bounds it.  A k-block (64 of K) of a pair tile is 512 clocks of MMA, reads 32 KB and receives 32 KB of shared
 // memory per SM, which together is the full 128 bytes per clock of its port.  Loads from L2 are not the limit (a
@@ -339,18 +341,14 @@ struct alignas(16) TileEntry {
     uint32_t tile;           // tile_m | tile_n << 16
     uint32_t flags;
     uint32_t tiles_n, slot;
-    uint64_t partials;       // split tile: FP32 tile of its first share
-    uint32_t counters;       // split tile: counter words of its first share, this share (bits 24-26), shares - 1 (28-30)
-    uint32_t k_first;        // first k-block of this share
 };
-static_assert(sizeof(TileEntry) == 80, "control region layout");
+static_assert(sizeof(TileEntry) == 64, "control region layout");
 constexpr uint32_t kRing = 4;
 // flags of an entry
 constexpr uint32_t kTileAMn = 1u, kTileBMn = 2u, kTileMirror = 4u;
 constexpr uint32_t kTileShared = 8u;      // B is the A tile: loaded once, read twice
 constexpr uint32_t kTileDependent = 16u;  // the operands were written by this launch
 constexpr uint32_t kTileEnd = 32u;        // no more tiles
-constexpr uint32_t kTileSplit = 64u;      // K is split: this is one share of the tile
 constexpr int kTileEpiShift = 8, kTileScaleShift = 12, kTileIterShift = 16, kTileNShift = 24;
 
 // Fills in everything but `flags` bits that come from the list entry.  The MMA's N is the width of the tile that
@@ -366,7 +364,6 @@ __device__ __forceinline__ void fill_entry(TileEntry &e, const GemmProblem *p, u
     e.M = p->M;
     e.N = p->N;
     e.num_kb = (p->K + kGemmBlockK - 1) / kGemmBlockK;
-    e.k_first = 0;
     e.tiles_n = p->tiles_n;
     const bool last = epilogue == kEpiApplyLast;
     e.out = last ? p->out32 : p->out16;
@@ -387,9 +384,8 @@ __global__ void __launch_bounds__((Cfg<BN, PAIR>::kThreads), 1)
 k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ tiles,
           uint32_t tile_count, uint32_t epilogue_arg, int f16, GemmCoefficients coef,
           const float *__restrict__ slot_scale, uint32_t scale_pow_arg, uint32_t *status, ChainSync *sync,
-          uint32_t slot_count, SplitScratch split_scratch) {
+          uint32_t slot_count) {
     using C = Cfg<BN, PAIR>;
-    constexpr bool SPLIT = BN == 128 && !CHAINED;   // lists of this form may hold split tiles
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *stage_base = smem;
@@ -483,18 +479,8 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                     if (!claim_slot()) { ok = false; break; }
                     TileEntry &e = ring[k % kRing];
                     fill_entry<BN, PAIR>(e, problems + tl.problem, tl.tile_m, tl.tile_n, epilogue_arg,
-                                         ((tl.reserved & 1u) ? kTileMirror : 0u) | (scale_pow_arg << kTileScaleShift));
+                                         (tl.reserved ? kTileMirror : 0u) | (scale_pow_arg << kTileScaleShift));
                     e.slot = tl.problem;
-                    if (SPLIT && tl.reserved >> 4 != 0u) {
-                        // k-blocks [total * share / shares, total * (share + 1) / shares)
-                        const uint32_t share = (tl.reserved >> 1) & 7u, shares = (tl.reserved >> 4) + 1u, total = e.num_kb;
-                        const uint32_t at = t - tile_stride - share;   // list position of the first share
-                        e.k_first = total * share / shares;
-                        e.num_kb = total * (share + 1u) / shares - e.k_first;
-                        e.partials = reinterpret_cast<uint64_t>(split_scratch.partials) + (size_t)at * kSplitTileBytes;
-                        e.counters = at * kSplitCounters | share << 24 | (shares - 1u) << 28;
-                        e.flags |= kTileSplit;
-                    }
                     if (k < 2) {
                         asm volatile("prefetch.tensormap [%0];" ::"l"(e.map_a) : "memory");
                         asm volatile("prefetch.tensormap [%0];" ::"l"(e.map_b) : "memory");
@@ -561,7 +547,7 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                 if (!mbar_wait(ring_full(k), ring_parity(k), abort_flag)) break;
                 const TileEntry &e = ring[k % kRing];
                 const uint32_t flags = e.flags, tile = e.tile;
-                const int num_kb = (int)e.num_kb, k_first = (int)e.k_first;
+                const int num_kb = (int)e.num_kb;
                 const uint64_t map_a = e.map_a, map_b = e.map_b;
                 mbar_arrive(ring_empty(k));
                 if (flags & kTileEnd) break;
@@ -590,7 +576,7 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                             if (shared) mbar_arrive(full_bar(stage));   // in the other producer's place
                         }
                         const uint32_t fb = leader_full + 8u * stage, dst = dst0 + stage * (uint32_t)C::kStageBytes;
-                        const int k0 = (k_first + kb) * kGemmBlockK;
+                        const int k0 = kb * kGemmBlockK;
                         if (mn) {   // 64 x 64 boxes: x = M or N index, y = K index
                             for (int j = 0; j < boxes; ++j) {
                                 tma_load_2d<PAIR>(dst + (2 * j) * kBoxBytes, map, fb, row0 + 128 * j, k0);
@@ -708,8 +694,6 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
             const size_t pitch = entry.pitch_bytes;
             const float4 *frag = reinterpret_cast<const float4 *>(entry.frag);
             const int tile_m = (int)(entry.tile & 0xffffu), tile_n = (int)(entry.tile >> 16);
-            float4 *const partials = reinterpret_cast<float4 *>(entry.partials);
-            const uint32_t split = entry.counters;
             // fragment scratch is indexed by 128-row sub-tiles
             const uint32_t tile_lin = (PAIR ? (uint32_t)tile_m * 2 + rank : (uint32_t)tile_m) * entry.tiles_n + tile_n;
             __syncwarp();
@@ -763,45 +747,6 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                 out_scale = scale_pow == 2u ? sv * sv : sv;
             }
             const bool scaled = out_scale != 1.0f;   // warp-uniform
-
-            // Split K: every share leaves its FP32 accumulator in memory (fragment order, one 32 x 64 block per warp) and
-            // the warp that finds itself last adds the shares up in their order, so the sum does not depend on who that
-            // is, and goes on with the epilogue; nobody waits.
-            const bool is_split = SPLIT && (flags & kTileSplit) != 0u;
-            const uint32_t shares = (split >> 28) + 1u;
-            const size_t part0 = (size_t)(c0 / 32) * 8 * kGemmBlockM + row_in_tile;
-            constexpr size_t kPartStride = kSplitTileBytes / 16;
-            if (is_split) {
-                float4 *mine = partials + (size_t)((split >> 24) & 7u) * kPartStride + part0;
-#pragma unroll 1
-                for (int sub = 0; sub < 2; ++sub) {
-                    uint32_t v[32];
-                    tc_ld32(taddr + 32 * sub, v);
-                    tc_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        __stcg(mine + (8 * sub + j) * kGemmBlockM, make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                                                               __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
-                }
-                tc_fence_before();
-                __threadfence();
-                __syncwarp();
-                uint32_t arrived = 0;
-                if (lane == 0) {
-                    mbar_arrive_cluster(tempty);
-                    uint32_t *counter = split_scratch.counters + (split & 0xffffffu) + (warp - C::kEpiWarp0);
-                    arrived = atomicAdd(counter, 1u);
-                    if (arrived + 1u == shares) *counter = 0u;   // as the next launch expects it
-                    __threadfence();
-                }
-                arrived = __shfl_sync(0xffffffffu, arrived, 0);
-                __syncwarp();
-                if (arrived + 1u != shares) {
-                    acc ^= 1u;
-                    if (acc == 0) acc_phase ^= 1u;
-                    continue;
-                }
-            }
 
             if (epilogue == kEpiApplyLast) {
                 // FP32 result in the storage layout: 32 columns (128 bytes) per staged slab
@@ -863,30 +808,9 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
 #pragma unroll
                 for (int sub = 0; sub < 2; ++sub) {
                     uint32_t v[32];
-                    if (is_split) {
-                        const float4 *p = partials + part0 + 8 * sub * kGemmBlockM;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float4 w = __ldcg(p + j * kGemmBlockM);
-                            v[4 * j] = __float_as_uint(w.x); v[4 * j + 1] = __float_as_uint(w.y);
-                            v[4 * j + 2] = __float_as_uint(w.z); v[4 * j + 3] = __float_as_uint(w.w);
-                        }
-                        for (uint32_t share = 1; share < shares; ++share) {
-                            p += kPartStride;
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const float4 w = __ldcg(p + j * kGemmBlockM);
-                                v[4 * j] = __float_as_uint(__uint_as_float(v[4 * j]) + w.x);
-                                v[4 * j + 1] = __float_as_uint(__uint_as_float(v[4 * j + 1]) + w.y);
-                                v[4 * j + 2] = __float_as_uint(__uint_as_float(v[4 * j + 2]) + w.z);
-                                v[4 * j + 3] = __float_as_uint(__uint_as_float(v[4 * j + 3]) + w.w);
-                            }
-                        }
-                    } else {
-                        tc_ld32(taddr + 32 * sub, v);
-                        tc_ld_wait();
-                    }
-                    if (sub == 1 && !hold && !is_split) {
+                    tc_ld32(taddr + 32 * sub, v);
+                    tc_ld_wait();
+                    if (sub == 1 && !hold) {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster(tempty);
@@ -1243,7 +1167,7 @@ template <int BN, bool PAIR, bool CHAINED>
 cudaError_t launch_impl(const GemmProblem *problems, const void *tiles, uint32_t tile_count, uint32_t epilogue,
                         int f16, const GemmCoefficients &coef, const float *slot_scale, uint32_t scale_pow,
                         uint32_t *status, void *sync, uint32_t slot_count, uint32_t debug_flags, int grid,
-                        cudaStream_t s, const SplitScratch &split) {
+                        cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     unsigned n_attr = 0;
@@ -1276,24 +1200,24 @@ cudaError_t launch_impl(const GemmProblem *problems, const void *tiles, uint32_t
     cfg.dynamicSmemBytes = Cfg<BN, PAIR>::kSmemBytes;
     cfg.stream = s;
     return cudaLaunchKernelEx(&cfg, k_ns_gemm<BN, PAIR, CHAINED>, problems, tiles, tile_count, epilogue, f16, coef,
-                              slot_scale, scale_pow, status, static_cast<ChainSync *>(sync), slot_count, split);
+                              slot_scale, scale_pow, status, static_cast<ChainSync *>(sync), slot_count);
 }
 
 template <bool CHAINED>
 cudaError_t dispatch(int block_n, int pair, const GemmProblem *problems, const void *tiles, uint32_t tile_count,
                      uint32_t epilogue, int f16, const GemmCoefficients &coef, const float *slot_scale,
                      uint32_t scale_pow, uint32_t *status, void *sync, uint32_t slot_count, uint32_t debug_flags,
-                     int grid, cudaStream_t s, const SplitScratch &split = {}) {
+                     int grid, cudaStream_t s) {
     if (tile_count == 0) return cudaSuccess;
     if (pair && block_n == 256)
         return launch_impl<256, true, CHAINED>(problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow,
-                                                  status, sync, slot_count, debug_flags, grid, s, split);
+                                                  status, sync, slot_count, debug_flags, grid, s);
     if (!pair && block_n == 256)
         return launch_impl<256, false, CHAINED>(problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow,
-                                                   status, sync, slot_count, debug_flags, grid, s, split);
+                                                   status, sync, slot_count, debug_flags, grid, s);
     if (!pair && block_n == 128)
         return launch_impl<128, false, CHAINED>(problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow,
-                                                   status, sync, slot_count, debug_flags, grid, s, split);
+                                                   status, sync, slot_count, debug_flags, grid, s);
     return cudaErrorInvalidValue;
 }
 
@@ -1354,11 +1278,11 @@ int gemm_resident_groups(int block_n, int pair, int sm_count) {
 cudaError_t launch_ns_gemm(int block_n, int pair, const GemmProblem *problems, const GemmTile *tiles,
                            uint32_t tile_count, uint32_t epilogue, int f16, float ca, float cb,
                            float cc, const float *slot_scale, uint32_t scale_pow, uint32_t *status,
-                           uint32_t debug_flags, int grid, cudaStream_t s, const SplitScratch &split) {
+                           uint32_t debug_flags, int grid, cudaStream_t s) {
     GemmCoefficients coef = {};
     coef.v[0] = ca; coef.v[1] = cb; coef.v[2] = cc;
     return dispatch<false>(block_n, pair, problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow, status,
-                           nullptr, 0u, debug_flags, grid, s, split);
+                           nullptr, 0u, debug_flags, grid, s);
 }
 bool ns_small_fits(uint32_t rows, uint32_t cols) { return std::min(rows, cols) <= 128u && std::max(rows, cols) <= 512u; }
 uint32_t ns_small_smem(uint32_t rows, uint32_t cols) {

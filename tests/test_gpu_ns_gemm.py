@@ -214,15 +214,16 @@ def test_tile_choice_agrees_with_the_oracle_on_both_sides_of_the_line():
 
 @pytest.mark.parametrize("deferred", [False, True])
 @pytest.mark.parametrize("shapes", [
-    [(3072, 768)],                              # four shares of twelve k-blocks
-    [(77, 1040), (1999, 64), (130, 16)],        # shares of unequal length, one matrix not split, ragged everywhere
-    [(200, 1536)],                              # shares of a wide matrix, tiles clipped in both directions
+    [(3072, 768)],                              # 36 Gram tiles of 128 x 128, each 48 k-blocks
+    [(77, 1040), (1999, 64), (130, 16)],        # ragged everywhere
+    [(200, 1536)],                              # wide, tiles clipped in both directions
 ])
-def test_split_gram_tiles(shapes, deferred):
-    """Few 128 x 128 Gram tiles with a long K are split; the shares add up to the product, launch after launch."""
+def test_few_gram_tiles_with_a_long_k(shapes, deferred):
+    """One iteration of 128 x 128 tiles, launch after launch, against FP64: every phase from the operands it has read."""
     rng = np.random.default_rng(17)
     xs = [_x0(rng, r, c, b2.OPERAND_BF16) for r, c in shapes]
     s = 0.75 if deferred else 1.0
+    ca, cb, cc = (float(v) for v in o.fixed_coefficients(1)[0])
     plan = b2.MuonPlan(shapes, scale_layout=b2.SCALES_RAW, tile_n=128, max_iterations=1,
                        normalize_mode=b2.NORMALIZE_DEFERRED if deferred else b2.NORMALIZE_TWO_PASS)
     first = None
@@ -235,17 +236,48 @@ def test_split_gram_tiles(shapes, deferred):
         torch.cuda.synchronize()
         assert plan.status() == 0
         got = [[host(plan.scratch(i, w).float()).copy() for w in (5, 6, 1)] for i in range(len(shapes))]
-        if first is not None:   # which share comes last must not matter
+        if first is not None:   # every launch gives the same bits
             assert all(np.array_equal(u, v) for a, b in zip(first, got) for u, v in zip(a, b))
         first = got
+    half_ulp, eps = 2.0 ** -8, 2.0 ** -24   # one rounding to BF16: half a unit in the last place, 2^-9 .. 2^-8 relative
     for x, (r, c), (g16, q16, u) in zip(xs, shapes, got):
         n = min(r, c)
         xd = (x if r <= c else x.T).astype(np.float64)
         G = xd @ xd.T * s * s
-        g16 = g16.reshape(n, -1)[:, :n]
-        # one rounding to BF16 (half a unit in the last place, 2^-9 .. 2^-8 relative) on top of FP32 sums of max(r, c) products
-        bound = 2.0 ** -8 * np.abs(G) + max(r, c) * 2.0 ** -24 * s * s * (np.abs(xd) @ np.abs(xd).T)
-        assert np.all(np.abs(g16 - G) <= bound)
+        g16, q16 = (v.reshape(n, -1)[:, :n].astype(np.float64) for v in (g16, q16))
+        # FP32 sums of max(r, c) products, the scaling included
+        g_sum = (max(r, c) + 2) * eps * s * s * (np.abs(xd) @ np.abs(xd).T)
+        assert np.all(np.abs(g16 - G) <= half_ulp * np.abs(G) + g_sum)
+        # Q = c G16 G16 + b G + a I: FP32 sums of n products and two fused multiply-adds, then one rounding to BF16
+        Q = cc * (g16 @ g16) + cb * G + ca * np.eye(n)
+        q_sum = (n + 4) * eps * (abs(cc) * (np.abs(g16) @ np.abs(g16)) + abs(cb) * np.abs(G) + abs(ca)) + abs(cb) * g_sum
+        assert np.all(np.abs(q16 - Q) <= half_ulp * (np.abs(Q) + q_sum) + q_sum)
+        want = s * (q16 @ xd)
+        got_u = (u.reshape(r, c) if r <= c else u.reshape(r, c).T).astype(np.float64)
+        assert np.all(np.abs(got_u - want) <= (n + 2) * eps * s * (np.abs(q16) @ np.abs(xd)))
+
+
+@pytest.mark.parametrize("company", [
+    [(512, 256), (256, 256), (256, 1024), (384, 128)],   # few more tiles of 128 x 128
+    [(64, 64)],
+    [(768, 768)] * 5,
+    [(2304, 768)] * 9,                                   # two-CTA tiles
+])
+@pytest.mark.parametrize("shape", [(768, 256), (512, 256), (384, 128), (3072, 768), (200, 1536), (77, 1040)])
+def test_result_of_a_matrix_does_not_depend_on_its_company(shape, company):
+    """A rank of a sharded run and a single GPU compute the same bits: whatever tiles a plan takes for the matrices it
+    holds, every sum runs over K in one order."""
+    rng = np.random.default_rng(shape[0])
+    x = _x0(rng, *shape, b2.OPERAND_BF16)
+    others = [_x0(rng, r, c, b2.OPERAND_BF16) for r, c in company]
+    results = []
+    for at, shapes, xs in ((0, [shape], [x]), (0, [shape] + company, [x] + others), (len(company), company + [shape], others + [x])):
+        plan = _run(shapes, b2.OPERAND_BF16, 5, o.fixed_coefficients(5), 0, xs)
+        results.append([host(plan.scratch(at, w).float()).copy() for w in (1, 5, 6, 7)])
+        plan.close()
+    for other in results[1:]:
+        for w, a, b in zip(("U", "Gram", "Q", "X1"), results[0], other):
+            assert np.array_equal(a, b), (w, float(np.abs(a - b).max()))
 
 
 def test_one_cta_loop_with_more_matrices_than_sms():
