@@ -456,7 +456,7 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
     e = gemm_configure(L.bn, L.pair);
     if (e != cudaSuccess) { delete p; return (int)e; }
     if (L.small_smem) {
-        e = ns_small_configure(L.small_smem);
+        e = ns_small_configure();
         if (e != cudaSuccess) { delete p; return (int)e; }
     }
     p->resident_groups = (uint32_t)std::max(gemm_resident_groups(L.bn, L.pair, p->dev.sm_count), 0);

@@ -1285,13 +1285,19 @@ cudaError_t launch_ns_gemm(int block_n, int pair, const GemmProblem *problems, c
                            nullptr, 0u, debug_flags, grid, s);
 }
 bool ns_small_fits(uint32_t rows, uint32_t cols) { return std::min(rows, cols) <= 128u && std::max(rows, cols) <= 512u; }
+namespace {
+// what the largest matrix that fits needs: G and Q, two panels each, and an operand of eight
+constexpr uint32_t kSmallMaxSmem = 1024u + 12u * kSmallPanel;
+static_assert(kSmallMaxSmem <= (uint32_t)kSmemLimit, "one SM holds the largest matrix");
+}  // namespace
 uint32_t ns_small_smem(uint32_t rows, uint32_t cols) {
     const uint32_t x = rows > cols ? 2u * ((rows + 127u) / 128u) : (cols + 63u) / 64u;
     // at least half of an SM's: a second CTA on it would only wait for the first one's tensor memory, all of which it takes
     return std::max(1024u + (4u + x) * kSmallPanel, 116u * 1024u);
 }
-cudaError_t ns_small_configure(uint32_t smem_bytes) {
-    return cudaFuncSetAttribute(k_ns_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+// The limit belongs to the function, not to a plan: it is always the largest, so that no plan takes it from another.
+cudaError_t ns_small_configure() {
+    return cudaFuncSetAttribute(k_ns_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
 }
 cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, const GemmProblem *apply0, const GemmProblem *apply1,
                             const GemmProblem *last, uint32_t slot_count, uint32_t iterations, int f16, int last16,

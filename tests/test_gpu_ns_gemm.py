@@ -290,3 +290,19 @@ def test_one_cta_loop_with_more_matrices_than_sms():
         results.append([host(plan.scratch(i, 1)).copy() for i in range(len(shapes))])
     for i, (a, b) in enumerate(zip(*results)):
         assert np.array_equal(a, b) and np.array_equal(a, results[0][i % 3]), i
+
+
+def test_a_plan_made_later_leaves_an_earlier_one_working():
+    """Plans of the one-CTA loop need 116 to 193 KB of shared memory; the kernel's limit is one for all of them."""
+    rng = np.random.default_rng(2)
+    shapes = [(128, 512), (64, 64)]
+    xs = [_x0(rng, r, c, b2.OPERAND_BF16) for r, c in shapes]
+    args = b2.MuonMegaUpdateArgs(coefficients=o.fixed_coefficients(5))
+    plans = [b2.MuonPlan([s], scale_layout=b2.SCALES_RAW) for s in shapes]   # the largest first, both alive
+    for plan, x, s in zip(plans, xs, shapes):
+        plan.scratch(0, 0).copy_(dev(x).to(torch.bfloat16))
+        b2.OptimizerModule().muon_polar(plan, args)
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        alone = _run([s], b2.OPERAND_BF16, 5, o.fixed_coefficients(5), 128, [x])   # per phase
+        assert torch.equal(plan.scratch(0, 1), alone.scratch(0, 1))
