@@ -211,6 +211,8 @@ __device__ __forceinline__ void atomic_max_nonneg(float *addr, float v) {
 
 // First statement of every streaming kernel: the next launch of the stream may begin, and this one goes on once the launch
 // in front of it has ended and its stores are visible (programmatic dependent launch; a no-op without the attribute).
+// A kernel may therefore be running while what it will read is still being written (the clip scale, NorMuon factors), so
+// these kernels read nothing through the read-only path: no __ldg, no const __restrict__.
 __device__ __forceinline__ void stream_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

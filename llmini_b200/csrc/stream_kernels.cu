@@ -99,7 +99,7 @@ __device__ __forceinline__ float qk_clip_factor(const b2_muon_slot_descriptor &d
     if (factors == nullptr || d.qk_clip_factor_offset == 0xffffffffu || d.qk_clip_head_dim == 0) return 1.0f;
     if (row >= 2u * d.cols) return 1.0f;
     const uint32_t in_block = row >= d.cols ? row - d.cols : row;   // row % cols for row < 2 cols
-    return __ldg(factors + d.qk_clip_factor_offset + in_block / d.qk_clip_head_dim);
+    return factors[d.qk_clip_factor_offset + in_block / d.qk_clip_head_dim];
 }
 
 struct ChunkCtx {
@@ -167,7 +167,7 @@ k_muon_momentum_sumsq(const b2_muon_slot_descriptor *slots, const uint32_t *pref
                       float *amax_x) {
     stream_enter();
     const int tid = threadIdx.x;
-    if (mp.d_grad_scale) mp.grad_scale = __ldg(mp.d_grad_scale);
+    if (mp.d_grad_scale) mp.grad_scale = *mp.d_grad_scale;
     for (uint32_t c0 = 2 * blockIdx.x; c0 < total_chunks; c0 += 2 * gridDim.x) {
         float local[2] = {0.0f, 0.0f};
         QuadRaw<VS> raw[2][2];
@@ -238,7 +238,7 @@ k_muon_normalize(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, u
                  MomentumParams mp, const float *inv_norm, const uint64_t *x0_ptrs, const uint64_t *u_ptrs, int f16) {
     stream_enter();
     const int tid = threadIdx.x;
-    if (mp.d_grad_scale) mp.grad_scale = __ldg(mp.d_grad_scale);
+    if (mp.d_grad_scale) mp.grad_scale = *mp.d_grad_scale;
     for (uint32_t c = blockIdx.x; c < total_chunks; c += gridDim.x) {
         const uint32_t slot = find_slot(prefix, slot_count, c);
         const b2_muon_slot_descriptor *d = slots + slot;
@@ -285,8 +285,8 @@ __device__ __forceinline__ SymExpLin symexp_for_slot(const UpdateParams &up, uin
             float v[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                const float z = __ldg(reinterpret_cast<const float *>(p[2 * k]));
-                const float x = __ldg(reinterpret_cast<const float *>(p[2 * k + 1]));
+                const float z = *reinterpret_cast<const float *>(p[2 * k]);
+                const float x = *reinterpret_cast<const float *>(p[2 * k + 1]);
                 v[k] = z + up.beta * (x - z);
             }
             s.exponential = v[0]; s.linear = v[1]; s.curvature = v[2];
@@ -304,10 +304,10 @@ __device__ __forceinline__ void neuron_factors(const ChunkCtx &cx, const UpdateP
     const float *fp = reinterpret_cast<const float *>(up.factor_ptrs[cx.slot]);
     const float sc = with_scale ? up.slot_stats[cx.slot * 4] : 1.0f;
     if (cx.d.rows >= cx.d.cols) {
-        const float f = with_scale ? __ldg(fp + row) * sc : __ldg(fp + row);
+        const float f = with_scale ? fp[row] * sc : fp[row];
         nf[0] = nf[1] = nf[2] = nf[3] = f;
     } else {
-        const float4 f = __ldg(reinterpret_cast<const float4 *>(fp + (i - row * cx.d.cols)));
+        const float4 f = *reinterpret_cast<const float4 *>(fp + (i - row * cx.d.cols));
         nf[0] = f.x; nf[1] = f.y; nf[2] = f.z; nf[3] = f.w;
         if (with_scale) {
 #pragma unroll
@@ -744,7 +744,7 @@ k_muon_sign_update(const b2_muon_slot_descriptor *slots, const uint32_t *prefix,
     stream_enter();
     __shared__ float warp_ax[kThreads / 32], warp_ay[kThreads / 32];
     const int tid = threadIdx.x;
-    if (mp.d_grad_scale) mp.grad_scale = __ldg(mp.d_grad_scale);
+    if (mp.d_grad_scale) mp.grad_scale = *mp.d_grad_scale;
     for (uint32_t c = blockIdx.x; c < total_chunks; c += gridDim.x) {
         ChunkCtx cx = chunk_ctx(slots, prefix, slot_count, c);
         float *grad = reinterpret_cast<float *>(cx.d.grad);
@@ -849,7 +849,7 @@ __device__ __forceinline__ SymExpLin symexp_resolve(const SymExpLinParams &p, fl
         float v[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const float z = __ldg(p.scales[2 * k]), x = __ldg(p.scales[2 * k + 1]);
+            const float z = *p.scales[2 * k], x = *p.scales[2 * k + 1];
             v[k] = z + schedule_beta * (x - z);
         }
         s.exponential = v[0]; s.linear = v[1]; s.curvature = v[2];
@@ -1334,7 +1334,7 @@ k_adamw(float *z, float *x, float *grad, float *m1, float *m2, float *amax, Adam
         const float *d_grad_scale, uint32_t len) {
     stream_enter();
     __shared__ float warp_part[kThreads / 32];
-    if (d_grad_scale) a.grad_scale = __ldg(d_grad_scale);
+    if (d_grad_scale) a.grad_scale = *d_grad_scale;
     const int tid = threadIdx.x;
     const float decay = 1.0f - a.lr * a.wd;
     const bool aligned = ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(x) |
@@ -1413,7 +1413,7 @@ k_adamw_multi(const b2_adamw_slot_descriptor *t, uint32_t count, uint32_t total_
     stream_enter();
     __shared__ float warp_part[kThreads / 32];
     const int tid = threadIdx.x;
-    if (d_grad_scale) a.grad_scale = __ldg(d_grad_scale);
+    if (d_grad_scale) a.grad_scale = *d_grad_scale;
     const float decay = 1.0f - a.lr * a.wd;
     for (uint32_t c = blockIdx.x; c < total_chunks; c += gridDim.x) {
         const uint32_t slot = find_adam_slot(t, count, c);

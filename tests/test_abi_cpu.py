@@ -131,3 +131,21 @@ def test_one_pass_prepare_is_refused_for_f16_operands():
     h = C.c_void_p()
     n = L.b2_muon_workspace_bytes(rows, cols, 1, C.byref(opt))
     assert L.b2_muon_plan_create(C.byref(h), rows, cols, 1, C.byref(opt), 1024, n, None) == _ffi.ERROR_INVALID_VALUE
+
+
+def test_streaming_kernels_wait_before_they_read_and_read_coherently():
+    """Launches that may start before the one in front of them has ended (csrc/stream_kernels.cu): every kernel so launched
+    waits in its first statement, and nothing is read through the read-only path, which is for data that no running kernel
+    writes (the clip scale and the NorMuon factors are written by the kernel in front)."""
+    import re
+
+    csrc = os.path.join(os.path.dirname(os.path.abspath(_ffi.__file__)), "csrc")
+    with open(os.path.join(csrc, "stream_kernels.cu")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    for form in ("__ldg(", "__restrict__", "ld.global.nc"):
+        assert form not in text, form
+    launched = set(re.findall(r"stream_launch\([^;]*?\b(k_\w+)", text))
+    assert len(launched) >= 20
+    for kernel in launched:
+        body = re.search(r"__global__[^;{]*\b" + kernel + r"\(.*?\)\s*\{\s*(\w+\(\);)", text, re.S)
+        assert body and body.group(1) == "stream_enter();", kernel

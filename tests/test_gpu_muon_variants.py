@@ -529,3 +529,58 @@ def test_normuon_without_state_buffer_is_the_plain_update():
     for a, b in zip(*outs):
         for u, v in zip(a, b):
             assert np.array_equal(u, v)
+
+
+@pytest.mark.parametrize("finish", ["normuon", "hyperball", "sign"])
+def test_a_chain_of_calls_equals_the_same_calls_with_a_wait_after_each(finish):
+    """Every kernel of a step may start before the one in front of it has ended, and what it reads (clip scale, factors,
+    statistics, maxima) may still be being written then: three steps with other values each."""
+    shapes = [(48, 160), (160, 48), (96, 96), (512, 1040)]
+    opt = b2.OptimizerModule()
+
+    def run(wait):
+        rng = np.random.default_rng(8)
+        slots = []
+        for r, c in shapes:
+            n = r * c
+            s = _slot(r, c, U.gradients(rng, n), o.bf16_bits(U.weights(rng, n, 1e-3)), U.weights(rng, n), U.weights(rng, n),
+                      o.bf16_bits(np.abs(U.weights(rng, n, 1e-6))))
+            s.second_momentum = dev(np.abs(U.weights(rng, max(r, c), 1e-3)) + F(1e-4))
+            slots.append(s)
+        plan, table = b2.MuonPlan(shapes, scale_layout=b2.SCALES_RAW), b2.slot_table(slots)
+        scale, norm = torch.zeros(1, device="cuda"), torch.zeros(1, device="cuda")
+        cuts = [(s.grad.data_ptr() + 4 * a, min(2048, r * c - a)) for s, (r, c) in zip(slots, shapes) for a in range(0, r * c, 2048)]
+        clip = dict(chunk_ptrs=torch.tensor([p for p, _ in cuts], dtype=torch.int64, device="cuda"),
+                    chunk_lens=torch.tensor([n for _, n in cuts], dtype=torch.int32, device="cuda"),
+                    chunk_sums=torch.zeros(len(cuts), device="cuda"), extra_sums=None, scale=scale, norm=norm,
+                    chunk_count=len(cuts), extra_sum_count=0, max_norm=0.5, apply=False)
+        args = b2.MuonMegaUpdateArgs(learning_rate=0.02, average_coefficient=0.5, schedule_beta=0.3, variance_adaptive=True,
+                                     bias_correction_inv=1.25, grad_scale_device=scale, normuon=finish == "normuon",
+                                     coefficients=o.fixed_coefficients(5))
+        calls = [lambda: opt.clip_gradients(**clip)]
+        if finish == "sign":
+            calls.append(lambda: opt.muon_tma_sign_update_deferred_quantization(plan, table, args))
+        else:
+            calls += [lambda: opt.muon_tma_prepare_polar(plan, table, args), lambda: opt.muon_polar(plan, args)]
+            calls.append(lambda: opt.muon_tma_finish_hyperball_update_deferred_quantization(plan, table, args) if finish == "hyperball"
+                         else opt.muon_tma_finish_update_deferred_quantization(plan, table, args))
+        calls.append(lambda: opt.muon_materialize_training_weights(plan, table))
+        torch.cuda.synchronize()
+        scales = []
+        for _ in range(3):
+            for call in calls:
+                call()
+                if wait:
+                    torch.cuda.synchronize()
+            scales.append(scale.clone())
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        plan.close()
+        return scales, [(s.grad, s.momentum, s.variance, s.z_master, s.x_master, s.second_momentum, s.bytes, s.scales,
+                         s.global_scale) for s in slots]
+
+    (sa, a), (sb, b) = run(False), run(True)
+    assert all(torch.equal(u, v) for u, v in zip(sa, sb)) and len({float(v) for v in sb}) > 1
+    for shape, u, v in zip(shapes, a, b):
+        for k, (x, y) in enumerate(zip(u, v)):
+            assert torch.equal(x, y), (shape, k)
