@@ -115,8 +115,7 @@ struct SlotLayout {
 struct Layout {
     std::vector<SlotLayout> slots;
     std::vector<uint32_t> chunk_prefix;  // slot_count + 1
-    std::vector<uint32_t> unit_prefix;   // slot_count + 1: NorMuon work units (32 rows or unit_cols columns)
-    uint32_t unit_cols = 128;
+    std::vector<uint32_t> unit_prefix;   // slot_count + 1: NorMuon work units (runs of rows or of columns)
     std::vector<uint32_t> items;         // work list of the fused update + encode launch
     std::vector<uint32_t> group_item_begin;   // groups + 1 entries: where each finish group's part of `items` begins
     uint32_t chain_tiles = 0;            // entries of the chained Newton-Schulz work list (0: not built)
@@ -276,14 +275,10 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
     }
     L.chunk_prefix[count] = chunks;
     L.total_chunks = chunks;
-    uint64_t wide_columns = 0;
-    for (uint32_t s = 0; s < count; ++s)
-        if (rows[s] < cols[s]) wide_columns += (cols[s] + 127u) / 128u;
-    L.unit_cols = wide_columns >= kTileRuleSms ? 128u : 32u;
     L.unit_prefix.assign(count + 1, 0);
     for (uint32_t s = 0; s < count; ++s) {
         uint32_t units = 0;
-        if ((uint64_t)rows[s] * cols[s] != 0) units = rows[s] >= cols[s] ? (rows[s] + B2_NORMUON_ROWS_PER_UNIT - 1) / B2_NORMUON_ROWS_PER_UNIT : (cols[s] + L.unit_cols - 1) / L.unit_cols;
+        if ((uint64_t)rows[s] * cols[s] != 0) units = rows[s] >= cols[s] ? (rows[s] + B2_NORMUON_ROWS_PER_UNIT - 1) / B2_NORMUON_ROWS_PER_UNIT : (cols[s] + B2_NORMUON_COLS_PER_UNIT - 1) / B2_NORMUON_COLS_PER_UNIT;
         L.unit_prefix[s + 1] = L.unit_prefix[s] + units;
     }
     // ---- metadata region (uploaded at plan creation) ----
@@ -388,7 +383,6 @@ struct b2_muon_plan {
         NeuronView nv;
         nv.unit_prefix = at<uint32_t>(layout.off_unit_prefix);
         nv.total_units = layout.unit_prefix.back();
-        nv.unit_cols = layout.unit_cols;
         nv.factor_ptrs = at<uint64_t>(layout.off_factor_ptrs);
         nv.partials = at<double>(layout.off_unit_partials);
         nv.slot_stats = at<float>(layout.off_slot_stats);

@@ -25,12 +25,12 @@ struct MomentumParams {
     float bias_correction_inv;
 };
 #define B2_NORMUON_ROWS_PER_UNIT 32
+#define B2_NORMUON_COLS_PER_UNIT 64
 // NorMuon / Hyperball scratch of a plan: work units are B2_NORMUON_ROWS_PER_UNIT rows (slots with rows >= cols) or
-// `unit_cols` (32 or 128) columns (rows < cols) of one slot; `unit_prefix` counts them like `chunk_prefix` counts chunks.
+// B2_NORMUON_COLS_PER_UNIT columns (rows < cols) of one slot; `unit_prefix` counts them like `chunk_prefix` counts chunks.
 struct NeuronView {
     const uint32_t *unit_prefix;   // device, slot_count + 1 entries
     uint32_t total_units;
-    uint32_t unit_cols;
     const uint64_t *factor_ptrs;   // device, per slot: f32[max(rows, cols)] factors
     double *partials;              // device, 4 per unit: raw, scaled, parameter, dot
     float *slot_stats;             // device, 4 per slot: normuon_scale, update_norm, radius, dot

@@ -458,19 +458,21 @@ k_muon_update(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint
 // NorMuon second moment per neuron, and the Hyperball statistics when `hyperball` is set:
 // crates/cuda-kernels/src/gpt/optimizer/muon/fused/tma_split.rs:285-443.  U is in the storage
 // layout here, so a neuron's values are one row (rows >= cols: a warp per row) or one column
-// (rows < cols: COLS columns per CTA, the threads striding over the rows); both read whole 128-byte lines or more.  Per
-// unit four partial sums leave the CTA: raw, scaled, parameter, dot.
-// COLS = 0 handles the row-neuron units, the others the column-neuron ones; each instance skips the
+// (rows < cols: B2_NORMUON_COLS_PER_UNIT columns per CTA, the threads striding over the rows); both read whole 128-byte
+// lines or more.  Per unit four partial sums leave the CTA: raw, scaled, parameter, dot.
+// COLS = 0 handles the row-neuron units, COLS = 1 the column-neuron ones; each instance skips the
 // other's units, so the register-hungry column form (eight loads in flight per thread) does not
 // take the occupancy of the row form down with it.
-// COLS = 128 where that gives every SM a unit, else 32: a matrix of a thousand columns is nine units of 128, each a chain
-// of round trips over its rows (ragged plan of 5 matrices: 19 us, with 32 columns 9; GPT-2 medium: 80 us, with 32 103).
+// The width of a column unit sets the order of a neuron's sum, so it is one width for every matrix in every plan: chosen by
+// the number of units in a plan, it let a matrix's bits depend on its company.  Narrow units give a lone matrix more CTAs,
+// each with a shorter chain of round trips; wide ones read longer pieces of a row.  NorMuon finish with 32 / 64 / 128 columns
+// (us): ragged plan of 5 matrices 24.9 / 25.8 / 28.9, one 768 x 3072 18.8 / 20.5 / 22.8, GPT-2 medium 1523 / 1494 / 1478.
 template <int COLS>
 __global__ void __launch_bounds__(kThreads, COLS ? 2 : 4)
 k_normuon_stats(const b2_muon_slot_descriptor *slots, uint32_t slot_count, NeuronView nv, const uint64_t *u_ptrs,
                 int hyperball) {
     stream_enter();
-    constexpr uint32_t kUnitCols = COLS ? COLS : 4, kQuads = kUnitCols / 4, kRowLanes = kThreads / kQuads;
+    constexpr uint32_t kUnitCols = COLS ? B2_NORMUON_COLS_PER_UNIT : 4, kQuads = kUnitCols / 4, kRowLanes = kThreads / kQuads;
     __shared__ float col_raw[COLS ? kRowLanes : 1][kUnitCols], col_dot[COLS ? kRowLanes : 1][kUnitCols];
     __shared__ double part[kThreads / 32][4];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1812,10 +1814,7 @@ cudaError_t launch_normuon_stats(const SlotView &v, const NeuronView &nv, const 
                                  cudaStream_t s) {
     if (nv.total_units == 0) return cudaSuccess;
     stream_launch(kPlain, k_normuon_stats<0>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
-    if (nv.unit_cols == 128)
-        stream_launch(kOverlapped, k_normuon_stats<128>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
-    else
-        stream_launch(kOverlapped, k_normuon_stats<32>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
+    stream_launch(kOverlapped, k_normuon_stats<1>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
     stream_launch(kOverlapped, k_normuon_reduce, v.slot_count, kThreads, s, v.slots, nv);
     return cudaGetLastError();
 }

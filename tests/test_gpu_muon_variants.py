@@ -584,3 +584,41 @@ def test_a_chain_of_calls_equals_the_same_calls_with_a_wait_after_each(finish):
     for shape, u, v in zip(shapes, a, b):
         for k, (x, y) in enumerate(zip(u, v)):
             assert torch.equal(x, y), (shape, k)
+
+
+@pytest.mark.parametrize("hyperball", [False, True])
+@pytest.mark.parametrize("shape", [(96, 400), (300, 1040), (77, 112), (16, 2064), (1000, 16), (384, 128)])
+def test_neuron_statistics_do_not_depend_on_the_company(shape, hyperball):
+    """The same matrix alone, among few and among many columns: equal bits, as on a rank of a sharded run."""
+    rng = np.random.default_rng(shape[0])
+    r, c = shape
+    u, z = (rng.standard_normal(r * c) * 0.05).astype(F), U.weights(rng, r * c)
+    sm = (0.01 + 0.02 * rng.random(max(r, c))).astype(F)
+    opt, results = b2.OptimizerModule(), []
+    for company in ([], [(40, 48)], [(32, 2064)] * 10):
+        shapes = company + [shape]
+        slots = [_slot(a, b, np.zeros(a * b, F), np.zeros(a * b, np.uint16), np.full(a * b, 0.02, F), np.zeros(a * b, F))
+                 for a, b in company] + [_slot(r, c, np.zeros(r * c, F), np.zeros(r * c, np.uint16), z, z)]
+        for s in slots[:-1]:
+            s.second_momentum = torch.full((max(s.rows, s.cols),), 0.01, device="cuda")
+        slots[-1].second_momentum = dev(sm)
+        plan, table = b2.MuonPlan(shapes, scale_layout=b2.SCALES_RAW), b2.slot_table(slots)
+        opt.muon_tma_prepare_polar(plan, table, b2.MuonMegaUpdateArgs(mu=1.0, grad_scale=0.0, iterations=1))
+        for k in range(len(company)):
+            plan.scratch(k, 1).fill_(0.05)
+        at = len(company)
+        plan.scratch(at, 1).copy_(dev(u).view(r, c))
+        args = b2.MuonMegaUpdateArgs(learning_rate=0.02, weight_decay=0.025, average_coefficient=0.3, schedule_beta=0.6,
+                                     normuon=True)
+        if hyperball:
+            opt.muon_tma_finish_hyperball_update_deferred_quantization(plan, table, args)
+        else:
+            opt.muon_tma_finish_update_deferred_quantization(plan, table, args)
+        torch.cuda.synchronize()
+        stats = host(plan.scratch(at, 9).view(torch.float32)).copy()
+        results.append([host(slots[-1].second_momentum), host(plan.scratch(at, 8).view(torch.float32)).copy(),
+                        stats if hyperball else stats[:2], host(slots[-1].z_master), host(slots[-1].x_master), host(slots[-1].grad)])
+        plan.close()
+    for other in results[1:]:
+        for name, a, b in zip(("second moment", "factors", "slot statistics", "z", "x", "y"), results[0], other):
+            assert np.array_equal(a, b), (name, float(np.abs(a - b).max()))
