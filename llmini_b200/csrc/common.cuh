@@ -218,6 +218,20 @@ __device__ __forceinline__ void stream_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Coherent loads that the compiler may move across this kernel's stores, for small tables that no store of this kernel
+// touches (a plain load waits for the stores in front of it, which could alias it).  The address has to come out of a
+// load behind stream_enter(): that dependence is what keeps these behind the wait.
+__device__ __forceinline__ float ld_table(const float *p) {
+    float v;
+    asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_table4(const float *p) {
+    float4 v;
+    asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
 // ---- streaming loads/stores ------------------------------------------------------------------
 __device__ __forceinline__ float4 ld_stream(const float *p) {
     return __ldcs(reinterpret_cast<const float4 *>(p));

@@ -99,7 +99,7 @@ __device__ __forceinline__ float qk_clip_factor(const b2_muon_slot_descriptor &d
     if (factors == nullptr || d.qk_clip_factor_offset == 0xffffffffu || d.qk_clip_head_dim == 0) return 1.0f;
     if (row >= 2u * d.cols) return 1.0f;
     const uint32_t in_block = row >= d.cols ? row - d.cols : row;   // row % cols for row < 2 cols
-    return factors[d.qk_clip_factor_offset + in_block / d.qk_clip_head_dim];
+    return ld_table(factors + d.qk_clip_factor_offset + in_block / d.qk_clip_head_dim);
 }
 
 struct ChunkCtx {
@@ -285,8 +285,8 @@ __device__ __forceinline__ SymExpLin symexp_for_slot(const UpdateParams &up, uin
             float v[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                const float z = *reinterpret_cast<const float *>(p[2 * k]);
-                const float x = *reinterpret_cast<const float *>(p[2 * k + 1]);
+                const float z = ld_table(reinterpret_cast<const float *>(p[2 * k]));
+                const float x = ld_table(reinterpret_cast<const float *>(p[2 * k + 1]));
                 v[k] = z + up.beta * (x - z);
             }
             s.exponential = v[0]; s.linear = v[1]; s.curvature = v[2];
@@ -304,10 +304,10 @@ __device__ __forceinline__ void neuron_factors(const ChunkCtx &cx, const UpdateP
     const float *fp = reinterpret_cast<const float *>(up.factor_ptrs[cx.slot]);
     const float sc = with_scale ? up.slot_stats[cx.slot * 4] : 1.0f;
     if (cx.d.rows >= cx.d.cols) {
-        const float f = with_scale ? fp[row] * sc : fp[row];
+        const float f = with_scale ? ld_table(fp + row) * sc : ld_table(fp + row);
         nf[0] = nf[1] = nf[2] = nf[3] = f;
     } else {
-        const float4 f = *reinterpret_cast<const float4 *>(fp + (i - row * cx.d.cols));
+        const float4 f = ld_table4(fp + (i - row * cx.d.cols));
         nf[0] = f.x; nf[1] = f.y; nf[2] = f.z; nf[3] = f.w;
         if (with_scale) {
 #pragma unroll
