@@ -128,6 +128,7 @@ struct Layout {
     int symmetric = 0;  // 1: Gram / Poly compute the upper triangle of tiles only (square tiles)
     int tile_m = 128;
     uint32_t small_smem = 0;   // shared memory of the one-CTA-per-matrix loop, 0 where some matrix is too large for it
+    bool small_ragged = false; // some row count is no multiple of 16
     size_t off_prefix, off_partials, off_inv_norm, off_amax_x, off_status, off_x0_ptrs, off_x1_ptrs, off_u_ptrs, off_maps,
         off_problems, off_tiles_nn, off_tiles_out, off_unit_prefix, off_factor_ptrs, off_unit_partials, off_slot_stats,
         off_items, off_fused_sync, off_chain, off_gp, off_chain_sync, off_meta_end, total;
@@ -257,6 +258,7 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
             if ((uint64_t)rows[s] * cols[s] == 0) continue;
             if (!ns_small_fits(rows[s], cols[s])) { L.small_smem = 0; break; }
             L.small_smem = std::max(L.small_smem, ns_small_smem(rows[s], cols[s]));
+            L.small_ragged = L.small_ragged || rows[s] % 16 != 0;
         }
     }
     L.slots.resize(count);
@@ -711,7 +713,7 @@ int b2_muon_polar(b2_muon_plan *plan, const b2_muon_step_args *a, void *stream) 
         if (small)
             return (int)launch_ns_small(probs + (size_t)kGram0 * count, probs + (size_t)kPoly * count, probs + (size_t)kApply0 * count,
                                         probs + (size_t)kApply1 * count, probs + (size_t)kLast0 * count, count, a->iterations, f16,
-                                        plan->options.update_input == B2_UPDATE_16BIT, coef, scale, L.small_smem, status, s);
+                                        plan->options.update_input == B2_UPDATE_16BIT, coef, scale, L.small_smem, L.small_ragged, status, s);
         return (int)launch_ns_chain(L.bn, L.pair, probs, plan->at<ChainTile>(L.off_chain), L.chain_tiles, f16, coef, scale,
                                     status, plan->ws + L.off_chain_sync, count, plan->options.measure_flags, grid, s);
     }

@@ -191,14 +191,15 @@ cudaError_t launch_ns_gemm(int block_n, int pair, const GemmProblem *problems, c
 
 // The whole loop of every matrix in one launch, one CTA per matrix: for plans all of whose matrices pass ns_small_fits.
 // The problem arrays are those of the plan's first slot (`apply0` writes the second operand buffer, `apply1` the first);
-// `smem_bytes` is the largest ns_small_smem of the plan.  `slot_scale` as above, for the first iteration.  At most kMaxChainIterations iterations.
+// `smem_bytes` is the largest ns_small_smem of the plan, `ragged` that some row count is no multiple of 16.  `slot_scale` as
+// above, for the first iteration.  At most kMaxChainIterations iterations.
 bool ns_small_fits(uint32_t rows, uint32_t cols);
 uint32_t ns_small_smem(uint32_t rows, uint32_t cols);
 cudaError_t ns_small_configure();   // once before the first launch on a device
 cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, const GemmProblem *apply0, const GemmProblem *apply1,
                             const GemmProblem *last, uint32_t slot_count, uint32_t iterations, int f16, int last16,
-                            const GemmCoefficients &coef, const float *slot_scale, uint32_t smem_bytes, uint32_t *status,
-                            cudaStream_t s);
+                            const GemmCoefficients &coef, const float *slot_scale, uint32_t smem_bytes, bool ragged,
+                            uint32_t *status, cudaStream_t s);
 
 // The ticketed launch over a ChainTile list.  `fused_list`: the list holds kEpiGramPoly entries, whose second part
 // waits for tiles with LARGER tickets of the same matrix; a CTA then never holds a ticket it has not started

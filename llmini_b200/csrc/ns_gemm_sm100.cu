@@ -930,8 +930,11 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
 // swizzle), read K-major along a row and MN-major across rows, so one copy serves both GEMMs it takes part in:
 //   wide (rows <= cols)  Gram K-major,  X' = Q X with X as an MN-major B;   tall  Gram MN-major,  X' = X Q with X as a
 //   K-major A.
-// What TMA fills in beyond the matrix is zero and stays zero, so nothing needs a bound but the stores.  Rounding points,
-// operand values and the order of every sum are those of k_ns_gemm.
+// What TMA fills in beyond the matrix is zero and stays zero, so that MMAs, whose K goes in steps of 16, need no bound.  It
+// stays zero by itself while everything is finite.  RAGGED, for plans with a row count that is no multiple of 16 (columns
+// always are): what an MMA may read again is cleared, because 0 times an infinity is not 0; a template parameter because the
+// code for it costs the others 3 % (64 x 64: 18.1 -> 18.6 us).  Rounding points, operand values and the order of every sum
+// are those of k_ns_gemm.
 constexpr int kSmallThreads = 256;
 constexpr uint32_t kSmallPanel = 128 * 128;   // bytes: 128 rows x 64 16-bit values
 constexpr uint32_t kSmallTmemCols = 512;
@@ -945,6 +948,7 @@ struct SmallLoop {
 
 __device__ __forceinline__ uint32_t small_swizzled(uint32_t row, uint32_t chunk) { return row * 128u + ((chunk ^ (row & 7u)) << 4); }
 
+template <bool RAGGED>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__ poly, const GemmProblem *__restrict__ apply0,
            const GemmProblem *__restrict__ apply1, const GemmProblem *__restrict__ last, SmallLoop loop,
@@ -1047,6 +1051,12 @@ k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__
             // each warp takes 64 columns of its 32 rows: one panel of G (and of Q)
             uint8_t *g_out = reinterpret_cast<uint8_t *>(gram[slot].out16), *q_out = reinterpret_cast<uint8_t *>(poly[slot].out16);
             const uint32_t pitch = gram[slot].pitch16;
+            auto clear_columns = [&](uint32_t col, uint32_t *v) {   // those from n on, of 32 from `col`
+                if (!RAGGED || (n & 15u) == 0u || col + 32u <= n) return;
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    if (col + j >= n) v[j] = 0u;
+            };
             auto store_nn = [&](uint8_t *panel0, uint8_t *global, uint32_t col, const uint32_t *v) {   // 32 columns from `col`
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -1068,6 +1078,7 @@ k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__
                 tc_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * s2);
+                clear_columns(col, v);
                 store_nn(g_panels, g_out, col, v);
             }
             hand_over();
@@ -1093,6 +1104,7 @@ k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__
                     // store/plain.rs:175-178: fma(c, acc, fma(b, base, identity))
                     v[j] = __float_as_uint(fmaf(cc, __uint_as_float(v[j]), fmaf(cb, __uint_as_float(h[j]) * s2, ident)));
                 }
+                clear_columns(col, v);
                 store_nn(q_panels, q_out, col, v);
             }
             hand_over();
@@ -1127,6 +1139,10 @@ k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__
                 const uint32_t c0 = tall ? (t & 127u) : t, r = tall ? (t >> 7) * 128u + row : row;
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * s1);
+                if (RAGGED && r >= rows) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = 0u;
+                }
                 if (out32) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
@@ -1297,12 +1313,14 @@ uint32_t ns_small_smem(uint32_t rows, uint32_t cols) {
 }
 // The limit belongs to the function, not to a plan: it is always the largest, so that no plan takes it from another.
 cudaError_t ns_small_configure() {
-    return cudaFuncSetAttribute(k_ns_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
+    const cudaError_t e = cudaFuncSetAttribute(k_ns_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_ns_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
 }
 cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, const GemmProblem *apply0, const GemmProblem *apply1,
                             const GemmProblem *last, uint32_t slot_count, uint32_t iterations, int f16, int last16,
-                            const GemmCoefficients &coef, const float *slot_scale, uint32_t smem_bytes, uint32_t *status,
-                            cudaStream_t s) {
+                            const GemmCoefficients &coef, const float *slot_scale, uint32_t smem_bytes, bool ragged,
+                            uint32_t *status, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1314,7 +1332,7 @@ cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, co
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = s;
     SmallLoop loop = {iterations, f16, last16, coef};
-    return cudaLaunchKernelEx(&cfg, k_ns_small, gram, poly, apply0, apply1, last, loop, slot_scale, status);
+    return cudaLaunchKernelEx(&cfg, ragged ? k_ns_small<true> : k_ns_small<false>, gram, poly, apply0, apply1, last, loop, slot_scale, status);
 }
 size_t chain_sync_bytes(uint32_t slot_count) { return sizeof(ChainSync) + sizeof(uint32_t) * slot_count; }
 uint32_t chain_epilogue_warps(int block_n, int pair) { return (uint32_t)(4 * (block_n / 64)) * (pair ? 2u : 1u); }

@@ -194,6 +194,25 @@ def test_one_cta_loop_equals_the_per_phase_launches_bit_for_bit(fmt, iterations,
             assert np.array_equal(u, v), (shape, w, float(np.abs(u - v).max()))
 
 
+@pytest.mark.parametrize("fmt", [b2.OPERAND_BF16, b2.OPERAND_F16])
+@pytest.mark.parametrize("kind", ["nan", "inf", "overflow"])
+def test_one_cta_loop_treats_non_finite_values_as_the_per_phase_launches_do(kind, fmt):
+    rng = np.random.default_rng(1)
+    xs = [_x0(rng, r, c, fmt) for r, c in SMALL]
+    for x in xs:
+        if kind == "overflow":
+            x *= F(3e4 if fmt == b2.OPERAND_F16 else 1e30)   # the Gram matrix leaves the operand type's range
+        else:
+            x[x.shape[0] // 2, x.shape[1] // 2] = F(kind)
+    for iterations in (1, 2):
+        a, b = (_run(SMALL, fmt, iterations, o.fixed_coefficients(iterations), tile_n, xs) for tile_n in (0, 128))
+        for i, shape in enumerate(SMALL):
+            for w, name in (1, "U"), (5, "G"), (6, "Q"):
+                assert np.array_equal(host(a.scratch(i, w).float()), host(b.scratch(i, w).float()), equal_nan=True), (shape, name)
+        a.close()
+        b.close()
+
+
 def test_tile_choice_agrees_with_the_oracle_on_both_sides_of_the_line():
     """One layer of width 512 takes 128 x 128 tiles, three of width 768 take pairs; mixed with odd row counts."""
     rng = np.random.default_rng(3)
