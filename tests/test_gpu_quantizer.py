@@ -181,3 +181,19 @@ def test_quantise_round_trip_property_large():
     bound = sc * t.global_scale * 1.0 + 1e-12
     blockmax = x.abs().view(-1, 16).max(dim=1).values.repeat_interleave(16)
     assert bool(((deq - x).abs() <= bound + blockmax * 0.07).all())
+
+
+def test_long_tensors_in_interleaved_runs_bit_exact():
+    """Where a CTA's share is 64 chunks or more it takes runs of 16 chunks, interleaved with the others': 16 CTAs (of 128
+    threads, more never fit) on every SM have 64 each here, and the last runs are uneven and end in a part of a chunk."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = (sms * 16 * 64 + 5) * 2048 + 48
+    x = torch.randn(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)).mul_(0.02)
+    q = b2.Nvfp4QuantModule()
+    amax = x.abs().max().reshape(1)
+    got = [torch.full((s,), 255, dtype=torch.uint8, device="cuda") for s in (n // 2, n // 16)] + [torch.zeros(1, device="cuda")]
+    q.fp32_to_nvfp4_four_six(x, amax, *got, n // 16, b2.SCALES_RAW)
+    want = q.debug_quantize_literal(x, amax)
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b.view_as(a))

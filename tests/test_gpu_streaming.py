@@ -496,3 +496,60 @@ def test_materialize_training_weights_for_all_slots():
         assert gs == ogs and np.array_equal(host(s.bytes), codes)
         assert np.array_equal(host(s.scales), o.csf_encode(raw, r, c))
     plan.close()
+
+
+@pytest.mark.parametrize("call", ["materialize_schedule_free", "materialize_master", "apply_adamw_update", "clip and fp32 adamw"])
+def test_captured_calls_replay_as_the_calls_themselves(call):
+    """Their launches may overlap the one in front of them, a memset included; a captured graph keeps that order: replayed
+    on other values it gives the bits of the eager call."""
+    rows, k = 129, 384                      # 24 chunks of 2048 values and a part of one
+    n = rows * k
+    opt = b2.OptimizerModule()
+    names = ("z_master", "x_master", "grad", "first_moment", "second_moment")
+    hp = dict(learning_rate=2e-4, weight_decay=0.005, beta1=0.9, beta2=0.95, beta1_correction=0.19, beta2_correction=0.0975,
+              eps=1e-10, average_coefficient=0.5, schedule_beta=0.3, grad_scale=0.7)
+
+    def buffers():
+        t = b2.Nvfp4Tensor.empty(rows, k)
+        q = dict(bytes=t.bytes, scales=t.scales, global_scale=t.global_scale, amax=torch.zeros(1, device="cuda"))
+        b = {name: torch.zeros(n, device="cuda") for name in names}
+        b["chunk_amax"] = torch.zeros((n + 2047) // 2048, device="cuda")
+        cuts = range(0, n, 4096)
+        clip = dict(chunk_ptrs=torch.tensor([b["grad"].data_ptr() + 4 * a for a in cuts], dtype=torch.int64, device="cuda"),
+                    chunk_lens=torch.tensor([min(4096, n - a) for a in cuts], dtype=torch.int32, device="cuda"),
+                    chunk_sums=torch.zeros(len(cuts), device="cuda"), scale=torch.zeros(1, device="cuda"),
+                    norm=torch.zeros(1, device="cuda"))
+        return q, b, clip
+
+    def run(q, b, clip):
+        if call == "materialize_schedule_free":
+            opt.materialize_schedule_free(**q, z_master=b["z_master"], x_master=b["x_master"], len=n, scale_rows=rows, scale_k=k, beta=0.4)
+        elif call == "materialize_master":
+            opt.materialize_master(q["bytes"], q["scales"], q["global_scale"], b["x_master"], q["amax"], b["chunk_amax"], n)
+        elif call == "apply_adamw_update":
+            opt.apply_adamw_update(**q, **b, len=n, **hp)
+        else:
+            opt.clip_gradients(**clip, extra_sums=None, chunk_count=clip["chunk_sums"].numel(), extra_sum_count=0, max_norm=0.1, apply=False)
+            opt.apply_fp32_adamw_update(**{name: b[name] for name in names}, len=n, grad_scale_device=clip["scale"], **hp)
+
+    captured = buffers()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(*captured)
+    rng, seen = np.random.default_rng(6), set()
+    for step in range(3):
+        eager = buffers()
+        values = {"z_master": U.weights(rng, n), "x_master": U.weights(rng, n), "grad": U.gradients(rng, n) * F(step + 1),
+                  "first_moment": U.weights(rng, n, 1e-3), "second_moment": np.abs(U.weights(rng, n, 1e-6))}
+        for _, b, _ in (captured, eager):
+            for name in names:
+                b[name].copy_(dev(values[name]))
+        graph.replay()
+        run(*eager)
+        torch.cuda.synchronize()
+        for got, want in zip(captured, eager):
+            for name, t in want.items():
+                if name != "chunk_ptrs":
+                    assert torch.equal(got[name], t), (step, name)
+        seen.add((float(eager[0]["amax"]), float(eager[2]["scale"])))
+    assert len(seen) == 3   # every replay had something else to find
