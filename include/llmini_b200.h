@@ -248,7 +248,9 @@ int b2_muon_sign_update_deferred_quantization(b2_muon_plan *plan, const b2_muon_
 /* Scratch views for tests and tracing (the reference's `MUON_TMA_TRACE`,
  * src/training/optimizer_muon/tma.rs:1210-1276).  which: 0 = X0 (16-bit, [rows][cols]),
  * 1 = Newton-Schulz result U (f32, [rows][cols]; with B2_UPDATE_16BIT the result is in the operand buffer 0 or 7
- * that the last iteration wrote: 7 for an odd iteration count, 0 for an even one), 2 = inverse norm (f32[1]),
+ * that the last iteration wrote: 7 for an odd iteration count, 0 for an even one.  A two-pass b2_muon_prepare_polar
+ * with `variance_adaptive` uses it as scratch: from there to b2_muon_polar it holds the update before its
+ * normalisation, not the last step's result), 2 = inverse norm (f32[1]),
  * 3 = max|x'| (f32[1]), 4 = device status word (u32[1], plan-wide).
  * 5 = Gram (16-bit, [n][ld]) and 6 = polynomial Q (16-bit, [n][ld]) of the LAST iteration,
  * 7 = the second operand buffer X1, 8 = NorMuon factors (f32[max(rows, cols)]),

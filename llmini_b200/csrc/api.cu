@@ -165,9 +165,9 @@ bool triangle_of_128(const uint32_t *rows, const uint32_t *cols, uint32_t count)
 // and for its epilogue.  Few tiles: the longest one decides, and small tiles on many SMs win; many tiles: the pair, which
 // loads half as many bytes per FLOP, wins.  The constants (us) are fitted to the Newton-Schulz stage of 24 plans of 1 to
 // 48 matrices, 64 to 6400 wide, in each configuration (mostly within 15 %).
-// Measured, pairs -> 128 x 128 (us): one 3072 x 768 242 -> 166, one layer of width 384 173 -> 119, 768 267 -> 206, 1024
-// 345 -> 325, the six largest matrices of a layer pair of width 768 298 -> 253; on the other side of the line two layers
-// of width 768 308 -> 318, four 494 -> 526, four of width 1024 883 -> 959.
+// Measured, pairs -> 128 x 128 (us): one 3072 x 768 241 -> 164, one layer of width 384 171 -> 117, 768 270 -> 206, 1024
+// 350 -> 327, the six largest matrices of a layer pair of width 768 300 -> 255; on the other side of the line two layers
+// of width 768 312 -> 321, four 498 -> 530, four of width 1024 980 -> 1104.
 void pick_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t count, const b2_muon_options &o, int &bn, int &pair) {
     if (o.tile_override == 128 || o.tile_override == 256) { bn = (int)o.tile_override; pair = 0; return; }
     if (o.tile_override == 512) { bn = 256; pair = 1; return; }
@@ -250,8 +250,10 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
     if (o.measure_flags & 4u) L.symmetric = 0;   // all tiles of the symmetric outputs
 #endif
     // One CTA per matrix runs the whole loop where every matrix fits it and neither a tile shape nor another schedule was
-    // asked for (Newton-Schulz stage, per phase -> one CTA each: three of 64 x 64 at most 66 -> 20 us, one layer of width
-    // 128 84 -> 57, twelve 89 -> 58).
+    // asked for (Newton-Schulz stage, 128 x 128 tiles per phase -> one CTA each: three of 64 x 64 at most 66 -> 18 us, one
+    // layer of width 128 83 -> 56, twelve 86 -> 56).  Not bounded in their number: beyond one matrix per SM the CTAs run in
+    // waves, the launches per phase in more tiles each (pairs, the tiles before there was a choice, against one CTA each:
+    // 149 of 64 x 64 104 -> 35 us, 1000 340 -> 124; 149 of 128 x 512 181 -> 113, 1000 827 -> 447).
     L.small_smem = 0;
     if (o.tile_override == 0 && o.ns_schedule == B2_NS_PER_PHASE) {
         for (uint32_t s = 0; s < count; ++s) {

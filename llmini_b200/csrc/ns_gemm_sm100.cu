@@ -25,13 +25,16 @@
 // tiles of a small plan over several CTAs took one 3072 x 768 from 166 to 150 us and broke that.)
 //
 // What bounds it.  A k-block (64 of K) of a pair tile is 512 clocks of MMA, reads 32 KB and receives 32 KB of shared
-// memory per SM, which together is the full 128 bytes per clock of its port.  Loads from L2 are not the limit (a
-// load-only kernel draws 60 bytes per clock into every SM at once, 128 into one alone; a k-block needs 63).  What kept
-// the pipe waiting were the single threads of the roles: one TMA producer took 400 to 590 clocks to issue the copies of
+// memory per SM, which together is the full 128 bytes per clock of its port.  Loads from L2 would let it run at
+// 0.95 of that (a load-only kernel draws 60 bytes per clock into every SM at once, 128 into one alone; a k-block at full
+// rate takes 63).  What kept the pipe waiting longer were the single threads of the roles: one TMA producer took 400 to 590 clocks to issue the copies of
 // a k-block, the MMA thread 390 to issue and 190 to wait, and both read the tile list and the problem table (two
 // dependent L2 reads) between tiles.  Two producers, a warp-uniform MMA loop and a scheduler warp that keeps a ring
-// of decoded tiles in shared memory took a k-block from 690-900 to 560-715 clocks; Newton-Schulz of GPT-2 XL,
-// sustained under the 1000 W cap, from 46.2 to 40.8 ms.
+// of decoded tiles in shared memory took a k-block from 690-900 to 560-715 clocks.  The Newton-Schulz stage inside the
+// step, before and after on one box: GPT-2 small 1.39 -> 1.36 ms, medium 5.51 -> 5.16, XL 42.5 -> 39.3 (medium and XL under
+// the 1000 W cap: the clock, and with it these times, differs from box to box by 5 %).  What is left on GPT-2 small is the
+// epilogue: with twelve k-blocks a tile its stores take as long as the MMAs, in 96 registers a thread with 72 bytes of
+// spills.
 //
 // Three ways to launch the loop (the template parameter CHAINED separates the first from the other two), and a fourth for
 // matrices that fit one SM (k_ns_small below):
