@@ -231,9 +231,11 @@ k_muon_momentum_sumsq(const b2_muon_slot_descriptor *slots, const uint32_t *pref
 
 // Second pass: X0 = r16(u * inv) in the storage layout [rows][cols] (momentum.rs:56-63 and normalize.rs:137-143; operand
 // rounding .../polar/fused/stage.rs:51-55).  No transpose: the GEMMs read either orientation.  STORED = 0 computes u
-// again and stores the BF16 momentum; STORED = 1 reads the u that the first pass left.
+// again and stores the BF16 momentum; STORED = 1 reads the u that the first pass left.  STORED = 0 takes the two halves of a
+// chunk one after the other, eight CTAs per SM: with all loads in front (six CTAs) the mixed reads and writes of large plans
+// were slower (both passes: GPT-2 medium 855 -> 929 us, small 244 -> 261), and a lone 3072 x 768 gained 0.4 of 10.2.
 template <int STORED>
-__global__ void __launch_bounds__(kThreads, 6)
+__global__ void __launch_bounds__(kThreads, STORED ? 6 : 8)
 k_muon_normalize(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint32_t slot_count, uint32_t total_chunks,
                  MomentumParams mp, const float *inv_norm, const uint64_t *x0_ptrs, const uint64_t *u_ptrs, int f16) {
     stream_enter();
@@ -253,12 +255,12 @@ k_muon_normalize(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, u
             const uint32_t i = base + h * (kChunk / 2);
             if (i >= len) continue;
             if (STORED) raw[h].g = ld_stream(reinterpret_cast<const float *>(u_ptrs[slot]) + i);
-            else raw[h] = quad_load<0>(grad, mom, nullptr, i, true);
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t i = base + h * (kChunk / 2);
             if (i >= len) continue;
+            if (!STORED) raw[h] = quad_load<0>(grad, mom, nullptr, i, true);
             float u[4] = {raw[h].g.x, raw[h].g.y, raw[h].g.z, raw[h].g.w};
             if (!STORED) {
                 const Quad q = momentum_quad<0>(raw[h], mp);
