@@ -82,6 +82,20 @@ bool make_map(CUtensorMap *m, void *base, int elem_bytes, uint64_t rows, uint64_
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same tensor of 16-bit values as a stack of 64-column strips, box = 64 columns x 64 rows x 2 strips: what an MN-major
+// operand of 128 rows needs per k-block, in one copy.  In the last strip of a tensor whose columns are no multiple of 64 the
+// columns beyond it hold what follows in memory (of the next row, or of the workspace behind the tensor), not zero: they are
+// rows or columns of the product that nothing stores.
+bool make_strip_map(CUtensorMap *m, void *base, uint64_t rows, uint64_t cols) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return false;
+    cuuint64_t dims[3] = {64, rows, (cols + 63) / 64};
+    cuuint64_t strides[2] = {cols * 2, 128};
+    cuuint32_t box[3] = {64, 64, 2}, estr[3] = {1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // crates/cuda-kernels/src/gpt/optimizer/muon/polar/fused/coefficients.rs:9-42
 void reference_coefficients(uint32_t iter, float &a, float &b, float &c) {
     static const float raw[5][3] = {{8.287212f, -23.595886f, 17.300388f},
@@ -104,11 +118,12 @@ double slot_flops(uint32_t rows, uint32_t cols) {
 }
 
 enum ProblemType { kGram0 = 0, kGram1, kPoly, kApply0, kApply1, kLast0, kLast1, kProblemTypes };
-// load maps: *K = box 64 (K) x 128 rows for K-major use, *M = box 64 x 64 for MN-major use
-enum MapKind { kLX0K = 0, kLX1K, kLX0M, kLX1M, kLG, kLQ, kMapsPerSlot };
+// load maps: *K, G and Q = box 64 (K) x 128 rows for K-major use, *M = box 64 x 64 for MN-major use and, like *64, for K-major
+// use by CTAs that stage 64 rows, *T = two neighbouring 64 x 64 boxes for MN-major use
+enum MapKind { kLX0K = 0, kLX1K, kLX0M, kLX1M, kLX0T, kLX1T, kLG, kLQ, kLG64, kLQ64, kMapsPerSlot };
 
 struct SlotLayout {
-    uint32_t rows, cols, n, m, ldg, tiles_m_nn, tiles_n_nn, sub_m_nn;
+    uint32_t rows, cols, n, m, ldg, frag_units;
     uint64_t len;
     size_t off_x[2], off_u, off_g16, off_q16, off_frag, off_factors;
 };
@@ -123,10 +138,9 @@ struct Layout {
     uint32_t gp_tiles = 0;               // entries of ONE fused Gram + polynomial work list (0: not built); three lists
     uint32_t gp_widest = 0;              // most Gram tiles any one matrix has
     uint32_t total_chunks = 0;
-    int bn = 256;
-    int pair = 0;   // 1: two-CTA 256 x 256 tiles
-    int symmetric = 0;  // 1: Gram / Poly compute the upper triangle of tiles only (square tiles)
-    int tile_m = 128;
+    GemmShape nn = {256, 256, 1};    // tiles of Gram and Poly
+    GemmShape out = {256, 256, 1};   // tiles of Apply
+    int symmetric = 0;  // 1: Gram / Poly leave out the tiles below the diagonal
     uint32_t small_smem = 0;   // shared memory of the one-CTA-per-matrix loop, 0 where some matrix is too large for it
     bool small_ragged = false; // some row count is no multiple of 16
     size_t off_prefix, off_partials, off_inv_norm, off_amax_x, off_status, off_x0_ptrs, off_x1_ptrs, off_u_ptrs, off_maps,
@@ -242,13 +256,19 @@ void build_items(Layout &L, const std::vector<uint32_t> &first) {
     }
 }
 
+// Calls f(tile_m, tile_n, mirrored) for the tiles of an n x n output.  It is symmetric: a tile wholly below the diagonal is
+// left out of a triangle, and the tile that holds its transpose, wholly above, also stores that.
+template <typename F>
+void for_nn_tiles(const Layout &L, uint32_t n, F f) {
+    const uint32_t tm = (uint32_t)L.nn.tm, bn = (uint32_t)L.nn.bn;
+    for (uint32_t i = 0; i * tm < n; ++i)
+        for (uint32_t j = 0; j * bn < n; ++j) {
+            if (L.symmetric && (j + 1) * bn <= i * tm) continue;
+            f(i, j, L.symmetric && j * bn >= (i + 1) * tm);
+        }
+}
+
 bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, const b2_muon_options &o, Layout &L) {
-    pick_tiles(rows, cols, count, o, L.bn, L.pair);
-    L.tile_m = L.pair ? 256 : 128;
-    L.symmetric = L.pair || (L.bn == 128 && triangle_of_128(rows, cols, count)) ? 1 : 0;
-#ifdef B2_MEASURE
-    if (o.measure_flags & 4u) L.symmetric = 0;   // all tiles of the symmetric outputs
-#endif
     // One CTA per matrix runs the whole loop where every matrix fits it and neither a tile shape nor another schedule was
     // asked for (Newton-Schulz stage, 128 x 128 tiles per phase -> one CTA each: three of 64 x 64 at most 66 -> 18 us, one
     // layer of width 128 83 -> 56, twelve 86 -> 56).  Not bounded in their number: beyond one matrix per SM the CTAs run in
@@ -263,6 +283,10 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
             L.small_ragged = L.small_ragged || rows[s] % 16 != 0;
         }
     }
+    int bn = 256, pair = 0;
+    pick_tiles(rows, cols, count, o, bn, pair);
+    L.nn = L.out = GemmShape{pair ? 256 : 128, bn, pair};
+    L.symmetric = pair || (bn == 128 && triangle_of_128(rows, cols, count)) ? 1 : 0;
     L.slots.resize(count);
     L.chunk_prefix.assign(count + 1, 0);
     size_t off = 0;
@@ -303,13 +327,11 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
         sl.len = (uint64_t)rows[s] * cols[s];
         sl.n = std::min(rows[s], cols[s]); sl.m = std::max(rows[s], cols[s]);
         sl.ldg = (uint32_t)align_up(sl.n, 8);
-        sl.tiles_m_nn = (sl.n + L.tile_m - 1) / L.tile_m;
-        sl.tiles_n_nn = (sl.n + L.bn - 1) / L.bn;
-        sl.sub_m_nn = sl.tiles_m_nn * (L.tile_m / kGemmBlockM);  // 128-row sub-tiles (fragment scratch)
+        sl.frag_units = (sl.n + 31) / 32;
         if (sl.len == 0) continue;
-        L.tiles_nn += L.symmetric ? sl.tiles_m_nn * (sl.tiles_m_nn + 1) / 2 : sl.tiles_m_nn * sl.tiles_n_nn;
-        uint32_t M = rows[s] > cols[s] ? sl.m : sl.n, N = rows[s] > cols[s] ? sl.n : sl.m;
-        L.tiles_out += ((M + L.tile_m - 1) / L.tile_m) * ((N + L.bn - 1) / L.bn);
+        for_nn_tiles(L, sl.n, [&](uint32_t, uint32_t, bool) { ++L.tiles_nn; });
+        const uint32_t M = rows[s] > cols[s] ? sl.m : sl.n, N = rows[s] > cols[s] ? sl.n : sl.m;
+        L.tiles_out += ((M + L.out.tm - 1) / L.out.tm) * ((N + L.out.bn - 1) / L.out.bn);
     }
     L.off_tiles_nn = take((size_t)std::max(L.tiles_nn, 1u) * sizeof(GemmTile));
     L.off_tiles_out = take((size_t)std::max(L.tiles_out, 1u) * sizeof(GemmTile));
@@ -342,7 +364,7 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
         sl.off_u = take(sl.len * 4);
         sl.off_g16 = take((size_t)sl.n * sl.ldg * 2);
         sl.off_q16 = take((size_t)sl.n * sl.ldg * 2);
-        sl.off_frag = take((size_t)sl.sub_m_nn * sl.tiles_n_nn * kGemmBlockM * L.bn * 4);
+        sl.off_frag = take((size_t)((sl.n + kGemmBlockM - 1) / kGemmBlockM) * kGemmBlockM * sl.frag_units * 32 * 4);
         sl.off_factors = take((size_t)sl.m * 4);
     }
     L.total = off;
@@ -451,13 +473,14 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
     Layout &L = p->layout;
     if (!build_layout(rows, cols, slot_count, o, L) || L.total > workspace_bytes) { delete p; return B2_ERROR_INVALID_VALUE; }
     p->ws = static_cast<uint8_t *>(d_workspace);
-    e = gemm_configure(L.bn, L.pair);
+    e = gemm_configure(L.nn);
+    if (e == cudaSuccess) e = gemm_configure(L.out);
     if (e != cudaSuccess) { delete p; return (int)e; }
     if (L.small_smem) {
         e = ns_small_configure();
         if (e != cudaSuccess) { delete p; return (int)e; }
     }
-    p->resident_groups = (uint32_t)std::max(gemm_resident_groups(L.bn, L.pair, p->dev.sm_count), 0);
+    p->resident_groups = (uint32_t)std::max(gemm_resident_groups(L.nn, p->dev.sm_count), 0);
 
     p->meta.assign(L.off_meta_end, 0);
     uint8_t *h = p->meta.data();
@@ -488,27 +511,37 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
         ok &= make_map(ms + kLX1K, p->ws + sl.off_x[1], 2, sl.rows, sl.cols, xp, 64, 128);
         ok &= make_map(ms + kLX0M, p->ws + sl.off_x[0], 2, sl.rows, sl.cols, xp, 64, 64);
         ok &= make_map(ms + kLX1M, p->ws + sl.off_x[1], 2, sl.rows, sl.cols, xp, 64, 64);
+        ok &= make_strip_map(ms + kLX0T, p->ws + sl.off_x[0], sl.rows, sl.cols);
+        ok &= make_strip_map(ms + kLX1T, p->ws + sl.off_x[1], sl.rows, sl.cols);
         ok &= make_map(ms + kLG, p->ws + sl.off_g16, 2, sl.n, sl.n, gp, 64, 128);
         ok &= make_map(ms + kLQ, p->ws + sl.off_q16, 2, sl.n, sl.n, gp, 64, 128);
+        ok &= make_map(ms + kLG64, p->ws + sl.off_g16, 2, sl.n, sl.n, gp, 64, 64);
+        ok &= make_map(ms + kLQ64, p->ws + sl.off_q16, 2, sl.n, sl.n, gp, 64, 64);
         const bool tall = sl.rows > sl.cols;
         const uint64_t frag = reinterpret_cast<uint64_t>(p->ws + sl.off_frag);
+        // the map whose boxes fit the rows that a CTA stages of A or of B
+        auto pick = [&](int rows_of_tile, int pair, int map128, int map64) {
+            return dmap(s, (pair ? rows_of_tile / 2 : rows_of_tile) == 64 ? map64 : map128);
+        };
         for (int b = 0; b < 2; ++b) {
             GemmProblem &g = probs[(size_t)(kGram0 + b) * slot_count + s];
-            g.map_a = g.map_b = dmap(s, (tall ? kLX0M : kLX0K) + b);
+            g.map_a = pick(L.nn.tm, L.nn.pair, (tall ? kLX0T : kLX0K) + b, kLX0M + b);
+            g.map_b = pick(L.nn.bn, L.nn.pair, (tall ? kLX0T : kLX0K) + b, kLX0M + b);
             g.out16 = reinterpret_cast<uint64_t>(p->ws + sl.off_g16);
             g.pitch16 = sl.ldg;
             g.frag32 = frag;
             g.M = g.N = sl.n; g.K = sl.m;
             g.a_mn_major = g.b_mn_major = tall ? 1u : 0u;
-            g.tiles_n = sl.tiles_n_nn;
+            g.frag_units = sl.frag_units;
             for (int last = 0; last < 2; ++last) {
                 GemmProblem &a = probs[(size_t)((last ? kLast0 : kApply0) + b) * slot_count + s];
                 if (tall) {  // Y' = Y Q : A = Y [m][n] K-major, B = Q [n][n] K-major
-                    a.map_a = dmap(s, kLX0K + b); a.map_b = dmap(s, kLQ);
+                    a.map_a = pick(L.out.tm, L.out.pair, kLX0K + b, kLX0M + b);
+                    a.map_b = pick(L.out.bn, L.out.pair, kLQ, kLQ64);
                     a.a_mn_major = 0; a.b_mn_major = 0;
                     a.M = sl.m; a.N = sl.n;
                 } else {     // X' = Q X : A = Q K-major, B = X [n][m] read as MN-major
-                    a.map_a = dmap(s, kLQ); a.map_b = dmap(s, kLX0M + b);
+                    a.map_a = pick(L.out.tm, L.out.pair, kLQ, kLQ64); a.map_b = pick(L.out.bn, L.out.pair, kLX0T + b, kLX0M + b);
                     a.a_mn_major = 0; a.b_mn_major = 1;
                     a.M = sl.n; a.N = sl.m;
                 }
@@ -517,16 +550,16 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
                 a.pitch16 = sl.cols;
                 a.out32 = reinterpret_cast<uint64_t>(p->ws + sl.off_u);
                 a.pitch32 = sl.cols;
-                a.tiles_n = (a.N + L.bn - 1) / L.bn;
             }
         }
         GemmProblem &q = probs[(size_t)kPoly * slot_count + s];
-        q.map_a = q.map_b = dmap(s, kLG);
+        q.map_a = pick(L.nn.tm, L.nn.pair, kLG, kLG64);
+        q.map_b = pick(L.nn.bn, L.nn.pair, kLG, kLG64);
         q.out16 = reinterpret_cast<uint64_t>(p->ws + sl.off_q16);
         q.pitch16 = sl.ldg;
         q.frag32 = frag;
         q.M = q.N = q.K = sl.n;
-        q.tiles_n = sl.tiles_n_nn;
+        q.frag_units = sl.frag_units;
     }
     if (!ok) { delete p; return B2_ERROR_NOT_SUPPORTED; }
     // tile lists, most expensive slots first so the round-robin over CTAs ends evenly
@@ -541,22 +574,16 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
     GemmTile *tnn = reinterpret_cast<GemmTile *>(h + L.off_tiles_nn);
     GemmTile *tout = reinterpret_cast<GemmTile *>(h + L.off_tiles_out);
     uint32_t inn = 0, iout = 0;
-    for (uint32_t s : order) {
-        const SlotLayout &sl = L.slots[s];
-        for (uint32_t i = 0; i < sl.tiles_m_nn; ++i)
-            for (uint32_t j = 0; j < sl.tiles_n_nn; ++j) {
-                // square tiles: G and Q are symmetric, so only tiles on or above the
-                // diagonal are computed and the others are written as transposes
-                if (L.symmetric && j < i) continue;
-                tnn[inn++] = GemmTile{(uint16_t)s, (uint16_t)i, (uint16_t)j, (uint16_t)((L.symmetric && j > i) ? 1 : 0)};
-            }
-    }
+    for (uint32_t s : order)
+        for_nn_tiles(L, L.slots[s].n, [&](uint32_t i, uint32_t j, bool mirrored) {
+            tnn[inn++] = GemmTile{(uint16_t)s, (uint16_t)i, (uint16_t)j, (uint16_t)(mirrored ? 1 : 0)};
+        });
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return L.slots[a].n > L.slots[b].n; });
     for (uint32_t s : order) {
         const SlotLayout &sl = L.slots[s];
         const bool tall = sl.rows > sl.cols;
         uint32_t M = tall ? sl.m : sl.n, N = tall ? sl.n : sl.m;
-        uint32_t tm = (M + L.tile_m - 1) / L.tile_m, tn = (N + L.bn - 1) / L.bn;
+        uint32_t tm = (M + L.out.tm - 1) / L.out.tm, tn = (N + L.out.bn - 1) / L.out.bn;
         for (uint32_t i = 0; i < tm; ++i)
             for (uint32_t j = 0; j < tn; ++j) tout[iout++] = GemmTile{(uint16_t)s, (uint16_t)i, (uint16_t)j, 0};
     }
@@ -565,7 +592,7 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
         // of a tile = progress increments of its matrix's earlier phases (every tile is finished by `warps`
         // epilogue warps).
         ChainTile *ct = reinterpret_cast<ChainTile *>(h + L.off_chain);
-        const uint32_t warps = chain_epilogue_warps(L.bn, L.pair);
+        const uint32_t warps = chain_epilogue_warps(L.nn);
         std::vector<uint32_t> done(slot_count, 0), nn_tiles(slot_count, 0), out_tiles(slot_count, 0);
         for (uint32_t i = 0; i < inn; ++i) ++nn_tiles[tnn[i].problem];
         for (uint32_t i = 0; i < iout; ++i) ++out_tiles[tout[i].problem];
@@ -600,7 +627,7 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
         // Gram tile, publishes its 16-bit form, waits for the matrix's other Gram tiles (need2) and goes on to the
         // polynomial tile of the same position.  The progress counts start from zero in every launch.
         ChainTile *gp = reinterpret_cast<ChainTile *>(h + L.off_gp);
-        const uint32_t warps = chain_epilogue_warps(L.bn, L.pair);
+        const uint32_t warps = chain_epilogue_warps(L.nn);
         std::vector<uint32_t> nn_tiles(slot_count, 0);
         for (uint32_t i = 0; i < inn; ++i) ++nn_tiles[tnn[i].problem];
         L.gp_widest = 0;
@@ -716,7 +743,7 @@ int b2_muon_polar(b2_muon_plan *plan, const b2_muon_step_args *a, void *stream) 
             return (int)launch_ns_small(probs + (size_t)kGram0 * count, probs + (size_t)kPoly * count, probs + (size_t)kApply0 * count,
                                         probs + (size_t)kApply1 * count, probs + (size_t)kLast0 * count, count, a->iterations, f16,
                                         plan->options.update_input == B2_UPDATE_16BIT, coef, scale, L.small_smem, L.small_ragged, status, s);
-        return (int)launch_ns_chain(L.bn, L.pair, probs, plan->at<ChainTile>(L.off_chain), L.chain_tiles, f16, coef, scale,
+        return (int)launch_ns_chain(L.nn, probs, plan->at<ChainTile>(L.off_chain), L.chain_tiles, f16, coef, scale,
                                     status, plan->ws + L.off_chain_sync, count, plan->options.measure_flags, grid, s);
     }
     // The fused form needs all Gram tiles of a matrix in flight at once: one CTA (pair) each.
@@ -742,18 +769,18 @@ int b2_muon_polar(b2_muon_plan *plan, const b2_muon_step_args *a, void *stream) 
             GemmCoefficients coef = {};
             coef.v[0] = ca; coef.v[1] = cb; coef.v[2] = cc;
             const uint32_t list = it == 0 ? 0u : ((it & 1u) ? 1u : 2u);
-            e = launch_ns_chain(L.bn, L.pair, probs, plan->at<ChainTile>(L.off_gp) + (size_t)list * L.gp_tiles, L.gp_tiles,
+            e = launch_ns_chain(L.nn, probs, plan->at<ChainTile>(L.off_gp) + (size_t)list * L.gp_tiles, L.gp_tiles,
                                 f16, coef, scale, status, plan->ws + L.off_chain_sync, count, dbg, grid, s, true);
         } else {
             if (mask & 1u)
-                e = launch_ns_gemm(L.bn, L.pair, probs + (size_t)(kGram0 + b) * count, tnn, L.tiles_nn, kEpiGram, f16, ca, cb,
+                e = launch_ns_gemm(L.nn, probs + (size_t)(kGram0 + b) * count, tnn, L.tiles_nn, kEpiGram, f16, ca, cb,
                                    cc, scale, 2u, status, dbg, grid, s);
             if (e == cudaSuccess && (mask & 2u))
-                e = launch_ns_gemm(L.bn, L.pair, probs + (size_t)kPoly * count, tnn, L.tiles_nn, kEpiPoly, f16, ca, cb, cc,
+                e = launch_ns_gemm(L.nn, probs + (size_t)kPoly * count, tnn, L.tiles_nn, kEpiPoly, f16, ca, cb, cc,
                                    nullptr, 0u, status, dbg, grid, s);
         }
         if (e == cudaSuccess && (mask & 4u))
-            e = launch_ns_gemm(L.bn, L.pair, probs + (size_t)((last ? kLast0 : kApply0) + b) * count, tout, L.tiles_out,
+            e = launch_ns_gemm(L.out, probs + (size_t)((last ? kLast0 : kApply0) + b) * count, tout, L.tiles_out,
                                last ? kEpiApplyLast : kEpiApply, f16, ca, cb, cc, scale, 1u, status, dbg, grid, s);
     }
     return (int)e;

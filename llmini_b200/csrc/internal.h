@@ -128,16 +128,16 @@ enum GemmEpilogue : uint32_t {
 // One GEMM of one slot: D[M][N] = A * B^T with A, B described by TMA maps.  Lives in device
 // memory; built once per plan.
 struct alignas(16) GemmProblem {
-    uint64_t map_a;      // device address of the CUtensorMap of operand A (16-bit; box 64 x 128
-                         // rows when K-major, 64 x 64 when MN-major)
+    uint64_t map_a;      // device address of the CUtensorMap of operand A (16-bit; K-major: boxes of 64 x the rows that a CTA
+                         // stages, at most 128; MN-major: 64 x 64)
     uint64_t map_b;
     uint64_t out16;      // 16-bit result, row-major with `pitch16` elements per row — unused for kEpiApplyLast
     uint64_t out32;      // f32 result, row-major with `pitch32` elements per row — kEpiApplyLast only
-    uint64_t frag32;     // f32 accumulator tiles in fragment order (Gram writes, Poly reads)
+    uint64_t frag32;     // f32 Gram values, [128 rows][32-column unit][float4 index][row] (Gram writes, Poly reads)
     uint32_t M, N, K;
     uint32_t a_mn_major;  // 0: A is [M][K] K-contiguous; 1: A is [K][M] M-contiguous
     uint32_t b_mn_major;  // 0: B is [N][K]; 1: B is [K][N]
-    uint32_t tiles_n;     // number of BN-wide tile columns (for frag32 addressing)
+    uint32_t frag_units;  // 32-column units per row of frag32
     uint32_t pitch16;     // >= N, a multiple of 8 (columns N .. pitch16 of a row are padding and may be written)
     uint32_t pitch32;
 };
@@ -177,14 +177,18 @@ struct alignas(16) ChainTile {
 };
 static_assert(sizeof(ChainTile) == 32, "ChainTile is read as two 16-byte words");
 
-cudaError_t gemm_configure(int block_n, int pair);
+// Tile of a launch: tm x bn, computed by one CTA or by a pair of CTAs: 256 x 256 (pair), 128 x 256, 128 x 128.
+struct GemmShape {
+    int tm, bn, pair;
+};
+cudaError_t gemm_configure(const GemmShape &shape);
 // CTAs (pairs of CTAs when `pair`) of the ticketed kernel that the device runs at the same time, 0 if unknown.
 // Call after gemm_configure.
-int gemm_resident_groups(int block_n, int pair, int sm_count);
+int gemm_resident_groups(const GemmShape &shape, int sm_count);
 // `slot_scale` (may be null): per-slot scalars s; the Gram epilogue multiplies the accumulator by s^scale_pow
 // (scale_pow = 2) and the Apply epilogues by s (scale_pow = 1).  Used by the first iteration after a
 // one-pass prepare, whose operand is not normalised yet.
-cudaError_t launch_ns_gemm(int block_n, int pair, const GemmProblem *problems, const GemmTile *tiles,
+cudaError_t launch_ns_gemm(const GemmShape &shape, const GemmProblem *problems, const GemmTile *tiles,
                            uint32_t tile_count, uint32_t epilogue, int f16, float ca, float cb,
                            float cc, const float *slot_scale, uint32_t scale_pow, uint32_t *status,
                            uint32_t debug_flags, int grid, cudaStream_t s);
@@ -207,8 +211,8 @@ cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, co
 // than the launch has CTAs (pairs).  `sync` is chain_sync_bytes(slot_count) of device memory, zeroed once by
 // the owner; every launch leaves it zeroed.  chain_epilogue_warps: progress-count increments per finished tile.
 size_t chain_sync_bytes(uint32_t slot_count);
-uint32_t chain_epilogue_warps(int block_n, int pair);
-cudaError_t launch_ns_chain(int block_n, int pair, const GemmProblem *problems, const ChainTile *tiles,
+uint32_t chain_epilogue_warps(const GemmShape &shape);
+cudaError_t launch_ns_chain(const GemmShape &shape, const GemmProblem *problems, const ChainTile *tiles,
                             uint32_t tile_count, int f16, const GemmCoefficients &coef, const float *slot_scale,
                             uint32_t *status, void *sync, uint32_t slot_count, uint32_t debug_flags, int grid,
                             cudaStream_t s, bool fused_list = false);

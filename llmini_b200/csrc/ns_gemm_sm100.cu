@@ -11,30 +11,36 @@
 //   Apply  X' = Q X                      (reference: tiles.rs:14-38)
 // Operands are read in their storage orientation: an operand whose reduction dimension is
 // the slow one is described to the tensor core as MN-major, so no transpose is ever
-// materialised.  16-bit results leave through a shared-memory slab and coalesced stores; the FP32 Gram
-// tile that the polynomial epilogue needs is kept in a private fragment-ordered scratch so
-// both sides access it fully coalesced.
+// materialised.  Results go from registers straight to memory, a whole 32-byte sector per lane; the FP32 Gram
+// values that the polynomial epilogue needs are kept in a private scratch in the order of the
+// registers, so both sides access it fully coalesced.
 //
-// Two tile configurations:
-//   PAIR  : a cluster of two CTAs computes a 256 x 256 tile with cta_group::2 MMAs.  Each
-//           CTA stages its own 128 rows of A and half (128 rows) of B, so a k-block costs
-//           32 KB of loads per SM instead of 48 KB.  No multicast load is used.
-//   single: one CTA computes 128 x BN (BN = 128 or 256).  128 x 128 is for plans of few tiles (the rule is in api.cu).
+// Tiles (the choice is in api.cu):
+//   PAIR  : a cluster of two CTAs computes 256 x 256 with cta_group::2 MMAs.  Each CTA stages half of the rows of A and half of
+//           those of B, so a k-block costs 32 KB of loads per SM instead of 48 KB.  No multicast load is used.
+//   single: one CTA computes 128 x BN (BN = 128 or 256).
 // In every configuration a tile's sum runs over all of K in one order, so a matrix's result does not depend on which
 // other matrices share its plan: a sharded run and a single GPU compute the same bits.  (Splitting K of the long Gram
 // tiles of a small plan over several CTAs took one 3072 x 768 from 166 to 150 us and broke that.)
 //
-// What bounds it.  A k-block (64 of K) of a pair tile is 512 clocks of MMA, reads 32 KB and receives 32 KB of shared
-// memory per SM, which together is the full 128 bytes per clock of its port.  Loads from L2 would let it run at
-// 0.95 of that (a load-only kernel draws 60 bytes per clock into every SM at once, 128 into one alone; a k-block at full
-// rate takes 63).  What kept the pipe waiting longer were the single threads of the roles: one TMA producer took 400 to 590 clocks to issue the copies of
-// a k-block, the MMA thread 390 to issue and 190 to wait, and both read the tile list and the problem table (two
-// dependent L2 reads) between tiles.  Two producers, a warp-uniform MMA loop and a scheduler warp that keeps a ring
-// of decoded tiles in shared memory took a k-block from 690-900 to 560-715 clocks.  The Newton-Schulz stage inside the
-// step, before and after on one box: GPT-2 small 1.39 -> 1.36 ms, medium 5.51 -> 5.16, XL 42.5 -> 39.3 (medium and XL under
-// the 1000 W cap: the clock, and with it these times, differs from box to box by 5 %).  What is left on GPT-2 small is the
-// epilogue: with twelve k-blocks a tile its stores take as long as the MMAs, in 96 registers a thread with 72 bytes of
-// spills.
+// What bounds it.
+//   Many tiles.  A k-block (64 of K) of a 256 x 256 pair tile is 512 clocks of MMA, in which an SM takes in 32 KB, the 64
+//   bytes per clock that it can (every shape comes to that rate, with 12 CTAs running or with 148), and its shared memory
+//   serves 32 KB read and 32 KB written, 128 bytes per clock.  k-blocks take 510 to 630 clocks.  Beyond that the 1000 W cap
+//   decides: with real data the clock falls to 1.4 - 1.7 GHz (GPT-2 small) and 1.1 - 1.4 (XL), where the same launches on
+//   operands of zeros keep 1.8.  What the epilogue does to shared memory therefore counts twice, in port time and in energy:
+//   through a slab for whole-line stores every result byte passed the port three times; directly from registers it passes
+//   once (Newton-Schulz loop, before and after: 48 matrices of GPT-2 small 1284 -> 1213 us, six layers of XL 4625 -> 4450).
+//   Whole lines without the slab, by exchanging pieces between the four lanes of a row, were slower for pairs (Apply of six
+//   XL layers 334 -> 364 us).
+//   Few tiles.  A launch is a chain: 2.0 us from the end of the launch in front to griddepcontrol.wait, 1.2 us to the first
+//   MMA, the k-blocks at what an SM takes in (512 clocks where a CTA stages 32 KB of a k-block, 256 where it stages 16),
+//   and the epilogue, 1400 clocks for 32 columns a warp.  That was 2500 while the arrival that hands an accumulator back had
+//   release semantics at cluster scope, which waits for the thread's stores.
+//   One thread issues a copy in 200 to 400 clocks, so each operand has a producer of its own and takes one copy per k-block;
+//   an MN-major operand of 128 rows is one copy of a three-dimensional map instead of two (six layers of XL 4280 -> 4160 us).
+//   The MMA loop is warp-uniform, and a scheduler warp keeps a ring of decoded tiles in shared memory: the tile list and the
+//   problem table are two dependent reads of L2.
 //
 // Three ways to launch the loop (the template parameter CHAINED separates the first from the other two), and a fourth for
 // matrices that fit one SM (k_ns_small below):
@@ -59,28 +65,35 @@ namespace b2 {
 namespace {
 
 constexpr int kBoxBytes = 64 * 128;          // 64 rows x 128 bytes
-constexpr int kABytes = 2 * kBoxBytes;       // 128 x 64 16-bit operand tile
-constexpr int kSlabBytes = 32 * 128;         // per-warp store staging: 32 rows x 128 bytes
 constexpr int kSmemLimit = 227 * 1024;
 constexpr uint32_t kSpinLimit = 1u << 24;    // hard cap on polls, whatever the timer says
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 
-template <int BN, bool PAIR>
+// TM x BN is the tile of a CTA, or of a pair of CTAs; a pair's CTAs hold half of its rows of A and half of its rows of B each.
+template <int TM, int BN, bool PAIR>
 struct Cfg {
-    static constexpr int kBRows = PAIR ? 128 : BN;   // rows of B this CTA stages per k-block
-    static constexpr int kBBytes = (kBRows / 64) * kBoxBytes;
-    static constexpr int kStageBytes = kABytes + kBBytes;
+    static constexpr int kTileM = TM;
+    static constexpr int kRows = PAIR ? TM / 2 : TM;        // output rows of this CTA, and rows of A it stages per k-block
+    static constexpr int kBRows = PAIR ? BN / 2 : BN;       // rows of B this CTA stages per k-block
+    static constexpr int kABytes = kRows * 128, kBBytes = kBRows * 128;
+    static constexpr int kKbBytes = kABytes + kBBytes;
+    // k-blocks per pipeline stage: with 16 KB each, one per stage would leave the roles 256 clocks for a barrier round
+    static constexpr int kStageKb = kKbBytes <= 16 * 1024 ? 2 : 1;
+    static constexpr int kStageBytes = kStageKb * kKbBytes;
+    // An accumulator of 64 rows per CTA lies in all 128 lanes: columns 0 .. BN/2-1 in lanes 0 .. 63, the others above.
+    static constexpr int kAccCols = kRows == 64 ? BN / 2 : BN;
     // warp 0: TMA producer of A, warp 1: MMA issuer, then four epilogue warps (one per TMEM lane quarter) for every
-    // 64 columns of the tile, the TMA producer of B and the tile scheduler
-    static constexpr int kEpiWarps = 4 * (BN / 64);
+    // kEpiCols tensor-memory columns, the TMA producer of B and the tile scheduler
+    static constexpr int kEpiCols = BN == 256 ? 64 : 32;
+    static constexpr int kEpiWarps = 4 * (kAccCols / kEpiCols);
     static constexpr int kProducerA = 0, kMmaWarp = 1, kEpiWarp0 = 2, kProducerB = 2 + kEpiWarps, kSchedulerWarp = 3 + kEpiWarps;
     static constexpr int kThreads = 32 * (4 + kEpiWarps);
-    static constexpr int kStagingBytes = kEpiWarps * kSlabBytes;
-    static constexpr int kTmemCols = 2 * BN;
+    static constexpr int kTmemCols = 2 * kAccCols;
     static constexpr int kBarrierBytes = 768;   // mbarriers, flags, the tile ring and the hand-over ring of the chained launch
-    static constexpr int kStages = (kSmemLimit - kStagingBytes - kBarrierBytes - 1024) / kStageBytes;
-    static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
-    static constexpr int kTileM = PAIR ? 256 : 128;  // rows of the (cluster) tile
+    static_assert(kRows == 128 || (kRows == 64 && kBRows == 64), "boxes of the operand maps");
+    static constexpr int kMaxStages = (kSmemLimit - kBarrierBytes - 1024) / kStageBytes;
+    static constexpr int kStages = kMaxStages < 8 ? kMaxStages : 8;
+    static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 1024;
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -110,9 +123,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// arrive on a barrier given by its shared::cluster address (own or peer CTA)
+// Arrive on a barrier given by its shared::cluster address (own or peer CTA).  For tensor memory that has been read, whose order
+// tcgen05.fence::before_thread_sync keeps; release semantics at cluster scope would make the thread wait for its stores.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -250,6 +264,19 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, uint64_t map, uint32_t
             ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
             : "memory");
 }
+template <bool PAIR>
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, uint64_t map, uint32_t bar, int x, int y, int z) {
+    if (PAIR)
+        asm volatile(
+            "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+            ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+            : "memory");
+    else
+        asm volatile(
+            "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+            ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+            : "memory");
+}
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -308,6 +335,12 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t *r) {
         : "r"(taddr)
         : "memory");
 }
+// 32 bytes, one sector, to a 32-byte aligned address
+__device__ __forceinline__ void st_global_32(void *p, const uint32_t *v) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor, 128-byte swizzle, descriptor version 1 (sm_100).
@@ -343,7 +376,7 @@ struct alignas(16) TileEntry {
     uint32_t M, N, num_kb, pitch_bytes;
     uint32_t tile;           // tile_m | tile_n << 16
     uint32_t flags;
-    uint32_t tiles_n, slot;
+    uint32_t frag_units, slot;
 };
 static_assert(sizeof(TileEntry) == 64, "control region layout");
 constexpr uint32_t kRing = 4;
@@ -358,7 +391,7 @@ constexpr int kTileEpiShift = 8, kTileScaleShift = 12, kTileIterShift = 16, kTil
 // exists, rounded up: a 1600-wide output has a last tile column of 64, which a 256-wide MMA would spend four times as
 // long on.  K-major B: steps of 64 (a pair splits N in two halves of at least 32 rows); MN-major B: steps of 128, so
 // that each half is made of whole 64-element swizzle atoms.
-template <int BN, bool PAIR>
+template <typename C, int BN, bool PAIR>
 __device__ __forceinline__ void fill_entry(TileEntry &e, const GemmProblem *p, uint32_t tile_m, uint32_t tile_n, uint32_t epilogue,
                                            uint32_t flags) {
     e.map_a = p->map_a;
@@ -367,7 +400,7 @@ __device__ __forceinline__ void fill_entry(TileEntry &e, const GemmProblem *p, u
     e.M = p->M;
     e.N = p->N;
     e.num_kb = (p->K + kGemmBlockK - 1) / kGemmBlockK;
-    e.tiles_n = p->tiles_n;
+    e.frag_units = p->frag_units;
     const bool last = epilogue == kEpiApplyLast;
     e.out = last ? p->out32 : p->out16;
     e.pitch_bytes = last ? p->pitch32 * 4u : p->pitch16 * 2u;
@@ -375,25 +408,25 @@ __device__ __forceinline__ void fill_entry(TileEntry &e, const GemmProblem *p, u
     const uint32_t a_mn = p->a_mn_major, b_mn = p->b_mn_major;
     const uint32_t step = b_mn ? 128u : 64u;
     const uint32_t left = e.N - tile_n * BN;
-    const uint32_t n_mma = min((uint32_t)BN, (left + step - 1u) / step * step);
-    // a diagonal tile of X X^T or G G: this CTA's 128 rows of B are its 128 rows of A, in the same shared-memory layout
-    const bool shared = (PAIR || BN == 128) && tile_m == tile_n && e.map_a == e.map_b && a_mn == b_mn && n_mma == (uint32_t)BN;
+    // (64 rows per CTA: always BN, which fixes where the columns lie in tensor memory)
+    const uint32_t n_mma = C::kRows == 64 ? (uint32_t)BN : min((uint32_t)BN, (left + step - 1u) / step * step);
+    // a diagonal tile of X X^T or G G: this CTA's rows of B are its rows of A, in the same shared-memory layout
+    const bool shared = C::kTileM == BN && tile_m == tile_n && e.map_a == e.map_b && a_mn == b_mn && n_mma == (uint32_t)BN;
     e.flags = flags | (a_mn ? kTileAMn : 0u) | (b_mn ? kTileBMn : 0u) | (shared ? kTileShared : 0u) |
               (epilogue << kTileEpiShift) | ((n_mma / 32u) << kTileNShift);
 }
 
-template <int BN, bool PAIR, bool CHAINED>
-__global__ void __launch_bounds__((Cfg<BN, PAIR>::kThreads), 1)
+template <int TM, int BN, bool PAIR, bool CHAINED>
+__global__ void __launch_bounds__((Cfg<TM, BN, PAIR>::kThreads), 1)
 k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ tiles,
           uint32_t tile_count, uint32_t epilogue_arg, int f16, GemmCoefficients coef,
           const float *__restrict__ slot_scale, uint32_t scale_pow_arg, uint32_t *status, ChainSync *sync,
           uint32_t slot_count) {
-    using C = Cfg<BN, PAIR>;
+    using C = Cfg<TM, BN, PAIR>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *stage_base = smem;
-    uint8_t *staging = smem + C::kStages * C::kStageBytes;
-    uint8_t *control = staging + C::kStagingBytes;
+    uint8_t *control = smem + C::kStages * C::kStageBytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(control);
     // bars: full[S], empty[S], tmem_full[2], tmem_empty[2], ring_full[kRing], ring_empty[kRing]
     constexpr int kBars = 2 * C::kStages + 4 + 2 * (int)kRing;
@@ -481,7 +514,7 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                     if (t < tile_count) next = list[t];
                     if (!claim_slot()) { ok = false; break; }
                     TileEntry &e = ring[k % kRing];
-                    fill_entry<BN, PAIR>(e, problems + tl.problem, tl.tile_m, tl.tile_n, epilogue_arg,
+                    fill_entry<C, BN, PAIR>(e, problems + tl.problem, tl.tile_m, tl.tile_n, epilogue_arg,
                                          (tl.reserved ? kTileMirror : 0u) | (scale_pow_arg << kTileScaleShift));
                     e.slot = tl.problem;
                     if (k < 2) {
@@ -524,7 +557,7 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                         }
                         if (!claim_slot()) { ok = false; break; }
                         TileEntry &e = ring[k % kRing];
-                        fill_entry<BN, PAIR>(e, problems + (part ? d.x : c.x), c.y & 0xffffu, c.y >> 16,
+                        fill_entry<C, BN, PAIR>(e, problems + (part ? d.x : c.x), c.y & 0xffffu, c.y >> 16,
                                              two ? (part ? kEpiPolyFused : kEpiGramHold) : epilogue,
                                              flags | (need != 0u ? kTileDependent : 0u));
                         e.slot = slot;
@@ -565,29 +598,36 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                 const bool mn = (flags & (as_b ? kTileBMn : kTileAMn)) != 0u;
                 const int n_half = (int)(flags >> kTileNShift) * 16;   // half of the MMA's N
                 const int row0 = as_b ? (int)(tile >> 16) * BN + (PAIR ? (int)rank * n_half : 0)
-                                      : (int)(tile & 0xffffu) * C::kTileM + (int)rank * 128;
-                // PAIR: both CTAs' copies complete on the leader's barrier, which expects the bytes of both
-                const uint32_t bytes = (as_b ? (uint32_t)C::kBBytes : (uint32_t)kABytes) * (PAIR ? 2u : 1u);
-                const uint32_t dst0 = smem_u32(stage_base) + (as_b ? (uint32_t)kABytes : 0u);
-                const int boxes = as_b ? C::kBRows / 128 : 1;
-                for (int kb = 0; kb < num_kb; ++kb) {
+                                      : (int)(tile & 0xffffu) * C::kTileM + (int)rank * C::kRows;
+                const uint32_t dst0 = smem_u32(stage_base) + (as_b ? (uint32_t)C::kABytes : 0u);
+                const int operand_rows = as_b ? C::kBRows : C::kRows;
+                for (int kb = 0; kb < num_kb; kb += C::kStageKb) {
                     turn ^= 1u;
                     if (!shared || turn == (for_b ? 1u : 0u)) {
+                        const int subs = min(C::kStageKb, num_kb - kb);
                         if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { ok = false; break; }
                         if (!PAIR || rank == 0) {
-                            mbar_expect_tx(full_bar(stage), bytes);
+                            // PAIR: both CTAs' copies complete on the leader's barrier, which expects the bytes of both
+                            mbar_expect_tx(full_bar(stage), (uint32_t)(operand_rows * 128 * subs) * (PAIR ? 2u : 1u));
                             if (shared) mbar_arrive(full_bar(stage));   // in the other producer's place
                         }
-                        const uint32_t fb = leader_full + 8u * stage, dst = dst0 + stage * (uint32_t)C::kStageBytes;
-                        const int k0 = kb * kGemmBlockK;
-                        if (mn) {   // 64 x 64 boxes: x = M or N index, y = K index
-                            for (int j = 0; j < boxes; ++j) {
-                                tma_load_2d<PAIR>(dst + (2 * j) * kBoxBytes, map, fb, row0 + 128 * j, k0);
-                                tma_load_2d<PAIR>(dst + (2 * j + 1) * kBoxBytes, map, fb, row0 + 128 * j + 64, k0);
+                        const uint32_t fb = leader_full + 8u * stage;
+#pragma unroll
+                        for (int sub = 0; sub < C::kStageKb; ++sub) {
+                            if (sub >= subs) break;
+                            const uint32_t dst = dst0 + stage * (uint32_t)C::kStageBytes + sub * C::kKbBytes;
+                            const int k0 = (kb + sub) * kGemmBlockK;
+                            if (C::kRows == 64) {   // (B has 64 rows too) one box of 64 x 64: x = M or N index, y = K index, or K, rows
+                                tma_load_2d<PAIR>(dst, map, fb, mn ? row0 : k0, mn ? k0 : row0);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < (C::kBRows > 128 ? 2 : 1); ++j) {
+                                    if (128 * j >= operand_rows) break;
+                                    // 128 rows: two boxes of 64 x 64, z = M or N index / 64, or one of 64 (K) x 128
+                                    if (mn) tma_load_3d<PAIR>(dst + j * 16384, map, fb, 0, k0, row0 / 64 + 2 * j);
+                                    else tma_load_2d<PAIR>(dst + j * 16384, map, fb, k0, row0 + 128 * j);
+                                }
                             }
-                        } else {    // 64 (K) x 128 (rows) boxes
-                            for (int j = 0; j < boxes; ++j)
-                                tma_load_2d<PAIR>(dst + (2 * j) * kBoxBytes, map, fb, k0, row0 + 128 * j);
                         }
                     }
                     if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
@@ -614,21 +654,27 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
                 const uint32_t idesc = instr_desc(C::kTileM, (int)(flags >> kTileNShift) * 32, f16, a_mn, b_mn);
                 // leading byte offset (unused by a K-major operand) and the step of 16 in K, in units of 16 bytes
                 const uint64_t a0 = desc0 + ((uint64_t)(a_mn ? kBoxBytes >> 4 : 1) << 16);
-                const uint64_t b0 = desc0 + ((uint64_t)(b_mn ? kBoxBytes >> 4 : 1) << 16) + (flags & kTileShared ? 0u : (uint32_t)(kABytes >> 4));
+                const uint64_t b0 = desc0 + ((uint64_t)(b_mn ? kBoxBytes >> 4 : 1) << 16) + (flags & kTileShared ? 0u : (uint32_t)(C::kABytes >> 4));
                 const uint32_t a_step = a_mn ? 128u : 2u, b_step = b_mn ? 128u : 2u;
                 if (!__all_sync(0xffffffffu, mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag))) break;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem + acc * BN;
-                for (uint32_t kb = 0; kb < num_kb; ++kb) {
+                const uint32_t d_tmem = tmem + acc * C::kAccCols;
+                for (uint32_t kb = 0; kb < num_kb; kb += C::kStageKb) {
                     if (!__all_sync(0xffffffffu, mbar_wait(full_bar(stage), phase, abort_flag))) { ok = false; break; }
                     tc_fence_after();
                     const uint64_t ad = a0 + stage * (uint32_t)(C::kStageBytes >> 4), bd = b0 + stage * (uint32_t)(C::kStageBytes >> 4);
                     if (elect_one()) {
 #pragma unroll
-                        for (uint32_t j = 0; j < kGemmBlockK / 16; ++j)
-                            tc_mma<PAIR>(d_tmem, ad + j * a_step, bd + j * b_step, idesc, j != 0 ? 1u : (uint32_t)(kb != 0));
+                        for (uint32_t sub = 0; sub < (uint32_t)C::kStageKb; ++sub) {
+                            if (C::kStageKb > 1 && kb + sub >= num_kb) break;
+#pragma unroll
+                            for (uint32_t j = 0; j < kGemmBlockK / 16; ++j)
+                                tc_mma<PAIR>(d_tmem, ad + sub * (uint32_t)(C::kKbBytes >> 4) + j * a_step,
+                                             bd + sub * (uint32_t)(C::kKbBytes >> 4) + j * b_step, idesc,
+                                             sub != 0 || j != 0 ? 1u : (uint32_t)(kb != 0));
+                        }
                         tc_commit<PAIR>(empty_bar(stage));
-                        if (kb + 1 == num_kb) tc_commit<PAIR>(tfull_bar(acc));
+                        if (kb + C::kStageKb >= num_kb) tc_commit<PAIR>(tfull_bar(acc));
                     }
                     __syncwarp();
                     if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
@@ -639,40 +685,16 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
         }
     } else {
         // ------------------------------------------------------------------ epilogue warps
-        // Warp w may read TMEM lanes 32 (w % 4) .. +31; the four warps of a lane quarter each take
-        // one 64-column chunk of the tile, so an accumulator buffer is free again after ONE chunk
-        // has been read and a tile's epilogue takes a quarter of the time it would on one warp.
+        // Warp w may read TMEM lanes 32 (w % 4) .. +31; the warps of a lane quarter each take kEpiCols columns, so an
+        // accumulator buffer is free again after that many have been read.  Results go from registers to memory in 32-byte
+        // pieces, one whole sector per lane: through a slab in shared memory, for stores of whole 128-byte lines, every byte
+        // would pass the shared-memory port twice more, and that port is what the MMAs and their operands fill.
         const int q = warp & 3;
         const int chunk = (warp - C::kEpiWarp0) >> 2;
-        const int c0 = chunk * 64;
-        // Results leave through a per-warp 4 KB slab in shared memory and plain 128-bit global stores: the warp
-        // writes its 32 rows into the slab (one row per lane, 16-byte chunks XOR-swizzled by the row so that the
-        // fill and the copy-out are both conflict-free), then copies it out with eight lanes per row, so every
-        // store instruction writes whole 128-byte lines.  Plain stores need no bulk-group wait before the slab
-        // is refilled or the launch ends, and a fence orders them before the progress count of a chained launch.
-        uint8_t *slab = staging + (size_t)(warp - C::kEpiWarp0) * kSlabBytes;
-        // 32 rows x 128 bytes, swizzled -> row-major tensor; rows >= row_limit and bytes >= byte_limit are dropped
-        auto slab_to_global = [&](uint8_t *base, size_t pitch_bytes, int row0, int row_limit, int byte0, int byte_limit) {
-#pragma unroll 2
-            for (int i = 0; i < 8; ++i) {
-                const int r = 4 * i + (lane >> 3), c = lane & 7;
-                const uint4 w = *reinterpret_cast<const uint4 *>(slab + r * 128 + ((c ^ (r & 7)) << 4));
-                const int gr = row0 + r, gb = byte0 + 16 * c;
-                if (gr < row_limit && gb < byte_limit)
-                    *reinterpret_cast<uint4 *>(base + (size_t)gr * pitch_bytes + gb) = w;
-            }
-        };
-        // 64 rows x 64 bytes, plain row-major (the transposed block of a symmetric output)
-        auto slab_t_to_global = [&](uint8_t *base, size_t pitch_bytes, int row0, int row_limit, int byte0, int byte_limit) {
-#pragma unroll 2
-            for (int i = 0; i < 8; ++i) {
-                const int r = 8 * i + (lane >> 2), c = lane & 3;
-                const uint4 w = *reinterpret_cast<const uint4 *>(slab + r * 64 + 16 * c);
-                const int gr = row0 + r, gb = byte0 + 16 * c;
-                if (gr < row_limit && gb < byte_limit)
-                    *reinterpret_cast<uint4 *>(base + (size_t)gr * pitch_bytes + gb) = w;
-            }
-        };
+        const int taddr_col = chunk * C::kEpiCols;
+        // rows and columns of the tile: 64 rows per CTA lie in two halves of the lanes
+        const int c0 = taddr_col + (C::kRows == 64 ? (q >> 1) * (BN / 2) : 0);
+        const int row_in_cta = 32 * (C::kRows == 64 ? q & 1 : q) + lane;
         const uint32_t tempty_leader0 = PAIR ? map_to_cta(tempty_bar(0), 0) : tempty_bar(0);
         uint32_t acc = 0, acc_phase = 0;
         // Chained launch: a finished tile is published to the other CTAs by raising its matrix's progress count
@@ -695,10 +717,9 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
             const uint32_t flags = entry.flags, M = entry.M, N = entry.N, slot = entry.slot;
             uint8_t *out = reinterpret_cast<uint8_t *>(entry.out);
             const size_t pitch = entry.pitch_bytes;
-            const float4 *frag = reinterpret_cast<const float4 *>(entry.frag);
+            const uint64_t entry_frag = entry.frag;
             const int tile_m = (int)(entry.tile & 0xffffu), tile_n = (int)(entry.tile >> 16);
-            // fragment scratch is indexed by 128-row sub-tiles
-            const uint32_t tile_lin = (PAIR ? (uint32_t)tile_m * 2 + rank : (uint32_t)tile_m) * entry.tiles_n + tile_n;
+            const uint32_t frag_units = entry.frag_units;
             __syncwarp();
             if (lane == 0) mbar_arrive(ring_empty(k));
             if (flags & kTileEnd) break;
@@ -717,30 +738,29 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
             // symmetric outputs (Gram, Poly): tiles below the diagonal are not computed; the tile
             // above writes them as its transpose (reference: tiles/symmetric.rs:76-92)
             const bool mirror = (flags & kTileMirror) != 0u;
-            const int m0 = tile_m * C::kTileM + (int)rank * 128, n0 = tile_n * BN;
-            const int row_in_tile = 32 * q + lane;
-            const int grow = m0 + row_in_tile;
-            const int slab_row0 = m0 + 32 * q;
-            // fragment order: [128-row sub-tile][32-column unit][float4 index][row]
-            const size_t unit0 = ((size_t)tile_lin * (BN / 32) + (size_t)(c0 / 32)) * 8;
+            const int grow = tile_m * C::kTileM + (int)rank * C::kRows + row_in_cta;   // this lane's row
+            const int warp_row0 = grow - lane, col0 = tile_n * BN + c0;
+            const bool in_range = col0 < (int)N && warp_row0 < (int)M;   // warp-uniform
+            // FP32 Gram values: [128 rows][32-column unit][float4 index][row]
+            float4 *frag = reinterpret_cast<float4 *>(entry_frag) +
+                           ((size_t)(grow / kGemmBlockM) * frag_units + (size_t)(col0 / 32)) * (8 * kGemmBlockM) + grow % kGemmBlockM;
 
             // The polynomial epilogue needs the FP32 Gram tile: fetch the first 32 columns before the accumulator is
             // ready so the latency hides behind the MMAs.  (Chained: an entry is in the ring only once the matrix's
             // Gram phase is complete.)
             float4 g[8];
-            if (epilogue == kEpiPoly) {
+            if (epilogue == kEpiPoly && in_range) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) g[j] = __ldcg(frag + (unit0 + j) * kGemmBlockM + row_in_tile);
+                for (int j = 0; j < 8; ++j) g[j] = __ldcg(frag + j * kGemmBlockM);
             }
             if (CHAINED && unpublished != kNoSlot && !__all_sync(0xffffffffu, mbar_test(tfull_bar(acc), acc_phase))) publish();
             if (!__all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), acc_phase, abort_flag))) break;
             tc_fence_after();
-            const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + acc * BN + c0;
+            const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + acc * C::kAccCols + taddr_col;
             // fused: the Gram accumulator of this tile sits in the other buffer
-            const uint32_t held_taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (acc ^ 1u) * BN + c0;
+            const uint32_t held_taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (acc ^ 1u) * C::kAccCols + taddr_col;
             const uint32_t tempty = tempty_leader0 + 8u * acc;
             const uint32_t held_tempty = tempty_leader0 + 8u * (acc ^ 1u);
-            const bool in_range = n0 + c0 < (int)N && slab_row0 < (int)M;   // warp-uniform
             // One-pass prepare: the operand of the first iteration is the un-normalised update, and
             // s = 1 / (1.01 |u| + 1e-7) of the tile's matrix enters here: G = (s s) X X^T, X1 = s (Q X).
             // (A fused polynomial part scales the held Gram accumulator, not its own.)
@@ -751,69 +771,41 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
             }
             const bool scaled = out_scale != 1.0f;   // warp-uniform
 
-            if (epilogue == kEpiApplyLast) {
-                // FP32 result in the storage layout: 32 columns (128 bytes) per staged slab
-#pragma unroll 1
-                for (int sub = 0; sub < 2; ++sub) {
-                    uint32_t v[32];
-                    tc_ld32(taddr + 32 * sub, v);
-                    tc_ld_wait();
-                    if (sub == 1) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(tempty);
-                    }
-                    if (!in_range || n0 + c0 + 32 * sub >= (int)N) continue;
-                    if (CHAINED && sub == 1 && unpublished != kNoSlot) publish();
-                    if (scaled) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * out_scale);
-                    }
-                    __syncwarp();   // the copy-out of the previous slab is done in every lane
+            for (int sub = 0; sub < C::kEpiCols / 32; ++sub) {
+                constexpr int kLastSub = C::kEpiCols / 32 - 1;
+                const int col = col0 + 32 * sub;
+                uint32_t packed[16];
+                if (CHAINED && fused) {
+                    // two halves of 16 columns: this tile's accumulator and the held Gram accumulator, which enters as the
+                    // unfused form would have read it back from memory
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        uint4 w = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                        *reinterpret_cast<uint4 *>(slab + lane * 128 + ((j ^ (lane & 7)) << 4)) = w;
-                    }
-                    __syncwarp();
-                    slab_to_global(out, pitch, slab_row0, (int)M, (n0 + c0 + 32 * sub) * 4, (int)pitch);
-                }
-            } else {
-                // 16-bit result: the chunk's 64 columns are read in two halves of 32 and packed
-                uint32_t packed[32];
-                if (fused) {
-                    // four quarters of 16 columns: this tile's accumulator and the held Gram accumulator, which
-                    // enters as the unfused form would have read it back from memory
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
+                    for (int half = 0; half < 2; ++half) {
                         uint32_t v[16], h[16];
-                        tc_ld16(taddr + 16 * k, v);
-                        tc_ld16(held_taddr + 16 * k, h);
+                        tc_ld16(taddr + 32 * sub + 16 * half, v);
+                        tc_ld16(held_taddr + 32 * sub + 16 * half, h);
                         tc_ld_wait();
-                        if (k == 3) {
+                        if (sub == kLastSub && half == 1) {
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) { mbar_arrive_cluster(tempty); mbar_arrive_cluster(held_tempty); }
                         }
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
-                            const int gcol = n0 + c0 + 16 * k + j;
-                            const float ident = (gcol == grow) ? ca : 0.0f;
+                            const float ident = (col + 16 * half + j == grow) ? ca : 0.0f;
                             const float base = scaled ? __uint_as_float(h[j]) * out_scale : __uint_as_float(h[j]);
                             // store/plain.rs:175-178: fma(c, acc, fma(b, base, identity))
                             v[j] = __float_as_uint(fmaf(cc, __uint_as_float(v[j]), fmaf(cb, base, ident)));
                         }
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
-                            packed[8 * k + j] = pack_operands(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), f16);
+                            packed[8 * half + j] = pack_operands(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), f16);
                     }
                 } else {
-#pragma unroll
-                for (int sub = 0; sub < 2; ++sub) {
                     uint32_t v[32];
                     tc_ld32(taddr + 32 * sub, v);
                     tc_ld_wait();
-                    if (sub == 1 && !hold) {
+                    if (sub == kLastSub && !hold) {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster(tempty);
@@ -822,62 +814,73 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * out_scale);
                     }
-                    if (epilogue == kEpiGram || epilogue == kEpiPoly) {
-                        const size_t unit = unit0 + 8 * sub;
+                    if (epilogue == kEpiApplyLast) {   // FP32 result in the storage layout
+                        if (CHAINED && unpublished != kNoSlot) publish();
+                        if (in_range && grow < (int)M) {
+                            uint8_t *dst = out + (size_t)grow * pitch + (size_t)col * 4;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (col * 4 + 32 * j < (int)pitch) st_global_32(dst + 32 * j, v + 8 * j);
+                        }
+                        continue;
+                    }
+                    if (in_range && col < (int)N && (epilogue == kEpiGram || epilogue == kEpiPoly)) {
+                        float4 *unit = frag + (size_t)sub * (8 * kGemmBlockM);
                         if (epilogue == kEpiGram) {
-                            float4 *fw = const_cast<float4 *>(frag);
 #pragma unroll
                             for (int j = 0; j < 8; ++j)
-                                __stcg(fw + (unit + j) * kGemmBlockM + row_in_tile,
+                                __stcg(unit + j * kGemmBlockM,
                                        make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
                                                    __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
                         } else {
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
-                                const float gv[4] = {g[j].x, g[j].y, g[j].z, g[j].w};
+                                const float gg[4] = {g[j].x, g[j].y, g[j].z, g[j].w};
 #pragma unroll
                                 for (int e = 0; e < 4; ++e) {
-                                    const int gcol = n0 + c0 + 32 * sub + 4 * j + e;
-                                    const float ident = (gcol == grow) ? ca : 0.0f;
+                                    const float ident = (col + 4 * j + e == grow) ? ca : 0.0f;
                                     // store/plain.rs:175-178: fma(c, acc, fma(b, base, identity))
-                                    v[4 * j + e] = __float_as_uint(
-                                        fmaf(cc, __uint_as_float(v[4 * j + e]), fmaf(cb, gv[e], ident)));
+                                    v[4 * j + e] = __float_as_uint(fmaf(cc, __uint_as_float(v[4 * j + e]), fmaf(cb, gg[e], ident)));
                                 }
                             }
-                            if (sub == 0) {   // the other 32 columns, while this half is packed
+                            if (sub < kLastSub && col + 32 < (int)N) {   // the next 32 columns, while these are packed and stored
 #pragma unroll
-                                for (int j = 0; j < 8; ++j) g[j] = __ldcg(frag + (unit + 8 + j) * kGemmBlockM + row_in_tile);
+                                for (int j = 0; j < 8; ++j) g[j] = __ldcg(unit + (8 + j) * kGemmBlockM);
                             }
                         }
                     }
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        packed[16 * sub + j] = pack_operands(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), f16);
-                }
+                        packed[j] = pack_operands(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), f16);
                 }
                 if (CHAINED && unpublished != kNoSlot) publish();
-                if (in_range) {
-                    __syncwarp();   // the copy-out of the previous slab is done in every lane
+                if (in_range && col < (int)N) {
+                    if (grow < (int)M) {
+                        uint8_t *dst = out + (size_t)grow * pitch + (size_t)col * 2;
+                        if ((pitch & 31u) == 0u) {
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const uint4 w = make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
-                        *reinterpret_cast<uint4 *>(slab + lane * 128 + ((j ^ (lane & 7)) << 4)) = w;
+                            for (int j = 0; j < 2; ++j)
+                                if (col * 2 + 32 * j < (int)pitch) st_global_32(dst + 32 * j, packed + 8 * j);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (col * 2 + 16 * j < (int)pitch)
+                                    *reinterpret_cast<uint4 *>(dst + 16 * j) =
+                                        make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+                        }
                     }
-                    __syncwarp();
-                    slab_to_global(out, pitch, slab_row0, (int)M, (n0 + c0) * 2, (int)pitch);
                     if (mirror) {
-                        // transposed 64 x 32 block (rows = this chunk's columns), plain row-major
-                        // 64-byte rows: lanes pair up so every lane stores two rows of one column
-                        __syncwarp();
+                        // the transposed block: lanes pair up, the even one stores two rows of one column, the odd one two of
+                        // the next, so a store writes 64 bytes of two rows of the result
+                        uint8_t *dst = out + (size_t)(col + (lane & 1)) * pitch + (size_t)(warp_row0 + (lane & ~1)) * 2;
+                        const bool inside = (warp_row0 + (lane & ~1)) * 2 < (int)pitch;
 #pragma unroll
-                        for (int c = 0; c < 64; c += 2) {
+                        for (int c = 0; c < 32; c += 2) {
                             const uint32_t mine = packed[c >> 1];
                             const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
-                            const uint32_t out = (lane & 1) ? __byte_perm(other, mine, 0x7632) : __byte_perm(mine, other, 0x5410);
-                            *reinterpret_cast<uint32_t *>(slab + (c + (lane & 1)) * 64 + (lane & ~1) * 2) = out;
+                            const uint32_t two = (lane & 1) ? __byte_perm(other, mine, 0x7632) : __byte_perm(mine, other, 0x5410);
+                            if (inside && col + c + (lane & 1) < (int)M) *reinterpret_cast<uint32_t *>(dst + (size_t)c * pitch) = two;
                         }
-                        __syncwarp();
-                        slab_t_to_global(out, pitch, n0 + c0, (int)M, slab_row0 * 2, (int)pitch);
                     }
                 }
             }
@@ -1182,11 +1185,12 @@ k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kSmallTmemCols) : "memory");
 }
 
-template <int BN, bool PAIR, bool CHAINED>
+template <int TM, int BN, bool PAIR, bool CHAINED>
 cudaError_t launch_impl(const GemmProblem *problems, const void *tiles, uint32_t tile_count, uint32_t epilogue,
                         int f16, const GemmCoefficients &coef, const float *slot_scale, uint32_t scale_pow,
                         uint32_t *status, void *sync, uint32_t slot_count, uint32_t debug_flags, int grid,
                         cudaStream_t s) {
+    using C = Cfg<TM, BN, PAIR>;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     unsigned n_attr = 0;
@@ -1215,51 +1219,51 @@ cudaError_t launch_impl(const GemmProblem *problems, const void *tiles, uint32_t
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
-    cfg.blockDim = dim3((unsigned)Cfg<BN, PAIR>::kThreads, 1, 1);
-    cfg.dynamicSmemBytes = Cfg<BN, PAIR>::kSmemBytes;
+    cfg.blockDim = dim3((unsigned)C::kThreads, 1, 1);
+    cfg.dynamicSmemBytes = C::kSmemBytes;
     cfg.stream = s;
-    return cudaLaunchKernelEx(&cfg, k_ns_gemm<BN, PAIR, CHAINED>, problems, tiles, tile_count, epilogue, f16, coef,
+    return cudaLaunchKernelEx(&cfg, k_ns_gemm<TM, BN, PAIR, CHAINED>, problems, tiles, tile_count, epilogue, f16, coef,
                               slot_scale, scale_pow, status, static_cast<ChainSync *>(sync), slot_count);
 }
 
-template <bool CHAINED>
-cudaError_t dispatch(int block_n, int pair, const GemmProblem *problems, const void *tiles, uint32_t tile_count,
-                     uint32_t epilogue, int f16, const GemmCoefficients &coef, const float *slot_scale,
-                     uint32_t scale_pow, uint32_t *status, void *sync, uint32_t slot_count, uint32_t debug_flags,
-                     int grid, cudaStream_t s) {
-    if (tile_count == 0) return cudaSuccess;
-    if (pair && block_n == 256)
-        return launch_impl<256, true, CHAINED>(problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow,
-                                                  status, sync, slot_count, debug_flags, grid, s);
-    if (!pair && block_n == 256)
-        return launch_impl<256, false, CHAINED>(problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow,
-                                                   status, sync, slot_count, debug_flags, grid, s);
-    if (!pair && block_n == 128)
-        return launch_impl<128, false, CHAINED>(problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow,
-                                                   status, sync, slot_count, debug_flags, grid, s);
-    return cudaErrorInvalidValue;
-}
+template <int TM, int BN, bool PAIR>
+struct Shape {
+    static constexpr bool is(const GemmShape &g) { return g.tm == TM && g.bn == BN && (g.pair != 0) == PAIR; }
+};
+// Calls f<TM, BN, PAIR>() for the shape, from those that exist with (CHAINED) or without the ticketed form.
+#define B2_FOR_SHAPE(shape, F, ...)                                                  \
+    if (Shape<256, 256, true>::is(shape)) return F<256, 256, true>(__VA_ARGS__);      \
+    if (Shape<128, 256, false>::is(shape)) return F<128, 256, false>(__VA_ARGS__);    \
+    if (Shape<128, 128, false>::is(shape)) return F<128, 128, false>(__VA_ARGS__);
 
-template <int BN, bool PAIR>
+template <int TM, int BN, bool PAIR>
+cudaError_t launch_plain(const GemmProblem *problems, const GemmTile *tiles, uint32_t tile_count, uint32_t epilogue, int f16,
+                         const GemmCoefficients &coef, const float *slot_scale, uint32_t scale_pow, uint32_t *status,
+                         uint32_t debug_flags, int grid, cudaStream_t s) {
+    return launch_impl<TM, BN, PAIR, false>(problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow, status,
+                                            nullptr, 0u, debug_flags, grid, s);
+}
+template <int TM, int BN, bool PAIR>
+cudaError_t launch_ticketed(const GemmProblem *problems, const ChainTile *tiles, uint32_t tile_count, int f16,
+                            const GemmCoefficients &coef, const float *slot_scale, uint32_t *status, void *sync,
+                            uint32_t slot_count, uint32_t debug_flags, int grid, cudaStream_t s, bool fused_list) {
+    // the epilogue argument of the plain launch carries the list kind here
+    return launch_impl<TM, BN, PAIR, true>(problems, tiles, tile_count, fused_list ? 1u : 0u, f16, coef, slot_scale, 0u, status,
+                                           sync, slot_count, debug_flags, grid, s);
+}
+template <int TM, int BN, bool PAIR>
+cudaError_t configure_plain() {
+    return cudaFuncSetAttribute(k_ns_gemm<TM, BN, PAIR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TM, BN, PAIR>::kSmemBytes);
+}
+template <int TM, int BN, bool PAIR>
 cudaError_t configure_both() {
-    cudaError_t e = cudaFuncSetAttribute(k_ns_gemm<BN, PAIR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Cfg<BN, PAIR>::kSmemBytes);
+    const cudaError_t e = configure_plain<TM, BN, PAIR>();
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_ns_gemm<BN, PAIR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                Cfg<BN, PAIR>::kSmemBytes);
+    return cudaFuncSetAttribute(k_ns_gemm<TM, BN, PAIR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TM, BN, PAIR>::kSmemBytes);
 }
-
-}  // namespace
-
-cudaError_t gemm_configure(int block_n, int pair) {
-    if (pair && block_n == 256) return configure_both<256, true>();
-    if (!pair && block_n == 256) return configure_both<256, false>();
-    if (!pair && block_n == 128) return configure_both<128, false>();
-    return cudaErrorInvalidValue;
-}
-namespace {
-template <int BN, bool PAIR>
+template <int TM, int BN, bool PAIR>
 int resident_groups(int sm_count) {
+    using C = Cfg<TM, BN, PAIR>;
     if (PAIR) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
@@ -1270,38 +1274,41 @@ int resident_groups(int sm_count) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         cfg.gridDim = dim3((unsigned)(sm_count & ~1), 1, 1);
-        cfg.blockDim = dim3((unsigned)Cfg<BN, PAIR>::kThreads, 1, 1);
-        cfg.dynamicSmemBytes = Cfg<BN, PAIR>::kSmemBytes;
+        cfg.blockDim = dim3((unsigned)C::kThreads, 1, 1);
+        cfg.dynamicSmemBytes = C::kSmemBytes;
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, k_ns_gemm<BN, PAIR, true>, &cfg) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&clusters, k_ns_gemm<TM, BN, PAIR, true>, &cfg) != cudaSuccess) {
             (void)cudaGetLastError();
             return 0;
         }
         return clusters;
     }
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ns_gemm<BN, PAIR, true>, Cfg<BN, PAIR>::kThreads,
-                                                      Cfg<BN, PAIR>::kSmemBytes) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ns_gemm<TM, BN, PAIR, true>, C::kThreads, C::kSmemBytes) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
     }
     return per_sm > 0 ? sm_count : 0;   // one CTA per SM is all a launch ever uses
 }
 }  // namespace
-int gemm_resident_groups(int block_n, int pair, int sm_count) {
-    if (pair && block_n == 256) return resident_groups<256, true>(sm_count);
-    if (!pair && block_n == 256) return resident_groups<256, false>(sm_count);
-    if (!pair && block_n == 128) return resident_groups<128, false>(sm_count);
+
+cudaError_t gemm_configure(const GemmShape &shape) {
+    B2_FOR_SHAPE(shape, configure_both)
+    return cudaErrorInvalidValue;
+}
+int gemm_resident_groups(const GemmShape &shape, int sm_count) {
+    B2_FOR_SHAPE(shape, resident_groups, sm_count)
     return 0;
 }
-cudaError_t launch_ns_gemm(int block_n, int pair, const GemmProblem *problems, const GemmTile *tiles,
+cudaError_t launch_ns_gemm(const GemmShape &shape, const GemmProblem *problems, const GemmTile *tiles,
                            uint32_t tile_count, uint32_t epilogue, int f16, float ca, float cb,
                            float cc, const float *slot_scale, uint32_t scale_pow, uint32_t *status,
                            uint32_t debug_flags, int grid, cudaStream_t s) {
+    if (tile_count == 0) return cudaSuccess;
     GemmCoefficients coef = {};
     coef.v[0] = ca; coef.v[1] = cb; coef.v[2] = cc;
-    return dispatch<false>(block_n, pair, problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow, status,
-                           nullptr, 0u, debug_flags, grid, s);
+    B2_FOR_SHAPE(shape, launch_plain, problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow, status, debug_flags, grid, s)
+    return cudaErrorInvalidValue;
 }
 bool ns_small_fits(uint32_t rows, uint32_t cols) { return std::min(rows, cols) <= 128u && std::max(rows, cols) <= 512u; }
 namespace {
@@ -1338,14 +1345,22 @@ cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, co
     return cudaLaunchKernelEx(&cfg, ragged ? k_ns_small<true> : k_ns_small<false>, gram, poly, apply0, apply1, last, loop, slot_scale, status);
 }
 size_t chain_sync_bytes(uint32_t slot_count) { return sizeof(ChainSync) + sizeof(uint32_t) * slot_count; }
-uint32_t chain_epilogue_warps(int block_n, int pair) { return (uint32_t)(4 * (block_n / 64)) * (pair ? 2u : 1u); }
-cudaError_t launch_ns_chain(int block_n, int pair, const GemmProblem *problems, const ChainTile *tiles,
+namespace {
+template <int TM, int BN, bool PAIR>
+uint32_t epilogue_warps() { return (uint32_t)Cfg<TM, BN, PAIR>::kEpiWarps * (PAIR ? 2u : 1u); }
+}  // namespace
+uint32_t chain_epilogue_warps(const GemmShape &shape) {
+    B2_FOR_SHAPE(shape, epilogue_warps)
+    return 0;
+}
+cudaError_t launch_ns_chain(const GemmShape &shape, const GemmProblem *problems, const ChainTile *tiles,
                             uint32_t tile_count, int f16, const GemmCoefficients &coef, const float *slot_scale,
                             uint32_t *status, void *sync, uint32_t slot_count, uint32_t debug_flags, int grid,
                             cudaStream_t s, bool fused_list) {
-    // the epilogue argument of the plain launch carries the list kind here
-    return dispatch<true>(block_n, pair, problems, tiles, tile_count, fused_list ? 1u : 0u, f16, coef, slot_scale, 0u,
-                          status, sync, slot_count, debug_flags, grid, s);
+    if (tile_count == 0) return cudaSuccess;
+    B2_FOR_SHAPE(shape, launch_ticketed, problems, tiles, tile_count, f16, coef, slot_scale, status, sync, slot_count, debug_flags, grid, s,
+                 fused_list)
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace b2
