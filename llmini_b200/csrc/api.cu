@@ -159,61 +159,103 @@ bool valid_shape(uint32_t rows, uint32_t cols, const b2_muon_options &o) {
     return true;
 }
 
-// G and Q are symmetric: with square tiles, those below the diagonal can be written as transposes of those above instead
-// of being computed.  Pairs always do that.  With 128 x 128 tiles the transposed store makes a tile's epilogue longer,
-// which pays only where the tiles are more than one wave: one 3072 x 768 (36 tiles) 166 us in full, 176 as a triangle;
-// six layers of width 384 (216 tiles) 216 us in full, 189 as a triangle.
+// Tile shapes of a plan.  tile_override = 128 / 256 forces one CTA per 128 x that many, 512 the pair's 256 x 256; 0 picks
+// the cheapest by estimated time, for Gram and polynomial together (the FP32 Gram tiles and the triangle go from one to the
+// other) and for Apply.  The ticketed schedules run one shape throughout, of those that exist in that form.
+//
+// What a shape costs.  An SM takes in 64 bytes per clock, so a k-block (64 of K) takes 512 clocks where a CTA stages 32 KB
+// (128 x 128, and the pair's 256 x 256, which are four of those) and 256 where it stages 16 KB (the pair's 128 x 128).  Few
+// tiles: the longest decides, and the small ones of a pair win; many: FLOPs per byte, and the large ones win.  A launch takes
+// a fixed time (about 2 us from the end of the launch in front to the first read, 1 us to the first MMA, pipeline fill and
+// last epilogue), a tile so long per k-block and for itself, at least a minimum (its epilogue), and the tiles are dealt round
+// the groups in order of their K, so the first group has the most.  Constants (us) fitted to each phase of 40 plans, one
+// to 192 matrices of 160 to 6400, in each shape (median error 3 %; against the best choice of each phase the picks lose 1 %
+// on average and at most 9 %).  G and Q are symmetric: a triangle leaves out the tiles below the diagonal, whose transposes
+// make the epilogue of the others longer, which pays only beyond one wave.
+// Measured, all of 128 x 128 on one CTA (the smallest shape before) -> the choice, Newton-Schulz loop in us: one 3072 x 768
+// 170 -> 125, one layer of width 320 117 -> 88, four 146 -> 131, five ragged matrices 172 -> 121.
 constexpr uint32_t kTileRuleSms = 148;   // of a B200; not asked of the device, because the workspace size depends on it
-bool triangle_of_128(const uint32_t *rows, const uint32_t *cols, uint32_t count) {
-    uint64_t full = 0;
-    for (uint32_t s = 0; s < count; ++s) {
-        if ((uint64_t)rows[s] * cols[s] == 0) continue;
-        const uint64_t t = (std::min(rows[s], cols[s]) + 127u) / 128u;
-        full += t * t;
+struct TileCost {
+    GemmShape shape;
+    int triangle;
+    bool ticketed;
+    double fixed, per_k_block, per_tile, least;
+};
+void pick_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t count, const b2_muon_options &o, Layout &L) {
+    const GemmShape pair256 = {256, 256, 1}, pair128 = {128, 128, 1}, one256 = {128, 256, 0}, one128 = {128, 128, 0};
+    if (o.tile_override || L.small_smem) {
+        L.nn = L.out = L.small_smem || o.tile_override == 128 ? one128 : o.tile_override == 256 ? one256 : pair256;
+        uint64_t full = 0;   // tiles of 128 x 128: a triangle of them beyond one wave, the pairs' always
+        for (uint32_t s = 0; s < count; ++s)
+            if ((uint64_t)rows[s] * cols[s] != 0) full += (uint64_t)((std::min(rows[s], cols[s]) + 127u) / 128u) * ((std::min(rows[s], cols[s]) + 127u) / 128u);
+        L.symmetric = L.nn.pair || (L.nn.bn == 128 && full > kTileRuleSms) ? 1 : 0;
+        return;
     }
-    return full > kTileRuleSms;
-}
-// Tile configuration: tile_override = 128 / 256 forces the single-CTA kernel with that width, 512 the two-CTA pair; 0
-// picks the cheapest by estimated time.  A phase (one launch) takes a fixed time (launch, prologue, pipeline fill, last
-// epilogue) plus the longer of its longest tile and its share of all tiles; a tile takes so long per k-block (64 of K)
-// and for its epilogue.  Few tiles: the longest one decides, and small tiles on many SMs win; many tiles: the pair, which
-// loads half as many bytes per FLOP, wins.  The constants (us) are fitted to the Newton-Schulz stage of 24 plans of 1 to
-// 48 matrices, 64 to 6400 wide, in each configuration (mostly within 15 %).
-// Measured, pairs -> 128 x 128 (us): one 3072 x 768 241 -> 164, one layer of width 384 171 -> 117, 768 270 -> 206, 1024
-// 350 -> 327, the six largest matrices of a layer pair of width 768 300 -> 255; on the other side of the line two layers
-// of width 768 312 -> 321, four 498 -> 530, four of width 1024 980 -> 1104.
-void pick_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t count, const b2_muon_options &o, int &bn, int &pair) {
-    if (o.tile_override == 128 || o.tile_override == 256) { bn = (int)o.tile_override; pair = 0; return; }
-    if (o.tile_override == 512) { bn = 256; pair = 1; return; }
-    struct Config { uint32_t tm, tn; double groups; bool triangle; double fixed, per_k_block, epilogue; };
-    const Config config[3] = {{128, 128, kTileRuleSms, triangle_of_128(rows, cols, count), 5.0, 0.27, 1.9},
-                              {128, 256, kTileRuleSms, false, 7.0, 0.39, 2.5},
-                              {256, 256, kTileRuleSms / 2, true, 7.0, 0.37, 2.5}};
-    double best_time = 0.0;
-    int best = -1;
-    for (int ci = 0; ci < 3; ++ci) {
-        const Config &c = config[ci];
-        double longest[3] = {0, 0, 0}, total[3] = {0, 0, 0};   // Gram, polynomial, apply
-        for (uint32_t s = 0; s < count; ++s) {
-            if ((uint64_t)rows[s] * cols[s] == 0) continue;
-            const uint32_t n = std::min(rows[s], cols[s]), m = std::max(rows[s], cols[s]);
-            auto tiles = [](uint32_t v, uint32_t t) { return (double)((v + t - 1) / t); };
-            const bool tall = rows[s] > cols[s];
-            const double a = tiles(n, c.tm), nn = c.triangle ? a * (a + 1.0) / 2.0 : a * tiles(n, c.tn);
-            const double out = tall ? tiles(m, c.tm) * tiles(n, c.tn) : a * tiles(m, c.tn);
-            const double k_gram = c.per_k_block * tiles(m, kGemmBlockK), k_rest = c.per_k_block * tiles(n, kGemmBlockK);
-            longest[0] = std::max(longest[0], k_gram);
-            longest[1] = longest[2] = std::max(longest[1], k_rest);
-            total[0] += nn * (k_gram + c.epilogue);
-            total[1] += nn * (k_rest + c.epilogue);
-            total[2] += out * (k_rest + c.epilogue);
+    const TileCost nn[5] = {{pair256, 1, true, 4.7, 0.350, 2.1, 0.9}, {pair128, 0, false, 3.6, 0.126, 0.72, 0.95},
+                            {pair128, 1, false, 3.6, 0.131, 0.92, 0.5}, {one128, 0, true, 3.1, 0.268, 1.1, 1.75},
+                            {one128, 1, true, 3.2, 0.280, 1.36, 1.25}};
+    const TileCost out[3] = {{pair256, 0, true, 4.8, 0.274, 1.6, 1.3}, {pair128, 0, false, 3.6, 0.121, 0.62, 1.0},
+                             {one128, 0, true, 3.2, 0.249, 0.87, 1.75}};
+    std::vector<uint32_t> by_m, by_n;
+    for (uint32_t s = 0; s < count; ++s)
+        if ((uint64_t)rows[s] * cols[s] != 0) by_m.push_back(s);
+    by_n = by_m;
+    auto n_of = [&](uint32_t s) { return std::min(rows[s], cols[s]); };
+    auto m_of = [&](uint32_t s) { return std::max(rows[s], cols[s]); };
+    std::stable_sort(by_m.begin(), by_m.end(), [&](uint32_t a, uint32_t b) { return m_of(a) > m_of(b); });
+    std::stable_sort(by_n.begin(), by_n.end(), [&](uint32_t a, uint32_t b) { return n_of(a) > n_of(b); });
+    auto tiles = [](uint64_t v, int t) { return (v + t - 1) / t; };
+    // time of a launch: `tiles_of(s)` tiles per matrix with a sum over `k_of(s)` each
+    auto launch = [&](const TileCost &c, const std::vector<uint32_t> &order, auto tiles_of, auto k_of) {
+        const uint64_t groups = c.shape.pair ? kTileRuleSms / 2 : kTileRuleSms;
+        uint64_t at = 0;
+        double t = c.fixed;
+        for (uint32_t s : order) {
+            const uint64_t n = tiles_of(s), first_group = (at + n + groups - 1) / groups - (at + groups - 1) / groups;
+            t += (double)first_group * std::max(c.per_k_block * (double)tiles(k_of(s), kGemmBlockK) + c.per_tile, c.least);
+            at += n;
         }
-        double time = 0.0;
-        for (int k = 0; k < 3; ++k) time += c.fixed + std::max(longest[k], total[k] / c.groups);
-        if (best < 0 || time < best_time) { best = ci; best_time = time; }
+        return t;
+    };
+    auto time_nn = [&](const TileCost &c) {
+        auto tiles_of = [&](uint32_t s) {
+            const uint64_t t = tiles(n_of(s), c.shape.tm);
+            return c.triangle ? t * (t + 1) / 2 : t * t;
+        };
+        return launch(c, by_m, tiles_of, m_of) + launch(c, by_m, tiles_of, n_of);
+    };
+    auto time_out = [&](const TileCost &c) {
+        return launch(c, by_n, [&](uint32_t s) { return tiles(rows[s], c.shape.tm) * tiles(cols[s], c.shape.bn); }, n_of);
+    };
+    const bool ticketed = o.ns_schedule != B2_NS_PER_PHASE;
+    double best_nn = 0.0, best_out = 0.0;
+    for (const TileCost &c : nn) {
+        if (ticketed && !c.ticketed) continue;
+        double t = time_nn(c);
+        if (ticketed)
+            for (const TileCost &a : out)
+                if (a.shape.pair == c.shape.pair && a.shape.bn == c.shape.bn) t += time_out(a);
+        if (best_nn == 0.0 || t < best_nn) {
+            best_nn = t;
+            L.nn = c.shape;
+            L.symmetric = c.triangle;
+        }
     }
-    bn = (int)config[best].tn;
-    pair = best == 2;
+    for (const TileCost &c : out) {
+        if (ticketed && (c.shape.pair != L.nn.pair || c.shape.bn != L.nn.bn)) continue;
+        const double t = time_out(c);
+        if (best_out == 0.0 || t < best_out) {
+            best_out = t;
+            L.out = c.shape;
+        }
+    }
+#ifdef B2_MEASURE
+    // bits 8-10 of the flags: tiles of Gram and Poly, 11: triangle, 12-14: tiles of Apply
+    const GemmShape all[4] = {pair256, pair128, one128, one256};
+    const uint32_t f = o.measure_flags >> 8;
+    if (f & 7) { L.nn = all[((f & 7) - 1) & 3]; L.symmetric = (f >> 3) & 1; }
+    if ((f >> 4) & 7) L.out = all[(((f >> 4) & 7) - 1) & 3];
+#endif
 }
 
 // Work list of the fused update + encode launch, for the slot groups [first[g], first[g + 1]): the lists of the
@@ -283,10 +325,7 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
             L.small_ragged = L.small_ragged || rows[s] % 16 != 0;
         }
     }
-    int bn = 256, pair = 0;
-    pick_tiles(rows, cols, count, o, bn, pair);
-    L.nn = L.out = GemmShape{pair ? 256 : 128, bn, pair};
-    L.symmetric = pair || (bn == 128 && triangle_of_128(rows, cols, count)) ? 1 : 0;
+    pick_tiles(rows, cols, count, o, L);
     L.slots.resize(count);
     L.chunk_prefix.assign(count + 1, 0);
     size_t off = 0;

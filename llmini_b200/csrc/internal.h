@@ -177,7 +177,8 @@ struct alignas(16) ChainTile {
 };
 static_assert(sizeof(ChainTile) == 32, "ChainTile is read as two 16-byte words");
 
-// Tile of a launch: tm x bn, computed by one CTA or by a pair of CTAs: 256 x 256 (pair), 128 x 256, 128 x 128.
+// Tile of a launch: tm x bn, computed by one CTA or by a pair of CTAs.  256 x 256 (pair), 128 x 256 and 128 x 128 exist in
+// the plain and the ticketed form, the pairs' 128 x 128 in the plain one.
 struct GemmShape {
     int tm, bn, pair;
 };

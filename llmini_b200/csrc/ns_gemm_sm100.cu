@@ -16,8 +16,9 @@
 // registers, so both sides access it fully coalesced.
 //
 // Tiles (the choice is in api.cu):
-//   PAIR  : a cluster of two CTAs computes 256 x 256 with cta_group::2 MMAs.  Each CTA stages half of the rows of A and half of
-//           those of B, so a k-block costs 32 KB of loads per SM instead of 48 KB.  No multicast load is used.
+//   PAIR  : a cluster of two CTAs computes 256 x 256 or 128 x 128 with cta_group::2 MMAs.  Each CTA stages half of the rows
+//           of A and half of those of B, so a k-block of 256 x 256 costs 32 KB of loads per SM instead of 48 KB, and one of
+//           128 x 128 16 KB instead of the 32 KB that one CTA needs for it.  No multicast load is used.
 //   single: one CTA computes 128 x BN (BN = 128 or 256).
 // In every configuration a tile's sum runs over all of K in one order, so a matrix's result does not depend on which
 // other matrices share its plan: a sharded run and a single GPU compute the same bits.  (Splitting K of the long Gram
@@ -1235,6 +1236,8 @@ struct Shape {
     if (Shape<256, 256, true>::is(shape)) return F<256, 256, true>(__VA_ARGS__);      \
     if (Shape<128, 256, false>::is(shape)) return F<128, 256, false>(__VA_ARGS__);    \
     if (Shape<128, 128, false>::is(shape)) return F<128, 128, false>(__VA_ARGS__);
+#define B2_FOR_PLAIN_SHAPE(shape, F, ...)                                            \
+    if (Shape<128, 128, true>::is(shape)) return F<128, 128, true>(__VA_ARGS__);
 
 template <int TM, int BN, bool PAIR>
 cudaError_t launch_plain(const GemmProblem *problems, const GemmTile *tiles, uint32_t tile_count, uint32_t epilogue, int f16,
@@ -1294,6 +1297,7 @@ int resident_groups(int sm_count) {
 
 cudaError_t gemm_configure(const GemmShape &shape) {
     B2_FOR_SHAPE(shape, configure_both)
+    B2_FOR_PLAIN_SHAPE(shape, configure_plain)
     return cudaErrorInvalidValue;
 }
 int gemm_resident_groups(const GemmShape &shape, int sm_count) {
@@ -1308,6 +1312,7 @@ cudaError_t launch_ns_gemm(const GemmShape &shape, const GemmProblem *problems, 
     GemmCoefficients coef = {};
     coef.v[0] = ca; coef.v[1] = cb; coef.v[2] = cc;
     B2_FOR_SHAPE(shape, launch_plain, problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow, status, debug_flags, grid, s)
+    B2_FOR_PLAIN_SHAPE(shape, launch_plain, problems, tiles, tile_count, epilogue, f16, coef, slot_scale, scale_pow, status, debug_flags, grid, s)
     return cudaErrorInvalidValue;
 }
 bool ns_small_fits(uint32_t rows, uint32_t cols) { return std::min(rows, cols) <= 128u && std::max(rows, cols) <= 512u; }

@@ -278,6 +278,36 @@ def test_few_gram_tiles_with_a_long_k(shapes, deferred):
         assert np.all(np.abs(got_u - want) <= (n + 2) * eps * s * (np.abs(q16) @ np.abs(xd)))
 
 
+@pytest.mark.parametrize("fmt,deferred", [(b2.OPERAND_BF16, True), (b2.OPERAND_F16, False)])
+@pytest.mark.parametrize("shapes", [
+    [(130, 528)],                                        # K of 9 and 3 k-blocks: the last stage of two is half full
+    [(129, 144), (144, 256), (2000, 16)],                # one row or 16 columns into the second tile; one k-block
+    [(1000, 1040), (77, 1040), (200, 208), (48, 1600)],  # rows no multiple of 8, 16 or 64; columns not of 64
+    [(960, 320), (320, 320), (1280, 320), (320, 1280)],  # MN-major on one side, K-major on the other
+    [(768, 768)] * 3 + [(3072, 768)],                    # more tiles than one wave: triangles
+])
+def test_small_pair_tiles_equal_one_cta_tiles_bit_for_bit(shapes, fmt, deferred):
+    """Plans of few tiles take the pairs' 128 x 128 for Gram and polynomial, and some for Apply; a sum runs over K in the
+    same order in every shape."""
+    rng = np.random.default_rng(sum(r for r, _ in shapes))
+    xs = [_x0(rng, r, c, fmt) for r, c in shapes]
+    results = []
+    for tile_n in (0, 128):
+        plan = b2.MuonPlan(shapes, operand_format=fmt, scale_layout=b2.SCALES_RAW, tile_n=tile_n, max_iterations=3,
+                           normalize_mode=b2.NORMALIZE_DEFERRED if deferred else b2.NORMALIZE_TWO_PASS)
+        for i, x in enumerate(xs):
+            plan.scratch(i, 0).copy_(dev(x).to(plan.scratch(i, 0).dtype))
+            plan.scratch(i, 2).view(torch.float32).fill_(0.75)   # read by a one-pass plan only
+        b2.OptimizerModule().muon_polar(plan, b2.MuonMegaUpdateArgs(iterations=3, coefficients=o.fixed_coefficients(3)))
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        results.append([[host(plan.scratch(i, w).float()).copy() for w in (5, 6, 7, 1)] for i in range(len(shapes))])
+        plan.close()
+    for shape, a, b in zip(shapes, *results):
+        for w, u, v in zip(("Gram", "Q", "X1", "U"), a, b):
+            assert np.isfinite(u).all() and np.array_equal(u, v), (shape, w)
+
+
 @pytest.mark.parametrize("company", [
     [(512, 256), (256, 256), (256, 1024), (384, 128)],   # few more tiles of 128 x 128
     [(64, 64)],
