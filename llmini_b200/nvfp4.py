@@ -17,8 +17,15 @@ from . import _ffi
 from ._ffi import SCALES_CSF, SCALES_RAW, SCALES_SM100, check
 
 
+# The handle of the current stream without a Stream object around it: 0.4 us instead of 3.2, of the 10 that a call on one
+# small tensor takes.  (torch keeps the shorter way for its own generated code; where a build has none, the public one does.)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _ptr(t: torch.Tensor) -> int:
@@ -67,7 +74,7 @@ def scales_to_sm100(scales: torch.Tensor, src_layout: int, rows: int, cols: int)
     kind::mxf4nvf4.block_scale` operands use; every byte of the result is written."""
     out = torch.empty(sm100_scales_bytes(rows, cols), dtype=torch.uint8, device=scales.device)
     check(_ffi.lib().b2_nvfp4_scales_to_sm100(scales.data_ptr(), src_layout, rows, cols, out.data_ptr(),
-                                              torch.cuda.current_stream().cuda_stream), "nvfp4_scales_to_sm100")
+                                              _stream()), "nvfp4_scales_to_sm100")
     return out
 
 

@@ -18,13 +18,10 @@ from . import _ffi
 from ._ffi import (AdamWSlotDescriptor, AdamWUpdateArgs as _CAdam, GradientClipArgs as _CClip, MuonOptions, MuonSlotDescriptor, MuonStepArgs, OPERAND_BF16,
                    NORMALIZE_DEFERRED, NORMALIZE_TWO_PASS, NS_CHAINED, NS_FUSED_GRAM_POLY, NS_PER_PHASE, OPERAND_F16, UPDATE_16BIT, UPDATE_F32, QUANTIZE_X, QUANTIZE_Y, SCALES_CSF, SCALES_RAW, SCALES_SM100,
                    ScheduleFreeMaterializeArgs as _CSf, check)
-from .nvfp4 import Nvfp4QuantModule, sm100_scales_bytes, zero_scales
+from .nvfp4 import Nvfp4QuantModule, _stream, sm100_scales_bytes, zero_scales
 
 U32_MAX = 0xFFFFFFFF
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+_Pointers6 = C.c_void_p * 6
 
 
 def _ptr(t: Optional[torch.Tensor]) -> int:
@@ -303,7 +300,7 @@ class OptimizerModule:
                  **_ignored):
         # symexp_lin_scales: `SymExpLinScaleRefs`, six f32[1] device tensors (exponential z, x; linear z, x;
         # curvature z, x), or None for unit scales
-        ptrs = (C.c_void_p * 6)(*[_ptr(t) for t in (symexp_lin_scales or [None] * 6)])
+        ptrs = _Pointers6(*[_ptr(t) for t in symexp_lin_scales]) if symexp_lin_scales else _Pointers6()
         return _CSf(_ptr(bytes), _ptr(scales), _ptr(global_scale), _ptr(z_master), _ptr(x_master),
                     _ptr(precomputed_values), _ptr(amax), len, scale_rows, scale_k, beta, symexp_lin_beta, scale_layout,
                     ptrs)
