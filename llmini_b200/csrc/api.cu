@@ -1029,6 +1029,16 @@ int b2_nvfp4_scales_to_sm100(const uint8_t *d_scales, uint32_t src_layout, uint3
 int b2_materialize_master(uint8_t *d_bytes, uint8_t *d_scales, float *d_global_scale, const float *d_master,
                           float *d_amax, float *d_chunk_amax, uint32_t len, uint32_t scale_layout, void *stream) {
     if (len % 16 != 0 || len > kMaxFlatElements) return B2_ERROR_INVALID_VALUE;
+    if (quantize_chain_fits(len, false, false) && reinterpret_cast<uintptr_t>(d_master) % 16 == 0) {
+        // what the two calls below would refuse
+        if (!d_bytes || !d_scales || !d_global_scale || !d_master || !d_amax || !d_chunk_amax) return B2_ERROR_INVALID_VALUE;
+        if (scale_layout > B2_SCALES_RAW || (scale_layout == B2_SCALES_CSF && len % 128 != 0)) return B2_ERROR_INVALID_VALUE;
+        DeviceInfo d;
+        const cudaError_t e = device_info(d);
+        if (e != cudaSuccess) return (int)e;
+        return (int)launch_quantize_chain(d_master, nullptr, nullptr, 0.0f, nullptr, d_amax, d_chunk_amax, d_bytes, d_scales,
+                                          d_global_scale, len, (int)scale_layout, stream_grid_cap(d), as_stream(stream));
+    }
     int rc = b2_tensor_amax_f32(d_master, d_chunk_amax, d_amax, len, stream);
     if (rc) return rc;
     return b2_fp32_to_nvfp4_four_six(d_master, d_amax, d_bytes, d_scales, d_global_scale, len / 16, scale_layout, stream);
@@ -1074,8 +1084,11 @@ int b2_materialize_schedule_free(const b2_schedule_free_materialize_args *a, voi
     cudaError_t e = device_info(d);
     if (e != cudaSuccess) return (int)e;
     cudaStream_t s = as_stream(stream);
-    e = cudaMemsetAsync(a->amax, 0, sizeof(float), s);  // launcher/update.rs:14-23 (zero_amax)
     const SymExpLinParams sp = symexp_params(a);
+    if (quantize_chain_fits(a->len, true, a->symexp_lin_beta > 0.0f))
+        return (int)launch_quantize_chain(nullptr, a->z_master, a->x_master, a->beta, &sp, a->amax, nullptr, a->bytes, a->scales,
+                                          a->global_scale, a->len, (int)a->scale_layout, stream_grid_cap(d), s);
+    e = cudaMemsetAsync(a->amax, 0, sizeof(float), s);  // launcher/update.rs:14-23 (zero_amax)
     if (e == cudaSuccess)
         e = launch_schedule_free_amax(a->z_master, a->x_master, a->beta, a->len, a->amax, stream_grid_cap(d), s, &sp);
     if (e == cudaSuccess)

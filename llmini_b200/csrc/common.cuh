@@ -168,7 +168,21 @@ __device__ __forceinline__ size_t sm100_scale_offset(uint32_t row, uint32_t kb, 
 // ---- SymExpLin forward (crates/cuda-kernels/src/gpt/optimizer/symexp_lin.rs:8-26) -------------
 struct SymExpLin {
     float beta, exponential, linear, curvature;
+    float inv_beta;   // 1 / beta where div_uniform may use it, else 0
 };
+// What SymExpLin::inv_beta holds: the reciprocal, rounded to nearest, of a divisor that is far from the ends of the range.
+__device__ __forceinline__ float uniform_reciprocal(float b) { return b >= 0x1p-40f && b <= 0x1p40f ? 1.0f / b : 0.0f; }
+// a / b, correctly rounded, for many a and one b.  Markstein (Computation of elementary functions on the IBM RISC System/6000
+// processor, IBM J. Res. Dev. 34, 1990): with r = 1 / b rounded to nearest and q within an ulp of a / b, the remainder
+// a - q b is exact in one fma and q + r (a - q b), rounded, is a / b rounded.  a r may be further off than an ulp, so the same
+// step brings it there first.  The caller has made sure that no step leaves the normal range (uniform_divides).
+__device__ __forceinline__ float div_uniform(float a, float b, float r) {
+    float q = a * r;
+    q = fmaf(r, fmaf(-q, b, a), q);
+    return fmaf(r, fmaf(-q, b, a), q);
+}
+// 2^-60 <= |a| < 2^61: a quotient by a divisor of uniform_reciprocal, and its remainder (2^-24 of a at least), are normal
+__device__ __forceinline__ bool uniform_divides(float a) { return ((__float_as_uint(a) >> 23) & 0xffu) - 67u < 121u; }
 // exp_f32 of the reference: ex2.approx.ftz.f32(x * log2(e)) (crates/cuda-kernels/src/utils/float_ptx.rs:46-51)
 __device__ __forceinline__ float exp_approx(float x) {
     float r;
@@ -191,6 +205,32 @@ __device__ __forceinline__ float symexp_forward(float raw, const SymExpLin &s) {
     if (sign == 0.0f) return 0.0f;
     const float exponential = s.exponential * (exp_approx(s.beta * s.curvature * fabsf(raw)) - 1.0f) / s.beta;
     return sign * (exponential + s.linear * raw / s.beta);
+}
+// The schedule-free values z + beta (x - z) of four elements, transformed.  Without branches per element where all eight
+// dividends allow (raw = 0 and what is not finite fail the test on `l`): a large tensor is bound by these instructions.
+__device__ __forceinline__ float4 schedule_quad(float4 z, float4 x, float beta, const SymExpLin &s) {
+    float v[4] = {z.x + beta * (x.x - z.x), z.y + beta * (x.y - z.y), z.z + beta * (x.z - z.z), z.w + beta * (x.w - z.w)};
+    if (s.beta > 0.0f) {
+        float e[4], l[4];
+        bool ok = s.inv_beta != 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            e[i] = s.exponential * (exp_approx(s.beta * s.curvature * fabsf(v[i])) - 1.0f);
+            l[i] = s.linear * v[i];
+            ok = ok && uniform_divides(e[i]) && uniform_divides(l[i]);
+        }
+        if (ok) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float t = div_uniform(e[i], s.beta, s.inv_beta) + div_uniform(l[i], s.beta, s.inv_beta);
+                v[i] = __uint_as_float(__float_as_uint(t) ^ (__float_as_uint(v[i]) & 0x80000000u));   // sign(v) t
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = symexp_forward(v[i], s);
+        }
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
 }
 
 // ---- reductions ----------------------------------------------------------------------------

@@ -86,6 +86,12 @@ cudaError_t launch_quantize_flat(const float *x, const float *z, const float *xm
                                  int mode, const float *amax, uint8_t *fp4, uint8_t *scales,
                                  float *gs, uint32_t group_count, int scale_layout, int grid_cap,
                                  cudaStream_t s, const SymExpLinParams *symexp = nullptr);
+// Maximum and encode of one tensor as a chain of overlapping launches, for tensors that pass quantize_chain_fits: of `src`,
+// leaving chunk maxima and maximum, or (src null) of the schedule-free values of z and xm, leaving the maximum.
+bool quantize_chain_fits(uint32_t len, bool schedule, bool transform);
+cudaError_t launch_quantize_chain(const float *src, const float *z, const float *xm, float beta, const SymExpLinParams *symexp,
+                                  float *amax, float *chunk_amax, uint8_t *fp4, uint8_t *scales, float *gs, uint32_t len,
+                                  int scale_layout, int grid_cap, cudaStream_t s);
 cudaError_t launch_schedule_free_amax(const float *z, const float *x, float beta, uint32_t len,
                                       float *amax, int grid_cap, cudaStream_t s,
                                       const SymExpLinParams *symexp = nullptr);

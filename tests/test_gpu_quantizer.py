@@ -197,3 +197,61 @@ def test_long_tensors_in_interleaved_runs_bit_exact():
     torch.cuda.synchronize()
     for a, b in zip(got, want):
         assert torch.equal(a, b.view_as(a))
+
+
+@pytest.mark.parametrize("chunks,tail", [(1, 0), (0, 16), (1, 48), (1279, 2032), (1280, 16), (6143, 2032), (6144, 16)])
+def test_one_tensor_calls_equal_their_parts(chunks, tail):
+    """Maximum and encode of one tensor as a chain of launches, up to 1280 chunks of 2048 values (schedule-free pairs up to 6144,
+    with the transform all): the same bits as the maximum and the quantiser called one after the other."""
+    n = chunks * 2048 + tail
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    z, x = (torch.randn(n, device="cuda", generator=gen).mul_(0.02) for _ in range(2))
+    opt, q, beta = b2.OptimizerModule(), b2.Nvfp4QuantModule(), 0.7
+
+    def buffers():
+        return [torch.full((n // 2,), 255, dtype=torch.uint8, device="cuda"), torch.full((n // 16,), 255, dtype=torch.uint8, device="cuda"),
+                torch.full((1,), -1.0, device="cuda")], torch.full((1,), 7.0, device="cuda"), torch.full(((n + 2047) // 2048,), 7.0, device="cuda")
+
+    for source in ("master", "schedule", "transform"):
+        got, amax, chunk = buffers()
+        want, want_amax, want_chunk = buffers()
+        if source == "master":
+            opt.materialize_master(got[0], got[1], got[2], x, amax, chunk, n, b2.SCALES_RAW)
+            q.tensor_amax_f32(x, want_chunk, want_amax, n)
+            q.fp32_to_nvfp4_four_six(x, want_amax, *want, n // 16, b2.SCALES_RAW)
+            assert torch.equal(chunk, want_chunk)
+        else:
+            kw = dict(z_master=z, x_master=x, len=n, scale_rows=n // 16, scale_k=16, beta=beta, scale_layout=b2.SCALES_RAW,
+                      symexp_lin_beta=12.5 if source == "transform" else 0.0)
+            opt.materialize_schedule_free(bytes=got[0], scales=got[1], global_scale=got[2], amax=amax, **kw)
+            y = z + (x - z) * beta
+            if source == "schedule":
+                q.tensor_amax_f32(y, want_chunk, want_amax, n)
+            else:   # the maximum is checked below, value by value
+                want_amax.copy_(amax)
+            opt.materialize_schedule_free_precomputed(bytes=want[0], scales=want[1], global_scale=want[2], amax=want_amax,
+                                                      precomputed_values=y if source == "schedule" else None, **kw)
+        torch.cuda.synchronize()
+        assert torch.equal(amax, want_amax), source
+        for a, b in zip(got, want):
+            assert torch.equal(a, b), source
+
+
+@pytest.mark.parametrize("symexp", [12.5, 0.37, 1.0 / 3.0, 2.0 ** -20, 1.9999999])
+def test_transform_divides_as_the_division_does(symexp):
+    """Four values that are all far from the ends of the range are divided by multiplication with the reciprocal and two
+    remainder steps, correctly rounded; a zero among them sends the four to the division.  The maximum shows the value itself."""
+    rng = np.random.default_rng(11)
+    values = (np.exp(rng.uniform(np.log(1e-7), np.log(3.0 / max(symexp, 0.1)), 150)) * rng.choice([-1.0, 1.0], 150)).astype(F)
+    opt = b2.OptimizerModule()
+    t = b2.Nvfp4Tensor.empty(1, 16, b2.SCALES_RAW)
+    out = torch.zeros(2, len(values), device="cuda")
+    for i, v in enumerate(values):
+        for way, four in enumerate(([v, v, v, v], [v, v, v, 0.0])):
+            x = dev(np.array(four * 4, F))
+            opt.materialize_schedule_free(bytes=t.bytes, scales=t.scales, global_scale=t.global_scale, amax=out[way, i:i + 1], z_master=x,
+                                          x_master=x, len=16, scale_rows=1, scale_k=16, beta=0.5, scale_layout=b2.SCALES_RAW,
+                                          symexp_lin_beta=symexp)
+    torch.cuda.synchronize()
+    a, b = host(out)
+    assert np.array_equal(a, b) and len(np.unique(a)) > 100
