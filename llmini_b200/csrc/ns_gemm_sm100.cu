@@ -336,6 +336,28 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t *r) {
         : "r"(taddr)
         : "memory");
 }
+// 16 lanes x 64 consecutive 32-bit columns, in the layout of an MMA accumulator: thread i receives columns 8 j + 2 (i % 4) and
+// the next one of row i / 4 in r[4 j], r[4 j + 1], those of row 8 + i / 4 in r[4 j + 2], r[4 j + 3].
+__device__ __forceinline__ void tc_ld_16x64(uint32_t taddr, uint32_t *r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+// Four words of each of four neighbouring lanes, transposed: word k of lane s becomes word s of lane k.
+__device__ __forceinline__ void quad_transpose(uint32_t &w0, uint32_t &w1, uint32_t &w2, uint32_t &w3, uint32_t lane) {
+    const bool odd = lane & 1u, high = lane & 2u;
+    const uint32_t p = __shfl_xor_sync(0xffffffffu, odd ? w0 : w1, 1), r = __shfl_xor_sync(0xffffffffu, odd ? w2 : w3, 1);
+    if (odd) { w0 = p; w2 = r; } else { w1 = p; w3 = r; }
+    const uint32_t t = __shfl_xor_sync(0xffffffffu, high ? w0 : w2, 2), u = __shfl_xor_sync(0xffffffffu, high ? w1 : w3, 2);
+    if (high) { w0 = t; w1 = u; } else { w2 = t; w3 = u; }
+}
 // 32 bytes, one sector, to a 32-byte aligned address
 __device__ __forceinline__ void st_global_32(void *p, const uint32_t *v) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
@@ -940,22 +962,30 @@ k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ til
 // What TMA fills in beyond the matrix is zero and stays zero, so that MMAs, whose K goes in steps of 16, need no bound.  It
 // stays zero by itself while everything is finite.  RAGGED, for plans with a row count that is no multiple of 16 (columns
 // always are): what an MMA may read again is cleared, because 0 times an infinity is not 0; a template parameter because the
-// code for it costs the others 3 % (64 x 64: 18.1 -> 18.6 us).  Rounding points, operand values and the order of every sum
-// are those of k_ns_gemm.
-constexpr int kSmallThreads = 256;
+// code for it costs the others 3 %.  Rounding points, operand values and the order of every sum are those of k_ns_gemm.
+// What bounds it: the chain of a phase.  For 64 x 64 that is 330 clocks of MMAs and their barrier, 210 to 360 of reading,
+// converting and storing 32 columns a warp, 220 of proxy fence and block barrier, and 100 to 500 between them; up to
+// 128 x 512 the MMAs (64 clocks each) and the conversion of 128 x 128 blocks (600 clocks).  So nothing is done for padding
+// (units of 32 x 32 that lie beyond G and Q are neither computed nor stored), a warp of its own issues, the inner product of
+// the polynomial is formed while its MMAs run, the blocks of Apply have a barrier each, and what memory keeps of G, Q and the
+// operands leaves as bulk copies.  Newton-Schulz loop, before and after: 64 x 64 34800 -> 21600 clocks, 128 x 128 49900 ->
+// 31600, 128 x 512 103600 -> 61000; whole steps: 64-wide fixture 32.8 -> 24.5 us, one layer of width 128 70.7 -> 46.1, twelve
+// 86.8 -> 63.5.  (In twelve layers the larger dimension is 512 and a matrix has one SM to itself.)
+constexpr int kSmallWarps = 8;                       // of the epilogue; one more issues MMAs and copies
+constexpr int kSmallThreads = 32 * (kSmallWarps + 1);
 constexpr uint32_t kSmallPanel = 128 * 128;   // bytes: 128 rows x 64 16-bit values
 constexpr uint32_t kSmallTmemCols = 512;
+constexpr uint32_t kSmallBlocks = 4;          // of 128 columns of tensor memory: a result of up to 128 x 512
 
 struct SmallLoop {
     uint32_t iterations;
-    int f16;
     int last16;           // the last result leaves in the operand type (into the operand buffer that is its turn)
     GemmCoefficients coef;
 };
 
 __device__ __forceinline__ uint32_t small_swizzled(uint32_t row, uint32_t chunk) { return row * 128u + ((chunk ^ (row & 7u)) << 4); }
 
-template <bool RAGGED>
+template <bool RAGGED, int F16>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__ poly, const GemmProblem *__restrict__ apply0,
            const GemmProblem *__restrict__ apply1, const GemmProblem *__restrict__ last, SmallLoop loop,
@@ -963,24 +993,34 @@ k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *g_panels = smem, *q_panels = smem + 2 * kSmallPanel, *x_panels = smem + 4 * kSmallPanel;
-    __shared__ uint64_t bars[2];              // operand loaded; MMAs of a phase retired
+    __shared__ uint64_t bars[2 + kSmallBlocks];   // operand loaded; MMAs of Gram or Poly retired; those of a block of Apply
     __shared__ uint32_t tmem_slot, abort_word;
+    __shared__ float coef[3 * kMaxChainIterations];
     volatile uint32_t *abort_flag = &abort_word;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t slot = blockIdx.x;
-    const uint32_t load_bar = smem_u32(bars), mma_bar = load_bar + 8;
+    const uint32_t load_bar = smem_u32(bars), mma_bar = load_bar + 8, block_bar = load_bar + 16;
     const GemmProblem *ap = apply0 + slot;
     const uint32_t rows = ap->M, cols = ap->N;   // of the storage layout
     const bool empty = rows == 0u;
     const bool tall = gram[slot].a_mn_major != 0u;
+    const bool issuer = warp == kSmallWarps;
     const uint32_t n = tall ? cols : rows;
+    // maps of 64 x 128 boxes, and results in memory: they belong to the plan.  (The second operand buffer's problems follow the
+    // first one's, a matrix per CTA.)
+    const uint64_t x0_map = tall ? ap->map_a : gram[slot].map_a, x1_map = tall ? apply1[slot].map_a : gram[gridDim.x + slot].map_a;
+    const uint64_t g_map = poly[slot].map_a, q_map = tall ? ap->map_b : ap->map_a;
+    uint8_t *out32 = reinterpret_cast<uint8_t *>(last[slot].out32);
     const uint32_t panels = tall ? 2u : (cols + 63u) / 64u, blocks = tall ? (rows + 127u) / 128u : 1u;
 
     if (threadIdx.x == 0) {
         mbar_init(load_bar, 1);
         mbar_init(mma_bar, 1);
+        for (uint32_t j = 0; j < kSmallBlocks; ++j) mbar_init(block_bar + 8u * j, 1);
         abort_word = 0;
         fence_async_smem();
+#pragma unroll
+        for (uint32_t i = 0; i < 3 * kMaxChainIterations; ++i) coef[i] = loop.coef.v[i];
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(kSmallTmemCols)
@@ -995,32 +1035,40 @@ k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     if (!empty) {
-        if (threadIdx.x == 0) {
-            const uint64_t map = tall ? ap->map_a : gram[slot].map_a;   // 64 x 128 boxes of the first operand buffer
+        if (threadIdx.x == 32 * kSmallWarps) {
             mbar_expect_tx(load_bar, panels * blocks * kSmallPanel);
             for (uint32_t p = 0; p < panels; ++p)
                 for (uint32_t j = 0; j < blocks; ++j)
-                    tma_load_2d<false>(smem_u32(x_panels) + (p * blocks + j) * kSmallPanel, map, load_bar, (int)(64 * p), (int)(128 * j));
+                    tma_load_2d<false>(smem_u32(x_panels) + (p * blocks + j) * kSmallPanel, x0_map, load_bar, (int)(64 * p), (int)(128 * j));
         }
         const float slot_s = slot_scale != nullptr ? __ldcg(slot_scale + slot) : 1.0f;
-        const int f16 = loop.f16;
-        const uint32_t q = warp & 3, half = warp >> 2;
+        const uint32_t q = warp & 3, half = (warp >> 2) & 1;
         const uint32_t row = 32 * q + lane;                          // TMEM lane
         const uint32_t lane_base = tmem + ((32u * q) << 16);
-        const uint32_t g_addr = smem_u32(g_panels), q_addr = smem_u32(q_panels), x_addr = smem_u32(x_panels);
         const uint32_t k16_n = (n + 15u) / 16u;                       // steps of 16 over the smaller dimension
-        uint32_t phase = 0;
+        // What there is of G and Q in units of 32 x 32: a warp whose 32 rows lie beyond it only waits, and the two warps of a
+        // lane quarter take its units in turn.
+        const uint32_t units_n = (n + 31u) / 32u;
+        const bool active = !issuer && q < units_n;
+        const uint64_t g_desc = smem_desc(smem_u32(g_panels), 16, 1024), q_desc = smem_desc(smem_u32(q_panels), 16, 1024);
+        const uint64_t x_k_desc = smem_desc(smem_u32(x_panels), 16, 1024);                                           // read along a row
+        const uint64_t x_mn_desc = smem_desc(smem_u32(x_panels), (tall ? blocks : 1u) * kSmallPanel, 1024);          // read across rows
+        constexpr uint32_t kPanel16 = kSmallPanel >> 4;                // a panel in the descriptors' units of 16 bytes
+        auto k_step = [](uint32_t k) { return (k >> 2) * kPanel16 + (k & 3u) * 2u; };   // 16 columns along 64-column panels
+        // What a plan keeps in memory of G, Q and the operands leaves as bulk copies of the panels, beside the MMAs.  (Stored by the
+        // epilogue, a row per lane, they were a quarter of the time of a 128 x 512 matrix.)
+        auto store_panels = [&](uint64_t map, uint32_t smem_addr, uint32_t count, uint32_t rows128) {
+            for (uint32_t p = 0; p < count; ++p)
+                for (uint32_t j = 0; j < rows128; ++j)
+                    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"((int)(64 * p)),
+                                 "r"((int)(128 * j)), "r"(smem_addr + (p * rows128 + j) * kSmallPanel)
+                                 : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        };
         (void)mbar_wait(load_bar, 0, abort_flag);   // on expiry the flag ends the loop at its next barrier
-        // MMAs of a phase by one thread of warp 0, then everybody waits for them
-        auto run = [&](auto &&issue) {
-            if (warp == 0 && elect_one()) {
-                tc_fence_after();
-                issue();
-                tc_commit<false>(mma_bar);
-            }
+        auto wait_mma = [&](uint32_t bar, uint32_t parity) {
             __syncwarp();
-            (void)mbar_wait(mma_bar, phase, abort_flag);
-            phase ^= 1u;
+            (void)mbar_wait(bar, parity, abort_flag);
             tc_fence_after();
         };
         // what this thread stored to shared memory is visible to the next phase's MMAs, and its TMEM reads are done
@@ -1029,151 +1077,209 @@ k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__
             tc_fence_before();
             __syncthreads();
         };
-        __syncthreads();
-        // coefficients without indexing the argument block by a register
-        for (uint32_t it = 0; it < loop.iterations; ++it) {
-            float ca = loop.coef.v[0], cb = loop.coef.v[1], cc = loop.coef.v[2];
-#pragma unroll
-            for (uint32_t i = 1; i < kMaxChainIterations; ++i)
-                if (it == i) { ca = loop.coef.v[3 * i]; cb = loop.coef.v[3 * i + 1]; cc = loop.coef.v[3 * i + 2]; }
-            const bool final = it + 1 == loop.iterations;
-            const float s1 = it == 0 ? slot_s : 1.0f, s2 = s1 * s1;
-            // ---- Gram: columns 0 .. 127 of tensor memory
-            run([&] {
-                const uint32_t idesc = instr_desc(128, 128, f16, tall ? 1u : 0u, tall ? 1u : 0u);
-                if (tall) {
-                    const uint32_t steps = (rows + 15u) / 16u;
-                    for (uint32_t k = 0; k < steps; ++k) {
-                        const uint64_t d = smem_desc(x_addr + k * 2048u, blocks * kSmallPanel, 1024);
-                        tc_mma<false>(tmem, d, d, idesc, k != 0);
-                    }
-                } else {
-                    const uint32_t steps = (cols + 15u) / 16u;
-                    for (uint32_t k = 0; k < steps; ++k) {
-                        const uint64_t d = smem_desc(x_addr + (k >> 2) * kSmallPanel + (k & 3u) * 32u, 16, 1024);
-                        tc_mma<false>(tmem, d, d, idesc, k != 0);
-                    }
-                }
-            });
-            // each warp takes 64 columns of its 32 rows: one panel of G (and of Q)
-            uint8_t *g_out = reinterpret_cast<uint8_t *>(gram[slot].out16), *q_out = reinterpret_cast<uint8_t *>(poly[slot].out16);
-            const uint32_t pitch = gram[slot].pitch16;
-            auto clear_columns = [&](uint32_t col, uint32_t *v) {   // those from n on, of 32 from `col`
-                if (!RAGGED || (n & 15u) == 0u || col + 32u <= n) return;
+        auto pack8 = [&](const uint32_t *v) {
+            uint4 w;
+            w.x = pack_operands(__uint_as_float(v[0]), __uint_as_float(v[1]), F16);
+            w.y = pack_operands(__uint_as_float(v[2]), __uint_as_float(v[3]), F16);
+            w.z = pack_operands(__uint_as_float(v[4]), __uint_as_float(v[5]), F16);
+            w.w = pack_operands(__uint_as_float(v[6]), __uint_as_float(v[7]), F16);
+            return w;
+        };
+        auto clear_columns = [&](uint32_t col, uint32_t *v) {   // those from n on, of 32 from `col`
+            if (RAGGED && (n & 15u) != 0u && col + 32u > n) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j)
                     if (col + j >= n) v[j] = 0u;
-            };
-            auto store_nn = [&](uint8_t *panel0, uint8_t *global, uint32_t col, const uint32_t *v) {   // 32 columns from `col`
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint4 w;
-                    w.x = pack_operands(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]), f16);
-                    w.y = pack_operands(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]), f16);
-                    w.z = pack_operands(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]), f16);
-                    w.w = pack_operands(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]), f16);
-                    const uint32_t c = col + 8 * j;
-                    *reinterpret_cast<uint4 *>(panel0 + (c >> 6) * kSmallPanel + small_swizzled(row, (c & 63u) >> 3)) = w;
-                    if (final && row < n && c < pitch) *reinterpret_cast<uint4 *>(global + ((size_t)row * pitch + c) * 2) = w;
-                }
-            };
-#pragma unroll 1
-            for (uint32_t sub = 0; sub < 2; ++sub) {
-                const uint32_t col = 64 * half + 32 * sub;
-                uint32_t v[32];
-                tc_ld32(lane_base + col, v);
-                tc_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * s2);
-                clear_columns(col, v);
-                store_nn(g_panels, g_out, col, v);
             }
-            hand_over();
-            // ---- Poly: columns 128 .. 255; the Gram accumulator stays where it is
-            run([&] {
-                const uint32_t idesc = instr_desc(128, 128, f16, 0u, 0u);
-                for (uint32_t k = 0; k < k16_n; ++k) {
-                    const uint64_t d = smem_desc(g_addr + (k >> 2) * kSmallPanel + (k & 3u) * 32u, 16, 1024);
-                    tc_mma<false>(tmem + 128u, d, d, idesc, k != 0);
-                }
-            });
-#pragma unroll 1
-            for (uint32_t sub = 0; sub < 2; ++sub) {
-                const uint32_t col = 64 * half + 32 * sub;
-                uint32_t v[32], h[32];
-                tc_ld32(lane_base + 128u + col, v);
-                tc_ld32(lane_base + col, h);
-                tc_ld_wait();
+        };
+        // byte offsets of this thread's row in a panel, for the four 16-byte pieces of a unit's 64 bytes
+        uint32_t piece[2][4];
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    // rows and columns beyond the matrix stay zero
-                    const float ident = (col + j == row && row < n) ? ca : 0.0f;
-                    // store/plain.rs:175-178: fma(c, acc, fma(b, base, identity))
-                    v[j] = __float_as_uint(fmaf(cc, __uint_as_float(v[j]), fmaf(cb, __uint_as_float(h[j]) * s2, ident)));
-                }
-                clear_columns(col, v);
-                store_nn(q_panels, q_out, col, v);
-            }
-            hand_over();
-            // ---- Apply: one 128 x 128 block of the result per 128 columns of tensor memory
-            run([&] {
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) piece[u][j] = small_swizzled(row, (uint32_t)(4 * u + j));
+        auto store_unit = [&](uint8_t *panel, uint32_t unit, const uint4 *w) {   // into the panel that holds 32-column unit `unit`
+#pragma unroll
+            for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4 *>(panel + ((unit & 1u) ? piece[1][j] : piece[0][j])) = w[j];
+        };
+        __syncthreads();
+        for (uint32_t it = 0; it < loop.iterations; ++it) {
+            const float ca = coef[3 * it], cb = coef[3 * it + 1], cc = coef[3 * it + 2];
+            const bool final = it + 1 == loop.iterations;
+            const bool scaled = it == 0 && slot_s != 1.0f;
+            const float s1 = slot_s, s2 = s1 * s1;
+            auto store_nn = [&](uint8_t *panels0, uint32_t unit, const uint32_t *v) {
+                uint4 w[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) w[j] = pack8(v + 8 * j);
+                store_unit(panels0 + (unit >> 1) * kSmallPanel, unit, w);
+            };
+            // ---- Gram: columns 0 .. 127 of tensor memory
+            if (issuer && elect_one()) {
+                tc_fence_after();
+                // (read across rows, N is made of whole 64-column swizzle atoms)
+                const uint32_t idesc = instr_desc(128, (int)(tall ? (n + 63u) / 64u * 64u : 32 * units_n), F16, tall ? 1u : 0u, tall ? 1u : 0u);
                 if (tall) {
-                    const uint32_t idesc = instr_desc(128, 128, f16, 0u, 0u);
-                    for (uint32_t j = 0; j < blocks; ++j)
+                    const uint32_t steps = (rows + 15u) / 16u;
+                    for (uint32_t k = 0; k < steps; ++k) tc_mma<false>(tmem, x_mn_desc + 128u * k, x_mn_desc + 128u * k, idesc, k != 0);
+                } else {
+                    const uint32_t steps = (cols + 15u) / 16u;
+                    for (uint32_t k = 0; k < steps; ++k) tc_mma<false>(tmem, x_k_desc + k_step(k), x_k_desc + k_step(k), idesc, k != 0);
+                }
+                tc_commit<false>(mma_bar);
+            }
+            uint32_t base[2][32];   // the Gram accumulator, which the polynomial starts from
+            if (!issuer) wait_mma(mma_bar, 0);
+            if (active) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t unit = half + 2 * u;
+                    if (unit >= units_n) break;   // warp-uniform
+                    tc_ld32(lane_base + 32 * unit, base[u]);
+                    tc_ld_wait();
+                    if (scaled) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) base[u][j] = __float_as_uint(__uint_as_float(base[u][j]) * s2);
+                    }
+                    uint32_t v[32];
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = base[u][j];
+                    clear_columns(32 * unit, v);
+                    store_nn(g_panels, unit, v);
+                }
+            }
+            hand_over();
+            // ---- Poly: columns 128 .. 255
+            if (issuer && elect_one()) {
+                tc_fence_after();
+                const uint32_t idesc = instr_desc(128, (int)(32 * units_n), F16, 0u, 0u);
+                for (uint32_t k = 0; k < k16_n; ++k) tc_mma<false>(tmem + 128u, g_desc + k_step(k), g_desc + k_step(k), idesc, k != 0);
+                tc_commit<false>(mma_bar);
+                if (final) store_panels(g_map, smem_u32(g_panels), (n + 63u) / 64u, 1u);
+            }
+            if (active) {   // store/plain.rs:175-178: fma(c, acc, fma(b, base, identity)): the inner one while the MMAs run
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t unit = half + 2 * u;
+                    if (unit >= units_n) break;
+                    if (unit == q) {   // on the diagonal; rows and columns beyond the matrix stay zero
+                        const float a = row < n ? ca : 0.0f;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) base[u][j] = __float_as_uint(fmaf(cb, __uint_as_float(base[u][j]), j == lane ? a : 0.0f));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) base[u][j] = __float_as_uint(fmaf(cb, __uint_as_float(base[u][j]), 0.0f));
+                    }
+                }
+            }
+            if (!issuer) wait_mma(mma_bar, 1);   // (two completions per iteration)
+            if (active) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t unit = half + 2 * u;
+                    if (unit >= units_n) break;
+                    uint32_t v[32];
+                    tc_ld32(lane_base + 128u + 32 * unit, v);
+                    tc_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(fmaf(cc, __uint_as_float(v[j]), __uint_as_float(base[u][j])));
+                    clear_columns(32 * unit, v);
+                    store_nn(q_panels, unit, v);
+                }
+            }
+            hand_over();
+            // ---- Apply: a block of 128 columns of tensor memory is 128 x 128 of the result, with a barrier of its own, so that
+            // the first ones are converted while the MMAs of the others run.  A block's result goes where only its own MMAs
+            // have read: the same panels (wide), the same rows (tall).
+            if (issuer && elect_one()) {
+                tc_fence_after();
+                // the copies of the panels that this phase overwrites have been read
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                if (tall) {
+                    const uint32_t idesc = instr_desc(128, (int)(32 * units_n), F16, 0u, 0u);
+                    for (uint32_t j = 0; j < blocks; ++j) {
                         for (uint32_t k = 0; k < k16_n; ++k)
-                            tc_mma<false>(tmem + 128u * j,
-                                          smem_desc(x_addr + ((k >> 2) * blocks + j) * kSmallPanel + (k & 3u) * 32u, 16, 1024),
-                                          smem_desc(q_addr + (k >> 2) * kSmallPanel + (k & 3u) * 32u, 16, 1024), idesc, k != 0);
+                            tc_mma<false>(tmem + 128u * j, x_k_desc + ((k >> 2) * blocks + j) * kPanel16 + (k & 3u) * 2u, q_desc + k_step(k),
+                                          idesc, k != 0);
+                        tc_commit<false>(block_bar + 8u * j);
+                    }
                 } else {
                     for (uint32_t p = 0; p < panels; p += 2) {
-                        const uint32_t idesc = instr_desc(128, p + 1 < panels ? 128 : 64, f16, 0u, 1u);
+                        const uint32_t idesc = instr_desc(128, p + 1 < panels ? 128 : 64, F16, 0u, 1u);
                         for (uint32_t k = 0; k < k16_n; ++k)
-                            tc_mma<false>(tmem + 64u * p, smem_desc(q_addr + (k >> 2) * kSmallPanel + (k & 3u) * 32u, 16, 1024),
-                                          smem_desc(x_addr + p * kSmallPanel + k * 2048u, kSmallPanel, 1024), idesc, k != 0);
+                            tc_mma<false>(tmem + 64u * p, q_desc + k_step(k), x_mn_desc + p * kPanel16 + 128u * k, idesc, k != 0);
+                        tc_commit<false>(block_bar + 4u * p);
                     }
                 }
-            });
-            const uint32_t columns = tall ? 128u * blocks : 64u * panels;
-            const bool out32 = final && !loop.last16;
-            uint8_t *out = reinterpret_cast<uint8_t *>(out32 ? last[slot].out32 : ((it & 1u) ? apply1 + slot : ap)->out16);
-            // the operand buffers in memory hold the last three operands of the loop, as with a launch per phase
-            const bool to_global = it + 3 >= loop.iterations;
+                if (final) store_panels(q_map, smem_u32(q_panels), (n + 63u) / 64u, 1u);
+            }
+            const bool fp32 = final && !loop.last16;
+            const uint32_t result_blocks = issuer ? 0u : tall ? blocks : (panels + 1) / 2;
 #pragma unroll 1
-            for (uint32_t t = 32 * half; t < columns; t += 64) {
-                uint32_t v[32];
-                tc_ld32(lane_base + t, v);
-                tc_ld_wait();
-                const uint32_t c0 = tall ? (t & 127u) : t, r = tall ? (t >> 7) * 128u + row : row;
+            for (uint32_t j = 0; j < result_blocks; ++j) {
+                wait_mma(block_bar + 8u * j, it & 1u);
+                const uint32_t r = tall ? 128 * j + row : row, units = tall ? units_n : min(4u, (cols - 128 * j + 31u) / 32u);
+                if (32 * q + (tall ? 128 * j : 0u) >= rows) continue;   // warp-uniform
+                if (fp32) {
+                    // 16 rows x 64 columns at a time; the four lanes of a row exchange pairs until each holds 32 bytes in a row, so
+                    // that a store writes whole 128-byte lines (128 x 128: 2800 clocks, 4600 with a row per lane)
+                    const uint32_t r0 = (tall ? 128 * j : 0u) + 32 * q + 16 * half + (lane >> 2);
+#pragma unroll 1
+                    for (uint32_t c = 0; c < units; c += 2) {
+                        uint32_t v[32];
+                        tc_ld_16x64(lane_base + ((16u * half) << 16) + 128 * j + 32 * c, v);
+                        tc_ld_wait();
+                        if (scaled) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * s1);
-                if (RAGGED && r >= rows) {
+                            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * s1);
+                        }
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = 0u;
-                }
-                if (out32) {
+                        for (int h = 0; h < 2; ++h) {       // rows r0 and r0 + 8
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (r < rows && c0 + 4 * j < cols)
-                            *reinterpret_cast<uint4 *>(out + ((size_t)r * cols + c0 + 4 * j) * 4) =
-                                make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                } else {
-                    uint8_t *panel0 = x_panels + (tall ? (t >> 7) * kSmallPanel : 0u);
+                            for (int g = 0; g < 2; ++g) {   // 32 columns each
+                                uint32_t a[4], b[4], w[8];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint4 w;
-                        w.x = pack_operands(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]), f16);
-                        w.y = pack_operands(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]), f16);
-                        w.z = pack_operands(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]), f16);
-                        w.w = pack_operands(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]), f16);
-                        const uint32_t c = c0 + 8 * j;
-                        *reinterpret_cast<uint4 *>(panel0 + (c >> 6) * blocks * kSmallPanel + small_swizzled(row, (c & 63u) >> 3)) = w;
-                        if (to_global && r < rows && c < cols) *reinterpret_cast<uint4 *>(out + ((size_t)r * cols + c) * 2) = w;
+                                for (int k = 0; k < 4; ++k) {
+                                    a[k] = v[16 * g + 4 * k + 2 * h];
+                                    b[k] = v[16 * g + 4 * k + 2 * h + 1];
+                                }
+                                quad_transpose(a[0], a[1], a[2], a[3], lane);
+                                quad_transpose(b[0], b[1], b[2], b[3], lane);
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) { w[2 * k] = a[k]; w[2 * k + 1] = b[k]; }
+                                const uint32_t r = r0 + 8 * h, col = (tall ? 0u : 128 * j) + 32 * (c + g) + 8 * (lane & 3);
+                                if (r < rows && col < cols) st_global_32(out32 + ((size_t)r * cols + col) * 4, w);
+                            }
+                        }
                     }
+                    continue;
+                }
+#pragma unroll 1
+                for (uint32_t unit = half; unit < units; unit += 2) {
+                    uint32_t v[32];
+                    tc_ld32(lane_base + 128 * j + 32 * unit, v);
+                    tc_ld_wait();
+                    if (scaled) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * s1);
+                    }
+                    if (RAGGED && r >= rows) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = 0u;
+                    }
+                    uint4 w[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) w[i] = pack8(v + 8 * i);
+                    store_unit(x_panels + (tall ? (unit >> 1) * blocks + j : 2 * j + (unit >> 1)) * kSmallPanel, unit, w);
                 }
             }
             hand_over();
             if (*abort_flag) break;   // a wait ran out: written before the barrier, so every thread sees it
+            // the operand buffers in memory hold the last three operands of the loop, as with a launch per phase
+            if (issuer && !fp32 && it + 3 >= loop.iterations && elect_one())
+                store_panels((it & 1u) ? x0_map : x1_map, smem_u32(x_panels), tall ? (n + 63u) / 64u : panels, blocks);
         }
+        if (issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         if (*abort_flag) {
             // copies or MMAs may still be in flight: give them time to land before the memory is released
             for (int i = 0; i < 4096; ++i) __nanosleep(512);
@@ -1328,9 +1434,10 @@ uint32_t ns_small_smem(uint32_t rows, uint32_t cols) {
 }
 // The limit belongs to the function, not to a plan: it is always the largest, so that no plan takes it from another.
 cudaError_t ns_small_configure() {
-    const cudaError_t e = cudaFuncSetAttribute(k_ns_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_ns_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
+    cudaError_t e = cudaSuccess;
+    for (auto *kernel : {k_ns_small<false, 0>, k_ns_small<false, 1>, k_ns_small<true, 0>, k_ns_small<true, 1>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
+    return e;
 }
 cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, const GemmProblem *apply0, const GemmProblem *apply1,
                             const GemmProblem *last, uint32_t slot_count, uint32_t iterations, int f16, int last16,
@@ -1346,8 +1453,9 @@ cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, co
     cfg.blockDim = dim3(kSmallThreads, 1, 1);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = s;
-    SmallLoop loop = {iterations, f16, last16, coef};
-    return cudaLaunchKernelEx(&cfg, ragged ? k_ns_small<true> : k_ns_small<false>, gram, poly, apply0, apply1, last, loop, slot_scale, status);
+    SmallLoop loop = {iterations, last16, coef};
+    auto *kernel = ragged ? (f16 ? k_ns_small<true, 1> : k_ns_small<true, 0>) : (f16 ? k_ns_small<false, 1> : k_ns_small<false, 0>);
+    return cudaLaunchKernelEx(&cfg, kernel, gram, poly, apply0, apply1, last, loop, slot_scale, status);
 }
 size_t chain_sync_bytes(uint32_t slot_count) { return sizeof(ChainSync) + sizeof(uint32_t) * slot_count; }
 namespace {

@@ -196,6 +196,29 @@ def test_one_cta_loop_equals_the_per_phase_launches_bit_for_bit(fmt, iterations,
             assert np.array_equal(u, v), (shape, w, float(np.abs(u - v).max()))
 
 
+@pytest.mark.parametrize("fmt,update16", [(b2.OPERAND_BF16, False), (b2.OPERAND_F16, True)])
+def test_one_cta_loop_at_the_edges_of_its_units(fmt, update16):
+    """G and Q in units of 32 x 32, results in blocks of 128: one and two units, three, a row beyond, a last block of 16."""
+    shapes = [(32, 32), (33, 64), (96, 96), (31, 160), (257, 112), (400, 32), (48, 384), (64, 272), (112, 512), (512, 96)]
+    rng = np.random.default_rng(4)
+    xs = [_x0(rng, r, c, fmt) for r, c in shapes]
+    results = []
+    for tile_n in (0, 128):
+        plan = b2.MuonPlan(shapes, operand_format=fmt, scale_layout=b2.SCALES_RAW, tile_n=tile_n, max_iterations=4,
+                           update_input=b2.UPDATE_16BIT if update16 else b2.UPDATE_F32)
+        for i, x in enumerate(xs):
+            plan.scratch(i, 0).copy_(dev(x).to(plan.scratch(i, 0).dtype))
+        b2.OptimizerModule().muon_polar(plan, b2.MuonMegaUpdateArgs(iterations=4, coefficients=o.fixed_coefficients(4)))
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        results.append([[host(plan.scratch(i, w).float()).copy() for w in ((0, 5, 6, 7) if update16 else (1, 5, 6, 7))] for i in range(len(shapes))])
+        plan.close()
+    for shape, a, b in zip(shapes, *results):
+        for u, v in zip(a, b):
+            assert np.array_equal(u, v), shape
+
+
+
 @pytest.mark.parametrize("fmt", [b2.OPERAND_BF16, b2.OPERAND_F16])
 @pytest.mark.parametrize("kind", ["nan", "inf", "overflow"])
 def test_one_cta_loop_treats_non_finite_values_as_the_per_phase_launches_do(kind, fmt):
