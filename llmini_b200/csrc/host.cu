@@ -54,9 +54,9 @@ size_t b2_csf_encode_host(const uint8_t *raw, size_t raw_len, size_t rows, size_
         return n;
     }
     // csf.rs:51-95 (encode_matrix)
-    int bytes = 1;
-    for (size_t i = 0; i < raw_len; ++i)
-        if (raw[i] >= 128) { bytes = 2; break; }
+    uint8_t all = 0;
+    for (size_t i = 0; i < raw_len; ++i) all |= raw[i];
+    const int bytes = all >= 128 ? 2 : 1;
     const size_t stride = 768 + 128 * (size_t)bytes;
     const size_t padded = (rows + 127) / 128 * 128;
     const size_t n = 128 + padded / 128 * (k / 128) * stride;
@@ -66,6 +66,7 @@ size_t b2_csf_encode_host(const uint8_t *raw, size_t raw_len, size_t rows, size_
     put_u32(out + 4, (uint32_t)rows);
     out[8] = (uint8_t)__builtin_ctzll(k / 16);
     out[9] = (uint8_t)(6 + bytes);
+    if (all == 0) return n;   // storage for a kernel to fill: 50304 x 768 in 0.4 ms instead of 4 to 5
     const size_t groups = k / 16;
     for (size_t row = 0; row < rows; ++row) {
         for (size_t kg = 0; kg < groups; kg += 8) {
