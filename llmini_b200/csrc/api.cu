@@ -448,6 +448,8 @@ struct b2_muon_plan {
         NeuronView nv;
         nv.unit_prefix = at<uint32_t>(layout.off_unit_prefix);
         nv.total_units = layout.unit_prefix.back();
+        nv.columns = false;
+        for (const SlotLayout &sl : layout.slots) nv.columns = nv.columns || (sl.len != 0 && sl.rows < sl.cols);
         nv.factor_ptrs = at<uint64_t>(layout.off_factor_ptrs);
         nv.partials = at<double>(layout.off_unit_partials);
         nv.slot_stats = at<float>(layout.off_slot_stats);

@@ -31,6 +31,7 @@ struct MomentumParams {
 struct NeuronView {
     const uint32_t *unit_prefix;   // device, slot_count + 1 entries
     uint32_t total_units;
+    bool columns;                  // some slot's neurons are its columns
     const uint64_t *factor_ptrs;   // device, per slot: f32[max(rows, cols)] factors
     double *partials;              // device, 4 per unit: raw, scaled, parameter, dot
     float *slot_stats;             // device, 4 per slot: normuon_scale, update_norm, radius, dot

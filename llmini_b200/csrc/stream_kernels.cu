@@ -470,10 +470,8 @@ k_muon_update(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint
 // each with a shorter chain of round trips; wide ones read longer pieces of a row.  NorMuon finish with 32 / 64 / 128 columns
 // (us): ragged plan of 5 matrices 24.9 / 25.8 / 28.9, one 768 x 3072 18.8 / 20.5 / 22.8, GPT-2 medium 1523 / 1494 / 1478.
 template <int COLS>
-__global__ void __launch_bounds__(kThreads, COLS ? 2 : 4)
-k_normuon_stats(const b2_muon_slot_descriptor *slots, uint32_t slot_count, NeuronView nv, const uint64_t *u_ptrs,
-                int hyperball) {
-    stream_enter();
+__device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slots, uint32_t slot_count, const NeuronView &nv,
+                                              const uint64_t *u_ptrs, int hyperball) {
     constexpr uint32_t kUnitCols = COLS ? B2_NORMUON_COLS_PER_UNIT : 4, kQuads = kUnitCols / 4, kRowLanes = kThreads / kQuads;
     __shared__ float col_raw[COLS ? kRowLanes : 1][kUnitCols], col_dot[COLS ? kRowLanes : 1][kUnitCols];
     __shared__ double part[kThreads / 32][4];
@@ -605,6 +603,21 @@ k_normuon_stats(const b2_muon_slot_descriptor *slots, uint32_t slot_count, Neuro
         }
         __syncthreads();
     }
+}
+
+// The two forms write to different slots, so they run side by side.  The columns' launch, behind the rows', reads at once: the
+// rows' does not begin before the Newton-Schulz result is complete (it is a plain launch), nor the columns' before the rows'.
+// It waits for the rows' at its end, so that what comes behind it finds both done.
+__global__ void __launch_bounds__(kThreads, 4)
+k_normuon_stats_rows(const b2_muon_slot_descriptor *slots, uint32_t slot_count, NeuronView nv, const uint64_t *u_ptrs, int hyperball) {
+    stream_enter();
+    normuon_stats<0>(slots, slot_count, nv, u_ptrs, hyperball);
+}
+__global__ void __launch_bounds__(kThreads, 2)
+k_normuon_stats_columns(const b2_muon_slot_descriptor *slots, uint32_t slot_count, NeuronView nv, const uint64_t *u_ptrs, int hyperball) {
+    chain_begin();
+    normuon_stats<1>(slots, slot_count, nv, u_ptrs, hyperball);
+    chain_wait();
 }
 
 // One CTA per slot: fixed-order sums of the unit partials, then the four slot scalars
@@ -1005,11 +1018,8 @@ template <int MODE, uint32_t RUN, typename F>
 __device__ __forceinline__ void encode_pipeline(uint32_t total_chunks, float beta, const SymExpLin sx, F target_of) {
     const uint32_t per = total_chunks / gridDim.x, rem = total_chunks % gridDim.x;
     const bool runs = RUN != 0 && per >= 4 * RUN;
-    // Runs are taken from the last one on, because some of what the pass in front has read last is still in L2 (maximum and
-    // encode: 16384 x 4096 101.5 -> 98.1 us, 65536 x 4096 387 -> 383).
-    uint32_t run = runs ? (total_chunks + RUN - 1) / RUN - blockIdx.x : 0u;   // one more than its index
-    uint32_t c = runs ? (run - 1) * RUN : blockIdx.x * per + min(blockIdx.x, rem);
-    uint32_t end = runs ? min(c + RUN, total_chunks) : c + per + (blockIdx.x < rem ? 1u : 0u);
+    uint32_t c = runs ? blockIdx.x * RUN : blockIdx.x * per + min(blockIdx.x, rem);
+    uint32_t end = runs ? c + RUN : c + per + (blockIdx.x < rem ? 1u : 0u);
     EncodeRaw<MODE> ra, rb;
     while (c < end) {
         EncodeTarget t = target_of(c);
@@ -1017,10 +1027,9 @@ __device__ __forceinline__ void encode_pipeline(uint32_t total_chunks, float bet
         const uint32_t left = (t.len - t.base + kChunk - 1) / kChunk;
         uint32_t n = max(min(left, end - c), 1u);   // never stands still, whatever the table says
         c += n;
-        if (RUN != 0 && runs && c == end && run > gridDim.x) {   // on to the next run
-            run -= gridDim.x;
-            c = (run - 1) * RUN;
-            end = c + RUN;
+        if (RUN != 0 && runs && c == end) {         // on to the next run
+            c += (gridDim.x - 1) * RUN;
+            end = min(c + RUN, total_chunks);
         }
         if (t.skip) continue;
         if (t.base == 0 && threadIdx.x == 0) *t.gs_out = t.gs;
@@ -1320,12 +1329,6 @@ k_schedule_free_amax(const float *z, const float *x, float beta, uint32_t len, f
 // 30.6 -> 25.9, 6144 x 2048 41.4 -> 37.7, 8192 x 2048 47.6 -> 49.2 (beyond, the encode that has the next chunk's loads in flight
 // wins); with the transform, whose arithmetic wants many small CTAs, 8192 x 2048 65.8 -> 59.7 and 16384 x 2048 123 -> 113.
 constexpr uint32_t kChainPlainChunks = 1280, kChainScheduleChunks = 6144;
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void chain_head() {
-    chain_wait();
-    chain_begin();
-}
 
 // Maximum of every chunk of `x` (head of the chain of a plain tensor).
 __global__ void __launch_bounds__(kThreads)
@@ -1531,13 +1534,7 @@ k_adamw(float *z, float *x, float *grad, float *m1, float *m2, float *amax, Adam
 
 // Multi-tensor AdamW: one table entry per tensor, chunks of all tensors in one flat list.
 __device__ __forceinline__ uint32_t find_adam_slot(const b2_adamw_slot_descriptor *t, uint32_t count, uint32_t c) {
-    uint32_t lo = 0, hi = count;
-    while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (t[mid].chunk_begin <= c) lo = mid;
-        else hi = mid;
-    }
-    return lo;
+    return find_last(count, c, [=](uint32_t i) { return t[i].chunk_begin; });
 }
 __global__ void k_adamw_multi_reset(const b2_adamw_slot_descriptor *t, uint32_t count) {
     stream_enter();
@@ -1779,7 +1776,7 @@ static cudaError_t stream_launch(LaunchKind kind, void (*kernel)(P...), int grid
     cfg.stream = s;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
-// Launches of a chain (k_chain_*): as above; they keep their own order (see there).
+// Launches that read before they wait (k_chain_*, k_normuon_stats_columns): why they may is said there.
 template <typename... P, typename... A>
 static cudaError_t launch_chained(void (*kernel)(P...), int grid, int threads, cudaStream_t s, A... args) {
     return stream_launch(kOverlapped, kernel, grid, threads, s, args...);
@@ -1953,8 +1950,9 @@ cudaError_t launch_muon_update_encode(const SlotView &v, const uint32_t *items, 
 cudaError_t launch_normuon_stats(const SlotView &v, const NeuronView &nv, const uint64_t *u_ptrs, int hyperball,
                                  cudaStream_t s) {
     if (nv.total_units == 0) return cudaSuccess;
-    stream_launch(kPlain, k_normuon_stats<0>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
-    stream_launch(kOverlapped, k_normuon_stats<1>, clamp_grid(nv.total_units, v.grid), kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
+    const int grid = clamp_grid(nv.total_units, v.grid);
+    stream_launch(kPlain, k_normuon_stats_rows, grid, kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
+    if (nv.columns) launch_chained(k_normuon_stats_columns, grid, kThreads, s, v.slots, v.slot_count, nv, u_ptrs, hyperball);
     stream_launch(kOverlapped, k_normuon_reduce, v.slot_count, kThreads, s, v.slots, nv);
     return cudaGetLastError();
 }
