@@ -515,10 +515,10 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
     if (!build_layout(rows, cols, slot_count, o, L) || L.total > workspace_bytes) { delete p; return B2_ERROR_INVALID_VALUE; }
     p->ws = static_cast<uint8_t *>(d_workspace);
     e = gemm_configure(L.nn);
-    if (e == cudaSuccess) e = gemm_configure(L.out);
+    if (e == cudaSuccess && (L.out.tm != L.nn.tm || L.out.bn != L.nn.bn || L.out.pair != L.nn.pair)) e = gemm_configure(L.out);
     if (e != cudaSuccess) { delete p; return (int)e; }
     if (L.small_smem) {
-        e = ns_small_configure();
+        e = ns_small_configure(L.small_ragged, o.operand_format == B2_OPERAND_F16);
         if (e != cudaSuccess) { delete p; return (int)e; }
     }
     p->resident_groups = (uint32_t)std::max(gemm_resident_groups(L.nn, p->dev.sm_count), 0);

@@ -207,7 +207,7 @@ cudaError_t launch_ns_gemm(const GemmShape &shape, const GemmProblem *problems, 
 // above, for the first iteration.  At most kMaxChainIterations iterations.
 bool ns_small_fits(uint32_t rows, uint32_t cols);
 uint32_t ns_small_smem(uint32_t rows, uint32_t cols);
-cudaError_t ns_small_configure();   // once before the first launch on a device
+cudaError_t ns_small_configure(bool ragged, int f16);   // once before the first launch of that kind on a device
 cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, const GemmProblem *apply0, const GemmProblem *apply1,
                             const GemmProblem *last, uint32_t slot_count, uint32_t iterations, int f16, int last16,
                             const GemmCoefficients &coef, const float *slot_scale, uint32_t smem_bytes, bool ragged,

@@ -1433,11 +1433,13 @@ uint32_t ns_small_smem(uint32_t rows, uint32_t cols) {
     return std::max(1024u + (4u + x) * kSmallPanel, 116u * 1024u);
 }
 // The limit belongs to the function, not to a plan: it is always the largest, so that no plan takes it from another.
-cudaError_t ns_small_configure() {
-    cudaError_t e = cudaSuccess;
-    for (auto *kernel : {k_ns_small<false, 0>, k_ns_small<false, 1>, k_ns_small<true, 0>, k_ns_small<true, 1>})
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
-    return e;
+namespace {
+auto small_kernel(bool ragged, int f16) {
+    return ragged ? (f16 ? k_ns_small<true, 1> : k_ns_small<true, 0>) : (f16 ? k_ns_small<false, 1> : k_ns_small<false, 0>);
+}
+}  // namespace
+cudaError_t ns_small_configure(bool ragged, int f16) {
+    return cudaFuncSetAttribute(small_kernel(ragged, f16), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallMaxSmem);
 }
 cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, const GemmProblem *apply0, const GemmProblem *apply1,
                             const GemmProblem *last, uint32_t slot_count, uint32_t iterations, int f16, int last16,
@@ -1454,8 +1456,7 @@ cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, co
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = s;
     SmallLoop loop = {iterations, last16, coef};
-    auto *kernel = ragged ? (f16 ? k_ns_small<true, 1> : k_ns_small<true, 0>) : (f16 ? k_ns_small<false, 1> : k_ns_small<false, 0>);
-    return cudaLaunchKernelEx(&cfg, kernel, gram, poly, apply0, apply1, last, loop, slot_scale, status);
+    return cudaLaunchKernelEx(&cfg, small_kernel(ragged, f16), gram, poly, apply0, apply1, last, loop, slot_scale, status);
 }
 size_t chain_sync_bytes(uint32_t slot_count) { return sizeof(ChainSync) + sizeof(uint32_t) * slot_count; }
 namespace {
