@@ -315,7 +315,8 @@ bool build_layout(const uint32_t *rows, const uint32_t *cols, uint32_t count, co
     // asked for (Newton-Schulz stage, 128 x 128 tiles per phase -> one CTA each: three of 64 x 64 at most 66 -> 18 us, one
     // layer of width 128 83 -> 56, twelve 86 -> 56).  Not bounded in their number: beyond one matrix per SM the CTAs run in
     // waves, the launches per phase in more tiles each (pairs, the tiles before there was a choice, against one CTA each:
-    // 149 of 64 x 64 104 -> 35 us, 1000 340 -> 124; 149 of 128 x 512 181 -> 113, 1000 827 -> 447).
+    // 149 of 64 x 64 104 -> 35 us, 1000 340 -> 124; 149 of 128 x 512 181 -> 113, 1000 827 -> 447; all before
+    // the loop itself became 1.6 times as fast, see k_ns_small).
     L.small_smem = 0;
     if (o.tile_override == 0 && o.ns_schedule == B2_NS_PER_PHASE) {
         for (uint32_t s = 0; s < count; ++s) {
@@ -514,14 +515,15 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
     Layout &L = p->layout;
     if (!build_layout(rows, cols, slot_count, o, L) || L.total > workspace_bytes) { delete p; return B2_ERROR_INVALID_VALUE; }
     p->ws = static_cast<uint8_t *>(d_workspace);
-    e = gemm_configure(L.nn);
-    if (e == cudaSuccess && (L.out.tm != L.nn.tm || L.out.bn != L.nn.bn || L.out.pair != L.nn.pair)) e = gemm_configure(L.out);
+    const bool ticketed = o.ns_schedule != B2_NS_PER_PHASE;
+    e = gemm_configure(L.nn, ticketed);
+    if (e == cudaSuccess && (L.out.tm != L.nn.tm || L.out.bn != L.nn.bn || L.out.pair != L.nn.pair)) e = gemm_configure(L.out, false);
     if (e != cudaSuccess) { delete p; return (int)e; }
     if (L.small_smem) {
         e = ns_small_configure(L.small_ragged, o.operand_format == B2_OPERAND_F16);
         if (e != cudaSuccess) { delete p; return (int)e; }
     }
-    p->resident_groups = (uint32_t)std::max(gemm_resident_groups(L.nn, p->dev.sm_count), 0);
+    if (ticketed) p->resident_groups = (uint32_t)std::max(gemm_resident_groups(L.nn, p->dev.sm_count), 0);
 
     p->meta.assign(L.off_meta_end, 0);
     uint8_t *h = p->meta.data();

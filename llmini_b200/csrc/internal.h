@@ -189,7 +189,7 @@ static_assert(sizeof(ChainTile) == 32, "ChainTile is read as two 16-byte words")
 struct GemmShape {
     int tm, bn, pair;
 };
-cudaError_t gemm_configure(const GemmShape &shape);
+cudaError_t gemm_configure(const GemmShape &shape, bool ticketed);   // `ticketed`: that form too
 // CTAs (pairs of CTAs when `pair`) of the ticketed kernel that the device runs at the same time, 0 if unknown.
 // Call after gemm_configure.
 int gemm_resident_groups(const GemmShape &shape, int sm_count);

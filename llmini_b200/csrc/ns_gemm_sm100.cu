@@ -1337,7 +1337,7 @@ template <int TM, int BN, bool PAIR>
 struct Shape {
     static constexpr bool is(const GemmShape &g) { return g.tm == TM && g.bn == BN && (g.pair != 0) == PAIR; }
 };
-// Calls f<TM, BN, PAIR>() for the shape, from those that exist with (CHAINED) or without the ticketed form.
+// Calls f<TM, BN, PAIR>() for the shape, from those that exist with or without the ticketed form.
 #define B2_FOR_SHAPE(shape, F, ...)                                                  \
     if (Shape<256, 256, true>::is(shape)) return F<256, 256, true>(__VA_ARGS__);      \
     if (Shape<128, 256, false>::is(shape)) return F<128, 256, false>(__VA_ARGS__);    \
@@ -1365,9 +1365,9 @@ cudaError_t configure_plain() {
     return cudaFuncSetAttribute(k_ns_gemm<TM, BN, PAIR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TM, BN, PAIR>::kSmemBytes);
 }
 template <int TM, int BN, bool PAIR>
-cudaError_t configure_both() {
+cudaError_t configure(bool ticketed) {
     const cudaError_t e = configure_plain<TM, BN, PAIR>();
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || !ticketed) return e;
     return cudaFuncSetAttribute(k_ns_gemm<TM, BN, PAIR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TM, BN, PAIR>::kSmemBytes);
 }
 template <int TM, int BN, bool PAIR>
@@ -1401,8 +1401,8 @@ int resident_groups(int sm_count) {
 }
 }  // namespace
 
-cudaError_t gemm_configure(const GemmShape &shape) {
-    B2_FOR_SHAPE(shape, configure_both)
+cudaError_t gemm_configure(const GemmShape &shape, bool ticketed) {
+    B2_FOR_SHAPE(shape, configure, ticketed)
     B2_FOR_PLAIN_SHAPE(shape, configure_plain)
     return cudaErrorInvalidValue;
 }
