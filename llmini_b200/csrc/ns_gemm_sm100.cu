@@ -983,6 +983,11 @@ struct SmallLoop {
     GemmCoefficients coef;
 };
 
+// Which of the loop's results the operand buffers in memory keep.  The buffers take turns, so after a launch per phase they
+// hold the last two 16-bit results.  Earlier ones are not stored: the bulk copies of two results to one buffer would be in
+// no order (what the issuer waits for before it reuses the panels is only that they have been read).
+__host__ __device__ constexpr bool small_keeps(uint32_t it, uint32_t iterations, bool last16) { return it + (last16 ? 2u : 3u) >= iterations; }
+
 __device__ __forceinline__ uint32_t small_swizzled(uint32_t row, uint32_t chunk) { return row * 128u + ((chunk ^ (row & 7u)) << 4); }
 
 template <bool RAGGED, int F16>
@@ -1275,8 +1280,7 @@ k_ns_small(const GemmProblem *__restrict__ gram, const GemmProblem *__restrict__
             }
             hand_over();
             if (*abort_flag) break;   // a wait ran out: written before the barrier, so every thread sees it
-            // the operand buffers in memory hold the last three operands of the loop, as with a launch per phase
-            if (issuer && !fp32 && it + 3 >= loop.iterations && elect_one())
+            if (issuer && !fp32 && small_keeps(it, loop.iterations, loop.last16 != 0) && elect_one())
                 store_panels((it & 1u) ? x0_map : x1_map, smem_u32(x_panels), tall ? (n + 63u) / 64u : panels, blocks);
         }
         if (issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");

@@ -1,0 +1,40 @@
+"""Rules of the kernels that a run on the GPU would only break now and then: read out of the sources, checked on the CPU."""
+import ctypes as C
+import os
+import re
+import subprocess
+
+import pytest
+
+from llmini_b200 import _ffi
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(_ffi.__file__)), "csrc")
+
+
+def _source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+@pytest.mark.parametrize("last16", [False, True])
+def test_one_cta_loop_stores_each_operand_buffer_once(tmp_path, last16):
+    """Bulk copies of separate groups to the same memory are in no order, so the one-CTA loop may store a buffer only once, and
+    has to leave in it what a launch per phase would.  Result `it` of the loop goes to buffer 1 - it % 2; the last one does so
+    only where it is a 16-bit result."""
+    text = _source("ns_gemm_sm100.cu")
+    rule = re.search(r"constexpr bool small_keeps\(uint32_t it, uint32_t iterations, bool last16\) \{[^}]*\}", text)
+    assert rule and "store_panels((it & 1u) ? x0_map : x1_map" in text
+    assert re.search(r"if \(issuer && !fp32 && small_keeps\(it, loop\.iterations, loop\.last16 != 0\) && elect_one\(\)\)\s*store_panels", text)
+    src, lib = tmp_path / "rule.cpp", tmp_path / "rule.so"
+    src.write_text("#include <cstdint>\n" + rule.group(0) +
+                   '\nextern "C" int keeps(uint32_t it, uint32_t n, int l) { return small_keeps(it, n, l != 0); }\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
+    keeps = C.CDLL(str(lib)).keeps
+    for iterations in range(1, 9):
+        results = [it for it in range(iterations) if last16 or it + 1 < iterations]   # in 16 bits
+        per_phase = {}
+        for it in results:
+            per_phase[1 - it % 2] = it
+        stored = [it for it in results if keeps(it, iterations, int(last16))]
+        assert len({1 - it % 2 for it in stored}) == len(stored), (iterations, stored)
+        assert {1 - it % 2: it for it in stored} == per_phase, (iterations, stored)
