@@ -71,7 +71,7 @@ constexpr uint32_t kSpinLimit = 1u << 24;    // hard cap on polls, whatever the 
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 
 // TM x BN is the tile of a CTA, or of a pair of CTAs; a pair's CTAs hold half of its rows of A and half of its rows of B each.
-template <int TM, int BN, bool PAIR>
+template <int TM, int BN, bool PAIR, bool CHAINED>
 struct Cfg {
     static constexpr int kTileM = TM;
     static constexpr int kRows = PAIR ? TM / 2 : TM;        // output rows of this CTA, and rows of A it stages per k-block
@@ -84,8 +84,11 @@ struct Cfg {
     // An accumulator of 64 rows per CTA lies in all 128 lanes: columns 0 .. BN/2-1 in lanes 0 .. 63, the others above.
     static constexpr int kAccCols = kRows == 64 ? BN / 2 : BN;
     // warp 0: TMA producer of A, warp 1: MMA issuer, then four epilogue warps (one per TMEM lane quarter) for every
-    // kEpiCols tensor-memory columns, the TMA producer of B and the tile scheduler
-    static constexpr int kEpiCols = BN == 256 ? 64 : 32;
+    // kEpiCols tensor-memory columns, the TMA producer of B and the tile scheduler.  Narrow tiles: 32 columns a warp shorten
+    // the epilogue, but in the ticketed form every warp publishes its part of a tile with a fence and an atomic, and twice as
+    // many of these cost more than that (128 x 128, one CTA, 32 -> 64 columns in the chained loop: one layer of width 768
+    // 247 -> 215 us, the eighth of GPT-2 small 302 -> 265; launch per phase 203 with 32).
+    static constexpr int kEpiCols = BN == 256 || CHAINED ? 64 : 32;
     static constexpr int kEpiWarps = 4 * (kAccCols / kEpiCols);
     static constexpr int kProducerA = 0, kMmaWarp = 1, kEpiWarp0 = 2, kProducerB = 2 + kEpiWarps, kSchedulerWarp = 3 + kEpiWarps;
     static constexpr int kThreads = 32 * (4 + kEpiWarps);
@@ -440,12 +443,12 @@ __device__ __forceinline__ void fill_entry(TileEntry &e, const GemmProblem *p, u
 }
 
 template <int TM, int BN, bool PAIR, bool CHAINED>
-__global__ void __launch_bounds__((Cfg<TM, BN, PAIR>::kThreads), 1)
+__global__ void __launch_bounds__((Cfg<TM, BN, PAIR, CHAINED>::kThreads), 1)
 k_ns_gemm(const GemmProblem *__restrict__ problems, const void *__restrict__ tiles,
           uint32_t tile_count, uint32_t epilogue_arg, int f16, GemmCoefficients coef,
           const float *__restrict__ slot_scale, uint32_t scale_pow_arg, uint32_t *status, ChainSync *sync,
           uint32_t slot_count) {
-    using C = Cfg<TM, BN, PAIR>;
+    using C = Cfg<TM, BN, PAIR, CHAINED>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *stage_base = smem;
@@ -1301,7 +1304,7 @@ cudaError_t launch_impl(const GemmProblem *problems, const void *tiles, uint32_t
                         int f16, const GemmCoefficients &coef, const float *slot_scale, uint32_t scale_pow,
                         uint32_t *status, void *sync, uint32_t slot_count, uint32_t debug_flags, int grid,
                         cudaStream_t s) {
-    using C = Cfg<TM, BN, PAIR>;
+    using C = Cfg<TM, BN, PAIR, CHAINED>;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     unsigned n_attr = 0;
@@ -1366,17 +1369,17 @@ cudaError_t launch_ticketed(const GemmProblem *problems, const ChainTile *tiles,
 }
 template <int TM, int BN, bool PAIR>
 cudaError_t configure_plain() {
-    return cudaFuncSetAttribute(k_ns_gemm<TM, BN, PAIR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TM, BN, PAIR>::kSmemBytes);
+    return cudaFuncSetAttribute(k_ns_gemm<TM, BN, PAIR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TM, BN, PAIR, false>::kSmemBytes);
 }
 template <int TM, int BN, bool PAIR>
 cudaError_t configure(bool ticketed) {
     const cudaError_t e = configure_plain<TM, BN, PAIR>();
     if (e != cudaSuccess || !ticketed) return e;
-    return cudaFuncSetAttribute(k_ns_gemm<TM, BN, PAIR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TM, BN, PAIR>::kSmemBytes);
+    return cudaFuncSetAttribute(k_ns_gemm<TM, BN, PAIR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<TM, BN, PAIR, true>::kSmemBytes);
 }
 template <int TM, int BN, bool PAIR>
 int resident_groups(int sm_count) {
-    using C = Cfg<TM, BN, PAIR>;
+    using C = Cfg<TM, BN, PAIR, true>;
     if (PAIR) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
@@ -1465,7 +1468,7 @@ cudaError_t launch_ns_small(const GemmProblem *gram, const GemmProblem *poly, co
 size_t chain_sync_bytes(uint32_t slot_count) { return sizeof(ChainSync) + sizeof(uint32_t) * slot_count; }
 namespace {
 template <int TM, int BN, bool PAIR>
-uint32_t epilogue_warps() { return (uint32_t)Cfg<TM, BN, PAIR>::kEpiWarps * (PAIR ? 2u : 1u); }
+uint32_t epilogue_warps() { return (uint32_t)Cfg<TM, BN, PAIR, true>::kEpiWarps * (PAIR ? 2u : 1u); }
 }  // namespace
 uint32_t chain_epilogue_warps(const GemmShape &shape) {
     B2_FOR_SHAPE(shape, epilogue_warps)
