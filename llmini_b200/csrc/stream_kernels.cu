@@ -859,14 +859,15 @@ k_muon_sign_update(const b2_muon_slot_descriptor *slots, const uint32_t *prefix,
 constexpr int kEncodeThreads = kChunk / 16;
 
 // Scalars of the transform: the three scales are schedule-free pairs themselves
-// (symexp_lin.rs:164-196: z + beta (x - z) with the SCHEDULE beta); no pointers = unit scales.
+// (symexp_lin.rs:164-196: z + beta (x - z) with the SCHEDULE beta); no pointers = unit scales.  They are trained, so they
+// change between two calls; read past L1, as launches that read before they wait have to (k_chain_*).
 __device__ __forceinline__ SymExpLin symexp_resolve(const SymExpLinParams &p, float schedule_beta) {
     SymExpLin s = {p.beta, 1.0f, 1.0f, 1.0f, uniform_reciprocal(p.beta)};
     if (p.beta > 0.0f && p.scales[0] != nullptr) {
         float v[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const float z = *p.scales[2 * k], x = *p.scales[2 * k + 1];
+            const float z = __ldcg(p.scales[2 * k]), x = __ldcg(p.scales[2 * k + 1]);
             v[k] = z + schedule_beta * (x - z);
         }
         s.exponential = v[0]; s.linear = v[1]; s.curvature = v[2];

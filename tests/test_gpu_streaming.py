@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import llmini_b200 as b2
+from llmini_b200 import _ffi
 from oracle import oracle as o
 from tests import _util as U
 from tests.gpu_util import bf16_bits, bf16_from_bits, decode_scales, dev, host, rcp_table
@@ -553,3 +554,55 @@ def test_captured_calls_replay_as_the_calls_themselves(call):
                     assert torch.equal(got[name], t), (step, name)
         seen.add((float(eager[0]["amax"]), float(eager[2]["scale"])))
     assert len(seen) == 3   # every replay had something else to find
+
+
+@pytest.mark.parametrize("front", ["weights", "scalars", "same outputs"])
+def test_one_tensor_chain_right_behind_the_kernels_that_write_its_inputs(front):
+    """The launches of materialize_schedule_free read before they wait for the one in front of them.  Behind the library's own
+    AdamW of the same masters, behind the update of the transform's scalars, and behind another such call on the same output
+    buffers: many steps without a wait give the bits of the same steps with one after every call."""
+    n, steps, beta = 300 * 2048 + 16, 24, 0.4
+    opt = b2.OptimizerModule()
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    randn = lambda std: torch.randn(n, device="cuda", generator=gen).mul_(std)
+    begin = dict(z_master=randn(0.02), x_master=randn(0.02), grad=randn(1e-3), first_moment=randn(1e-4), second_moment=randn(1e-3).square_())
+    other = dict(z_master=randn(0.03), x_master=randn(0.01))
+    names = [f"{part}_{kind}" for part in ("exponential", "linear", "curvature") for kind in ("z", "x", "grad", "first", "second")]
+    one = {k: 1.0 if k[-1] in "zx" else (0.3 if k.endswith("grad") else 0.0) for k in names}
+
+    def steps_of(wait):
+        state = {k: v.clone() for k, v in begin.items()}
+        scalars = {k: torch.full((1,), v, device="cuda") for k, v in one.items()}
+        desc = (_ffi.SymExpLinSlotDescriptor * 1)()
+        for k, t in scalars.items():
+            setattr(desc[0], k, t.data_ptr())
+        table = torch.from_numpy(np.frombuffer(bytes(desc), dtype=np.uint8).copy()).cuda()
+        refs = [scalars[f"{part}_{kind}"] for part in ("exponential", "linear", "curvature") for kind in "zx"]
+        outs = [dict(bytes=torch.zeros(n // 2, dtype=torch.uint8, device="cuda"), scales=torch.zeros(n // 16, dtype=torch.uint8, device="cuda"),
+                     global_scale=torch.zeros(1, device="cuda"), amax=torch.zeros(1, device="cuda")) for _ in range(steps)]
+        call = dict(len=n, scale_rows=n // 16, scale_k=16, beta=beta, scale_layout=b2.SCALES_RAW)
+        torch.cuda.synchronize()
+        for i, q in enumerate(outs):
+            masters = dict(z_master=state["z_master"], x_master=state["x_master"])
+            if front == "weights":
+                opt.apply_fp32_adamw_update(**state, len=n, learning_rate=1e-2, weight_decay=0.005, beta1=0.9, beta2=0.95, beta1_correction=0.19,
+                                            beta2_correction=0.0975, eps=1e-10, average_coefficient=0.5, schedule_beta=0.3, grad_scale=1.0)
+            elif front == "scalars":
+                opt.symexp_lin_scale_adamw_update(table, 1, 0.5, 0.05, 0.03, 0.1, 0.9, 0.95, 0.1, 0.05, 1.0e-10, 0.25)
+                call.update(symexp_lin_beta=12.5, symexp_lin_scales=refs)
+            else:
+                opt.materialize_schedule_free(**q, **(other if i % 2 else masters), **call)
+                masters = masters if i % 2 else other
+            if wait:
+                torch.cuda.synchronize()
+            opt.materialize_schedule_free(**q, **masters, **call)
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return outs
+
+    got, want = steps_of(False), steps_of(True)
+    for i, (a, b) in enumerate(zip(got, want)):
+        for key in a:
+            assert torch.equal(a[key], b[key]), (i, key)
+    assert len({float(q["amax"]) for q in want}) == (2 if front == "same outputs" else steps)

@@ -38,3 +38,22 @@ def test_one_cta_loop_stores_each_operand_buffer_once(tmp_path, last16):
         stored = [it for it in results if keeps(it, iterations, int(last16))]
         assert len({1 - it % 2 for it in stored}) == len(stored), (iterations, stored)
         assert {1 - it % 2: it for it in stored} == per_phase, (iterations, stored)
+
+
+def _function(text, name):
+    """The body of a function of the source, without its closing brace."""
+    head = re.search(r"\b" + name + r"\([^;{]*\{", text)
+    assert head, name
+    depth, at = 1, head.end()
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[at], 0)
+        at += 1
+    return text[head.end():at - 1]
+
+
+def test_transform_scalars_are_read_past_l1():
+    """The launches of the one-tensor chain resolve the transform's scalars before they wait for the launch in front of them:
+    L1 may still hold what an earlier kernel of the stream saw of these trained values."""
+    body = _function(_source("stream_kernels.cu"), "symexp_resolve")
+    reads = re.findall(r"(\S*)\(?p\.scales\[2 \* k[^\]]*\]\)?", body)
+    assert reads and all(r.startswith("__ldcg(") for r in reads), reads
