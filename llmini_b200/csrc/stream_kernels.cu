@@ -469,6 +469,10 @@ k_muon_update(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint
 // the number of units in a plan, it let a matrix's bits depend on its company.  Narrow units give a lone matrix more CTAs,
 // each with a shorter chain of round trips; wide ones read longer pieces of a row.  NorMuon finish with 32 / 64 / 128 columns
 // (us): ragged plan of 5 matrices 24.9 / 25.8 / 28.9, one 768 x 3072 18.8 / 20.5 / 22.8, GPT-2 medium 1523 / 1494 / 1478.
+// What COLS reads in front of its wait goes to L2, past the L1 of an SM that may hold what an earlier kernel saw.  (Plain loads
+// find the tables in L1 behind the rows: ragged plan of 5 matrices with Hyperball, whole call 153.8 us with them, 156.2 now.)
+template <int COLS, typename T>
+__device__ __forceinline__ T normuon_load(const T *p) { return COLS ? __ldcg(p) : *p; }
 template <int COLS>
 __device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slots, uint32_t slot_count, const NeuronView &nv,
                                               const uint64_t *u_ptrs, int hyperball) {
@@ -477,14 +481,14 @@ __device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slo
     __shared__ double part[kThreads / 32][4];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint32_t unit = blockIdx.x; unit < nv.total_units; unit += gridDim.x) {
-        const uint32_t slot = find_slot(nv.unit_prefix, slot_count, unit);
-        if ((slots[slot].rows < slots[slot].cols) != (COLS != 0)) continue;   // CTA-uniform
-        const b2_muon_slot_descriptor d = slots[slot];
-        const uint32_t local = unit - nv.unit_prefix[slot];
-        const float *U = reinterpret_cast<const float *>(u_ptrs[slot]);
-        const float *z = reinterpret_cast<const float *>(d.z_master);
-        float *state = reinterpret_cast<float *>(d.second_momentum);
-        float *factors = reinterpret_cast<float *>(nv.factor_ptrs[slot]);
+        const uint32_t slot = find_last(slot_count, unit, [=](uint32_t i) { return normuon_load<COLS>(nv.unit_prefix + i); });
+        const uint32_t rows = normuon_load<COLS>(&slots[slot].rows), cols = normuon_load<COLS>(&slots[slot].cols);
+        if ((rows < cols) != (COLS != 0)) continue;   // CTA-uniform
+        const uint32_t local = unit - normuon_load<COLS>(nv.unit_prefix + slot);
+        const float *U = reinterpret_cast<const float *>(normuon_load<COLS>(u_ptrs + slot));
+        const float *z = reinterpret_cast<const float *>(normuon_load<COLS>(&slots[slot].z_master));
+        float *state = reinterpret_cast<float *>(normuon_load<COLS>(&slots[slot].second_momentum));
+        float *factors = reinterpret_cast<float *>(normuon_load<COLS>(nv.factor_ptrs + slot));
         double s_raw = 0.0, s_scaled = 0.0, s_param = 0.0, s_dot = 0.0;  // meaningful on one thread per neuron
         if (!COLS) {
             // B2_NORMUON_ROWS_PER_UNIT rows per unit, kRowsPerWarp per warp, one after the other: the
@@ -495,15 +499,15 @@ __device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slo
             float old_state[kRowsPerWarp];
 #pragma unroll
             for (uint32_t j = 0; j < kRowsPerWarp; ++j)
-                old_state[j] = (lane == 0 && state && row0 + j < d.rows) ? __ldcg(state + row0 + j) : 0.0f;
+                old_state[j] = (lane == 0 && state && row0 + j < rows) ? __ldcg(state + row0 + j) : 0.0f;
 #pragma unroll
             for (uint32_t j = 0; j < kRowsPerWarp; ++j) {
                 const uint32_t row = row0 + j;
-                if (row >= d.rows) break;   // warp-uniform
+                if (row >= rows) break;   // warp-uniform
                 float raw = 0.0f, param = 0.0f, dot = 0.0f;
-                const size_t base = (size_t)row * d.cols;
+                const size_t base = (size_t)row * cols;
 #pragma unroll 4
-                for (uint32_t c = lane * 4; c < d.cols; c += 128) {
+                for (uint32_t c = lane * 4; c < cols; c += 128) {
                     const float4 u = *reinterpret_cast<const float4 *>(U + base + c);
                     raw = fmaf(u.x, u.x, raw); raw = fmaf(u.y, u.y, raw);
                     raw = fmaf(u.z, u.z, raw); raw = fmaf(u.w, u.w, raw);
@@ -519,7 +523,7 @@ __device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slo
                 if (lane == 0) {
                     float factor = 1.0f;
                     if (state) {
-                        const float mean = (float)r / (float)d.cols;
+                        const float mean = (float)r / (float)cols;
                         const float next = 0.95f * old_state[j] + (1.0f - 0.95f) * mean;
                         factor = 1.0f / sqrtf(fmaxf(next, 1.0e-10f));
                         state[row] = next;
@@ -533,18 +537,18 @@ __device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slo
             const uint32_t quad = tid % kQuads, row_lane = tid / kQuads;
             const uint32_t c0 = local * kUnitCols + quad * 4;
             float raw[4] = {0.f, 0.f, 0.f, 0.f}, dot[4] = {0.f, 0.f, 0.f, 0.f}, param = 0.0f;
-            if (c0 < d.cols) {
+            if (c0 < cols) {
                 // eight independent 128-bit loads in flight per thread
                 constexpr uint32_t kRowsInFlight = 8;
-                for (uint32_t r0 = row_lane; r0 < d.rows; r0 += kRowLanes * kRowsInFlight) {
+                for (uint32_t r0 = row_lane; r0 < rows; r0 += kRowLanes * kRowsInFlight) {
                     float4 u[kRowsInFlight], p[kRowsInFlight];
 #pragma unroll
                     for (uint32_t k = 0; k < kRowsInFlight; ++k) {
                         const uint32_t r = r0 + k * kRowLanes;
-                        const size_t at = (size_t)r * d.cols + c0;
-                        u[k] = r < d.rows ? *reinterpret_cast<const float4 *>(U + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        const size_t at = (size_t)r * cols + c0;
+                        u[k] = r < rows ? __ldcg(reinterpret_cast<const float4 *>(U + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
                         if (hyperball)
-                            p[k] = r < d.rows ? *reinterpret_cast<const float4 *>(z + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            p[k] = r < rows ? __ldcg(reinterpret_cast<const float4 *>(z + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
 #pragma unroll
                     for (uint32_t k = 0; k < kRowsInFlight; ++k) {
@@ -570,7 +574,7 @@ __device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slo
             s_param = (double)param;
             __syncthreads();
             const uint32_t col = local * kUnitCols + tid;
-            if (tid < kUnitCols && col < d.cols) {
+            if (tid < kUnitCols && col < cols) {
                 double r = 0.0, dd = 0.0;
 #pragma unroll 8
                 for (uint32_t w = 0; w < kRowLanes; ++w) {
@@ -579,8 +583,8 @@ __device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slo
                 }
                 float factor = 1.0f;
                 if (state) {
-                    const float mean = (float)r / (float)d.rows;
-                    const float next = 0.95f * state[col] + (1.0f - 0.95f) * mean;
+                    const float mean = (float)r / (float)rows;
+                    const float next = 0.95f * __ldcg(state + col) + (1.0f - 0.95f) * mean;
                     factor = 1.0f / sqrtf(fmaxf(next, 1.0e-10f));
                     state[col] = next;
                 }
@@ -605,9 +609,9 @@ __device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slo
     }
 }
 
-// The two forms write to different slots, so they run side by side.  The columns' launch, behind the rows', reads at once: the
-// rows' does not begin before the Newton-Schulz result is complete (it is a plain launch), nor the columns' before the rows'.
-// It waits for the rows' at its end, so that what comes behind it finds both done.
+// The two forms write to different slots, so they run side by side.  The columns' launch, behind the rows', reads at once, from
+// L2: the rows' does not begin before the Newton-Schulz result is complete and in L2 (it is a plain launch), nor the columns'
+// before the rows'.  It waits for the rows' at its end, so that what comes behind it finds both done.
 __global__ void __launch_bounds__(kThreads, 4)
 k_normuon_stats_rows(const b2_muon_slot_descriptor *slots, uint32_t slot_count, NeuronView nv, const uint64_t *u_ptrs, int hyperball) {
     stream_enter();

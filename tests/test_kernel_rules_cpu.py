@@ -57,3 +57,19 @@ def test_transform_scalars_are_read_past_l1():
     body = _function(_source("stream_kernels.cu"), "symexp_resolve")
     reads = re.findall(r"(\S*)\(?p\.scales\[2 \* k[^\]]*\]\)?", body)
     assert reads and all(r.startswith("__ldcg(") for r in reads), reads
+
+
+def test_column_statistics_read_past_l1():
+    """k_normuon_stats_columns reads before it waits: its tables, the Newton-Schulz result, the weights and the old second
+    moments all come from L2."""
+    text = _source("stream_kernels.cu")
+    body = _function(text, "normuon_stats")
+    head, rest = body.split("if (!COLS) {", 1)
+    columns = rest[rest.index("const uint32_t quad = tid % kQuads"):]
+    for table in (r"slots\[", r"nv\.unit_prefix\b", r"\bu_ptrs\b", r"nv\.factor_ptrs\b"):
+        reads = re.findall(r"(\S*?)&?" + table, head)
+        assert reads and all(r.endswith("normuon_load<COLS>(") for r in reads), (table, reads)
+    assert "slots[" not in columns and "*reinterpret_cast<const" not in columns
+    assert re.findall(r"\bstate\[col\]\s*(\S+)", columns) == ["="]
+    assert "0.95f * __ldcg(state + col)" in columns
+    assert "return COLS ? __ldcg(p) : *p;" in _function(text, "normuon_load")
