@@ -204,28 +204,32 @@ void pick_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t count, cons
     auto m_of = [&](uint32_t s) { return std::max(rows[s], cols[s]); };
     std::stable_sort(by_m.begin(), by_m.end(), [&](uint32_t a, uint32_t b) { return m_of(a) > m_of(b); });
     std::stable_sort(by_n.begin(), by_n.end(), [&](uint32_t a, uint32_t b) { return n_of(a) > n_of(b); });
-    auto tiles = [](uint64_t v, int t) { return (v + t - 1) / t; };
-    // time of a launch: `tiles_of(s)` tiles per matrix with a sum over `k_of(s)` each
-    auto launch = [&](const TileCost &c, const std::vector<uint32_t> &order, auto tiles_of, auto k_of) {
-        const uint64_t groups = c.shape.pair ? kTileRuleSms / 2 : kTileRuleSms;
-        uint64_t at = 0;
-        double t = c.fixed;
-        for (uint32_t s : order) {
-            const uint64_t n = tiles_of(s), first_group = (at + n + groups - 1) / groups - (at + groups - 1) / groups;
-            t += (double)first_group * std::max(c.per_k_block * (double)tiles(k_of(s), kGemmBlockK) + c.per_tile, c.least);
-            at += n;
-        }
-        return t;
+    auto tiles = [](uint32_t v, int t) { return (v + (uint32_t)t - 1u) / (uint32_t)t; };   // (fewer than 2^19 of any matrix)
+    // `n` more tiles are dealt round the groups: how many of them the first group gets; `turn` is the group that comes next
+    auto deal = [](uint32_t &turn, uint32_t n, uint32_t groups) {
+        const uint32_t end = turn + n, rounds = end / groups, before = turn != 0u;
+        turn = end - rounds * groups;
+        return (double)(rounds + (turn != 0u) - before);
     };
+    auto tile_time = [&](const TileCost &c, uint32_t k) { return std::max(c.per_k_block * (double)tiles(k, kGemmBlockK) + c.per_tile, c.least); };
+    auto groups_of = [](const TileCost &c) { return c.shape.pair ? kTileRuleSms / 2 : kTileRuleSms; };
     auto time_nn = [&](const TileCost &c) {
-        auto tiles_of = [&](uint32_t s) {
-            const uint64_t t = tiles(n_of(s), c.shape.tm);
-            return c.triangle ? t * (t + 1) / 2 : t * t;
-        };
-        return launch(c, by_m, tiles_of, m_of) + launch(c, by_m, tiles_of, n_of);
+        double gram = c.fixed, poly = c.fixed;
+        uint32_t turn = 0;
+        for (uint32_t s : by_m) {
+            const uint32_t t = tiles(n_of(s), c.shape.tm);
+            const double first_group = deal(turn, c.triangle ? t * (t + 1) / 2 : t * t, groups_of(c));
+            gram += first_group * tile_time(c, m_of(s));
+            poly += first_group * tile_time(c, n_of(s));
+        }
+        return gram + poly;
     };
     auto time_out = [&](const TileCost &c) {
-        return launch(c, by_n, [&](uint32_t s) { return tiles(rows[s], c.shape.tm) * tiles(cols[s], c.shape.bn); }, n_of);
+        double t = c.fixed;
+        uint32_t turn = 0;
+        for (uint32_t s : by_n)
+            t += deal(turn, tiles(rows[s], c.shape.tm) * tiles(cols[s], c.shape.bn), groups_of(c)) * tile_time(c, n_of(s));
+        return t;
     };
     const bool ticketed = o.ns_schedule != B2_NS_PER_PHASE;
     double best_nn = 0.0, best_out = 0.0;
@@ -536,9 +540,6 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
     if (!L.items.empty()) std::memcpy(h + L.off_items, L.items.data(), L.items.size() * sizeof(uint32_t));
     CUtensorMap *maps = reinterpret_cast<CUtensorMap *>(h + L.off_maps);
     GemmProblem *probs = reinterpret_cast<GemmProblem *>(h + L.off_problems);
-    auto dmap = [&](uint32_t s, int kind) {
-        return reinterpret_cast<uint64_t>(p->ws + L.off_maps + ((size_t)s * kMapsPerSlot + kind) * sizeof(CUtensorMap));
-    };
     bool ok = true;
     for (uint32_t s = 0; s < slot_count; ++s) {
         const SlotLayout &sl = L.slots[s];
@@ -550,21 +551,28 @@ int b2_muon_plan_create(b2_muon_plan **out, const uint32_t *rows, const uint32_t
         fp[s] = reinterpret_cast<uint64_t>(p->ws + sl.off_factors);
         CUtensorMap *ms = maps + (size_t)s * kMapsPerSlot;
         const uint64_t xp = (uint64_t)sl.cols * 2, gp = (uint64_t)sl.ldg * 2;
-        ok &= make_map(ms + kLX0K, p->ws + sl.off_x[0], 2, sl.rows, sl.cols, xp, 64, 128);
-        ok &= make_map(ms + kLX1K, p->ws + sl.off_x[1], 2, sl.rows, sl.cols, xp, 64, 128);
-        ok &= make_map(ms + kLX0M, p->ws + sl.off_x[0], 2, sl.rows, sl.cols, xp, 64, 64);
-        ok &= make_map(ms + kLX1M, p->ws + sl.off_x[1], 2, sl.rows, sl.cols, xp, 64, 64);
-        ok &= make_strip_map(ms + kLX0T, p->ws + sl.off_x[0], sl.rows, sl.cols);
-        ok &= make_strip_map(ms + kLX1T, p->ws + sl.off_x[1], sl.rows, sl.cols);
-        ok &= make_map(ms + kLG, p->ws + sl.off_g16, 2, sl.n, sl.n, gp, 64, 128);
-        ok &= make_map(ms + kLQ, p->ws + sl.off_q16, 2, sl.n, sl.n, gp, 64, 128);
-        ok &= make_map(ms + kLG64, p->ws + sl.off_g16, 2, sl.n, sl.n, gp, 64, 64);
-        ok &= make_map(ms + kLQ64, p->ws + sl.off_q16, 2, sl.n, sl.n, gp, 64, 64);
+        uint32_t made = 0;
+        // A map's address, encoded when it is first asked for: of the ten a plan's tile shapes use six.  (A plan of 192 matrices
+        // is made in 318 us; 383 with all ten and a tile choice of twice the work.)
+        auto dmap = [&](int kind) {
+            if (!(made >> kind & 1u)) {
+                made |= 1u << kind;
+                const bool second = kind == kLX1K || kind == kLX1M || kind == kLX1T;
+                uint8_t *x = p->ws + sl.off_x[second ? 1 : 0], *nn = p->ws + (kind == kLG || kind == kLG64 ? sl.off_g16 : sl.off_q16);
+                switch (kind) {
+                    case kLX0K: case kLX1K: ok &= make_map(ms + kind, x, 2, sl.rows, sl.cols, xp, 64, 128); break;
+                    case kLX0M: case kLX1M: ok &= make_map(ms + kind, x, 2, sl.rows, sl.cols, xp, 64, 64); break;
+                    case kLX0T: case kLX1T: ok &= make_strip_map(ms + kind, x, sl.rows, sl.cols); break;
+                    default: ok &= make_map(ms + kind, nn, 2, sl.n, sl.n, gp, 64, kind == kLG64 || kind == kLQ64 ? 64 : 128); break;
+                }
+            }
+            return reinterpret_cast<uint64_t>(p->ws + L.off_maps + ((size_t)s * kMapsPerSlot + kind) * sizeof(CUtensorMap));
+        };
         const bool tall = sl.rows > sl.cols;
         const uint64_t frag = reinterpret_cast<uint64_t>(p->ws + sl.off_frag);
         // the map whose boxes fit the rows that a CTA stages of A or of B
         auto pick = [&](int rows_of_tile, int pair, int map128, int map64) {
-            return dmap(s, (pair ? rows_of_tile / 2 : rows_of_tile) == 64 ? map64 : map128);
+            return dmap((pair ? rows_of_tile / 2 : rows_of_tile) == 64 ? map64 : map128);
         };
         for (int b = 0; b < 2; ++b) {
             GemmProblem &g = probs[(size_t)(kGram0 + b) * slot_count + s];
