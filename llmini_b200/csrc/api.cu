@@ -1102,7 +1102,7 @@ int b2_materialize_schedule_free(const b2_schedule_free_materialize_args *a, voi
                                           a->global_scale, a->len, (int)a->scale_layout, stream_grid_cap(d), s);
     e = cudaMemsetAsync(a->amax, 0, sizeof(float), s);  // launcher/update.rs:14-23 (zero_amax)
     if (e == cudaSuccess)
-        e = launch_schedule_free_amax(a->z_master, a->x_master, a->beta, a->len, a->amax, stream_grid_cap(d), s, &sp);
+        e = launch_schedule_free_amax(a->z_master, a->x_master, a->beta, a->len, a->amax, stream_grid_cap(d), s);
     if (e == cudaSuccess)
         e = launch_quantize_flat(nullptr, a->z_master, a->x_master, a->beta, 1, a->amax, a->bytes, a->scales,
                                  a->global_scale, a->len / 16, (int)a->scale_layout, stream_grid_cap(d), s, &sp);

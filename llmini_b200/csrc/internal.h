@@ -94,8 +94,7 @@ cudaError_t launch_quantize_chain(const float *src, const float *z, const float 
                                   float *amax, float *chunk_amax, uint8_t *fp4, uint8_t *scales, float *gs, uint32_t len,
                                   int scale_layout, int grid_cap, cudaStream_t s);
 cudaError_t launch_schedule_free_amax(const float *z, const float *x, float beta, uint32_t len,
-                                      float *amax, int grid_cap, cudaStream_t s,
-                                      const SymExpLinParams *symexp = nullptr);
+                                      float *amax, int grid_cap, cudaStream_t s);
 cudaError_t launch_adamw(const b2_adamw_update_args &a, int mode, int grid_cap,
                          cudaStream_t s);
 cudaError_t launch_adamw_multi(const b2_adamw_slot_descriptor *table, uint32_t count, uint32_t total_chunks,

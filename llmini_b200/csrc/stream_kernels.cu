@@ -1287,12 +1287,13 @@ k_tensor_amax_from_chunks(const float *chunk_amax, float *out, uint32_t count) {
     }
 }
 
-// `schedule_free_amax_kernel` (crates/cuda-kernels/src/gpt/optimizer/schedule_free/amax.rs:16-68).
+// `schedule_free_amax_kernel` (crates/cuda-kernels/src/gpt/optimizer/schedule_free/amax.rs:16-68), of long pairs without the
+// transform: the others are k_chain_schedule_amax's.
 __global__ void __launch_bounds__(kThreads)
-k_schedule_free_amax(const float *z, const float *x, float beta, uint32_t len, float *amax, SymExpLinParams sp) {
+k_schedule_free_amax(const float *z, const float *x, float beta, uint32_t len, float *amax) {
     stream_enter();
     __shared__ float warp_part[kThreads / 32];
-    const SymExpLin sx = symexp_resolve(sp, beta);
+    const SymExpLin identity = {0.0f, 1.0f, 1.0f, 1.0f};
     const int tid = threadIdx.x;
     const uint32_t chunks = (len + kChunk - 1) / kChunk;
     float m = 0.0f;
@@ -1302,11 +1303,11 @@ k_schedule_free_amax(const float *z, const float *x, float beta, uint32_t len, f
             uint32_t i = c * kChunk + h * (kChunk / 2) + tid * 4;
             if (i + 4 <= len) {
                 float4 zv = ld_stream(z + i), xv = ld_stream(x + i);
-                const float4 v = schedule_quad(zv, xv, beta, sx);
+                const float4 v = schedule_quad(zv, xv, beta, identity);
                 m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
             } else {
                 for (uint32_t j = i; j < len && j < i + 4; ++j)
-                    m = fmaxf(m, fabsf(symexp_forward(z[j] + beta * (x[j] - z[j]), sx)));
+                    m = fmaxf(m, fabsf(z[j] + beta * (x[j] - z[j])));
             }
         }
     }
@@ -2042,12 +2043,10 @@ cudaError_t launch_quantize_chain(const float *src, const float *z, const float 
     return e;
 }
 cudaError_t launch_schedule_free_amax(const float *z, const float *x, float beta, uint32_t len,
-                                      float *amax, int grid_cap, cudaStream_t s, const SymExpLinParams *symexp) {
-    SymExpLinParams sp = {};
-    if (symexp) sp = *symexp;
+                                      float *amax, int grid_cap, cudaStream_t s) {
     uint32_t chunks = (len + kChunk - 1) / kChunk;
     if (chunks == 0) return cudaSuccess;
-    stream_launch(kOverlapped, k_schedule_free_amax, clamp_grid(chunks, grid_cap), kThreads, s, z, x, beta, len, amax, sp);
+    stream_launch(kOverlapped, k_schedule_free_amax, clamp_grid(chunks, grid_cap), kThreads, s, z, x, beta, len, amax);
     return cudaGetLastError();
 }
 cudaError_t launch_adamw(const b2_adamw_update_args &a, int mode, int grid_cap,
