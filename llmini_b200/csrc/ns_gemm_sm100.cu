@@ -128,9 +128,10 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Arrive on a barrier given by its shared::cluster address (own or peer CTA).  For tensor memory that has been read, whose order
-// tcgen05.fence::before_thread_sync keeps; release semantics at cluster scope would make the thread wait for its stores.
+// tcgen05.fence::before_thread_sync keeps: relaxed, because release semantics at cluster scope would make the thread wait for
+// its stores.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
