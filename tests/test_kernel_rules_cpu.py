@@ -73,3 +73,62 @@ def test_column_statistics_read_past_l1():
     assert re.findall(r"\bstate\[col\]\s*(\S+)", columns) == ["="]
     assert "0.95f * __ldcg(state + col)" in columns
     assert "return COLS ? __ldcg(p) : *p;" in _function(text, "normuon_load")
+
+
+def _kernel(text, name):
+    """(parameters, body) of a kernel."""
+    head = re.search(r"__global__[^;{]*\b" + name + r"\(([^{]*)\)\s*\{", text)
+    assert head, name
+    return head.group(1), _function(text, name)
+
+
+def _check_early_reader(text, name):
+    """A kernel that lets the next launch begin and reads before it waits: it waits in every block, in front of that it stores
+    nothing to global memory, and reads it from L2 only."""
+    params, body = _kernel(text, name)
+    assert body.count("chain_wait();") == 1, name
+    early, late = body.split("chain_wait();")
+    assert "return" not in early, name
+    depth = early.count("{") - early.count("}")      # the wait itself: by every thread, or by the first of every block
+    assert depth == 0 or (depth == 1 and re.search(r"if \(tid == 0\) \{[^{}]*(\{[^{}]*\}[^{}]*)*$", early)), name
+    early = re.sub(r"\bsymexp_resolve\(sp, beta\)|encode_fetch<MODE, true>\(r, src, z, xm, len, base\)", "", early)
+    for param in params.split(","):
+        if "*" not in param:
+            continue
+        pointer = param.split("*")[-1].strip()
+        uses = re.findall(r"(.{0,48})(?<![\w.])" + pointer + r"\b", early)
+        assert all(re.search(r"__ldcg\(reinterpret_cast<const \w+ \*>\($", u) for u in uses), (name, pointer, uses)
+
+
+def test_launches_that_read_before_they_wait():
+    """What is launched by launch_chained may begin while the launch in front runs (csrc/stream_kernels.cu).  The first of a chain
+    waits and only then lets the next one begin, so that a launch that has begun finds every input of the call written; the
+    others are early readers.  The column statistics are the exception: they store before they wait, to slots that no launch in
+    flight looks at (the row statistics in front of them work on the other slots), and the plain launch of these is what their
+    inputs are complete before; all that they read is checked in test_column_statistics_read_past_l1."""
+    text = _source("stream_kernels.cu")
+    launched = re.findall(r"launch_chained\((k_\w+)", text)
+    assert sorted(set(launched)) == ["k_chain_chunk_amax", "k_chain_encode", "k_chain_schedule_amax", "k_chain_zero", "k_normuon_stats_columns"]
+    first = {name: re.match(r"\s*(\w+\(\);)", _kernel(text, name)[1]).group(1) for name in launched}
+    heads = {name for name in launched if first[name] == "chain_head();"}
+    assert heads == {"k_chain_zero", "k_chain_chunk_amax"}
+    assert re.fullmatch(r"\s*chain_wait\(\);\s*chain_begin\(\);\s*", _function(text + _source("common.cuh"), "chain_head"))
+    for name in set(launched) - heads:
+        assert first[name] == "chain_begin();", name
+        if name != "k_normuon_stats_columns":
+            _check_early_reader(text, name)
+    # a chain begins with its head ...
+    chain = _function(text, "launch_quantize_chain")
+    for branch in (chain[chain.index("if (src) {"):chain.index("return e;")], chain[chain.index("return e;"):]):
+        assert re.search(r"launch_chained\((k_\w+)", branch).group(1) in heads
+    # ... and the column statistics follow those of the rows, a plain launch of a kernel that waits in its first statement
+    assert re.search(r"stream_launch\(kPlain, k_normuon_stats_rows,[^;]*;\s*if \(nv\.columns\) launch_chained\(k_normuon_stats_columns,",
+                     _function(text, "launch_normuon_stats"))
+    assert re.fullmatch(r"\s*chain_begin\(\);\s*normuon_stats<1>\([^;]*\);\s*chain_wait\(\);\s*", _kernel(text, "k_normuon_stats_columns")[1])
+    assert re.fullmatch(r"\s*stream_enter\(\);\s*normuon_stats<0>\([^;]*\);\s*", _kernel(text, "k_normuon_stats_rows")[1])
+    # what the early readers share
+    fetch = _function(text, "encode_fetch")
+    direct, bounded = fetch.split("return;", 1)
+    assert re.search(r"if \(!L2_ONLY && ", direct)
+    assert re.findall(r"(L2_ONLY \? __ldcg)?\(?[^?;]*: ld_stream\((\w+) \+ e\)", bounded) == [("L2_ONLY ? __ldcg", p) for p in ("src", "z", "xm")]
+    assert "ld_stream" not in re.sub(r"L2_ONLY \? __ldcg\(reinterpret_cast<const float4 \*>\(\w+ \+ e\)\) : ld_stream\(\w+ \+ e\)", "", bounded)
