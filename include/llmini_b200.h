@@ -533,6 +533,11 @@ int b2_peer_status(const b2_peer_group *group, void *stream);
  * Synchronises `stream` before the launch. */
 int b2_debug_muon_fused_wait_expiry(b2_muon_plan *plan, const b2_muon_slot_descriptor *d_slots, uint32_t slot,
                                     uint64_t wait_ns, void *stream);
+/* The tile shapes that a plan of these matrices takes (needs no GPU): rows and columns of a tile of Gram and
+ * polynomial, whether a pair of CTAs computes it (1) or one (0), whether the tiles below the diagonal are left out
+ * and written as transposes; then rows, columns and pair of a tile of Apply. */
+int b2_debug_muon_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t slot_count,
+                        const b2_muon_options *options, uint32_t tiles[7]);
 /* Evaluates `rcp.approx.ftz.f32` (crates/cuda-kernels/src/utils/float_ptx.rs:31-33). */
 int b2_debug_rcp_approx_ftz(const float *d_in, float *d_out, uint32_t count, void *stream);
 /* Literal one-thread-per-group transcription of the reference quantiser

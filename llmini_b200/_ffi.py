@@ -174,6 +174,7 @@ def _declare(L: C.CDLL) -> None:
         "b2_peer_push": (i, [C.POINTER(PeerGroup), sz, sz, u32, vp]),
         "b2_peer_wait": (i, [C.POINTER(PeerGroup), u64, vp]),
         "b2_peer_status": (i, [C.POINTER(PeerGroup), vp]),
+        "b2_debug_muon_tiles": (i, [u32p, u32p, u32, C.POINTER(MuonOptions), u32p]),
         "b2_debug_muon_fused_wait_expiry": (i, [vp, vp, u32, u64, vp]),
         "b2_debug_rcp_approx_ftz": (i, [vp, vp, u32, vp]),
         "b2_debug_quantize_literal": (i, [vp, vp, vp, vp, vp, u32, vp]),

@@ -1228,6 +1228,15 @@ int b2_zero_f32_pointer_table(const uint64_t *d_pointers, uint32_t pointer_count
     return (int)launch_zero_pointer_table(d_pointers, pointer_count, as_stream(stream));
 }
 
+int b2_debug_muon_tiles(const uint32_t *rows, const uint32_t *cols, uint32_t slot_count, const b2_muon_options *options,
+                        uint32_t tiles[7]) {
+    if (!rows || !cols || slot_count == 0 || slot_count > 65535 || !tiles) return B2_ERROR_INVALID_VALUE;
+    Layout L;
+    if (!build_layout(rows, cols, slot_count, normalized(options), L)) return B2_ERROR_INVALID_VALUE;
+    const int out[7] = {L.nn.tm, L.nn.bn, L.nn.pair, L.symmetric, L.out.tm, L.out.bn, L.out.pair};
+    for (int k = 0; k < 7; ++k) tiles[k] = (uint32_t)out[k];
+    return B2_SUCCESS;
+}
 int b2_debug_muon_fused_wait_expiry(b2_muon_plan *plan, const b2_muon_slot_descriptor *d_slots, uint32_t slot,
                                     uint64_t wait_ns, void *stream) {
     if (!plan || !d_slots || wait_ns == 0 || wait_ns > 1000000000ull) return B2_ERROR_INVALID_VALUE;

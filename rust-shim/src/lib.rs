@@ -337,6 +337,8 @@ pub mod ffi {
         pub fn b2_peer_push(group: *const b2_peer_group, offset: usize, bytes: usize, ctas: u32, stream: CUstream) -> i32;
         pub fn b2_peer_wait(group: *const b2_peer_group, wait_ns: u64, stream: CUstream) -> i32;
         pub fn b2_peer_status(group: *const b2_peer_group, stream: CUstream) -> i32;
+        pub fn b2_debug_muon_tiles(rows: *const u32, cols: *const u32, slot_count: u32, options: *const b2_muon_options,
+                                   tiles: *mut u32) -> i32;
         pub fn b2_debug_muon_fused_wait_expiry(plan: *mut b2_muon_plan, d_slots: CUdeviceptr, slot: u32, wait_ns: u64,
                                                stream: CUstream) -> i32;
         pub fn b2_debug_rcp_approx_ftz(d_in: CUdeviceptr, d_out: CUdeviceptr, count: u32, stream: CUstream) -> i32;

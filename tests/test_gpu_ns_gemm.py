@@ -9,11 +9,14 @@ accumulate in a different order already differ by about 1e-2: the five-iteration
 relative L2 <= 2e-2 (the stated tolerance of the path), with a loose sanity bound of 1e-1 of the
 peak entry on the largest single-entry difference.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 import llmini_b200 as b2
+from llmini_b200 import _ffi
 from oracle import oracle as o
 from tests import _util as U
 from tests.gpu_util import dev, host
@@ -307,7 +310,7 @@ def test_few_gram_tiles_with_a_long_k(shapes, deferred):
     [(129, 144), (144, 256), (2000, 16)],                # one row or 16 columns into the second tile; one k-block
     [(1000, 1040), (77, 1040), (200, 208), (48, 1600)],  # rows no multiple of 8, 16 or 64; columns not of 64
     [(960, 320), (320, 320), (1280, 320), (320, 1280)],  # MN-major on one side, K-major on the other
-    [(768, 768)] * 3 + [(3072, 768)],                    # more tiles than one wave: triangles
+    [(768, 768)] * 3 + [(3072, 768)],                    # 144 tiles, just within one wave of CTAs; Apply in 256 x 256
 ])
 def test_small_pair_tiles_equal_one_cta_tiles_bit_for_bit(shapes, fmt, deferred):
     """Plans of few tiles take the pairs' 128 x 128 for Gram and polynomial, and some for Apply; a sum runs over K in the
@@ -321,6 +324,45 @@ def test_small_pair_tiles_equal_one_cta_tiles_bit_for_bit(shapes, fmt, deferred)
         for i, x in enumerate(xs):
             plan.scratch(i, 0).copy_(dev(x).to(plan.scratch(i, 0).dtype))
             plan.scratch(i, 2).view(torch.float32).fill_(0.75)   # read by a one-pass plan only
+        b2.OptimizerModule().muon_polar(plan, b2.MuonMegaUpdateArgs(iterations=3, coefficients=o.fixed_coefficients(3)))
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        results.append([[host(plan.scratch(i, w).float()).copy() for w in (5, 6, 7, 1)] for i in range(len(shapes))])
+        plan.close()
+    for shape, a, b in zip(shapes, *results):
+        for w, u, v in zip(("Gram", "Q", "X1", "U"), a, b):
+            assert np.isfinite(u).all() and np.array_equal(u, v), (shape, w)
+
+
+def _tiles(shapes, tile_n, fmt):
+    """(tile of Gram and polynomial, by a pair of CTAs, triangle of tiles, tile of Apply, by a pair) that a plan takes."""
+    n = len(shapes)
+    opt = _ffi.MuonOptions(fmt, b2.SCALES_RAW, 0, 3, tile_n)
+    out = (C.c_uint32 * 7)()
+    rows, cols = (C.c_uint32 * n)(*[r for r, _ in shapes]), (C.c_uint32 * n)(*[c for _, c in shapes])
+    assert b2.lib().b2_debug_muon_tiles(rows, cols, n, C.byref(opt), out) == 0
+    return (out[0], out[1]), bool(out[2]), bool(out[3]), (out[4], out[5]), bool(out[6])
+
+
+@pytest.mark.parametrize("fmt", [b2.OPERAND_BF16, b2.OPERAND_F16])
+@pytest.mark.parametrize("shapes,apply", [
+    ([(1920, 640), (640, 640), (2560, 640), (640, 2560)], ((128, 128), True)),      # whole tiles
+    ([(650, 656)] * 3, ((128, 128), False)),                                        # ten rows into the last tile, no multiple of 8
+    ([(1001, 1040), (700, 1200)], ((128, 128), False)),                             # an odd row count: G and Q have padding columns
+    ([(645, 656), (1300, 656), (645, 1312), (2000, 656)], ((256, 256), True)),      # both sides ragged
+])
+def test_triangles_of_small_pair_tiles_equal_full_one_cta_tiles_bit_for_bit(shapes, apply, fmt):
+    """Beyond one wave the pairs' 128 x 128 tiles leave out what lies below the diagonal and store it as transposes, 64 rows a
+    CTA with their columns in two halves of the lanes."""
+    assert _tiles(shapes, 0, fmt) == ((128, 128), True, True, *apply)
+    assert _tiles(shapes, 128, fmt) == ((128, 128), False, False, (128, 128), False)
+    rng = np.random.default_rng(sum(r for r, _ in shapes))
+    xs = [_x0(rng, r, c, fmt) for r, c in shapes]
+    results = []
+    for tile_n in (0, 128):
+        plan = b2.MuonPlan(shapes, operand_format=fmt, scale_layout=b2.SCALES_RAW, tile_n=tile_n, max_iterations=3)
+        for i, x in enumerate(xs):
+            plan.scratch(i, 0).copy_(dev(x).to(plan.scratch(i, 0).dtype))
         b2.OptimizerModule().muon_polar(plan, b2.MuonMegaUpdateArgs(iterations=3, coefficients=o.fixed_coefficients(3)))
         torch.cuda.synchronize()
         assert plan.status() == 0
