@@ -227,7 +227,7 @@ def test_one_tensor_calls_equal_their_parts(chunks, tail):
             y = z + (x - z) * beta
             if source == "schedule":
                 q.tensor_amax_f32(y, want_chunk, want_amax, n)
-            else:   # the maximum is checked below, value by value
+            else:   # (the maximum: test_transformed_maximum_over_many_chunks)
                 want_amax.copy_(amax)
             opt.materialize_schedule_free_precomputed(bytes=want[0], scales=want[1], global_scale=want[2], amax=want_amax,
                                                       precomputed_values=y if source == "schedule" else None, **kw)
@@ -255,3 +255,32 @@ def test_transform_divides_as_the_division_does(symexp):
     torch.cuda.synchronize()
     a, b = host(out)
     assert np.array_equal(a, b) and len(np.unique(a)) > 100
+
+
+@pytest.mark.parametrize("chunks,tail", [(0, 16), (1, 48), (3, 0), (1279, 2032), (6144, 16)])
+@pytest.mark.parametrize("at", ["first", "between", "last"])
+def test_transformed_maximum_over_many_chunks(chunks, tail, at):
+    """The transform with positive scales grows with |y|, so the maximum of a tensor is the transform of its largest value, which a
+    call on 16 values shows alone; it stands out by a third, which no rounding of the transform turns round."""
+    n = chunks * 2048 + tail
+    where = {"first": 0, "between": n // 2 + 5, "last": n - 1}[at]
+    gen = torch.Generator(device="cuda").manual_seed(n + where)
+    z, x = (torch.rand(n, device="cuda", generator=gen).sub_(0.5).mul_(0.3) for _ in range(2))
+    z[where] = -0.21
+    x[where] = -0.2
+    opt, scales = b2.OptimizerModule(), [torch.full((1,), v, device="cuda") for v in (1.1, 0.9, 0.8, 1.3, 1.2, 1.0)]
+    amax = torch.full((2,), 7.0, device="cuda")
+    outs = []
+    for i, (zz, xx) in enumerate(((z, x), (z[where:where + 1].repeat(16), x[where:where + 1].repeat(16)))):
+        m = zz.numel()
+        q = dict(bytes=torch.full((m // 2,), 255, dtype=torch.uint8, device="cuda"), scales=torch.full((m // 16,), 255, dtype=torch.uint8, device="cuda"),
+                 global_scale=torch.zeros(1, device="cuda"))
+        opt.materialize_schedule_free(**q, amax=amax[i:i + 1], z_master=zz, x_master=xx, len=m, scale_rows=m // 16, scale_k=16, beta=0.5,
+                                      scale_layout=b2.SCALES_RAW, symexp_lin_beta=12.5, symexp_lin_scales=scales)
+        outs.append(q)
+    torch.cuda.synchronize()
+    assert float(torch.max((z + (x - z) * 0.5).abs())) == float((z + (x - z) * 0.5)[where].abs()) and float(amax[0]) > 0.1
+    assert float(amax[0]) == float(amax[1])
+    assert torch.equal(outs[0]["global_scale"], outs[1]["global_scale"])
+    group = where // 16
+    assert outs[0]["scales"][group] == outs[1]["scales"][0]

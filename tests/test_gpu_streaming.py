@@ -606,3 +606,85 @@ def test_one_tensor_chain_right_behind_the_kernels_that_write_its_inputs(front):
         for key in a:
             assert torch.equal(a[key], b[key]), (i, key)
     assert len({float(q["amax"]) for q in want}) == (2 if front == "same outputs" else steps)
+
+
+@pytest.mark.parametrize("count", [33, 128, 129, 300])
+def test_a_step_on_many_matrices_equals_steps_on_few(count):
+    """A chunk finds its matrix among 128 at a time, above that by halving first: every streaming kernel of the step on plans on both
+    sides of these lines, empty matrices among the others, gives each matrix the bits it has in a plan of five."""
+    shapes = [[(16, 16), (0, 0), (130, 48), (7, 32), (48, 130 // 16 * 16)][i % 5] for i in range(count)]
+    opt = b2.OptimizerModule()
+    args = b2.MuonMegaUpdateArgs(grad_scale=0.5, learning_rate=0.02, average_coefficient=0.5, schedule_beta=0.3, iterations=3,
+                                 coefficients=o.fixed_coefficients(3), normuon=True)
+    gen = torch.Generator(device="cuda").manual_seed(count)
+    begin = []
+    for r, c in shapes:
+        randn = lambda std: torch.randn(r, c, device="cuda", generator=gen).mul_(std)
+        begin.append((randn(1e-3), randn(1e-3).to(torch.bfloat16), randn(0.02), randn(0.02), torch.rand(max(r, c), device="cuda", generator=gen).add_(1e-4)))
+
+    def run(first, last):
+        slots = [b2.MuonSlot.allocate(r, c, b2.SCALES_RAW) for r, c in shapes[first:last]]
+        for s, (g, m, z, x, second) in zip(slots, begin[first:last]):
+            for t, v in ((s.grad, g), (s.momentum, m), (s.z_master, z), (s.x_master, x)):
+                t.copy_(v)
+            s.second_momentum = second.clone()
+        table = b2.slot_table(slots)
+        plan = b2.MuonPlan(shapes[first:last], scale_layout=b2.SCALES_RAW, max_iterations=3)
+        opt.muon_tma_prepare_polar(plan, table, args)
+        opt.muon_polar(plan, args)
+        opt.muon_tma_finish_update_deferred_quantization(plan, table, args)
+        opt.muon_materialize_training_weights(plan, table)
+        first_step = [(s.grad.clone(), s.bytes.clone(), s.scales.clone(), s.global_scale.clone()) for s in slots]
+        for s, (g, *_) in zip(slots, begin[first:last]):
+            s.grad.copy_(g)
+        plain = b2.MuonPlan(shapes[first:last], scale_layout=b2.SCALES_RAW, max_iterations=3, normalize_mode=b2.NORMALIZE_DEFERRED)
+        opt.muon_mega_update(plain, table, b2.MuonMegaUpdateArgs(**{**vars(args), "normuon": False}))
+        torch.cuda.synchronize()
+        assert plan.status() == 0 and plain.status() == 0
+        out = [(*a, s.grad, s.momentum, s.z_master, s.x_master, s.second_momentum, s.schedule_amax, s.bytes, s.scales, s.global_scale)
+               for a, s in zip(first_step, slots)]
+        plan.close()
+        plain.close()
+        return out
+
+    many = run(0, count)
+    few = [r for at in range(0, count, 5) for r in run(at, min(at + 5, count))]
+    for i, (a, b) in enumerate(zip(many, few)):
+        if shapes[i] != (0, 0):
+            for k, (u, v) in enumerate(zip(a, b)):
+                assert torch.equal(u, v), (i, shapes[i], k)
+
+
+@pytest.mark.parametrize("count", [33, 128, 129, 300])
+def test_an_adamw_table_of_many_entries_equals_tables_of_few(count):
+    """The same for the pointer table of AdamW: update, requantisation and the deferred materialisation, entries of no values among
+    the others."""
+    opt = b2.OptimizerModule()
+    hp = dict(grad_scale=0.7, learning_rate=2e-4, weight_decay=0.005, beta1=0.9, beta2=0.95, beta1_correction=0.19,
+              beta2_correction=0.0975, eps=1e-10, average_coefficient=0.5, schedule_beta=0.3)
+    specs = [[(768, 0), (16, 1), (0, 0), (4112, 2), (2048, 1), (4099, 0)][i % 6] for i in range(count)]
+
+    def tensors():
+        gen = torch.Generator(device="cuda").manual_seed(count)
+        out = []
+        for n, mode in specs:
+            randn = lambda std: torch.randn(n, device="cuda", generator=gen).mul_(std)
+            t = dict(z_master=randn(0.02), x_master=randn(0.02), grad=randn(1e-3), first_moment=randn(1e-3), second_moment=randn(1e-3).square_(),
+                     len=n, mode=mode)
+            if mode:
+                t.update(amax=torch.full((1,), 7.0, device="cuda"), bytes=torch.zeros(n // 2, dtype=torch.uint8, device="cuda"),
+                         scales=torch.zeros(n // 16, dtype=torch.uint8, device="cuda"), global_scale=torch.zeros(1, device="cuda"),
+                         scale_layout=b2.SCALES_RAW)
+            out.append(t)
+        return out
+
+    many, few = tensors(), tensors()
+    for part in [many] + [few[at:at + 4] for at in range(0, count, 4)]:
+        table, entries, chunks = opt.adamw_table(part)
+        opt.apply_adamw_update_multi(table, entries, chunks, **hp)
+        opt.adamw_materialize_training_weights(table, entries, chunks, 0.3)
+        torch.cuda.synchronize()
+    for i, (a, b) in enumerate(zip(many, few)):
+        for key, v in a.items():
+            if torch.is_tensor(v):
+                assert torch.equal(v, b[key]), (i, specs[i], key)
