@@ -469,8 +469,7 @@ k_muon_update(const b2_muon_slot_descriptor *slots, const uint32_t *prefix, uint
 // the number of units in a plan, it let a matrix's bits depend on its company.  Narrow units give a lone matrix more CTAs,
 // each with a shorter chain of round trips; wide ones read longer pieces of a row.  NorMuon finish with 32 / 64 / 128 columns
 // (us): ragged plan of 5 matrices 24.9 / 25.8 / 28.9, one 768 x 3072 18.8 / 20.5 / 22.8, GPT-2 medium 1523 / 1494 / 1478.
-// What COLS reads in front of its wait goes to L2, past the L1 of an SM that may hold what an earlier kernel saw.  (Plain loads
-// find the tables in L1 behind the rows: ragged plan of 5 matrices with Hyperball, whole call 153.8 us with them, 156.2 now.)
+// What COLS reads in front of its wait goes to L2, past the L1 of an SM that may hold what an earlier kernel saw.
 template <int COLS, typename T>
 __device__ __forceinline__ T normuon_load(const T *p) { return COLS ? __ldcg(p) : *p; }
 template <int COLS>
@@ -546,9 +545,9 @@ __device__ __forceinline__ void normuon_stats(const b2_muon_slot_descriptor *slo
                     for (uint32_t k = 0; k < kRowsInFlight; ++k) {
                         const uint32_t r = r0 + k * kRowLanes;
                         const size_t at = (size_t)r * cols + c0;
-                        u[k] = r < rows ? __ldcg(reinterpret_cast<const float4 *>(U + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        u[k] = r < rows ? ld_l2(U + at) : make_float4(0.f, 0.f, 0.f, 0.f);
                         if (hyperball)
-                            p[k] = r < rows ? __ldcg(reinterpret_cast<const float4 *>(z + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            p[k] = r < rows ? ld_l2(z + at) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
 #pragma unroll
                     for (uint32_t k = 0; k < kRowsInFlight; ++k) {

@@ -72,6 +72,8 @@ def test_column_statistics_read_past_l1():
     assert "slots[" not in columns and "*reinterpret_cast<const" not in columns
     assert re.findall(r"\bstate\[col\]\s*(\S+)", columns) == ["="]
     assert "0.95f * __ldcg(state + col)" in columns
+    assert re.findall(r"(\w+\()?\b[Uz] \+", columns) == ["ld_l2(", "ld_l2("]
+    assert '"ld.relaxed.gpu.global.v4.f32' in _function(_source("common.cuh"), "ld_l2")
     assert "return COLS ? __ldcg(p) : *p;" in _function(text, "normuon_load")
 
 
