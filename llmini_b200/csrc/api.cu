@@ -169,9 +169,10 @@ bool valid_shape(uint32_t rows, uint32_t cols, const b2_muon_options &o) {
 // a fixed time (about 2 us from the end of the launch in front to the first read, 1 us to the first MMA, pipeline fill and
 // last epilogue), a tile so long per k-block and for itself, at least a minimum (its epilogue), and the tiles are dealt round
 // the groups in order of their K, so the first group has the most.  Constants (us) fitted to each phase of 40 plans, one
-// to 192 matrices of 160 to 6400, in each shape (median error 3 %; against the best choice of each phase the picks lose 1 %
-// on average and at most 9 %).  G and Q are symmetric: a triangle leaves out the tiles below the diagonal, whose transposes
-// make the epilogue of the others longer, which pays only beyond one wave.
+// to 192 matrices of 160 to 6400, in each shape (median error 3 %).  Against the best shape of each phase, measured on 40 plans
+// of one matrix to 12 layers and of widths 160 to 1600, the picks are the best in 28 and lose 0.6 % on average: on 60
+// matrices of width 320 7 %, elsewhere at most 3 %.  G and Q are symmetric: a triangle leaves out the tiles below the diagonal,
+// whose transposes make the epilogue of the others longer, which pays only beyond one wave.
 // Measured, all of 128 x 128 on one CTA (the smallest shape before) -> the choice, Newton-Schulz loop in us: one 3072 x 768
 // 170 -> 125, one layer of width 320 117 -> 88, four 146 -> 131, five ragged matrices 172 -> 121.
 constexpr uint32_t kTileRuleSms = 148;   // of a B200; not asked of the device, because the workspace size depends on it
